@@ -158,6 +158,7 @@ static void free_ctx(mic_ctx *ctx) {
   cudaFree(ctx->io_buf);
   for (int w = 0; w < 2; ++w) {
     if (ctx->sys[w].lu_exec) cudaGraphExecDestroy(ctx->sys[w].lu_exec);
+    mic_front_plan_free(ctx->sys[w].plan);
     cudaFree(ctx->sys[w].cnt);
     cudaFree(ctx->sys[w].col);
     cudaFree(ctx->sys[w].val);
@@ -165,11 +166,6 @@ static void free_ctx(mic_ctx *ctx) {
   }
   cudaFree(ctx->sys_scratch);
   cudaFree(ctx->lu_buf);
-  if (ctx->lu_side) {
-    cudaStreamDestroy(ctx->lu_side);
-    cudaEventDestroy(ctx->lu_ev[0]);
-    cudaEventDestroy(ctx->lu_ev[1]);
-  }
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
   for (int k = 0; k < 2; ++k)
     if (ctx->aux_ev[k]) cudaEventDestroy(ctx->aux_ev[k]);

@@ -1,0 +1,957 @@
+// mic_front_lu.cu -- direct solve of an assembled system on the device: LU factorisation with
+// partial pivoting in nested-dissection order, then the back substitution.  It stands in for
+// kspLinearSolve (kspLinearSolve.c:13-120) run as the reference's option files configure it,
+// `-stokes_ksp_type preonly -stokes_pc_type lu` and the same for `energy_`
+// (option_files/run_mumps.petscopt), i.e. one direct factorisation and solve per call.
+//
+// Order.  The grid's rows (equations) are bisected along the longer side again and again, down to
+// rectangles of a few nodes: a binary tree.  A column (unknown) is eliminated at the lowest tree
+// node whose rectangle holds every row that touches it.  Such a tree node is a dense front:
+//   rows     the rectangle's equations (a leaf), or the rows its two children have left over;
+//   columns  P pivot columns, then the columns its rows share with the rest of the grid (the
+//            border), then the right-hand side.
+// Every row that touches a pivot column is in the front, so partial pivoting over all of the
+// front's rows is partial pivoting over the whole column: the elimination is Gaussian elimination
+// with partial pivoting of the column-permuted matrix, whatever is zero or small inside a
+// subdomain (a Stokes subdomain's own block is singular: its pressures have a free constant).
+// After P steps the first P pivot rows are rows of U, and the other R - P rows, their border
+// columns and right-hand sides, go to the parent unchanged in number and without any sum: the
+// children's rows are stacked.  The forward substitution rides along as the last column.
+//
+// Why this order: eliminating the band from one end is a chain of n column steps, each a pivot
+// search, a reciprocal and an update (1.7 us a step; 31.6 ms for the 129 x 33 Stokes system, 862
+// for 513 x 129, 175 for 513 x 129 temperatures).  Here all fronts of one tree level are
+// eliminated side by side, so the chain is the sum over the levels of one front's pivots (797,
+// 3,197 and 1,278 columns), and for the two larger systems the work falls as well (17 G and 1.1 G
+// multiply-adds, against 61 G and 2.2 G in the band).
+//
+// Two forms of a level, chosen by estimated time (plan_level):
+//   small  the front in shared memory, one block per front, unblocked (k_front_small);
+//   large  the front in global memory, panels of NB columns: one block per front factors a panel
+//          in shared memory (k_front_panel), then the trailing tiles of every front are updated,
+//          each block forming its own piece of U12 (k_front_update).
+// FP64 multiply-adds bound the updates (2 per SM and clock); the panels and the small fronts are
+// bound by the latency of their column steps.  One CUDA graph holds all launches of a solve.
+#include <algorithm>
+#include <climits>
+#include <iterator>
+#include <new>
+#include <vector>
+
+#include "mic_internal.cuh"
+
+using namespace mic;
+
+namespace {
+
+struct Front {
+  int R, P, C;  // rows, pivot columns, columns (pivots, border, right-hand side)
+  int nA;       // rows that come from the first child (the second's follow)
+  int child;    // first child's index (the second follows); -1: a leaf
+  int x0, x1, y0, y1;  // the rectangle of nodes whose equations these are
+  int full;     // storage: 1 all R rows, C values each (panels); 0 the left-over rows, C - P each
+  int64_t f, u; // offsets of the front's rows and of its rows of U (doubles)
+  int64_t lb;   // panel buffer (doubles)
+  int64_t col;  // the pivots' and the border's unknowns (ints, C - 1)
+  int64_t map;  // child columns of this front's columns (2 C ints), or a leaf's slot table
+  int64_t act;  // row list of a front in panels (ints, R): pivot rows in order, then the others
+};
+
+// info[0]: smallest unknown with a zero pivot; info[1]: entries outside the assumed stencils;
+// info[2], info[3]: lower and upper band widths of the matrix in grid order (mic_system_band)
+constexpr int kInfo = 4;
+
+__device__ __forceinline__ int64_t bmap(int64_t r, int dof, int NX, int NY, int transpose) {
+  if (!transpose) return r;
+  const int64_t node = r / dof;
+  const int d = (int)(r % dof);
+  const int ix = (int)(node % NX), jy = (int)(node / NX);
+  return ((int64_t)ix * NY + jy) * dof + d;
+}
+
+// band widths with the nodes numbered along the shorter grid side (reported, and the size limit)
+__global__ void k_band_width(const int *__restrict__ cnt, const int *__restrict__ col, int width, int64_t n,
+                             int dof, int NX, int NY, int transpose, int *bw) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  int lo = 0, up = 0;
+  if (r < n) {
+    const int64_t bi = bmap(r, dof, NX, NY, transpose);
+    for (int k = 0; k < cnt[r]; ++k) {
+      const int64_t bj = bmap(col[r * width + k], dof, NX, NY, transpose);
+      lo = max(lo, (int)(bi - bj));
+      up = max(up, (int)(bj - bi));
+    }
+  }
+  lo = __reduce_max_sync(0xffffffffu, lo);
+  up = __reduce_max_sync(0xffffffffu, up);
+  if ((threadIdx.x & 31) == 0) {
+    if (lo > 0) atomicMax(&bw[0], lo);
+    if (up > 0) atomicMax(&bw[1], up);
+  }
+}
+
+struct SystemRows {  // the assembled rows (mic_systems.cu)
+  const int *cnt, *col;
+  const double *val, *rhs;
+  int width, dof, NX, NY;
+};
+
+// Largest |a| in a column by its high word (sign, exponent, 20 bits of mantissa): an integer key,
+// so the search costs no FP64 slot and one warp instruction per warp.  Rows whose keys agree
+// differ by less than 2^-20 relatively, as good a pivot.  -1 for a NaN.
+__device__ __forceinline__ int pivot_key(double a) {
+  const int h = (int)((unsigned long long)dbits(a) >> 32) & 0x7fffffff;
+  return h <= 0x7ff00000 ? h : -1;
+}
+
+// a column whose keys are all zero (every |a| below 2^-1042): the exact largest |a|, in order
+__device__ int pivot_slow(const double *col, int stride, int r0, int r1) {
+  long long best = -1;
+  int p = r0;
+  for (int r = r0; r < r1; ++r) {
+    const long long b = dbits(col[(int64_t)r * stride]) & 0x7fffffffffffffffLL;
+    if (b > best && b <= 0x7ff0000000000000LL) {
+      best = b;
+      p = r;
+    }
+  }
+  return p;
+}
+
+// (key, row) of the warp's best lane, in every lane
+__device__ __forceinline__ int2 warp_best(int key, int row) {
+  const int m = __reduce_max_sync(0xffffffffu, key);
+  const unsigned b = __ballot_sync(0xffffffffu, key == m);
+  return make_int2(m, __shfl_sync(0xffffffffu, row, __ffs(b) - 1));
+}
+
+// value of column c (of q's columns) in left-over row i of child k: where the child keeps it
+__device__ __forceinline__ const double *child_row(const Front &k, int i, const double *F, const int *act) {
+  return k.full ? F + k.f + (int64_t)act[k.act + k.P + i] * k.C + k.P : F + k.f + (int64_t)i * (k.C - k.P);
+}
+
+// ---- small fronts ------------------------------------------------------------------------
+// One block per front, the front in shared memory with an odd row stride, so that lanes taking
+// consecutive rows of one column meet no bank conflict.  A column step: the warps' best candidate
+// rows meet in shared memory, the pivot row changes places with row j and its reciprocal is formed
+// once, then a lane takes a row (its multiplier in a register) and the warps share out rows and
+// columns; the warps that update column j + 1 also find its candidates.  Two barriers a step.
+// The step is bound by this chain (about 1 us) until a front exceeds some 50,000 multiply-adds,
+// then by the FP64 pipe.
+constexpr int kSmallThreads = 256, kSmallWarps = kSmallThreads / 32;
+
+__global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__restrict__ fr, int first,
+                                                              const int *__restrict__ tab,
+                                                              const int *__restrict__ act, SystemRows sys,
+                                                              const double *__restrict__ Fin, double *F, double *U,
+                                                              int *info) {
+  extern __shared__ double A[];
+  __shared__ int2 red[32];
+  __shared__ double s_rcp;
+  const Front q = fr[first + blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int R = q.R, P = q.P, C = q.C, ld = C | 1;
+  if (q.child < 0) {
+    for (int e = tid; e < R * ld; e += kSmallThreads) A[e] = 0.0;
+    __syncthreads();
+    const int w = q.x1 - q.x0, tx = max(q.x0 - 1, 0), ty = max(q.y0 - 1, 0);
+    const int tw = min(q.x1 + 1, sys.NX) - tx, th = min(q.y1 + 1, sys.NY) - ty;
+    for (int r = tid; r < R; r += kSmallThreads) {
+      const int node = r / sys.dof, d = r % sys.dof;
+      const int64_t g = (int64_t)sys.dof * ((int64_t)(q.y0 + node / w) * sys.NX + q.x0 + node % w) + d;
+      const int n = sys.cnt[g];
+      for (int k = 0; k < n; ++k) {
+        const int c = sys.col[g * sys.width + k];
+        const int cn = c / sys.dof, cx = cn % sys.NX - tx, cy = cn / sys.NX - ty;
+        const bool in = cx >= 0 && cx < tw && cy >= 0 && cy < th;
+        const int pos = in ? tab[q.map + (cy * tw + cx) * sys.dof + c % sys.dof] : -1;
+        if (pos >= 0)
+          A[r * ld + pos] = sys.val[g * sys.width + k];
+        else
+          atomicAdd(&info[1], 1);
+      }
+      A[r * ld + C - 1] = sys.rhs[g];
+    }
+  } else {
+    const Front a = fr[q.child], b = fr[q.child + 1];
+    for (int r = warp; r < R; r += kSmallWarps) {
+      const bool fa = r < q.nA;
+      const double *src = fa ? child_row(a, r, Fin, act) : child_row(b, r - q.nA, Fin, act);
+      const int *m = tab + q.map + (fa ? 0 : C);
+      for (int c = lane; c < C; c += 32) {
+        const int s = m[c];
+        A[r * ld + c] = s >= 0 ? src[s] : 0.0;
+      }
+    }
+  }
+  __syncthreads();
+  int G = (R + 31) / 32;  // candidate entries waiting in red
+  for (int g = warp; g < G; g += kSmallWarps) {
+    const int r = g * 32 + lane;
+    const int2 best = warp_best(r < R ? pivot_key(A[r * ld]) : -1, r);
+    if (lane == 0) red[g] = best;
+  }
+  __syncthreads();
+  for (int j = 0; j < P; ++j) {
+    const int2 e = lane < G ? red[lane] : make_int2(-1, j);
+    const int2 best = warp_best(e.x, e.y);
+    int p = best.x < 0 ? j : best.y;  // all NaN: keep the diagonal
+    if (best.x == 0) {
+      p = pivot_slow(A + j, ld, j, R);
+      __syncthreads();  // every thread has read the column before rows move
+    }
+    for (int c = j + tid; c < C; c += kSmallThreads) {
+      const double up = A[p * ld + c], dn = A[j * ld + c];
+      A[j * ld + c] = up;
+      A[p * ld + c] = dn;
+      if (c == j) {
+        s_rcp = up != 0.0 ? 1.0 / up : 0.0;
+        if (up == 0.0) atomicMin(&info[0], tab[q.col + j]);
+      }
+    }
+    __syncthreads();
+    const double rcp = s_rcp;
+    const int n = R - j - 1;
+    G = (n + 31) / 32;
+    const int SL = max(1, kSmallWarps / max(G, 1));
+    for (int t = warp; t < G * SL; t += kSmallWarps) {
+      const int g = t % G, s = t / G, r = j + 1 + g * 32 + lane;
+      double *row = A + r * ld;
+      const double *piv = A + j * ld;
+      const double l = r < R ? row[j] * rcp : 0.0;
+      int c = j + 1 + s;
+      if (s == 0 && j + 1 < P) {  // the next column first, with its candidates
+        double v = 0.0;
+        if (r < R) {
+          v = row[c] - l * piv[c];
+          row[c] = v;
+        }
+        const int2 b = warp_best(r < R ? pivot_key(v) : -1, r);
+        if (lane == 0) red[g] = b;
+        c += SL;
+      }
+      if (r < R) {
+#pragma unroll 4
+        for (; c < C; c += SL) row[c] -= l * piv[c];
+      }
+    }
+    __syncthreads();
+  }
+  for (int r = warp; r < P; r += kSmallWarps)
+    for (int c = r + lane; c < C; c += 32) U[q.u + (int64_t)r * C + c] = A[r * ld + c];
+  for (int r = P + warp; r < R; r += kSmallWarps)
+    for (int c = P + lane; c < C; c += 32) F[q.f + (int64_t)(r - P) * (C - P) + c - P] = A[r * ld + c];
+}
+
+// ---- large fronts --------------------------------------------------------------------------
+
+// the children's left-over rows stacked, their columns placed; a warp per row
+__global__ void __launch_bounds__(256) k_front_gather(const Front *__restrict__ fr, int first,
+                                                     const int *__restrict__ tab, int *act,
+                                                     const double *__restrict__ Fin, double *F) {
+  const Front q = fr[first + blockIdx.x];
+  const int r = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= q.R) return;
+  if (lane == 0) act[q.act + r] = r;
+  const bool fa = r < q.nA;
+  const Front k = fr[q.child + (fa ? 0 : 1)];
+  const double *src = child_row(k, fa ? r : r - q.nA, Fin, act);
+  const int *m = tab + q.map + (fa ? 0 : q.C);
+  double *dst = F + q.f + (int64_t)r * q.C;
+  for (int c = lane; c < q.C; c += 32) {
+    const int s = m[c];
+    dst[c] = s >= 0 ? src[s] : 0.0;
+  }
+}
+
+// One panel: columns k0 .. k0 + NB - 1 of the rows not yet pivots, one block per front, the panel
+// in shared memory (odd stride NB + 1).  A thread keeps the same rows through a step: it forms
+// their multipliers, updates column j + 1 first and offers its best row for it, then the rest, so
+// that the search overlaps the update.  Rows move only inside the panel (with their numbers); in
+// the front they stay where they are, and the row list says which are pivots.
+template <int NB>
+__global__ void __launch_bounds__(1024) k_front_panel(const Front *__restrict__ fr, int first, int k0,
+                                                     const double *__restrict__ F, double *U, double *Lb, int *act,
+                                                     const int *__restrict__ tab, int *info) {
+  extern __shared__ double S[];
+  __shared__ int2 red[32];
+  __shared__ double s_rcp;
+  const Front q = fr[first + blockIdx.x];
+  if (k0 >= q.P) return;
+  constexpr int LD = NB + 1;
+  const int nb = min(NB, q.P - k0), na = q.R - k0;
+  int *id = reinterpret_cast<int *>(S + (int64_t)na * LD);
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  for (int r = tid; r < na; r += nt) id[r] = act[q.act + k0 + r];
+  __syncthreads();
+  for (int e = tid; e < na * NB; e += nt) {
+    const int r = e / NB, c = e % NB;
+    S[r * LD + c] = c < nb ? F[q.f + (int64_t)id[r] * q.C + k0 + c] : 0.0;
+  }
+  __syncthreads();
+  int key = -1, who = 0;
+  for (int r = tid; r < na; r += nt) {
+    const int k = pivot_key(S[r * LD]);
+    if (k > key) {
+      key = k;
+      who = r;
+    }
+  }
+  for (int j = 0; j < nb; ++j) {
+    const int2 mine = warp_best(key, who);
+    if (lane == 0) red[warp] = mine;
+    __syncthreads();
+    const int2 e = lane < nw ? red[lane] : make_int2(-1, j);
+    const int2 best = warp_best(e.x, e.y);
+    int p = best.x < 0 ? j : best.y;
+    if (best.x == 0) {
+      p = pivot_slow(S + j, LD, j, na);
+      __syncthreads();  // every thread has read the column before rows move
+    }
+    if (warp == 0) {
+      if (lane < NB) {
+        const double up = S[p * LD + lane], dn = S[j * LD + lane];
+        S[j * LD + lane] = up;
+        S[p * LD + lane] = dn;
+        if (lane == j) {
+          s_rcp = up != 0.0 ? 1.0 / up : 0.0;
+          if (up == 0.0) atomicMin(&info[0], tab[q.col + k0 + j]);
+        }
+      } else if (lane == NB) {
+        const int t = id[j];
+        id[j] = id[p];
+        id[p] = t;
+      }
+    }
+    __syncthreads();
+    const double rcp = s_rcp;
+    key = -1;
+    who = 0;
+    for (int r = j + 1 + tid; r < na; r += nt) {
+      double *row = S + r * LD;
+      const double *piv = S + j * LD;
+      const double l = row[j] * rcp;
+      row[j] = l;
+      if (j + 1 < nb) {
+        const double v = row[j + 1] - l * piv[j + 1];
+        row[j + 1] = v;
+        const int k = pivot_key(v);
+        if (k > key) {
+          key = k;
+          who = r;
+        }
+#pragma unroll 4
+        for (int c = j + 2; c < NB; ++c) row[c] -= l * piv[c];
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < nb * NB; e += nt) {  // U11
+    const int r = e / NB, c = e % NB;
+    if (c >= r && c < nb) U[q.u + (int64_t)(k0 + r) * q.C + k0 + c] = S[r * LD + c];
+  }
+  for (int e = tid; e < na * NB; e += nt) {  // multipliers (below the pivots), rows in list order
+    const int r = e / NB, c = e % NB;
+    Lb[q.lb + e] = (c < nb && r > c) ? S[r * LD + c] : 0.0;
+  }
+  for (int r = tid; r < na; r += nt) act[q.act + k0 + r] = id[r];
+}
+
+// U12 = L11^-1 A12 and A22 -= L21 U12 for the columns right of the panel, TR x TC tiles.  Each
+// block forms U12 of its own columns (NB^2 / 2 multiply-adds a column against NB TR for the tile:
+// 6% more work at TR = 128, 25% at 32, for one launch and one wait less per panel); the first row
+// of tiles also stores it.  The FP64 pipe is the bound: small tiles where there are too few large
+// ones to fill the SMs.
+template <int NB, int TR, int TC>
+__global__ void __launch_bounds__(256) k_front_update(const Front *__restrict__ fr, int first, int k0, double *F,
+                                                     double *U, const double *__restrict__ Lb,
+                                                     const int *__restrict__ act) {
+  constexpr int RT = TR / 16, CT = TC / 16;  // a thread's rows and columns
+  __shared__ double Us[NB][TC + 1];
+  __shared__ double Ls[TR][NB + 1];
+  __shared__ double L11[NB][NB + 1];
+  const Front q = fr[first + blockIdx.x];
+  if (k0 >= q.P) return;
+  const int nb = min(NB, q.P - k0);
+  const int c0 = k0 + nb + blockIdx.z * TC, r0 = nb + blockIdx.y * TR, na = q.R - k0;
+  if (c0 >= q.C || (r0 >= na && blockIdx.y > 0)) return;
+  const int tid = threadIdx.x, ti = tid / 16, tj = tid % 16;
+  const int *list = act + q.act + k0;
+  double *base = F + q.f;
+  const double *L = Lb + q.lb;
+  // the tile itself first: its loads overlap the triangular solve
+  double v[RT][CT];
+  int64_t at[RT];
+#pragma unroll
+  for (int a = 0; a < RT; ++a) {
+    const int r = r0 + ti + 16 * a;
+    at[a] = r < na ? (int64_t)list[r] * q.C : -1;
+#pragma unroll
+    for (int b = 0; b < CT; ++b) {
+      const int c = c0 + tj + 16 * b;
+      v[a][b] = (at[a] >= 0 && c < q.C) ? base[at[a] + c] : 0.0;
+    }
+  }
+  for (int e = tid; e < NB * TC; e += 256) {
+    const int k = e / TC, c = c0 + e % TC;
+    Us[k][e % TC] = (k < nb && c < q.C) ? base[(int64_t)list[k] * q.C + c] : 0.0;
+  }
+  for (int e = tid; e < NB * NB; e += 256) L11[e / NB][e % NB] = e / NB < nb ? L[e] : 0.0;
+  for (int e = tid; e < TR * NB; e += 256) {
+    const int r = r0 + e / NB;
+    Ls[e / NB][e % NB] = r < na ? L[(int64_t)r * NB + e % NB] : 0.0;
+  }
+  __syncthreads();
+  if (tid < TC) {
+    double u[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) u[k] = Us[k][tid];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+#pragma unroll
+      for (int k = j + 1; k < NB; ++k) u[k] -= L11[k][j] * u[j];
+    }
+#pragma unroll
+    for (int k = 0; k < NB; ++k) Us[k][tid] = u[k];
+    if (blockIdx.y == 0 && c0 + tid < q.C) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k)
+        if (k < nb) U[q.u + (int64_t)(k0 + k) * q.C + c0 + tid] = u[k];
+    }
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int k = 0; k < NB; ++k) {
+    double l[RT], u[CT];
+#pragma unroll
+    for (int a = 0; a < RT; ++a) l[a] = Ls[ti + 16 * a][k];
+#pragma unroll
+    for (int b = 0; b < CT; ++b) u[b] = Us[k][tj + 16 * b];
+#pragma unroll
+    for (int a = 0; a < RT; ++a)
+#pragma unroll
+      for (int b = 0; b < CT; ++b) v[a][b] -= l[a] * u[b];
+  }
+#pragma unroll
+  for (int a = 0; a < RT; ++a)
+#pragma unroll
+    for (int b = 0; b < CT; ++b) {
+      const int c = c0 + tj + 16 * b;
+      if (at[a] >= 0 && c < q.C) base[at[a] + c] = v[a][b];
+    }
+}
+
+// ---- back substitution ------------------------------------------------------------------
+
+// y -= U12 x_border in the right-hand side column of U, a warp per row (large fronts, whose rows
+// spread over the SMs; the small ones do it in k_front_back)
+__global__ void __launch_bounds__(256) k_front_border(const Front *__restrict__ fr, int first,
+                                                     const int *__restrict__ tab, double *U,
+                                                     const double *__restrict__ x) {
+  const Front q = fr[first + blockIdx.x];
+  const int r = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= q.P) return;
+  double *u = U + q.u + (int64_t)r * q.C;
+  double s = 0.0;
+#pragma unroll 4
+  for (int c = q.P + lane; c < q.C - 1; c += 32) s += u[c] * x[tab[q.col + c]];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) u[q.C - 1] -= s;
+}
+
+// U11 x = y, 32 rows at a time from the bottom, one block per front: a warp per row for the part
+// from solved unknowns (border: those of the border too), one warp for the 32 x 32 triangle with
+// all reciprocals formed at once
+__global__ void __launch_bounds__(1024) k_front_back(const Front *__restrict__ fr, int first,
+                                                    const int *__restrict__ tab, const double *__restrict__ U,
+                                                    double *x, int border) {
+  extern __shared__ double xs[];  // the front's unknowns: pivots, then (border) the border's
+  __shared__ double acc[32];
+  __shared__ double Ud[32][33];
+  const Front q = fr[first + blockIdx.x];
+  if (q.P == 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int *col = tab + q.col;
+  const int top = border ? q.C - 1 : q.P;
+  for (int c = q.P + tid; c < top; c += blockDim.x) xs[c] = x[col[c]];
+  __syncthreads();
+  for (int j1 = q.P; j1 > 0; j1 -= 32) {
+    const int j0 = max(j1 - 32, 0), nr = j1 - j0;
+    for (int w = warp; w < nr; w += nw) {
+      const double *u = U + q.u + (int64_t)(j0 + w) * q.C;
+      double s = 0.0;
+#pragma unroll 4
+      for (int c = j1 + lane; c < top; c += 32) s += u[c] * xs[c];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) acc[w] = u[q.C - 1] - s;
+      Ud[w][lane] = (lane >= w && lane < nr) ? u[j0 + lane] : 0.0;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      double a = lane < nr ? acc[lane] : 0.0;
+      const double rd = 1.0 / (lane < nr ? Ud[lane][lane] : 1.0);
+      for (int t = nr - 1; t >= 0; --t) {
+        const double xt = __shfl_sync(0xffffffffu, a * rd, t);
+        if (lane < t) a -= Ud[lane][t] * xt;
+        if (lane == t) a = xt;
+      }
+      if (lane < nr) {
+        xs[j0 + lane] = a;
+        x[col[j0 + lane]] = a;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---- the plan of a grid's solves ---------------------------------------------------------------
+
+// rows that touch unknown d of a node, relative to the node (the stencils of mic_systems.cu): the
+// velocities and the temperature are read by rows on either side, the pressure by rows at and
+// before its node only
+struct Reach {
+  int lo, hi;
+};
+Reach reach(int dof, int d) { return dof == 3 && d == 2 ? Reach{-1, 0} : Reach{-1, 1}; }
+
+struct Rect {
+  int x0, x1, y0, y1;
+};
+
+bool touches(const Rect &r, int x, int y, Reach e) {
+  return x + e.hi >= r.x0 && x + e.lo < r.x1 && y + e.hi >= r.y0 && y + e.lo < r.y1;
+}
+bool owns(const Rect &r, int x, int y, Reach e, int NX, int NY) {
+  return std::max(x + e.lo, 0) >= r.x0 && std::min(x + e.hi, NX - 1) < r.x1 && std::max(y + e.lo, 0) >= r.y0 &&
+         std::min(y + e.hi, NY - 1) < r.y1;
+}
+
+struct Level {
+  int first, count;          // fronts
+  int maxR, maxP, maxC, minP;
+  bool small;
+  int64_t nF, nL;            // doubles of row storage and of panel buffer
+  size_t smem_small;
+};
+
+constexpr size_t kMaxSmem = 227 * 1024 - 1024;  // dynamic shared memory (static parts stay below 1 KB)
+constexpr int kUpdateBlocks = 256;
+
+int panel_columns(int maxR) {  // panel width: the widest whose panel fits shared memory
+  for (int nb : {16, 8, 4})
+    if ((size_t)maxR * ((nb + 1) * sizeof(double) + sizeof(int)) <= kMaxSmem) return nb;
+  return 0;
+}
+
+}  // namespace
+
+struct mic_front_plan {
+  int dof = 0, NX = 0, NY = 0;
+  std::vector<Front> fronts;
+  std::vector<Level> levels;  // root first
+  std::vector<int> tab;
+  int64_t nF[2] = {0, 0}, nU = 0, nL = 0, nAct = 0;
+  Front *d_fronts = nullptr;
+  int *d_tab = nullptr;
+};
+
+namespace {
+
+// The level's form.  Small: blocks share the SMs, each front's multiply-adds on one SM (2 per
+// clock), about 1.1 us a column step.  Large: multiply-adds over all SMs at about 70% of the pipe,
+// 14 us a panel of 16 columns for its factorisation, its update's launch and its tail, 6 us for
+// the gather.  (Both sides measured on the levels of the 129 x 33 and 513 x 129 systems.)
+void plan_level(Level &L, const std::vector<Front> &fr, int nsm) {
+  double total = 0, most = 0;
+  for (int i = L.first; i < L.first + L.count; ++i) {
+    double w = 0;
+    for (int j = 0; j < fr[i].P; ++j) w += double(fr[i].R - j - 1) * (fr[i].C - j - 1);
+    total += w;
+    most = std::max(most, w);
+  }
+  const double clk = 1.9e3;  // per us
+  const double waves = (L.count + nsm - 1) / nsm;
+  const double small = std::max(waves * most, total / nsm) / 2 / clk * 1.25 + 1.1 * L.maxP;
+  const double large = total / (2.0 * nsm * clk) / 0.7 + 14.0 * ((L.maxP + 15) / 16) + 6.0;
+  L.smem_small = (size_t)L.maxR * (L.maxC | 1) * sizeof(double);
+  L.small = L.smem_small <= kMaxSmem && L.maxR <= 1024 && (fr[L.first].child < 0 || small <= large);
+}
+
+int build_plan(mic_front_plan &pl, int dof, int NX, int NY, int nsm) {
+  pl.dof = dof;
+  pl.NX = NX;
+  pl.NY = NY;
+  // rectangles, level by level; one split direction per level keeps a level's fronts alike.  A
+  // leaf side of at most 3 nodes (Stokes) or 5 (temperature)
+  const int leaf = dof == 3 ? 3 : 5;
+  std::vector<std::vector<Rect>> rects{{Rect{0, NX, 0, NY}}};
+  for (int dx = NX, dy = NY; std::max(dx, dy) > leaf;) {
+    const bool sx = dx >= dy;
+    std::vector<Rect> next;
+    for (const Rect &r : rects.back()) {
+      const int m = sx ? (r.x0 + r.x1) / 2 : (r.y0 + r.y1) / 2;
+      next.push_back(sx ? Rect{r.x0, m, r.y0, r.y1} : Rect{r.x0, r.x1, r.y0, m});
+      next.push_back(sx ? Rect{m, r.x1, r.y0, r.y1} : Rect{r.x0, r.x1, m, r.y1});
+    }
+    rects.push_back(next);
+    (sx ? dx : dy) = ((sx ? dx : dy) + 1) / 2;
+  }
+  const int nl = (int)rects.size();
+  int first = 0;
+  for (auto &v : rects) {
+    Level L = {};
+    L.first = first;
+    L.count = (int)v.size();
+    first += L.count;
+    pl.levels.push_back(L);
+  }
+  pl.fronts.assign(first, Front{});
+  std::vector<int> pos((size_t)dof * NX * NY, -1);
+  // leaves first: a parent's rows and columns follow from its children
+  for (int l = nl - 1; l >= 0; --l) {
+    Level &L = pl.levels[l];
+    L.minP = INT_MAX;
+    for (int i = 0; i < L.count; ++i) {
+      const Rect r = rects[l][i];
+      Front &q = pl.fronts[L.first + i];
+      q.x0 = r.x0;
+      q.x1 = r.x1;
+      q.y0 = r.y0;
+      q.y1 = r.y1;
+      const bool isleaf = l == nl - 1;
+      q.child = isleaf ? -1 : pl.levels[l + 1].first + 2 * i;
+      const int tx = std::max(r.x0 - 1, 0), tX = std::min(r.x1 + 1, NX);
+      const int ty = std::max(r.y0 - 1, 0), tY = std::min(r.y1 + 1, NY);
+      // columns: the unknowns this rectangle is the first to hold all rows of, then the others
+      // its rows touch that no child has eliminated
+      std::vector<int> piv, bor;
+      auto take = [&](int x, int y, int d) {
+        const Reach e = reach(dof, d);
+        if (!touches(r, x, y, e)) return;
+        (owns(r, x, y, e, NX, NY) ? piv : bor).push_back(dof * (y * NX + x) + d);
+      };
+      if (isleaf) {
+        q.R = dof * (r.x1 - r.x0) * (r.y1 - r.y0);
+        for (int y = ty; y < tY; ++y)
+          for (int x = tx; x < tX; ++x)
+            for (int d = 0; d < dof; ++d) take(x, y, d);
+      } else {  // every column left is on the border of a child
+        const Front &a = pl.fronts[q.child], &b = pl.fronts[q.child + 1];
+        const auto t = pl.tab.begin();
+        std::vector<int> all;  // (borders are in ascending order)
+        std::set_union(t + a.col + a.P, t + a.col + a.C - 1, t + b.col + b.P, t + b.col + b.C - 1,
+                       std::back_inserter(all));
+        for (int g : all) take(g / dof % NX, g / dof / NX, g % dof);
+        q.nA = a.R - a.P;
+        q.R = q.nA + b.R - b.P;
+      }
+      q.P = (int)piv.size();
+      q.C = q.P + (int)bor.size() + 1;
+      if (q.P > q.R) return MIC_ERR_SOLVE;
+      q.col = (int64_t)pl.tab.size();
+      pl.tab.insert(pl.tab.end(), piv.begin(), piv.end());
+      pl.tab.insert(pl.tab.end(), bor.begin(), bor.end());
+      for (int c = 0; c < q.C - 1; ++c) pos[pl.tab[q.col + c]] = c;
+      q.map = (int64_t)pl.tab.size();
+      if (isleaf) {
+        for (int y = ty; y < tY; ++y)
+          for (int x = tx; x < tX; ++x)
+            for (int d = 0; d < dof; ++d) {
+              const int g = dof * (y * NX + x) + d;
+              pl.tab.push_back(touches(r, x, y, reach(dof, d)) ? pos[g] : -1);
+            }
+      } else {
+        pl.tab.resize(pl.tab.size() + 2 * (size_t)q.C, -1);
+        for (int k = 0; k < 2; ++k) {
+          const Front &c = pl.fronts[q.child + k];
+          int *m = pl.tab.data() + q.map + (size_t)k * q.C;
+          for (int s = c.P; s < c.C - 1; ++s) m[pos[pl.tab[c.col + s]]] = s - c.P;
+          m[q.C - 1] = c.C - 1 - c.P;
+        }
+      }
+      L.maxR = std::max(L.maxR, q.R);
+      L.maxP = std::max(L.maxP, q.P);
+      L.maxC = std::max(L.maxC, q.C);
+      L.minP = std::min(L.minP, q.P);
+    }
+    plan_level(L, pl.fronts, nsm);
+    if (!L.small && panel_columns(L.maxR) == 0) return MIC_ERR_SOLVE;
+    for (int i = L.first; i < L.first + L.count; ++i) {
+      Front &q = pl.fronts[i];
+      q.full = L.small ? 0 : 1;
+      q.f = L.nF;
+      L.nF += q.full ? (int64_t)q.R * q.C : (int64_t)(q.R - q.P) * (q.C - q.P);
+      q.u = pl.nU;
+      pl.nU += (int64_t)q.P * q.C;
+      if (q.full) {
+        q.lb = L.nL;
+        L.nL += (int64_t)q.R * 16;
+        q.act = pl.nAct;
+        pl.nAct += q.R;
+      }
+    }
+    pl.nF[l & 1] = std::max(pl.nF[l & 1], L.nF);
+    pl.nL = std::max(pl.nL, L.nL);
+  }
+  return MIC_OK;
+}
+
+int ensure_lu(mic_ctx *ctx, size_t need) {
+  if (ctx->lu_bytes >= need) return MIC_OK;
+  cudaFree(ctx->lu_buf);
+  ctx->lu_buf = nullptr;
+  ctx->lu_bytes = 0;
+  if (cudaMalloc(&ctx->lu_buf, need) != cudaSuccess) return MIC_ERR_NOMEM;
+  ctx->lu_bytes = need;
+  return MIC_OK;
+}
+
+template <typename T>
+T *carve(unsigned char *&p, size_t count) {
+  T *r = reinterpret_cast<T *>(p);
+  p += ((count * sizeof(T) + 255) / 256) * 256;
+  return r;
+}
+size_t room(size_t bytes) { return ((bytes + 255) / 256) * 256; }
+
+struct Buffers {
+  int *info;
+  double *F[2], *U, *Lb;
+  int *act;
+};
+
+template <int NB>
+int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, int parity) {
+  double *F = B.F[parity];
+  for (int k0 = 0; k0 < L.maxP; k0 += NB) {
+    const int rows = L.maxR - k0;
+    const int threads = std::min(1024, std::max(128, (rows + 31) / 32 * 32));
+    {
+      MIC_KERNEL(ctx, "k_front_panel");
+      k_front_panel<NB><<<L.count, threads, (size_t)rows * ((NB + 1) * sizeof(double) + sizeof(int)), ctx->stream>>>(
+          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act, pl.d_tab, B.info);
+    }
+    // a front's trailing columns: the most any front has (its panel may be narrower than NB)
+    const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
+    auto tiles = [&](int tr, int tc) { return (int64_t)((cols + tc - 1) / tc) * ((below + tr - 1) / tr) * L.count; };
+    MIC_KERNEL(ctx, "k_front_update");
+    if (tiles(128, 64) >= 3LL * sm_count(ctx))
+      k_front_update<NB, 128, 64><<<dim3(L.count, (below + 127) / 128, (cols + 63) / 64), kUpdateBlocks, 0, ctx->stream>>>(
+          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act);
+    else if (tiles(64, 32) >= 2LL * sm_count(ctx))
+      k_front_update<NB, 64, 32><<<dim3(L.count, (below + 63) / 64, (cols + 31) / 32), kUpdateBlocks, 0, ctx->stream>>>(
+          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act);
+    else
+      k_front_update<NB, 32, 32><<<dim3(L.count, (below + 31) / 32, (cols + 31) / 32), kUpdateBlocks, 0, ctx->stream>>>(
+          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act);
+  }
+  return MIC_OK;
+}
+
+// every launch of one solve, on the context's stream
+int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, const SystemRows &sys, double *x) {
+  const int nl = (int)pl.levels.size();
+  for (int l = nl - 1; l >= 0; --l) {
+    const Level &L = pl.levels[l];
+    const double *Fin = B.F[(l + 1) & 1];
+    if (L.small) {
+      MIC_KERNEL(ctx, "k_front_small");
+      k_front_small<<<L.count, kSmallThreads, L.smem_small, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act, sys,
+                                                                         Fin, B.F[l & 1], B.U, B.info);
+      continue;
+    }
+    {
+      MIC_KERNEL(ctx, "k_front_gather");
+      k_front_gather<<<dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act,
+                                                                              Fin, B.F[l & 1]);
+    }
+    int e = MIC_OK;
+    switch (panel_columns(L.maxR)) {
+      case 16: e = large_level<16>(ctx, pl, L, B, l & 1); break;
+      case 8: e = large_level<8>(ctx, pl, L, B, l & 1); break;
+      default: e = large_level<4>(ctx, pl, L, B, l & 1); break;
+    }
+    if (e) return e;
+  }
+  for (int l = 0; l < nl; ++l) {
+    const Level &L = pl.levels[l];
+    // border part apart once a front's P x B block is more than one SM should read
+    const bool apart = L.maxC > L.maxP + 1 && ((int64_t)L.maxP * (L.maxC - L.maxP) > 8192 || L.maxC > 4096);
+    if (apart) {
+      MIC_KERNEL(ctx, "k_front_border");
+      k_front_border<<<dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x);
+    }
+    MIC_KERNEL(ctx, "k_front_back");
+    const int threads = L.maxP <= 16 ? 128 : L.maxP <= 64 ? 256 : 1024;
+    k_front_back<<<L.count, threads, sizeof(double) * (apart ? L.maxP : L.maxC), ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x,
+                                                                            apart ? 0 : 1);
+  }
+  return MIC_OK;
+}
+
+cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
+  cudaError_t e = cudaFuncSetAttribute(k_front_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_panel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_panel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_panel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  return e;
+}
+
+}  // namespace
+
+void mic_front_plan_free(mic_front_plan *pl) {
+  if (!pl) return;
+  cudaFree(pl->d_fronts);
+  cudaFree(pl->d_tab);
+  delete pl;
+}
+
+// the plan of a system's grid, made with its first solve and kept with the system (the grid of a
+// context never changes)
+static int ensure_plan(mic_ctx *ctx, mic_system_store &S, int dof) {
+  if (S.plan) return MIC_OK;
+  mic_front_plan *pl = new (std::nothrow) mic_front_plan();
+  if (!pl) return MIC_ERR_NOMEM;
+  int e;
+  try {
+    e = build_plan(*pl, dof, ctx->P.NX, ctx->P.NY, sm_count(ctx));
+  } catch (const std::bad_alloc &) {
+    e = MIC_ERR_NOMEM;
+  }
+  if (e) {
+    delete pl;
+    return e;
+  }
+  const size_t fb = sizeof(Front) * pl->fronts.size(), tb = sizeof(int) * pl->tab.size();
+  if (cudaMalloc((void **)&pl->d_fronts, fb) != cudaSuccess || cudaMalloc((void **)&pl->d_tab, tb) != cudaSuccess) {
+    cudaGetLastError();
+    mic_front_plan_free(pl);
+    return MIC_ERR_NOMEM;
+  }
+  cudaError_t ce = allow_smem();
+  if (ce == cudaSuccess)
+    ce = cudaMemcpyAsync(pl->d_fronts, pl->fronts.data(), fb, cudaMemcpyHostToDevice, ctx->stream);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(pl->d_tab, pl->tab.data(), tb, cudaMemcpyHostToDevice, ctx->stream);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
+  if (ce != cudaSuccess) {
+    mic_front_plan_free(pl);
+    return mic_fail_cuda(ctx, ce);
+  }
+  std::vector<int>().swap(pl->tab);  // the device copy is the one that is used
+  std::vector<Front>().swap(pl->fronts);
+  S.plan = pl;
+  return MIC_OK;
+}
+
+extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
+  if (!ctx || which < 0 || which > 1) return MIC_ERR_ARG;
+  cudaSetDevice(ctx->device);
+  mic_system_store &S = ctx->sys[which];
+  if (!S.cnt) return MIC_ERR_ARG;
+  const int NX = ctx->P.NX, NY = ctx->P.NY;
+  const int dof = which == 0 ? 3 : 1;
+  const int64_t n = S.n;
+  const int transpose = NX > NY ? 1 : 0;
+  int e;
+  auto band_width = [&](int *bw) {
+    MIC_KERNEL(ctx, "k_band_width");
+    k_band_width<<<grid_for(n), kBlock, 0, ctx->stream>>>(S.cnt, S.col, S.width, n, dof, NX, NY, transpose, bw);
+  };
+  // the solver's size limit, a band of 1,016 below the diagonal: only a grid whose shorter side
+  // could reach it has its band measured first
+  constexpr int kMaxBand = 1016;
+  if (dof * (std::min(NX, NY) + 2) + 2 > kMaxBand) {
+    if ((e = ensure_lu(ctx, 4096))) return e;
+    int *bw = static_cast<int *>(ctx->lu_buf), h[2];
+    MIC_CUDA_TRY(cudaMemsetAsync(bw, 0, 2 * sizeof(int), ctx->stream));
+    band_width(bw);
+    MIC_CUDA_TRY(cudaMemcpyAsync(h, bw, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (h[0] > kMaxBand) return MIC_ERR_SOLVE;
+  }
+  if ((e = ensure_plan(ctx, S, dof))) return e;
+  const mic_front_plan &pl = *S.plan;
+  const size_t need = 256 + room(sizeof(double) * pl.nF[0]) + room(sizeof(double) * pl.nF[1]) +
+                      room(sizeof(double) * pl.nU) + room(sizeof(double) * pl.nL) + room(sizeof(int) * pl.nAct);
+  if ((e = ensure_lu(ctx, need))) return e;
+  double *out = nullptr;
+  if (which == 0) {
+    if (!ctx->solution && cudaMalloc((void **)&ctx->solution, sizeof(double) * n) != cudaSuccess) return MIC_ERR_NOMEM;
+    out = ctx->solution;
+  } else {
+    out = ctx->nodal[MIC_NF_THIST];
+  }
+  unsigned char *p = static_cast<unsigned char *>(ctx->lu_buf);
+  Buffers B;
+  B.info = carve<int>(p, kInfo);
+  B.F[0] = carve<double>(p, pl.nF[0]);
+  B.F[1] = carve<double>(p, pl.nF[1]);
+  B.U = carve<double>(p, pl.nU);
+  B.Lb = carve<double>(p, pl.nL);
+  B.act = carve<int>(p, pl.nAct);
+  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY};
+  MIC_CUDA_TRY(cudaMemsetAsync(B.info, 0x7f, sizeof(int), ctx->stream));
+  MIC_CUDA_TRY(cudaMemsetAsync(B.info + 1, 0, sizeof(int) * (kInfo - 1), ctx->stream));
+  band_width(B.info + 2);
+  // The launches are the same for every solve of a system: captured once as a graph and replayed,
+  // so host launch cost stays off the chain of levels.  Not while launches are being timed one by
+  // one.
+  const bool graphable = !ctx->prof_on;
+  if (graphable && S.lu_exec && S.lu_key_buf == ctx->lu_buf) {
+    MIC_CUDA_TRY(cudaGraphLaunch(S.lu_exec, ctx->stream));
+    ctx->launches += S.lu_nodes;
+  } else if (graphable && cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
+    const long long l0 = ctx->launches;
+    e = solve_launches(ctx, pl, B, sys, out);
+    cudaGraph_t g = nullptr;
+    const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
+    if (e || ce != cudaSuccess) {
+      if (g) cudaGraphDestroy(g);
+      return e ? e : mic_fail_cuda(ctx, ce);
+    }
+    if (S.lu_exec) cudaGraphExecDestroy(S.lu_exec);
+    S.lu_exec = nullptr;
+    const cudaError_t ie = cudaGraphInstantiate(&S.lu_exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ie != cudaSuccess) {
+      S.lu_exec = nullptr;
+      return mic_fail_cuda(ctx, ie);
+    }
+    S.lu_nodes = ctx->launches - l0;
+    S.lu_key_buf = ctx->lu_buf;
+    MIC_CUDA_TRY(cudaGraphLaunch(S.lu_exec, ctx->stream));
+  } else {
+    cudaGetLastError();  // a stream that cannot be captured: launch directly
+    if ((e = solve_launches(ctx, pl, B, sys, out))) return e;
+  }
+  MIC_CUDA_TRY(cudaGetLastError());
+  int h[kInfo];
+  MIC_CUDA_TRY(cudaMemcpyAsync(h, B.info, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  S.factored = 1;
+  S.kl = h[2];
+  S.ku = h[3];
+  return h[0] == 0x7f7f7f7f && h[1] == 0 ? MIC_OK : MIC_ERR_SOLVE;
+}
+
+extern "C" int mic_solution_get(mic_ctx *ctx, int which, double *out) {
+  if (!ctx || !out || which < 0 || which > 1) return MIC_ERR_ARG;
+  cudaSetDevice(ctx->device);
+  const int64_t nn = (int64_t)ctx->P.NX * ctx->P.NY;
+  const double *src = which == 0 ? ctx->solution : ctx->nodal[MIC_NF_THIST];
+  if (!src) return MIC_ERR_ARG;
+  MIC_CUDA_TRY(cudaMemcpyAsync(out, src, sizeof(double) * (which == 0 ? 3 * nn : nn), cudaMemcpyDeviceToHost,
+                               ctx->stream));
+  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return MIC_OK;
+}
+
+extern "C" int mic_system_band(mic_ctx *ctx, int which, int *kl, int *ku) {
+  if (!ctx || which < 0 || which > 1) return MIC_ERR_ARG;
+  if (kl) *kl = ctx->sys[which].kl;
+  if (ku) *ku = ctx->sys[which].ku;
+  return MIC_OK;
+}

@@ -83,7 +83,7 @@ struct Params {  // everything a kernel needs besides the marker columns; passed
 }  // namespace mic
 
 // one assembled linear system: rows of at most `width` (column, value) entries, the right-hand
-// side, and the banded factorisation state
+// side, and the direct solver's state
 struct mic_system_store {
   int64_t n;
   int width;
@@ -91,13 +91,11 @@ struct mic_system_store {
   double *val, *rhs;
   double Kbond, Kcont;
   int factored;
-  int kl, ku;       // band widths of the last factorisation
-  int zero_pivot;   // first zero pivot of the last factorisation (-1: none)
-  // the factorisation's launches captured as a graph, valid for this buffer, size, band, panel
+  int kl, ku;       // band widths of the matrix in grid order
+  struct mic_front_plan *plan;  // the solver's fronts on this grid (mic_front_lu.cu)
+  // the solve's launches captured as a graph, valid for this buffer
   cudaGraphExec_t lu_exec;
   const void *lu_key_buf;
-  int64_t lu_key_n;
-  int lu_key_kl, lu_key_ku, lu_key_nb;
   long long lu_nodes;
 };
 
@@ -130,10 +128,8 @@ struct mic_ctx {
   mic_system_store sys[2];    // assembled systems: 0 Stokes (vep_system.c), 1 thermal
   void *sys_scratch;          // assembly scratch: geometry tables, scaled viscosities
   size_t sys_scratch_bytes;
-  void *lu_buf;               // banded factorisation storage (grown on demand)
+  void *lu_buf;               // the direct solver's storage (grown on demand)
   size_t lu_bytes;
-  cudaStream_t lu_side;       // second stream of the factorisation: the far part of each update
-  cudaEvent_t lu_ev[2];       // its two hand-offs (trsm done, far update done)
   cudaStream_t aux;           // second stream of a projection: its cell-centre partial sums run
   cudaEvent_t aux_ev[2];      // beside the basic-cell ones (fork, join)
   size_t io_bytes;
@@ -209,6 +205,7 @@ int mic_ensure_sorted(mic_ctx *ctx);  // bins + sorts if positions changed since
 // centres (stag -1), divided by the weights
 int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cudaStream_t s = nullptr);
 void mic_invalidate_sort(mic_ctx *ctx);
+void mic_front_plan_free(mic_front_plan *plan);  // (mic_front_lu.cu)
 int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out);
 int mic_ensure_geometry(mic_ctx *ctx);  // sorted columns + projection geometry
 // projectMarkersNodesAll2 again after a full pass on unchanged positions, densities, temperatures

@@ -349,12 +349,13 @@ int mic_form_thermal_system(mic_ctx *ctx, const mic_subduction_options *options,
 int mic_system_size(mic_ctx *ctx, int which, int64_t *nrows, int64_t *nnz);
 int mic_system_get(mic_ctx *ctx, int which, int32_t *rowptr, int32_t *cols, double *vals, double *rhs);
 /* kspLinearSolve (kspLinearSolve.c:13) as the reference's option files run it (preonly + LU,
- * option_files/run_mumps.petscopt): a direct solve on the device, banded LU with partial
- * pivoting.  The Stokes solution stays on the device for mic_retrieve_solutions(ctx, NULL, ...);
+ * option_files/run_mumps.petscopt): a direct solve on the device, LU with partial pivoting in
+ * nested-dissection order.  The Stokes solution stays on the device for mic_retrieve_solutions(ctx, NULL, ...);
  * the temperature goes to MIC_NF_THIST.  MIC_ERR_SOLVE for a zero pivot. */
 int mic_linear_solve(mic_ctx *ctx, int which);
 int mic_solution_get(mic_ctx *ctx, int which, double *out);
-/* band widths (lower, upper) the last solve of a system factorised */
+/* band widths (lower, upper) of the matrix the last solve of a system factorised, nodes numbered
+ * along the shorter grid side */
 int mic_system_band(mic_ctx *ctx, int which, int *kl, int *ku);
 
 /* One time step of main_subduction.c (227-460) without PETSc, everything on the device:
