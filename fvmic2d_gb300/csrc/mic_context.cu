@@ -166,6 +166,9 @@ static void free_ctx(mic_ctx *ctx) {
   }
   cudaFree(ctx->sys_scratch);
   cudaFree(ctx->lu_buf);
+  if (ctx->lu_chain) cudaStreamDestroy(ctx->lu_chain);
+  for (cudaEvent_t v : ctx->lu_ev)
+    if (v) cudaEventDestroy(v);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
   for (int k = 0; k < 2; ++k)
     if (ctx->aux_ev[k]) cudaEventDestroy(ctx->aux_ev[k]);

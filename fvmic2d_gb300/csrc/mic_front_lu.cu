@@ -29,11 +29,13 @@
 //   small  the front in shared memory, one block per front, unblocked (k_front_small);
 //   large  the front in global memory, panels of NB columns: one block per front factors a panel
 //          in shared memory (k_front_panel), then the trailing tiles of every front are updated,
-//          each block forming its own piece of U12 (k_front_update).
+//          each block forming its own piece of U12 (k_front_update): the next panel's columns
+//          first, the rest beside the next panel's factorisation.
 // FP64 multiply-adds bound the updates (2 per SM and clock); the panels and the small fronts are
 // bound by the latency of their column steps.  One CUDA graph holds all launches of a solve.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <iterator>
 #include <new>
 #include <vector>
@@ -54,7 +56,9 @@ struct Front {
   int64_t lb;   // panel buffer (doubles)
   int64_t col;  // the pivots' and the border's unknowns (ints, C - 1)
   int64_t map;  // child columns of this front's columns (2 C ints), or a leaf's slot table
-  int64_t act;  // row list of a front in panels (ints, R): pivot rows in order, then the others
+  int64_t act;  // two row lists of a front in panels (ints, 2 R), written in turn by its panels:
+                // pivot rows in order, then the others
+  int64_t left; // the left-over rows in the list its last panel wrote
 };
 
 // info[0]: smallest unknown with a zero pivot; info[1]: entries outside the assumed stencils;
@@ -104,18 +108,38 @@ __device__ __forceinline__ int pivot_key(double a) {
   return h <= 0x7ff00000 ? h : -1;
 }
 
-// a column whose keys are all zero (every |a| below 2^-1042): the exact largest |a|, in order
-__device__ int pivot_slow(const double *col, int stride, int r0, int r1) {
-  long long best = -1;
-  int p = r0;
-  for (int r = r0; r < r1; ++r) {
+// a column whose best key is 0 or none (every |a| below 2^-1042, or NaN): the exact largest |a| of
+// the rows not used, the first of them when there is no other
+__device__ int pivot_rare(const double *col, int stride, int rows, const int *used) {
+  long long best = -2;
+  int p = 0;
+  for (int r = 0; r < rows; ++r) {
+    if (used && used[r]) continue;
     const long long b = dbits(col[(int64_t)r * stride]) & 0x7fffffffffffffffLL;
-    if (b > best && b <= 0x7ff0000000000000LL) {
-      best = b;
+    const long long k = b <= 0x7ff0000000000000LL ? b : -1;
+    if (k > best) {
+      best = k;
       p = r;
     }
   }
   return p;
+}
+
+// 1 / p by Newton's iteration of third order from an FP32 reciprocal of p's mantissa: with
+// e = 1 - m r, |e| < 2^-22, r (1 + e + e^2) is 1 / m to e^3 < 2^-66, so to rounding, in three
+// dependent FP64 operations (a pivot's reciprocal is on the chain of every column step).  Pivots
+// whose reciprocal leaves the normal range are divided.
+__device__ __forceinline__ double pivot_rcp(double p) {
+  const unsigned long long b = (unsigned long long)dbits(p);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  if (ex < 8 || ex > 2038) return p != 0.0 ? 1.0 / p : 0.0;
+  const double m = __longlong_as_double((long long)((b & 0xfffffffffffffULL) | 0x3ff0000000000000ULL));
+  const float f = __uint_as_float(0x3f800000u | ((unsigned)(b >> 29) & 0x7fffffu));
+  const double r0 = f64_of(__frcp_rn(f));
+  const double e = fma(-m, r0, 1.0);
+  const double r = fma(r0, fma(e, e, e), r0);  // in (1/2, 1]
+  const long long rb = dbits(r) - ((long long)(ex - 1023) << 52);
+  return __longlong_as_double(rb | (long long)(b & 0x8000000000000000ULL));
 }
 
 // (key, row) of the warp's best lane, in every lane
@@ -127,7 +151,7 @@ __device__ __forceinline__ int2 warp_best(int key, int row) {
 
 // value of column c (of q's columns) in left-over row i of child k: where the child keeps it
 __device__ __forceinline__ const double *child_row(const Front &k, int i, const double *F, const int *act) {
-  return k.full ? F + k.f + (int64_t)act[k.act + k.P + i] * k.C + k.P : F + k.f + (int64_t)i * (k.C - k.P);
+  return k.full ? F + k.f + (int64_t)act[k.left + i] * k.C + k.P : F + k.f + (int64_t)i * (k.C - k.P);
 }
 
 // ---- small fronts ------------------------------------------------------------------------
@@ -137,14 +161,16 @@ __device__ __forceinline__ const double *child_row(const Front &k, int i, const 
 // once, then a lane takes a row (its multiplier in a register) and the warps share out rows and
 // columns; the warps that update column j + 1 also find its candidates.  Two barriers a step.
 // The step is bound by this chain (about 1 us) until a front exceeds some 50,000 multiply-adds,
-// then by the FP64 pipe.
-constexpr int kSmallThreads = 256, kSmallWarps = kSmallThreads / 32;
-
+// then by the FP64 pipe.  A row's values are read four at a time before any is written: the
+// compiler cannot tell the row from the pivot row, so a load written after a store would wait
+// for it.
+template <int kSmallThreads>
 __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__restrict__ fr, int first,
                                                               const int *__restrict__ tab,
                                                               const int *__restrict__ act, SystemRows sys,
                                                               const double *__restrict__ Fin, double *F, double *U,
                                                               int *info) {
+  constexpr int kSmallWarps = kSmallThreads / 32;
   extern __shared__ double A[];
   __shared__ int2 red[32];
   __shared__ double s_rcp;
@@ -195,9 +221,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   for (int j = 0; j < P; ++j) {
     const int2 e = lane < G ? red[lane] : make_int2(-1, j);
     const int2 best = warp_best(e.x, e.y);
-    int p = best.x < 0 ? j : best.y;  // all NaN: keep the diagonal
-    if (best.x == 0) {
-      p = pivot_slow(A + j, ld, j, R);
+    int p = best.y;
+    if (best.x <= 0) {
+      p = j + pivot_rare(A + j * ld + j, ld, R - j, nullptr);
       __syncthreads();  // every thread has read the column before rows move
     }
     for (int c = j + tid; c < C; c += kSmallThreads) {
@@ -205,7 +231,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
       A[j * ld + c] = up;
       A[p * ld + c] = dn;
       if (c == j) {
-        s_rcp = up != 0.0 ? 1.0 / up : 0.0;
+        s_rcp = pivot_rcp(up);
         if (up == 0.0) atomicMin(&info[0], tab[q.col + j]);
       }
     }
@@ -231,7 +257,16 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
         c += SL;
       }
       if (r < R) {
-#pragma unroll 4
+        for (; c + 3 * SL < C; c += 4 * SL) {
+          double v[4], u[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            v[i] = row[c + i * SL];
+            u[i] = piv[c + i * SL];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) row[c + i * SL] = v[i] - l * u[i];
+        }
         for (; c < C; c += SL) row[c] -= l * piv[c];
       }
     }
@@ -265,28 +300,53 @@ __global__ void __launch_bounds__(256) k_front_gather(const Front *__restrict__ 
 }
 
 // One panel: columns k0 .. k0 + NB - 1 of the rows not yet pivots, one block per front, the panel
-// in shared memory (odd stride NB + 1).  A thread keeps the same rows through a step: it forms
-// their multipliers, updates column j + 1 first and offers its best row for it, then the rest, so
-// that the search overlaps the update.  Rows move only inside the panel (with their numbers); in
-// the front they stay where they are, and the row list says which are pivots.
+// in shared memory (odd stride NB + 1).  Rows stay where they are; a list of the pivots' rows
+// stands for their interchanges, and the front's row list says which are pivots.
+// What bounds it is one SM's FP64 rate (a warp's FP64 instruction holds its quarter of the SM for
+// 64 cycles, measured) and the latency of the step, so a step j has two phases with a barrier
+// after each:
+//   each thread its rows' multipliers and their column j + 1, the warps' best rows for it;
+//   the other columns, shared out over all warps by rows and columns; meanwhile one warp forms
+//   the next pivot's reciprocal, which needs column j + 1 only.
+// Global loads go out in batches, and values are read four at a time before any is written (the
+// compiler cannot tell a row from the pivot row).
+constexpr int kPanelThreads = 512;
+constexpr int kPanelBytes = 8;  // per row besides its values: its number, whether it is a pivot
 template <int NB>
-__global__ void __launch_bounds__(1024) k_front_panel(const Front *__restrict__ fr, int first, int k0,
-                                                     const double *__restrict__ F, double *U, double *Lb, int *act,
-                                                     const int *__restrict__ tab, int *info) {
+__global__ void __launch_bounds__(kPanelThreads, 2)
+    k_front_panel(const Front *__restrict__ fr, int first, int k0, int turn, const double *__restrict__ F, double *U,
+                  double *Lb, int *act, const int *__restrict__ tab, int *info) {
   extern __shared__ double S[];
   __shared__ int2 red[32];
   __shared__ double s_rcp;
+  __shared__ int piv[NB];  // rows of the pivots so far
   const Front q = fr[first + blockIdx.x];
   if (k0 >= q.P) return;
-  constexpr int LD = NB + 1;
+  constexpr int LD = NB + 1, RW = 32 / NB, BATCH = 8;  // rows a warp loads at once, and how often
   const int nb = min(NB, q.P - k0), na = q.R - k0;
-  int *id = reinterpret_cast<int *>(S + (int64_t)na * LD);
+  int *id = reinterpret_cast<int *>(S + (int64_t)na * LD), *used = id + na;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  for (int r = tid; r < na; r += nt) id[r] = act[q.act + k0 + r];
-  __syncthreads();
-  for (int e = tid; e < na * NB; e += nt) {
-    const int r = e / NB, c = e % NB;
-    S[r * LD + c] = c < nb ? F[q.f + (int64_t)id[r] * q.C + k0 + c] : 0.0;
+  const int *list = act + q.act + (int64_t)turn * q.R + k0;
+  int *out = act + q.act + (int64_t)(1 - turn) * q.R + k0;
+  {
+    const int lc = lane % NB;
+    for (int r0 = warp * RW + lane / NB; r0 < na; r0 += nw * RW * BATCH) {
+      int k[BATCH];
+      double v[BATCH];
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) k[i] = r0 + i * nw * RW < na ? list[r0 + i * nw * RW] : -1;
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) v[i] = (k[i] >= 0 && lc < nb) ? F[q.f + (int64_t)k[i] * q.C + k0 + lc] : 0.0;
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i)
+        if (k[i] >= 0) {
+          S[(r0 + i * nw * RW) * LD + lc] = v[i];
+          if (lc == 0) {
+            id[r0 + i * nw * RW] = k[i];
+            used[r0 + i * nw * RW] = 0;
+          }
+        }
+    }
   }
   __syncthreads();
   int key = -1, who = 0;
@@ -297,129 +357,231 @@ __global__ void __launch_bounds__(1024) k_front_panel(const Front *__restrict__ 
       who = r;
     }
   }
-  for (int j = 0; j < nb; ++j) {
-    const int2 mine = warp_best(key, who);
-    if (lane == 0) red[warp] = mine;
-    __syncthreads();
-    const int2 e = lane < nw ? red[lane] : make_int2(-1, j);
-    const int2 best = warp_best(e.x, e.y);
-    int p = best.x < 0 ? j : best.y;
-    if (best.x == 0) {
-      p = pivot_slow(S + j, LD, j, na);
-      __syncthreads();  // every thread has read the column before rows move
-    }
-    if (warp == 0) {
-      if (lane < NB) {
-        const double up = S[p * LD + lane], dn = S[j * LD + lane];
-        S[j * LD + lane] = up;
-        S[p * LD + lane] = dn;
-        if (lane == j) {
-          s_rcp = up != 0.0 ? 1.0 / up : 0.0;
-          if (up == 0.0) atomicMin(&info[0], tab[q.col + k0 + j]);
+  // row groups and column shares of phase 2; the reciprocal's warp takes part only where there is
+  // more work than the others can share evenly
+  const int G = (na + 31) / 32, workers = G >= nw ? nw : nw - 1, CS = max(1, workers / G);
+  unsigned mine = 0;  // which of this thread's rows are pivots
+  for (int j = -1; j < nb; ++j) {
+    // phase 1 of step j (none before the first): multipliers, column j + 1
+    if (j >= 0) {
+      const double rcp = s_rcp;
+      const int p = piv[j];
+      const bool more = j + 1 < nb;
+      key = -1;
+      who = 0;
+      const double pn = more ? S[p * LD + j + 1] : 0.0;
+      unsigned bit = 1;
+      for (int r = tid; r < na; r += nt, bit <<= 1) {
+        if (r == p) {
+          mine |= bit;
+          used[r] = 1;
         }
-      } else if (lane == NB) {
-        const int t = id[j];
-        id[j] = id[p];
-        id[p] = t;
+        if (mine & bit) continue;
+        double *row = S + r * LD;
+        const double aj = row[j], an = more ? row[j + 1] : 0.0, l = aj * rcp;
+        row[j] = l;
+        if (more) {
+          const double v = an - l * pn;
+          row[j + 1] = v;
+          const int k = pivot_key(v);
+          if (k > key) {
+            key = k;
+            who = r;
+          }
+        }
+      }
+    }
+    if (j + 1 == nb) break;
+    const int2 offer = warp_best(key, who);
+    if (lane == 0) red[warp] = offer;
+    __syncthreads();
+    // phase 2: the pivot of column j + 1 and its reciprocal; the columns after it
+    if (warp == nw - 1) {
+      const int2 e = lane < nw ? red[lane] : make_int2(-1, 0);
+      const int2 best = warp_best(e.x, e.y);
+      int p = best.y;
+      if (best.x <= 0) p = pivot_rare(S + j + 1, LD, na, used);
+      if (lane == 0) {
+        const double v = S[p * LD + j + 1];
+        s_rcp = pivot_rcp(v);
+        piv[j + 1] = p;
+        if ((dbits(v) << 1) == 0) atomicMin(&info[0], tab[q.col + k0 + j + 1]);
+      }
+    }
+    if (j >= 0) {
+      const double *pr = S + piv[j] * LD;
+      for (int t = warp; t < G * CS; t += workers) {
+        const int r = (t % G) * 32 + lane;
+        if (warp >= workers || r >= na || used[r]) continue;
+        double *row = S + r * LD;
+        const double l = row[j];
+        for (int c = j + 2 + t / G; c < nb; c += 4 * CS) {
+          double v[4], u[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int ci = c + i * CS;
+            v[i] = ci < nb ? row[ci] : 0.0;
+            u[i] = ci < nb ? pr[ci] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (c + i * CS < nb) row[c + i * CS] = v[i] - l * u[i];
+        }
       }
     }
     __syncthreads();
-    const double rcp = s_rcp;
-    key = -1;
-    who = 0;
-    for (int r = j + 1 + tid; r < na; r += nt) {
-      double *row = S + r * LD;
-      const double *piv = S + j * LD;
-      const double l = row[j] * rcp;
-      row[j] = l;
-      if (j + 1 < nb) {
-        const double v = row[j + 1] - l * piv[j + 1];
-        row[j + 1] = v;
-        const int k = pivot_key(v);
-        if (k > key) {
-          key = k;
-          who = r;
-        }
-#pragma unroll 4
-        for (int c = j + 2; c < NB; ++c) row[c] -= l * piv[c];
-      }
-    }
   }
   __syncthreads();
-  for (int e = tid; e < nb * NB; e += nt) {  // U11
-    const int r = e / NB, c = e % NB;
-    if (c >= r && c < nb) U[q.u + (int64_t)(k0 + r) * q.C + k0 + c] = S[r * LD + c];
+  for (int e = tid; e < nb * NB; e += nt) {  // the pivots in order: U11 and the multipliers before it
+    const int k = e / NB, c = e % NB;
+    const double v = c < nb ? S[piv[k] * LD + c] : 0.0;
+    if (c >= k && c < nb) U[q.u + (int64_t)(k0 + k) * q.C + k0 + c] = v;
+    Lb[q.lb + e] = c < k ? v : 0.0;
+    if (c == 0) out[k] = id[piv[k]];
   }
-  for (int e = tid; e < na * NB; e += nt) {  // multipliers (below the pivots), rows in list order
-    const int r = e / NB, c = e % NB;
-    Lb[q.lb + e] = (c < nb && r > c) ? S[r * LD + c] : 0.0;
+  {  // the other rows in their order behind them
+    const int lc = lane % NB;
+    for (int r = warp * RW + lane / NB; r < na; r += nw * RW) {
+      if (used[r]) continue;
+      int pos = nb + r;
+#pragma unroll
+      for (int k = 0; k < NB; ++k) pos -= k < nb && piv[k] < r;
+      Lb[q.lb + (int64_t)pos * NB + lc] = lc < nb ? S[r * LD + lc] : 0.0;
+      if (lc == 0) out[pos] = id[r];
+    }
   }
-  for (int r = tid; r < na; r += nt) act[q.act + k0 + r] = id[r];
 }
 
-// U12 = L11^-1 A12 and A22 -= L21 U12 for the columns right of the panel, TR x TC tiles.  Each
-// block forms U12 of its own columns (NB^2 / 2 multiply-adds a column against NB TR for the tile:
-// 6% more work at TR = 128, 25% at 32, for one launch and one wait less per panel); the first row
-// of tiles also stores it.  The FP64 pipe is the bound: small tiles where there are too few large
-// ones to fill the SMs.
-template <int NB, int TR, int TC>
-__global__ void __launch_bounds__(256) k_front_update(const Front *__restrict__ fr, int first, int k0, double *F,
-                                                     double *U, const double *__restrict__ Lb,
-                                                     const int *__restrict__ act) {
-  constexpr int RT = TR / 16, CT = TC / 16;  // a thread's rows and columns
+// U12 = L11^-1 A12 of TC columns in shared memory, NB rows: four lanes a column, each every fourth
+// row, so that all warps take part (a warp's FP64 instruction holds a quarter of the SM for 64
+// cycles, whatever its lanes).  Threads from 4 TC on return; store: also to U.
+template <int NB, int TC>
+__device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB + 1], int tid, double *u_out, int ldu,
+                                          int nb, int cols, bool store) {
+  if (tid >= 4 * TC) return;  // whole warps
+  constexpr int PER = NB / 4;
+  const int part = tid & 3, c = tid >> 2;
+  double u[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) u[i] = Us[4 * i + part][c];
+#pragma unroll
+  for (int j = 0; j < NB - 1; ++j) {
+    const double uj = __shfl_sync(0xffffffffu, u[j / 4], (tid & 28) | (j & 3));
+#pragma unroll
+    for (int i = j / 4; i < PER; ++i)
+      if (4 * i + part > j) u[i] -= L11[4 * i + part][j] * uj;
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int k = 4 * i + part;
+    Us[k][c] = u[i];
+    if (store && k < nb && c < cols) u_out[(int64_t)k * ldu + c] = u[i];
+  }
+}
+
+// U12 of a panel apart, for updates so large that every tile forming its own piece would cost more
+// than a launch
+template <int NB>
+__global__ void __launch_bounds__(256) k_front_solve(const Front *__restrict__ fr, int first, int k0, int turn,
+                                                    const double *__restrict__ F, double *U,
+                                                    const double *__restrict__ Lb, const int *__restrict__ act) {
+  constexpr int TC = 64;
   __shared__ double Us[NB][TC + 1];
-  __shared__ double Ls[TR][NB + 1];
   __shared__ double L11[NB][NB + 1];
   const Front q = fr[first + blockIdx.x];
   if (k0 >= q.P) return;
+  const int nb = min(NB, q.P - k0), c0 = k0 + nb + blockIdx.y * TC, tid = threadIdx.x;
+  if (c0 >= q.C) return;
+  const int *list = act + q.act + (int64_t)(1 - turn) * q.R + k0;
+  double u[NB * TC / 256], l1 = 0.0;
+#pragma unroll
+  for (int i = 0; i < NB * TC / 256; ++i) {
+    const int e = tid + 256 * i, k = e / TC, c = c0 + e % TC;
+    u[i] = (k < nb && c < q.C) ? F[q.f + (int64_t)list[k] * q.C + c] : 0.0;
+  }
+  if (tid < NB * NB && tid / NB < nb) l1 = Lb[q.lb + tid];
+#pragma unroll
+  for (int i = 0; i < NB * TC / 256; ++i) Us[(tid + 256 * i) / TC][(tid + 256 * i) % TC] = u[i];
+  if (tid < NB * NB) L11[tid / NB][tid % NB] = l1;
+  __syncthreads();
+  solve_u12<NB, TC>(Us, L11, tid, U + q.u + (int64_t)k0 * q.C + c0, q.C, nb, q.C - c0, true);
+}
+
+// A22 -= L21 U12 for columns right of the panel, TR x TC tiles.  SOLVE: each block forms U12 of its
+// own columns (NB^2 / 2 multiply-adds a column against NB TR for the tile: 25% more work at
+// TR = 32, for one launch and one wait less per panel), and the first row of tiles stores it;
+// otherwise U12 is in U.  The FP64 pipe is the bound: small tiles where there are too few large
+// ones to fill the SMs evenly.  Columns coff .. coff + clen - 1 of those right of the panel: the
+// next panel's columns go first, on the chain of panels, the others beside the next panel's
+// factorisation.
+template <int NB, int TR, int TC, bool SOLVE>
+__global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
+    k_front_update(const Front *__restrict__ fr, int first, int k0, int turn, int coff, int clen, double *F, double *U,
+                   const double *__restrict__ Lb, const int *__restrict__ act) {
+  constexpr int RT = TR / 16, CT = TC / 16;  // a thread's rows and columns
+  __shared__ double Us[NB][TC + 1];
+  __shared__ double Ls[TR][NB + 1];
+  __shared__ double L11[SOLVE ? NB : 1][NB + 1];
+  const Front q = fr[first + blockIdx.x];
+  if (k0 >= q.P) return;
   const int nb = min(NB, q.P - k0);
-  const int c0 = k0 + nb + blockIdx.z * TC, r0 = nb + blockIdx.y * TR, na = q.R - k0;
-  if (c0 >= q.C || (r0 >= na && blockIdx.y > 0)) return;
+  const int cend = min(q.C, k0 + nb + coff + clen);
+  const int c0 = k0 + nb + coff + blockIdx.z * TC, r0 = nb + blockIdx.y * TR, na = q.R - k0;
+  if (c0 >= cend || (r0 >= na && (blockIdx.y > 0 || !SOLVE))) return;
   const int tid = threadIdx.x, ti = tid / 16, tj = tid % 16;
-  const int *list = act + q.act + k0;
+  const int *list = act + q.act + (int64_t)(1 - turn) * q.R + k0;
   double *base = F + q.f;
   const double *L = Lb + q.lb;
-  // the tile itself first: its loads overlap the triangular solve
+  // every load in flight before the first is stored or used
   double v[RT][CT];
   int64_t at[RT];
 #pragma unroll
   for (int a = 0; a < RT; ++a) {
     const int r = r0 + ti + 16 * a;
     at[a] = r < na ? (int64_t)list[r] * q.C : -1;
+  }
+#pragma unroll
+  for (int a = 0; a < RT; ++a)
 #pragma unroll
     for (int b = 0; b < CT; ++b) {
       const int c = c0 + tj + 16 * b;
-      v[a][b] = (at[a] >= 0 && c < q.C) ? base[at[a] + c] : 0.0;
+      v[a][b] = (at[a] >= 0 && c < cend) ? base[at[a] + c] : 0.0;
     }
-  }
-  for (int e = tid; e < NB * TC; e += 256) {
-    const int k = e / TC, c = c0 + e % TC;
-    Us[k][e % TC] = (k < nb && c < q.C) ? base[(int64_t)list[k] * q.C + c] : 0.0;
-  }
-  for (int e = tid; e < NB * NB; e += 256) L11[e / NB][e % NB] = e / NB < nb ? L[e] : 0.0;
-  for (int e = tid; e < TR * NB; e += 256) {
-    const int r = r0 + e / NB;
-    Ls[e / NB][e % NB] = r < na ? L[(int64_t)r * NB + e % NB] : 0.0;
+  {
+    constexpr int NU = (NB * TC + 255) / 256, NL = (TR * NB + 255) / 256;
+    double u[NU], l[NL], l1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      const int e = tid + 256 * i, k = e / TC, c = c0 + e % TC;
+      const bool in = e < NB * TC && k < nb && c < cend;
+      if (SOLVE)
+        u[i] = in ? base[(int64_t)list[k] * q.C + c] : 0.0;
+      else
+        u[i] = in ? U[q.u + (int64_t)(k0 + k) * q.C + c] : 0.0;
+    }
+    if (SOLVE && tid < NB * NB && tid / NB < nb) l1 = L[tid];
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+      const int e = tid + 256 * i, r = r0 + e / NB;
+      l[i] = (e < TR * NB && r < na) ? L[(int64_t)r * NB + e % NB] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      const int e = tid + 256 * i;
+      if (e < NB * TC) Us[e / TC][e % TC] = u[i];
+    }
+    if (SOLVE && tid < NB * NB) L11[tid / NB][tid % NB] = l1;
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+      const int e = tid + 256 * i;
+      if (e < TR * NB) Ls[e / NB][e % NB] = l[i];
+    }
   }
   __syncthreads();
-  if (tid < TC) {
-    double u[NB];
-#pragma unroll
-    for (int k = 0; k < NB; ++k) u[k] = Us[k][tid];
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-#pragma unroll
-      for (int k = j + 1; k < NB; ++k) u[k] -= L11[k][j] * u[j];
-    }
-#pragma unroll
-    for (int k = 0; k < NB; ++k) Us[k][tid] = u[k];
-    if (blockIdx.y == 0 && c0 + tid < q.C) {
-#pragma unroll
-      for (int k = 0; k < NB; ++k)
-        if (k < nb) U[q.u + (int64_t)(k0 + k) * q.C + c0 + tid] = u[k];
-    }
+  if (SOLVE) {
+    solve_u12<NB, TC>(Us, L11, tid, U + q.u + (int64_t)k0 * q.C + c0, q.C, nb, cend - c0, blockIdx.y == 0);
+    __syncthreads();
   }
-  __syncthreads();
 #pragma unroll 4
   for (int k = 0; k < NB; ++k) {
     double l[RT], u[CT];
@@ -437,7 +599,7 @@ __global__ void __launch_bounds__(256) k_front_update(const Front *__restrict__ 
 #pragma unroll
     for (int b = 0; b < CT; ++b) {
       const int c = c0 + tj + 16 * b;
-      if (at[a] >= 0 && c < q.C) base[at[a] + c] = v[a][b];
+      if (at[a] >= 0 && c < cend) base[at[a] + c] = v[a][b];
     }
 }
 
@@ -539,7 +701,7 @@ constexpr int kUpdateBlocks = 256;
 
 int panel_columns(int maxR) {  // panel width: the widest whose panel fits shared memory
   for (int nb : {16, 8, 4})
-    if ((size_t)maxR * ((nb + 1) * sizeof(double) + sizeof(int)) <= kMaxSmem) return nb;
+    if ((size_t)maxR * ((nb + 1) * sizeof(double) + kPanelBytes) <= kMaxSmem) return nb;
   return 0;
 }
 
@@ -557,22 +719,25 @@ struct mic_front_plan {
 
 namespace {
 
-// The level's form.  Small: blocks share the SMs, each front's multiply-adds on one SM (2 per
-// clock), about 1.1 us a column step.  Large: multiply-adds over all SMs at about 70% of the pipe,
-// 14 us a panel of 16 columns for its factorisation, its update's launch and its tail, 6 us for
-// the gather.  (Both sides measured on the levels of the 129 x 33 and 513 x 129 systems.)
+// The level's form, by estimated time (us).  Small: a front's multiply-adds on one SM (2 per
+// clock), 1.5 us a column step, 8 us to load and store.  Large: per panel of 16 columns, 28 us for
+// its factorisation and the launches, and the update's 32 x 32 tiles (padding included) over all
+// SMs at 5.4 us a tile; 9 us for the gather.  Measured on the levels of five systems: the lines
+// cross near 60 fronts of 100 x 170 (241 us small, 230 large); 256 fronts of 52 x 90 take 81 us
+// small and 280 large, 16 of 80 x 133 take 134 us small and 98 large.
 void plan_level(Level &L, const std::vector<Front> &fr, int nsm) {
-  double total = 0, most = 0;
+  double total = 0, most = 0, large = 9.0;
   for (int i = L.first; i < L.first + L.count; ++i) {
     double w = 0;
     for (int j = 0; j < fr[i].P; ++j) w += double(fr[i].R - j - 1) * (fr[i].C - j - 1);
     total += w;
     most = std::max(most, w);
+    for (int k1 = 16; k1 < fr[i].P + 16; k1 += 16)
+      large += 5.4 / nsm * ((fr[i].R - std::min(k1, fr[i].P) + 31) / 32) * ((fr[i].C - std::min(k1, fr[i].P) + 31) / 32);
   }
-  const double clk = 1.9e3;  // per us
-  const double waves = (L.count + nsm - 1) / nsm;
-  const double small = std::max(waves * most, total / nsm) / 2 / clk * 1.25 + 1.1 * L.maxP;
-  const double large = total / (2.0 * nsm * clk) / 0.7 + 14.0 * ((L.maxP + 15) / 16) + 6.0;
+  large += 28.0 * ((L.maxP + 15) / 16);
+  const double waves = (L.count + nsm - 1) / nsm, clk = 1.9e3;
+  const double small = std::max(waves * most, total / nsm) / 2 / clk * 1.3 + 1.5 * L.maxP + 8.0;
   L.smem_small = (size_t)L.maxR * (L.maxC | 1) * sizeof(double);
   L.small = L.smem_small <= kMaxSmem && L.maxR <= 1024 && (fr[L.first].child < 0 || small <= large);
 }
@@ -686,8 +851,10 @@ int build_plan(mic_front_plan &pl, int dof, int NX, int NY, int nsm) {
       if (q.full) {
         q.lb = L.nL;
         L.nL += (int64_t)q.R * 16;
+        const int nb = panel_columns(L.maxR), panels = (q.P + nb - 1) / nb;
         q.act = pl.nAct;
-        pl.nAct += q.R;
+        q.left = q.act + (panels & 1 ? q.R : 0) + q.P;
+        pl.nAct += 2 * q.R;
       }
     }
     pl.nF[l & 1] = std::max(pl.nF[l & 1], L.nF);
@@ -720,31 +887,78 @@ struct Buffers {
   int *act;
 };
 
+template <int NB, int TR, int TC, bool SOLVE>
+void update(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, double *F, int k0, int turn,
+            int rows, int coff, int cols, cudaStream_t st) {
+  MIC_KERNEL_ON(ctx, "k_front_update", st);
+  k_front_update<NB, TR, TC, SOLVE>
+      <<<dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC), kUpdateBlocks, 0, st>>>(
+          pl.d_fronts, L.first, k0, turn, coff, cols, F, B.U, B.Lb + turn * pl.nL, B.act);
+}
+
+// One level in panels.  The chain (panel, then its update of the next panel's columns) runs on the
+// context's high-priority stream; the rest of each update runs on the main stream beside the next
+// panel, and the next panel's own update waits for it.  Row lists and panel buffers alternate, so
+// a panel does not overwrite what the update before it still reads.
 template <int NB>
-int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, int parity) {
-  double *F = B.F[parity];
-  for (int k0 = 0; k0 < L.maxP; k0 += NB) {
+int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, double *F) {
+  cudaStream_t main = ctx->stream, chain = ctx->lu_chain;
+  MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], main));
+  MIC_CUDA_TRY(cudaStreamWaitEvent(chain, ctx->lu_ev[0], 0));
+  bool far = false;
+  for (int k0 = 0, turn = 0; k0 < L.maxP; k0 += NB, turn ^= 1) {
     const int rows = L.maxR - k0;
-    const int threads = std::min(1024, std::max(128, (rows + 31) / 32 * 32));
+    const int threads = rows <= 256 ? 256 : kPanelThreads;
     {
-      MIC_KERNEL(ctx, "k_front_panel");
-      k_front_panel<NB><<<L.count, threads, (size_t)rows * ((NB + 1) * sizeof(double) + sizeof(int)), ctx->stream>>>(
-          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act, pl.d_tab, B.info);
+      MIC_KERNEL_ON(ctx, "k_front_panel", chain);
+      k_front_panel<NB><<<L.count, threads, (size_t)rows * ((NB + 1) * sizeof(double) + kPanelBytes), chain>>>(
+          pl.d_fronts, L.first, k0, turn, F, B.U, B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
     }
-    // a front's trailing columns: the most any front has (its panel may be narrower than NB)
+    // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
-    auto tiles = [&](int tr, int tc) { return (int64_t)((cols + tc - 1) / tc) * ((below + tr - 1) / tr) * L.count; };
-    MIC_KERNEL(ctx, "k_front_update");
-    if (tiles(128, 64) >= 3LL * sm_count(ctx))
-      k_front_update<NB, 128, 64><<<dim3(L.count, (below + 127) / 128, (cols + 63) / 64), kUpdateBlocks, 0, ctx->stream>>>(
-          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act);
-    else if (tiles(64, 32) >= 2LL * sm_count(ctx))
-      k_front_update<NB, 64, 32><<<dim3(L.count, (below + 63) / 64, (cols + 31) / 32), kUpdateBlocks, 0, ctx->stream>>>(
-          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act);
-    else
-      k_front_update<NB, 32, 32><<<dim3(L.count, (below + 31) / 32, (cols + 31) / 32), kUpdateBlocks, 0, ctx->stream>>>(
-          pl.d_fronts, L.first, k0, F, B.U, B.Lb, B.act);
+    // Ahead only where the update leaves SMs idle: once its multiply-adds alone take longer than a
+    // panel (about 25 us at 2 per SM and clock), both wait for the same FP64 pipes and the split
+    // costs (513 x 129 Stokes: 54.3 ms with every update split, 51.6 with none; 129 x 33: 2.46 and 2.79)
+    const double us = (double)cols * below * NB * L.count / (2.0 * 1.9e3 * sm_count(ctx));
+    const bool ahead = k0 + NB < L.maxP && cols > NB && us < 25.0;
+    const int near = ahead ? NB : 0, rest = cols - near;
+    cudaStream_t st = ahead ? main : chain;
+    if (ahead) {
+      MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], chain));
+      MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
+    }
+    if (far) MIC_CUDA_TRY(cudaStreamWaitEvent(chain, ctx->lu_ev[1], 0));
+    if (ahead) update<NB, 64, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+    // the tile whose blocks, padding and triangular solves included, take the least time on the
+    // fullest SM (multiply-adds, 2 per clock; 600 clocks a block to start and end)
+    const double nsm = sm_count(ctx);
+    auto cost = [&](int tr, int tc, bool solve) {
+      const double n = (double)((rest + tc - 1) / tc) * ((below + tr - 1) / tr) * L.count;
+      return std::ceil(n / nsm) * (0.5 * tc * NB * (tr + (solve ? NB / 2 : 0)) + 600.0);
+    };
+    const double c32 = cost(32, 32, true), c6432 = cost(64, 32, true), c64 = cost(64, 64, false) + 8000.0,
+                 c128 = cost(128, 64, false) + 8000.0;  // (8,000 clocks: U12's launch and solve)
+    const double best = std::min(std::min(c32, c6432), std::min(c64, c128));
+    if (best == c64 || best == c128) {
+      {
+        MIC_KERNEL_ON(ctx, "k_front_solve", st);
+        k_front_solve<NB><<<dim3(L.count, (cols + 63) / 64), 256, 0, st>>>(pl.d_fronts, L.first, k0, turn, F, B.U,
+                                                                         B.Lb + turn * pl.nL, B.act);
+      }
+      if (best == c64)
+        update<NB, 64, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+      else
+        update<NB, 128, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+    } else if (best == c6432) {
+      update<NB, 64, 32, true>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+    } else {
+      update<NB, 32, 32, true>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+    }
+    far = ahead;
+    if (ahead) MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[1], main));
   }
+  MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], chain));
+  MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
   return MIC_OK;
 }
 
@@ -756,8 +970,13 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     const double *Fin = B.F[(l + 1) & 1];
     if (L.small) {
       MIC_KERNEL(ctx, "k_front_small");
-      k_front_small<<<L.count, kSmallThreads, L.smem_small, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act, sys,
-                                                                         Fin, B.F[l & 1], B.U, B.info);
+      // (more warps where one front fills an SM's shared memory)
+      if (L.smem_small > kMaxSmem / 2)
+        k_front_small<512><<<L.count, 512, L.smem_small, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act, sys,
+                                                                        Fin, B.F[l & 1], B.U, B.info);
+      else
+        k_front_small<256><<<L.count, 256, L.smem_small, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act, sys,
+                                                                        Fin, B.F[l & 1], B.U, B.info);
       continue;
     }
     {
@@ -767,9 +986,9 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     }
     int e = MIC_OK;
     switch (panel_columns(L.maxR)) {
-      case 16: e = large_level<16>(ctx, pl, L, B, l & 1); break;
-      case 8: e = large_level<8>(ctx, pl, L, B, l & 1); break;
-      default: e = large_level<4>(ctx, pl, L, B, l & 1); break;
+      case 16: e = large_level<16>(ctx, pl, L, B, B.F[l & 1]); break;
+      case 8: e = large_level<8>(ctx, pl, L, B, B.F[l & 1]); break;
+      default: e = large_level<4>(ctx, pl, L, B, B.F[l & 1]); break;
     }
     if (e) return e;
   }
@@ -790,7 +1009,9 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
 }
 
 cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
-  cudaError_t e = cudaFuncSetAttribute(k_front_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  cudaError_t e = cudaFuncSetAttribute(k_front_small<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_small<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_panel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
   if (e == cudaSuccess)
@@ -873,9 +1094,16 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
     if (h[0] > kMaxBand) return MIC_ERR_SOLVE;
   }
   if ((e = ensure_plan(ctx, S, dof))) return e;
+  if (!ctx->lu_chain) {
+    int least = 0, most = 0;
+    MIC_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &most));
+    for (cudaEvent_t &v : ctx->lu_ev)
+      if (!v) MIC_CUDA_TRY(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
+    MIC_CUDA_TRY(cudaStreamCreateWithPriority(&ctx->lu_chain, cudaStreamNonBlocking, most));
+  }
   const mic_front_plan &pl = *S.plan;
   const size_t need = 256 + room(sizeof(double) * pl.nF[0]) + room(sizeof(double) * pl.nF[1]) +
-                      room(sizeof(double) * pl.nU) + room(sizeof(double) * pl.nL) + room(sizeof(int) * pl.nAct);
+                      room(sizeof(double) * pl.nU) + room(sizeof(double) * 2 * pl.nL) + room(sizeof(int) * pl.nAct);
   if ((e = ensure_lu(ctx, need))) return e;
   double *out = nullptr;
   if (which == 0) {
@@ -890,7 +1118,7 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
   B.F[0] = carve<double>(p, pl.nF[0]);
   B.F[1] = carve<double>(p, pl.nF[1]);
   B.U = carve<double>(p, pl.nU);
-  B.Lb = carve<double>(p, pl.nL);
+  B.Lb = carve<double>(p, 2 * pl.nL);
   B.act = carve<int>(p, pl.nAct);
   const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY};
   MIC_CUDA_TRY(cudaMemsetAsync(B.info, 0x7f, sizeof(int), ctx->stream));

@@ -130,6 +130,8 @@ struct mic_ctx {
   size_t sys_scratch_bytes;
   void *lu_buf;               // the direct solver's storage (grown on demand)
   size_t lu_bytes;
+  cudaStream_t lu_chain;      // the solver's chain of panels (high priority); its hand-offs with
+  cudaEvent_t lu_ev[2];       // the updates on the main stream
   cudaStream_t aux;           // second stream of a projection: its cell-centre partial sums run
   cudaEvent_t aux_ev[2];      // beside the basic-cell ones (fork, join)
   size_t io_bytes;

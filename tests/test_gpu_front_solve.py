@@ -77,3 +77,22 @@ def test_zero_column_is_refused_and_the_context_stays_usable():
     x = P.solution(P.THERMAL)
     assert np.max(np.abs(A @ x - b)) <= 1e-12 * np.max(np.abs(A).sum(axis=1)) * np.max(np.abs(x))
     P.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(260, 90), (430, 430), (770, 760)])
+def test_tall_fronts_residual(nx, ny):
+    """Temperatures on grids whose top fronts need panels of 16, 8 and 4 columns to fit a block's
+    shared memory, and whose updates take every tile size: the residual stays at rounding level
+    (a diagonally dominant matrix, no growth: n eps at most, 2e-10 at the largest, in practice a few
+    eps; bound 1e-12)."""
+    P, so = _problem(nx, ny)
+    P.enforceThermalBCs1(so)
+    P.formThermalSystem(so, 3.0e11)
+    P.linear_solve(P.THERMAL)
+    x = P.solution(P.THERMAL)
+    rp, c, v, b = P.system(P.THERMAL)
+    assert np.all(np.isfinite(x))
+    r = np.add.reduceat(v * x[c], rp[:-1]) - b
+    a = np.add.reduceat(np.abs(v), rp[:-1])
+    assert np.max(np.abs(r)) <= 1e-12 * np.max(a) * np.max(np.abs(x))
+    P.close()
