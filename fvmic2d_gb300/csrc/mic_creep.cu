@@ -67,122 +67,253 @@ __global__ void k_creep_samples(unsigned long long seed, int64_t n, CreepConfig 
   target[m] = (float)(u - kLn1e6 - (double)mref);
 }
 
-// ---- training: per-block forward/backward with deterministic partial gradients -------
+// ---- training: forward/backward per cluster of blocks, deterministic gradient sums -------
 
-constexpr int kTB = 128;  // samples per block
+constexpr int kTB = 128;  // samples per gradient sum: one cluster of kTC blocks
+constexpr int kTC = 4;    // blocks per cluster, kTS samples each
+constexpr int kTS = kTB / kTC, kTThreads = 256, kTN = kH / (kTThreads / 32);  // a warp's neurons
+
+// One block's shared memory.  [n][s] arrays hold a neuron's value for the block's samples (a lane a
+// sample: no bank conflicts); q arrays a quarter of the neurons for all the cluster's samples.
+struct TrainSmem {
+  float w2t[kH][kH];      // W2 by input neuron (forward); with w2 the cluster's h1 afterwards
+  float w2[kH][kH];       // W2 by output neuron (backward)
+  float h1t[kH][kTS];
+  float h1[kTS][kH + 4];
+  float h2t[kH][kTS], dz2t[kH][kTS], dz1t[kH][kTS];
+  float dz2q[kH / kTC][kTB + 4], dz1q[kH / kTC][kTB + 4], h2q[kH / kTC][kTB + 4];
+  float w1[kH * 4], b1[kH], b2[kH], w3[kH];
+  float f[kTS][4], fq[kTB][4];
+  float dy[kTS], dyq[kTB];
+  float loss;
+};
+
+__device__ __forceinline__ void train_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// a float of another block of the cluster, at the place `mine` has in this one
+__device__ __forceinline__ float peer_float(const float *mine, unsigned rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(mine), r;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+  return v;
+}
 
 // Loss = mean over the batch of (y - t)^2 with t = (log10 s - out_mu) / out_sigma.
-// part[block][kNTrain] receives the block's gradient sums; lpart[block] its loss sum.
-__global__ void __launch_bounds__(kTB) k_train_fwdbwd(const float *__restrict__ p, const float *__restrict__ feat,
-                                                      const float *__restrict__ target,
-                                                      const int *__restrict__ index, int64_t nb, float inv_batch,
-                                                      float *__restrict__ part, float *__restrict__ lpart) {
-  extern __shared__ float sm[];
-  float *w2s = sm;                    // 64*64
-  float *h1s = w2s + kH * kH;         // [128][64]
-  float *h2s = h1s + kTB * kH;        // [128][64]
-  float *dz2s = h2s + kTB * kH;       // [128][64]
-  float *dz1s = dz2s + kTB * kH;      // [128][64]
-  float *fs = dz1s + kTB * kH;        // [128][4]
-  float *dys = fs + kTB * 4;          // [128]
-  const int t = threadIdx.x;
-  for (int q = t; q < kH * kH; q += kTB) w2s[q] = bf16_round(p[kOffW2 + q]);
-  const int64_t b = (int64_t)blockIdx.x * kTB + t;
+// part[cluster][kNTrain] receives the cluster's gradient sums over its 128 samples, in sample
+// order; lpart[cluster] its loss sum.
+//
+// A batch of 4,096 is 32 such sums.  One block per sum with a thread per sample used 32 SMs and ran
+// 79 us, every thread's 64 x 64 products in a row.  Here a sum is a cluster of four blocks, each with
+// a quarter of the samples for the forward and backward passes (a lane a sample, a warp eight
+// neurons, W2 broadcast from shared memory) and a quarter of the neurons for the gradient sums,
+// whose inputs it reads from the others' shared memory.  Every sum keeps its order, so the
+// parameters come out bit for bit the same.  79 -> 15 us; a step with k_train_reduce 88 -> 22 us.
+__global__ void __cluster_dims__(kTC, 1, 1) __launch_bounds__(kTThreads)
+    k_train_fwdbwd(const float *__restrict__ p, const float *__restrict__ feat, const float *__restrict__ target,
+                   const int *__restrict__ index, int64_t nb, float inv_batch, float *__restrict__ part,
+                   float *__restrict__ lpart) {
+  extern __shared__ __align__(16) unsigned char train_raw[];
+  TrainSmem &S = *reinterpret_cast<TrainSmem *>(train_raw);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, n0 = warp * kTN;
+  const unsigned rank = blockIdx.x % kTC;  // the block's rank in its cluster (one-dimensional grid)
+  const int64_t cluster = blockIdx.x / kTC;
+  const int64_t b = cluster * kTB + rank * kTS + lane;
   const bool valid = b < nb;
   const int s = valid ? index[b] : 0;
+  {
+    float w[kH * kH / kTThreads];
+#pragma unroll
+    for (int i = 0; i < kH * kH / kTThreads; ++i) w[i] = p[kOffW2 + t + i * kTThreads];
+#pragma unroll
+    for (int i = 0; i < kH * kH / kTThreads; ++i) {
+      const int q = t + i * kTThreads;
+      w[i] = bf16_round(w[i]);
+      S.w2[q / kH][q % kH] = w[i];
+      S.w2t[q % kH][q / kH] = w[i];
+    }
+  }
+  S.w1[t] = p[kOffW1 + t];
+  if (t < kH) {
+    S.b1[t] = p[kOffB1 + t];
+    S.b2[t] = p[kOffB2 + t];
+    S.w3[t] = p[kOffW3 + t];
+  }
   float f[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) f[i] = valid ? feat[4 * (int64_t)s + i] : 0.0f;
+  const float goal = valid ? target[s] : 0.0f, mu = p[kOffNorm], sigma = p[kOffNorm + 1], b3 = p[kOffB3];
   __syncthreads();
-  // forward, keeping pre-activations for the backward pass
-  float z1[kH], h1[kH];
+  float z1[kTN], z2[kTN];
 #pragma unroll
-  for (int n = 0; n < kH; ++n) {
-    float z = p[kOffB1 + n];
+  for (int j = 0; j < kTN; ++j) {
+    const int n = n0 + j;
+    float z = S.b1[n];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) z = fmaf(p[kOffW1 + 4 * n + i], f[i], z);
-    z1[n] = z;
-    h1[n] = silu(z);
-    h1s[t * kH + n] = h1[n];
+    for (int i = 0; i < 4; ++i) z = fmaf(S.w1[4 * n + i], f[i], z);
+    z1[j] = z;
+    const float h = silu(z);
+    S.h1t[n][lane] = h;
+    S.h1[lane][n] = h;
+    z2[j] = S.b2[n];
   }
-  float y = p[kOffB3];
-  for (int n = 0; n < kH; ++n) {
-    float z = p[kOffB2 + n];
-#pragma unroll 16
-    for (int k = 0; k < kH; ++k) z = fmaf(w2s[n * kH + k], h1[k], z);
-    const float h2 = silu(z);
-    h2s[t * kH + n] = h2;
-    dz2s[t * kH + n] = z;  // pre-activation for now
-    y = fmaf(p[kOffW3 + n], h2, y);
+  if (warp == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S.f[lane][i] = f[i];
   }
-  const float tt = valid ? (target[s] - p[kOffNorm]) / p[kOffNorm + 1] : 0.0f;
-  const float err = valid ? (y - tt) : 0.0f;
-  const float dy = 2.0f * err * inv_batch;
-  dys[t] = dy;
-  // backward through layer 3 and the second activation
-  for (int n = 0; n < kH; ++n) {
-    const float z = dz2s[t * kH + n];
-    dz2s[t * kH + n] = dy * p[kOffW3 + n] * dsilu(z);
-  }
-  // dh1 = W2^T dz2, then through the first activation
-#pragma unroll 4
+  __syncthreads();
+#pragma unroll 8
   for (int k = 0; k < kH; ++k) {
-    float acc = 0.0f;
-    for (int n = 0; n < kH; ++n) acc = fmaf(w2s[n * kH + k], dz2s[t * kH + n], acc);
-    dz1s[t * kH + k] = acc * dsilu(z1[k]);
+    const float h = S.h1t[k][lane];
+#pragma unroll
+    for (int j = 0; j < kTN; ++j) z2[j] = fmaf(S.w2t[k][n0 + j], h, z2[j]);
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) fs[t * 4 + i] = f[i];
+  for (int j = 0; j < kTN; ++j) S.h2t[n0 + j][lane] = silu(z2[j]);
   __syncthreads();
-  // block partial gradients, each summed over the block's samples in index order
-  float *g = part + (size_t)blockIdx.x * kNTrain;
-  for (int q = t; q < kH * kH; q += kTB) {  // dW2[n][k] = sum dz2[n] h1[k]
-    const int n = q / kH, k = q % kH;
-    float acc = 0.0f;
-    for (int r = 0; r < kTB; ++r) acc = fmaf(dz2s[r * kH + n], h1s[r * kH + k], acc);
-    g[kOffW2 + q] = acc;
+  if (warp == 0) {
+    float y = b3;
+#pragma unroll 16
+    for (int n = 0; n < kH; ++n) y = fmaf(S.w3[n], S.h2t[n][lane], y);
+    const float tt = valid ? (goal - mu) / sigma : 0.0f;
+    const float err = valid ? (y - tt) : 0.0f;
+    S.dy[lane] = 2.0f * err * inv_batch;
+    float l = err * err;  // warp shuffles, then the cluster's warps in order
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+    if (lane == 0) S.loss = l;
   }
-  for (int q = t; q < kH * 4; q += kTB) {  // dW1[n][i] = sum dz1[n] f[i]
-    const int n = q / 4, i = q % 4;
-    float acc = 0.0f;
-    for (int r = 0; r < kTB; ++r) acc = fmaf(dz1s[r * kH + n], fs[r * 4 + i], acc);
-    g[kOffW1 + q] = acc;
+  __syncthreads();
+  const float dy = S.dy[lane];
+#pragma unroll
+  for (int j = 0; j < kTN; ++j) S.dz2t[n0 + j][lane] = dy * S.w3[n0 + j] * dsilu(z2[j]);
+  __syncthreads();
+  // dh1 = W2^T dz2, then through the first activation
+  float acc[kTN];
+#pragma unroll
+  for (int j = 0; j < kTN; ++j) acc[j] = 0.0f;
+#pragma unroll 8
+  for (int n = 0; n < kH; ++n) {
+    const float d = S.dz2t[n][lane];
+#pragma unroll
+    for (int j = 0; j < kTN; ++j) acc[j] = fmaf(S.w2[n][n0 + j], d, acc[j]);
   }
-  if (t < kH) {
-    float a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-    for (int r = 0; r < kTB; ++r) {
-      a1 += dz1s[r * kH + t];
-      a2 += dz2s[r * kH + t];
-      a3 = fmaf(dys[r], h2s[r * kH + t], a3);
+#pragma unroll
+  for (int j = 0; j < kTN; ++j) S.dz1t[n0 + j][lane] = acc[j] * dsilu(z1[j]);
+  train_cluster_sync();
+  // what this block's quarter of the neurons needs of the cluster's samples
+  float(*h1all)[kH] = reinterpret_cast<float(*)[kH]>(&S.w2t[0][0]);  // [kTB][kH]: w2t and w2 are read no more
+  const int q0 = rank * (kH / kTC);
+  {  // (all reads of a group in flight before the first is stored)
+    constexpr int W = kTThreads / 32, NH = kTB / W, NQ = kH / W;
+    float a[NH][2];
+#pragma unroll
+    for (int i = 0; i < NH; ++i) {
+      const int r = warp + i * W;
+      a[i][0] = peer_float(&S.h1[r % kTS][lane], r / kTS);
+      a[i][1] = peer_float(&S.h1[r % kTS][lane + 32], r / kTS);
     }
-    g[kOffB1 + t] = a1;
-    g[kOffB2 + t] = a2;
-    g[kOffW3 + t] = a3;
+#pragma unroll
+    for (int i = 0; i < NH; ++i) {
+      h1all[warp + i * W][lane] = a[i][0];
+      h1all[warp + i * W][lane + 32] = a[i][1];
+    }
+    float c[NQ][3];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const int e = warp + i * W, n = e % (kH / kTC);
+      const unsigned from = e / (kH / kTC);
+      c[i][0] = peer_float(&S.dz2t[q0 + n][lane], from);
+      c[i][1] = peer_float(&S.dz1t[q0 + n][lane], from);
+      c[i][2] = peer_float(&S.h2t[q0 + n][lane], from);
+    }
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const int e = warp + i * W, n = e % (kH / kTC), r = e / (kH / kTC) * kTS + lane;
+      S.dz2q[n][r] = c[i][0];
+      S.dz1q[n][r] = c[i][1];
+      S.h2q[n][r] = c[i][2];
+    }
   }
-  if (t == 0) {
+  if (t < kTB) {
+    const unsigned from = t / kTS;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S.fq[t][i] = peer_float(&S.f[t % kTS][i], from);
+    S.dyq[t] = peer_float(&S.dy[t % kTS], from);
+  }
+  float loss = 0.0f;
+  if (rank == 0 && t == 0)
+    for (unsigned w = 0; w < kTC; ++w) loss += peer_float(&S.loss, w);
+  __syncwarp();
+  train_cluster_sync();  // (the last read of another block's memory; also this block's barrier)
+  if (rank == 0 && t == 0) lpart[cluster] = loss;
+  // gradient sums over the cluster's samples in order: each thread one neuron and four inputs of W2
+  float *g = part + (size_t)cluster * kNTrain;
+  {
+    const int n = t / 16, k = (t % 16) * 4;
+    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
+    for (int r = 0; r < kTB; ++r) {
+      const float d = S.dz2q[n][r];
+      const float4 h = *reinterpret_cast<const float4 *>(&h1all[r][k]);
+      a[0] = fmaf(d, h.x, a[0]);
+      a[1] = fmaf(d, h.y, a[1]);
+      a[2] = fmaf(d, h.z, a[2]);
+      a[3] = fmaf(d, h.w, a[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) g[kOffW2 + (q0 + n) * kH + k + i] = a[i];
+  }
+  if (t < 64) {  // W1
+    const int n = t / 4, i = t % 4;
     float a = 0.0f;
-    for (int r = 0; r < kTB; ++r) a += dys[r];
+#pragma unroll 8
+    for (int r = 0; r < kTB; ++r) a = fmaf(S.dz1q[n][r], S.fq[r][i], a);
+    g[kOffW1 + 4 * (q0 + n) + i] = a;
+  } else if (t < 80) {
+    const int n = t - 64;
+    float a = 0.0f;
+#pragma unroll 8
+    for (int r = 0; r < kTB; ++r) a += S.dz1q[n][r];
+    g[kOffB1 + q0 + n] = a;
+  } else if (t >= 96 && t < 112) {
+    const int n = t - 96;
+    float a = 0.0f;
+#pragma unroll 8
+    for (int r = 0; r < kTB; ++r) a += S.dz2q[n][r];
+    g[kOffB2 + q0 + n] = a;
+  } else if (t >= 128 && t < 144) {
+    const int n = t - 128;
+    float a = 0.0f;
+#pragma unroll 8
+    for (int r = 0; r < kTB; ++r) a = fmaf(S.dyq[r], S.h2q[n][r], a);
+    g[kOffW3 + q0 + n] = a;
+  } else if (t == 160 && rank == 0) {
+    float a = 0.0f;
+#pragma unroll 8
+    for (int r = 0; r < kTB; ++r) a += S.dyq[r];
     g[kOffB3] = a;
-  }
-  // loss partial: warp shuffles then one value per block
-  float l = err * err;
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-  __shared__ float lw[kTB / 32];
-  if ((t & 31) == 0) lw[t >> 5] = l;
-  __syncthreads();
-  if (t == 0) {
-    float a = 0.0f;
-    for (int w = 0; w < kTB / 32; ++w) a += lw[w];
-    lpart[blockIdx.x] = a;
   }
 }
 
-// gradient = sum of the block partials in block order; optional Adam step
-__global__ void k_train_reduce(float *p, const float *part, int nblocks, float *grad, float *m_, float *v_, int step,
-                               float lr, int apply) {
+// The clusters' sums in order and Adam (apply); in the last block the losses' sum.  A thread waits
+// for as many loads as there are clusters, so eight are in flight at a time.  (Done by the last
+// cluster of k_train_step instead, it measured 27 us a step against 22.)
+__global__ void k_train_reduce(float *p, const float *__restrict__ part, int nblocks, float *grad, float *m_, float *v_,
+                               int step, float lr, int apply, const float *__restrict__ lpart, float *loss) {
+  if (blockIdx.x == gridDim.x - 1) {
+    if (threadIdx.x == 0) {
+      float s = 0.0f;
+#pragma unroll 8
+      for (int i = 0; i < nblocks; ++i) s += lpart[i];
+      *loss = s;
+    }
+    return;
+  }
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= kNTrain) return;
   float g = 0.0f;
+#pragma unroll 8
   for (int b = 0; b < nblocks; ++b) g += part[(size_t)b * kNTrain + q];
   if (grad) grad[q] = g;
   if (!apply) return;
@@ -195,13 +326,7 @@ __global__ void k_train_reduce(float *p, const float *part, int nblocks, float *
   const float vh = v / (1.0f - powf(b2, (float)step));
   p[q] -= lr * mh / (sqrtf(vh) + eps);
 }
-
-__global__ void k_sum_floats(const float *a, int n, float *out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  float s = 0.0f;
-  for (int i = 0; i < n; ++i) s += a[i];
-  *out = s;
-}
+constexpr int kReduceBlocks = (kNTrain + 255) / 256 + 1;  // parameters, then the losses
 
 // deterministic shuffle of sample indices for one epoch: the affine permutation
 // i -> (a i + c) mod n, with a coprime to n chosen on the host
@@ -306,7 +431,7 @@ int ensure_mlp(mic_ctx *ctx) {
   return MIC_OK;
 }
 
-size_t fwdbwd_smem() { return sizeof(float) * (kH * kH + 4 * kTB * kH + kTB * 4 + kTB); }
+
 
 // W2 of a host copy of the parameters rounded to BF16 (round to nearest even, as
 // __float2bfloat16_rn; the weights are finite)
@@ -504,19 +629,14 @@ extern "C" int mic_creep_mlp_grad(mic_ctx *ctx, const float *params, const float
   MIC_CUDA_TRY(cudaMemcpyAsync(fe, feat, sizeof(float) * 4 * n, cudaMemcpyHostToDevice, ctx->stream));
   MIC_CUDA_TRY(cudaMemcpyAsync(tg, target, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
   MIC_CUDA_TRY(cudaMemcpyAsync(ix, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
-  MIC_CUDA_TRY(cudaFuncSetAttribute(k_train_fwdbwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwdbwd_smem()));
+  MIC_CUDA_TRY(cudaFuncSetAttribute(k_train_fwdbwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
   {
     MIC_KERNEL(ctx, "k_train_fwdbwd");
-    k_train_fwdbwd<<<nblocks, kTB, fwdbwd_smem(), ctx->stream>>>(p, fe, tg, ix, n, 1.0f / n, part, lp);
+    k_train_fwdbwd<<<nblocks * kTC, kTThreads, sizeof(TrainSmem), ctx->stream>>>(p, fe, tg, ix, n, 1.0f / n, part, lp);
   }
   {
     MIC_KERNEL(ctx, "k_train_reduce");
-    k_train_reduce<<<(kNTrain + 255) / 256, 256, 0, ctx->stream>>>(p, part, nblocks, g, nullptr, nullptr, 0, 0.f,
-                                                                   0);
-  }
-  {
-    MIC_KERNEL(ctx, "k_sum_floats");
-    k_sum_floats<<<1, 32, 0, ctx->stream>>>(lp, nblocks, ls);
+    k_train_reduce<<<kReduceBlocks, 256, 0, ctx->stream>>>(p, part, nblocks, g, nullptr, nullptr, 0, 0.f, 0, lp, ls);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   MIC_CUDA_TRY(cudaMemcpyAsync(grad, g, sizeof(float) * kNTrain, cudaMemcpyDeviceToHost, ctx->stream));
@@ -566,7 +686,7 @@ extern "C" int mic_creep_train(mic_ctx *ctx, int64_t nsamples, int batch, int st
   }
   MIC_CUDA_TRY(cudaMemcpyAsync(ctx->mlp + kOffNorm, norm, sizeof(norm), cudaMemcpyHostToDevice, ctx->stream));
   MIC_CUDA_TRY(cudaMemsetAsync(am, 0, sizeof(float) * 2 * kNTrain, ctx->stream));
-  MIC_CUDA_TRY(cudaFuncSetAttribute(k_train_fwdbwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwdbwd_smem()));
+  MIC_CUDA_TRY(cudaFuncSetAttribute(k_train_fwdbwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
   const int64_t per_epoch = nsamples / batch;
   for (int s = 0; s < steps; ++s) {
     const int epoch = (int)(s / per_epoch);
@@ -578,21 +698,15 @@ extern "C" int mic_creep_train(mic_ctx *ctx, int64_t nsamples, int batch, int st
       k_epoch_order<<<grid_for(nsamples), kBlock, 0, ctx->stream>>>(ix, nsamples, a, c);
     }
     const int64_t off = (s % per_epoch) * (int64_t)batch;
-    {
-      MIC_KERNEL(ctx, "k_train_fwdbwd");
-      k_train_fwdbwd<<<nblocks, kTB, fwdbwd_smem(), ctx->stream>>>(ctx->mlp, fe, tg, ix + off, batch, 1.0f / batch,
-                                                                    part, lp);
-    }
     const float lrs = 0.5f * lr * (1.0f + cosf(3.14159265f * s / steps));
     {
-      MIC_KERNEL(ctx, "k_train_reduce");
-      k_train_reduce<<<(kNTrain + 255) / 256, 256, 0, ctx->stream>>>(ctx->mlp, part, nblocks, nullptr, am, av, s + 1,
-                                                                     lrs, 1);
+      MIC_KERNEL(ctx, "k_train_fwdbwd");
+      k_train_fwdbwd<<<nblocks * kTC, kTThreads, sizeof(TrainSmem), ctx->stream>>>(ctx->mlp, fe, tg, ix + off, batch,
+                                                                                  1.0f / batch, part, lp);
     }
-    {
-      MIC_KERNEL(ctx, "k_sum_floats");
-      k_sum_floats<<<1, 32, 0, ctx->stream>>>(lp, nblocks, lh + s);
-    }
+    MIC_KERNEL(ctx, "k_train_reduce");
+    k_train_reduce<<<kReduceBlocks, 256, 0, ctx->stream>>>(ctx->mlp, part, nblocks, nullptr, am, av, s + 1, lrs, 1, lp,
+                                                           lh + s);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   if (loss_hist) {
