@@ -974,6 +974,37 @@ __global__ void k_advect_coef(const double *__restrict__ vx, const double *__res
     cwz[k] = bil_coef_df(wz[w0], wz[w0 + 1], wz[w0 + NX], wz[w0 + NX + 1]);
   }
 }
+
+// The same on a grid periodic in x, in FP64 records: NX cells a row for all three fields, the last
+// one's right column wrapping to column 0, and no ghost column at the left wall.
+__global__ void k_advect_coef_periodic(const double *__restrict__ vx, const double *__restrict__ vy,
+                                       const double *__restrict__ wz, mic_bcinfo top, int NX, int NY, Bil4 *cvx,
+                                       Bil4 *cvy, Bil4 *cwz) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k >= (int64_t)NX * NY) return;
+  const int row = (int)(k / NX), i = (int)(k % NX), i1 = next_col(i, NX);
+  const size_t r0 = (size_t)row * NX;
+  const double vll = vx[r0 + i], vlr = vx[r0 + i1];
+  double vul = vll, vur = vlr;  // the top wall's ghost row: free slip
+  if (row > 0) {
+    vul = vx[r0 - NX + i];
+    vur = vx[r0 - NX + i1];
+  } else if (top.type[0] == 0) {
+    vul = 2.0 * top.value[0] - vll;
+    vur = 2.0 * top.value[0] - vlr;
+  }
+  cvx[k] = bil_coef(vul, vur, vll, vlr);
+  if (row + 1 < NY) {
+    cvy[k] = bil_coef(vy[r0 + i], vy[r0 + i1], vy[r0 + NX + i], vy[r0 + NX + i1]);
+    cwz[k] = bil_coef(wz[r0 + i], wz[r0 + i1], wz[r0 + NX + i], wz[r0 + NX + i1]);
+  }
+}
+// c0 + tx c1 + ty (c2 + tx c3), two 16-byte loads
+__device__ __forceinline__ double bil_eval(const Bil4 *__restrict__ cells, size_t k, double tx, double ty) {
+  const double2 a = __ldg(reinterpret_cast<const double2 *>(cells + k));
+  const double2 b = __ldg(reinterpret_cast<const double2 *>(cells + k) + 1);
+  return fma(ty, fma(tx, b.y, b.x), fma(tx, a.y, a.x));
+}
 #endif
 
 struct AdvectCols {
@@ -1162,6 +1193,9 @@ __device__ __forceinline__ double advect_marker(const Params &P, const AdvectCol
 // (markers.c:2120-2223).  Returns the rotated sxx.
 __device__ __forceinline__ double advect_tail(const Params &P, const AdvectCols &c, double dt, int64_t m, double X0,
                                               double Y0, const double *mvx, const double *mvy, const double *mwz) {
+  // loads before the first store (the compiler cannot tell the columns apart)
+  const double s11 = c.sxx[m], s22 = c.syy[m], s12 = c.sxy[m];
+  const double e11 = c.exx[m], e22 = c.eyy[m], e12 = c.exy[m], E0 = c.Eii[m];
 #ifdef MIC_EXACT
   const double VX = div6(mvx[0] + 2 * mvx[1] + 2 * mvx[2] + mvx[3]);
   const double VY = div6(mvy[0] + 2 * mvy[1] + 2 * mvy[2] + mvy[3]);
@@ -1189,7 +1223,6 @@ __device__ __forceinline__ double advect_tail(const Params &P, const AdvectCols 
       Xn += P.LX;
   }
   c.X[m] = Xn;
-  const double s11 = c.sxx[m], s22 = c.syy[m], s12 = c.sxy[m];
   double nsxx;
   if (P.jaumann) {
     // first-order Jaumann terms with wxy1 = wxy dt (markers.c:2147-2156)
@@ -1223,11 +1256,9 @@ __device__ __forceinline__ double advect_tail(const Params &P, const AdvectCols 
 #endif
   }
 #ifdef MIC_EXACT
-  const double e11 = c.exx[m], e22 = c.eyy[m], e12 = c.exy[m];
-  c.Eii[m] = c.Eii[m] + dt * sqrt(0.5 * (e11 * e11 + e22 * e22) + e12 * e12);
+  c.Eii[m] = E0 + dt * sqrt(0.5 * (e11 * e11 + e22 * e22) + e12 * e12);
 #else
-  const double e11 = c.exx[m], e22 = c.eyy[m], e12 = c.exy[m];
-  c.Eii[m] = fma(dt, sqrt(fma(e12, e12, 0.5 * fma(e11, e11, e22 * e22))), c.Eii[m]);
+  c.Eii[m] = fma(dt, sqrt(fma(e12, e12, 0.5 * fma(e11, e11, e22 * e22))), E0);
 #endif
   return nsxx;
 }
@@ -1303,8 +1334,9 @@ __device__ __forceinline__ double advect_tail_df(const Params &P, const AdvectCo
 
 // advectMarkersRK on a grid periodic in x (markers.c:1907-1913, 1928-1944, 1961-1966, 2014-2023):
 // the cell walk runs over cells -1 .. NX-1 (line -1 and NX are the seam's images), the vx and vy
-// cells are not clamped in x, node columns wrap, and the left wall has no ghost values.  The
-// reference's own divisions, in both builds (periodic grids are small).
+// cells are not clamped in x, node columns wrap, and the left wall has no ghost values.
+#ifdef MIC_EXACT
+// The FMA-free build: the reference's own divisions.
 __device__ double advect_marker_periodic(const Params &P, const AdvectCols &c, const double *__restrict__ vx,
                                          const double *__restrict__ vy, const double *__restrict__ wz,
                                          const mic_bcinfo &top, double dt, int64_t m, int ci, int cj) {
@@ -1381,6 +1413,68 @@ __device__ double advect_marker_periodic(const Params &P, const AdvectCols &c, c
   }
   return advect_tail(P, c, dt, m, X0, Y0, mvx, mvy, mwz);
 }
+#else
+// The product build, all in FP64: cell decisions on integer images, the first stage's fractions
+// from the binning, the others as correctly rounded quotients by the tabulated reciprocals
+// (div_sp), the fields by their cells' coefficient forms.  About 160 FP64 instructions a marker; with
+// the reference's ten divisions a stage and its products it took 660 (1,600,208 markers: 1671 us,
+// now 465).
+__device__ __forceinline__ double advect_marker_periodic(const Params &P, const AdvectCols &c, const Geo &g,
+                                                         const AdvectCoef &cv, double dt, int64_t m, int ci, int cj) {
+  const Bil4 *__restrict__ cvx = static_cast<const Bil4 *>(cv.cvx);
+  const Bil4 *__restrict__ cvy = static_cast<const Bil4 *>(cv.cvy);
+  const Bil4 *__restrict__ cwz = static_cast<const Bil4 *>(cv.cwz);
+  const int NX = P.NX, NY = P.NY;
+  const double X0 = c.X[m], Y0 = c.Y[m], hdt = 0.5 * dt;
+  double xcur = X0, ycur = Y0;
+  double mvx[4], mvy[4], mwz[4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const long long bx = ordered_bits(xcur), by = ordered_bits(ycur);
+    const bool okx = !nan_bits(dbits(xcur)), oky = !nan_bits(dbits(ycur));
+    int i = ci, j = cj;
+    if (okx) {
+      if (bx > P.xbits[i + 1]) {
+        while (bx > P.xbits[i + 1] && i < NX - 1) i++;
+      } else if (bx < P.xbits[i]) {
+        while (bx < P.xbits[i] && i > -1) i--;
+      }
+    }
+    if (oky) {
+      if (by > P.ybits[j + 1]) {
+        while (by > P.ybits[j + 1] && j < NY - 2) j++;
+      } else if (by < P.ybits[j]) {
+        while (by < P.ybits[j] && j > 0) j--;
+      }
+    }
+    int vxY = j, vyX = i;
+    if (oky && by < P.ycbits[vxY + 1]) vxY--;
+    if (vyX > -1 && okx && bx < P.xcbits[vyX + 1]) vyX--;
+    double fx, fy, ftx, fty;
+    if (s == 0) {
+      fx = g.gx0[m];
+      fy = g.gy0[m];
+      ftx = g.gx1[m];
+      fty = g.gy1[m];
+    } else {
+      fx = div_sp(xcur - P.x[i], P.hx[i], P.ix[i]);
+      fy = div_sp(ycur - P.y[j], P.hy[j], P.iy[j]);
+      ftx = div_sp(xcur - P.xc[vyX + 1], P.hxc[vyX + 1], P.ixc[vyX + 1]);
+      fty = div_sp(ycur - P.yc[vxY + 1], P.hyc[vxY + 1], P.iyc[vxY + 1]);
+    }
+    const size_t col = wrap_col(i, NX);
+    mvx[s] = bil_eval(cvx, (size_t)(vxY + 1) * NX + col, fx, fty);
+    mvy[s] = bil_eval(cvy, (size_t)j * NX + wrap_col(vyX, NX), ftx, fy);
+    mwz[s] = bil_eval(cwz, (size_t)j * NX + col, fx, fy);
+    if (s < 3) {
+      const double h = s < 2 ? hdt : dt;
+      xcur = fma(h, mvx[s], X0);
+      ycur = fma(h, mvy[s], Y0);
+    }
+  }
+  return advect_tail(P, c, dt, m, X0, Y0, mvx, mvy, mwz);
+}
+#endif
 
 // one marker; returns the bits of |sxx| after the rotation for an in-domain marker, else 0
 __device__ __forceinline__ long long advect_one(const Params &P, const AdvectCols &c, const Geo &g,
@@ -1392,8 +1486,12 @@ __device__ __forceinline__ long long advect_one(const Params &P, const AdvectCol
   if (m < n) {
     const int ci = c.cellX[m], cj = c.cellY[m];
     if (ci != -1) {
-      const double a = fabs(P.xper ? advect_marker_periodic(P, c, vx, vy, wz, top, dt, m, ci, cj)
-                                   : advect_marker(P, c, g, vx, vy, wz, cv, top, left, dt, m, ci, cj, wz_known));
+#ifdef MIC_EXACT
+      const double per = P.xper ? advect_marker_periodic(P, c, vx, vy, wz, top, dt, m, ci, cj) : 0.0;
+#else
+      const double per = P.xper ? advect_marker_periodic(P, c, g, cv, dt, m, ci, cj) : 0.0;
+#endif
+      const double a = fabs(P.xper ? per : advect_marker(P, c, g, vx, vy, wz, cv, top, left, dt, m, ci, cj, wz_known));
       if (a > 0.0) b = dbits(a);
     }
   }
@@ -2375,9 +2473,10 @@ static int advect_launch(mic_ctx *ctx, double dt, bool wz_known, bool with_max =
     c.exy = ctx->f64[C_EXY];
     AdvectCoef cv = {nullptr, nullptr, nullptr};
 #ifndef MIC_EXACT
-    if (!ctx->P.xper) {  // (the periodic advection interpolates the nodes directly)
+    {
       const int NX = ctx->P.NX, NY = ctx->P.NY;
       const size_t nn = (size_t)NX * NY;
+      static_assert(sizeof(BilDF) == sizeof(Bil4), "one buffer for either record");
       if (!ctx->adv_coef && cudaMalloc((void **)&ctx->adv_coef, 3 * nn * sizeof(BilDF)) != cudaSuccess) {
         ctx->adv_coef = nullptr;
         return MIC_ERR_NOMEM;
@@ -2385,9 +2484,16 @@ static int advect_launch(mic_ctx *ctx, double dt, bool wz_known, bool with_max =
       BilDF *cb = static_cast<BilDF *>(ctx->adv_coef);
       cv = {cb, cb + nn, cb + 2 * nn};
       MIC_KERNEL(ctx, "k_advect_coef");
-      k_advect_coef<<<grid_for((int64_t)nn), kBlock, 0, ctx->stream>>>(
-          ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop,
-          ctx->bcs.mechBCLeft, NX, NY, cb, cb + nn, cb + 2 * nn);
+      if (ctx->P.xper) {
+        Bil4 *cp = static_cast<Bil4 *>(ctx->adv_coef);
+        k_advect_coef_periodic<<<grid_for((int64_t)nn), kBlock, 0, ctx->stream>>>(
+            ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop, NX, NY, cp,
+            cp + nn, cp + 2 * nn);
+      } else {
+        k_advect_coef<<<grid_for((int64_t)nn), kBlock, 0, ctx->stream>>>(
+            ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop,
+            ctx->bcs.mechBCLeft, NX, NY, cb, cb + nn, cb + 2 * nn);
+      }
     }
     MIC_CUDA_TRY(cudaGetLastError());
 #endif
