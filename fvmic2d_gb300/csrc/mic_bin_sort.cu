@@ -10,11 +10,12 @@
 // basic cells in x (NX - 1, or NX on a grid periodic in x: markers.c:49, 73); out-of-domain
 // markers get key 4*NCX*(NY-1).  Cells stay contiguous and inside a cell the markers
 // of each quadrant are contiguous, so every staggered (cell-centre) cell's markers are four
-// runs.  An LSD radix sort with 8-bit digits (stable by construction) orders (key, index) pairs:
-// per 4096-marker tile a digit histogram, one exclusive scan over the digit-major
-// histogram matrix, then a scatter in which each tile ranks its items per digit with warp
-// match/ballot in index order.  Ties keep the current device order, so the result equals
-// a CPU stable sort of the current order.  cell_start[] brackets each cell's markers.
+// runs.  An LSD radix sort with 8-bit digits (stable by construction) orders (key, index) pairs.
+// The digit counts of every pass come with the cell location (they do not depend on the order), and
+// a pass is one kernel: each block ranks a tile's items per digit in index order (warp match), finds
+// what the tiles before it hold of each digit by looking back at their published counts, and writes
+// the tile out in digit order.  Ties keep the current device order, so the result equals a CPU
+// stable sort of the current order.  cell_start[] brackets each cell's markers.
 #include "mic_internal.cuh"
 
 using namespace mic;
@@ -22,10 +23,27 @@ using namespace mic;
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kItemsPerThread = 16;
-constexpr int kTile = kSortThreads * kItemsPerThread;  // 4096
 constexpr int kRadixBits = 8;
 constexpr int kBuckets = 1 << kRadixBits;
+constexpr int kMaxPasses = 4;
+// Items per thread of a pass: 16 (tiles of 4,096) where that fills the GPU; 4 up to 524,288 markers,
+// so that the small sorts spread over more SMs (65,536 markers: 64 tiles instead of 16).
+constexpr int kItemsLarge = 16, kItemsSmall = 4;
+constexpr int64_t kSmallSort = 1 << 19;
+inline int items_for(int64_t n) { return n <= kSmallSort ? kItemsSmall : kItemsLarge; }
+inline int64_t tiles_for(int64_t n) {
+  const int64_t t = (int64_t)kSortThreads * items_for(n);
+  return (n + t - 1) / t;
+}
+// scratch of one sort (ints): tile tickets of the passes, digit counts of the passes, and per pass
+// each tile's published counts
+constexpr int kOffTicket = 0, kOffCounts = 32, kOffTiles = kOffCounts + kMaxPasses * kBuckets;
+inline int64_t sort_ints(int64_t tiles, int passes) { return kOffTiles + (int64_t)passes * tiles * kBuckets; }
+inline int passes_for(int64_t ncells) {  // digits of the largest key, 4 ncells
+  int bits = 1;
+  while ((1LL << bits) <= 4 * ncells) ++bits;
+  return (bits + kRadixBits - 1) / kRadixBits;
+}
 
 // Largest i in [0, n-2] with g[i] <= v (markers.c:47-69), on bit patterns.
 __device__ __forceinline__ int bisect_bits(const long long *__restrict__ g, int n, long long v) {
@@ -57,53 +75,70 @@ __device__ __forceinline__ int locate_bits(const long long *__restrict__ g, int 
   return bisect_bits(g, n, v);
 }
 
-__global__ void k_find_cells(Params P, const double *__restrict__ X, const double *__restrict__ Y,
-                             int *__restrict__ cellX, int *__restrict__ cellY, int *__restrict__ cpu,
-                             int *__restrict__ key, int64_t n, Status *st) {
-  __shared__ unsigned long long s_out;
-  if (threadIdx.x == 0) s_out = 0;
-  __syncthreads();
-  const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (m < n) {
-    const long long bx = dbits(X[m]);
-    const long long by = dbits(Y[m]);
-    const long long ux = (bx == (long long)0x8000000000000000ULL) ? 0LL : bx;
-    const long long uy = (by == (long long)0x8000000000000000ULL) ? 0LL : by;
-    const long long blx = dbits(P.LX), bly = dbits(P.LY);
-    // X >= 0 && Y >= 0 && X <= LX && Y <= LY; NaN fails every test
-    const bool in = ux >= 0 && uy >= 0 && ux <= blx && uy <= bly;
-    const int hx = cellX[m], hy = cellY[m];  // the cell before this binning (any value)
-    int cx = -1, cy = -1, k = 4 * P.NCX * (P.NY - 1);
-    if (in) {
-      cx = locate_bits(P.xbits, P.NCX + 1, ux, hx);  // lines 0..NCX (periodic: line NX = LX)
-      cy = locate_bits(P.ybits, P.NY, uy, hy);
-      const int qx = ux >= nonneg_bits(P.xc[cx + 1]), qy = uy >= nonneg_bits(P.yc[cy + 1]);
-      k = 4 * (cy * P.NCX + cx) + 2 * qy + qx;
-    } else {
-      atomicAdd(&s_out, 1ULL);
+// digit counts of a warp's keys into shared memory; neighbouring markers share their high digits,
+// so a warp of one digit adds once
+__device__ __forceinline__ void count_digits(int (*h)[kBuckets], int passes, bool valid, int k) {
+  const unsigned in = __ballot_sync(0xffffffffu, valid);
+  if (in == 0) return;
+  for (int p = 0; p < passes; ++p) {
+    const int d = (k >> (p * kRadixBits)) & (kBuckets - 1);
+    const int d0 = __shfl_sync(0xffffffffu, d, __ffs(in) - 1);
+    if (__all_sync(0xffffffffu, !valid || d == d0)) {
+      if ((threadIdx.x & 31) == 0) atomicAdd(&h[p][d0], __popc(in));
+    } else if (valid) {
+      atomicAdd(&h[p][d], 1);
     }
-    cellX[m] = cx;
-    cellY[m] = cy;
-    cpu[m] = 0;
-    key[m] = k;
   }
-  __syncthreads();
-  if (threadIdx.x == 0 && s_out) atomicAdd(&st->n_out, s_out);
+}
+__device__ __forceinline__ void clear_digits(int (*h)[kBuckets], int passes) {
+  for (int b = threadIdx.x; b < passes * kBuckets; b += blockDim.x) (&h[0][0])[b] = 0;
+}
+__device__ __forceinline__ void add_digits(int (*h)[kBuckets], int passes, int *counts) {
+  for (int b = threadIdx.x; b < passes * kBuckets; b += blockDim.x)
+    if ((&h[0][0])[b]) atomicAdd(counts + b, (&h[0][0])[b]);
 }
 
-__global__ void k_radix_hist(const int *__restrict__ key, int64_t n, int shift, int *__restrict__ hist,
-                             int ntiles) {
-  __shared__ int cnt[kBuckets];
-  for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) cnt[b] = 0;
+// (a grid of a few blocks per SM walks the markers, so that few digit counts are added in memory)
+__global__ void k_find_cells(Params P, const double *__restrict__ X, const double *__restrict__ Y,
+                             int *__restrict__ cellX, int *__restrict__ cellY, int *__restrict__ cpu,
+                             int *__restrict__ key, int64_t n, int passes, int *counts, Status *st) {
+  __shared__ unsigned long long s_out;
+  __shared__ int h[kMaxPasses][kBuckets];
+  if (threadIdx.x == 0) s_out = 0;
+  clear_digits(h, passes);
   __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kTile;
-#pragma unroll 4
-  for (int r = 0; r < kItemsPerThread; ++r) {
-    const int64_t idx = base + (int64_t)r * kSortThreads + threadIdx.x;
-    if (idx < n) atomicAdd(&cnt[(key[idx] >> shift) & (kBuckets - 1)], 1);
+  for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t m = base + threadIdx.x;
+    int k = 0;
+    if (m < n) {
+      const long long bx = dbits(X[m]);
+      const long long by = dbits(Y[m]);
+      const long long ux = (bx == (long long)0x8000000000000000ULL) ? 0LL : bx;
+      const long long uy = (by == (long long)0x8000000000000000ULL) ? 0LL : by;
+      const long long blx = dbits(P.LX), bly = dbits(P.LY);
+      // X >= 0 && Y >= 0 && X <= LX && Y <= LY; NaN fails every test
+      const bool in = ux >= 0 && uy >= 0 && ux <= blx && uy <= bly;
+      const int hx = cellX[m], hy = cellY[m];  // the cell before this binning (any value)
+      int cx = -1, cy = -1;
+      k = 4 * P.NCX * (P.NY - 1);
+      if (in) {
+        cx = locate_bits(P.xbits, P.NCX + 1, ux, hx);  // lines 0..NCX (periodic: line NX = LX)
+        cy = locate_bits(P.ybits, P.NY, uy, hy);
+        const int qx = ux >= nonneg_bits(P.xc[cx + 1]), qy = uy >= nonneg_bits(P.yc[cy + 1]);
+        k = 4 * (cy * P.NCX + cx) + 2 * qy + qx;
+      } else {
+        atomicAdd(&s_out, 1ULL);
+      }
+      cellX[m] = cx;
+      cellY[m] = cy;
+      cpu[m] = 0;
+      key[m] = k;
+    }
+    count_digits(h, passes, m < n, k);
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) hist[(size_t)b * ntiles + blockIdx.x] = cnt[b];
+  add_digits(h, passes, counts);
+  if (threadIdx.x == 0 && s_out) atomicAdd(&st->n_out, s_out);
 }
 
 // In-place exclusive scan of an int array of length len, in blocks of 2048; block totals go
@@ -158,52 +193,183 @@ __global__ void k_scan_add(int *__restrict__ data, int64_t len, const int *__res
     if (base + k < len) data[base + k] += add;
 }
 
-__global__ void k_radix_scatter(const int *__restrict__ key_in, const int *__restrict__ val_in, int use_iota,
-                                int *__restrict__ key_out, int *__restrict__ val_out, int64_t n, int shift,
-                                const int *__restrict__ hist, int ntiles) {
-  __shared__ int tile_off[kBuckets];
-  __shared__ int run[kBuckets];
-  __shared__ int wcnt[kSortThreads / 32][kBuckets];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) {
-    tile_off[b] = hist[(size_t)b * ntiles + blockIdx.x];
-    run[b] = 0;
+// One pass of the sort.  Tiles are taken in order from a ticket, so the tiles a block waits for are
+// running or done.  A tile publishes per digit its own count, then (after looking back) the count of
+// all tiles up to it; a later tile adds counts backwards until it meets one of the latter, eight
+// tiles' words in flight at a time.  The wait is bounded: a block that gives up counts its tile's
+// markers in bad_cell (the binning then reports MIC_ERR_CELL) and leaves its items where they are.
+// Bound by the ranking (a chain of warp matches and shared-memory counts: half the issue slots, 15%
+// of HBM's rate); matching by eight ballots instead took 159 against 129 us, eight items a thread
+// 150.  The five launches of a pass (digit counts, three of their scan, scatter) became one: 16.8 M
+// markers 224 -> 129 us a pass, 65,536 markers 42 -> 10.
+constexpr unsigned kHas = 1u << 30, kUpTo = 2u << 30, kCount = kHas - 1;  // (2^30 markers of 440 B fit no GPU)
+constexpr int kLookRounds = 1 << 22;
+
+template <int IT>
+__global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__restrict__ key_in, const int *__restrict__ val_in,
+                                                            int use_iota, int *__restrict__ key_out,
+                                                            int *__restrict__ val_out, int64_t n, int shift,
+                                                            const int *__restrict__ counts, unsigned *tiles, int *ticket,
+                                                            unsigned long long *lost) {
+  constexpr int W = kSortThreads / 32, T = kSortThreads * IT;
+  __shared__ int wcnt[W][kBuckets];        // per warp and digit: count, then offset in the tile's digit
+  __shared__ int s_key[T], s_val[T];       // the tile in digit order
+  __shared__ int local[kBuckets], at[kBuckets];  // digit's first item in the tile; its place in the output
+  __shared__ int wsum[2][W];
+  __shared__ int s_tile, s_lost;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (t == 0) {
+    s_tile = atomicAdd(ticket, 1);
+    s_lost = 0;
   }
-  const unsigned lt_mask = (1u << lane) - 1u;
-  const int64_t base = (int64_t)blockIdx.x * kTile;
-  for (int r = 0; r < kItemsPerThread; ++r) {
-    for (int t = threadIdx.x; t < (kSortThreads / 32) * kBuckets; t += blockDim.x) (&wcnt[0][0])[t] = 0;
-    __syncthreads();
-    const int64_t idx = base + (int64_t)r * kSortThreads + threadIdx.x;
-    const bool valid = idx < n;
-    int k = 0, v = 0, d = kBuckets;  // invalid items form their own group and are never written
-    if (valid) {
-      k = key_in[idx];
-      v = use_iota ? (int)idx : val_in[idx];
-      d = (k >> shift) & (kBuckets - 1);
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int rank = __popc(peers & lt_mask);
-    if (valid && rank == 0) wcnt[warp][d] = __popc(peers);
-    __syncthreads();
-    // per digit: exclusive prefix over the warps of this round, then advance the running count
-    for (int b = threadIdx.x; b < kBuckets; b += blockDim.x) {
-      int acc = run[b];
 #pragma unroll
-      for (int w = 0; w < kSortThreads / 32; ++w) {
-        int c = wcnt[w][b];
-        wcnt[w][b] = acc;
-        acc += c;
+  for (int w = 0; w < W; ++w) wcnt[w][t] = 0;
+  __syncthreads();
+  const int tile = s_tile;
+  const int64_t first = (int64_t)tile * T, base = first + warp * (32 * IT) + lane;
+  int k[IT], v[IT], rank[IT];
+#pragma unroll
+  for (int r = 0; r < IT; ++r) {
+    const int64_t i = base + r * 32;
+    k[r] = i < n ? key_in[i] : 0;
+    v[r] = i < n ? (use_iota ? (int)i : val_in[i]) : 0;
+  }
+  const unsigned before = (1u << lane) - 1u;
+#pragma unroll
+  for (int r = 0; r < IT; ++r) {
+    const bool valid = base + r * 32 < n;
+    const int d = valid ? (k[r] >> shift) & (kBuckets - 1) : kBuckets;  // invalid: a group of their own
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const int c = valid ? wcnt[warp][d] : 0, mine = __popc(peers & before);
+    rank[r] = c + mine;
+    __syncwarp();
+    if (valid && mine == 0) wcnt[warp][d] = c + __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  // thread t: digit t
+  int count = 0;
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    const int c = wcnt[w][t];
+    wcnt[w][t] = count;
+    count += c;
+  }
+  volatile unsigned *slot = tiles + t;
+  slot[(int64_t)tile * kBuckets] = (tile == 0 ? kUpTo : kHas) | (unsigned)count;
+  // first places: of the digit among all markers, and in the tile
+  int a = counts[t], b = count;
+  const int a0 = a, b0 = b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+    if (lane >= o) {
+      a += x;
+      b += y;
+    }
+  }
+  if (lane == 31) {
+    wsum[0][warp] = a;
+    wsum[1][warp] = b;
+  }
+  __syncthreads();
+  a -= a0;
+  b -= b0;
+#pragma unroll
+  for (int w = 0; w < W; ++w)
+    if (w < warp) {
+      a += wsum[0][w];
+      b += wsum[1][w];
+    }
+  int run = 0;
+  if (tile > 0) {
+    constexpr int LB = 8;
+    int p = tile - 1, rounds = 0;
+    bool done = false;
+    while (!done) {
+      unsigned w[LB];
+#pragma unroll
+      for (int i = 0; i < LB; ++i) w[i] = p - i >= 0 ? (unsigned)slot[(int64_t)(p - i) * kBuckets] : (2u << 30);
+      int moved = 0;
+      bool open = true;
+#pragma unroll
+      for (int i = 0; i < LB; ++i) {
+        if (open && !done && (w[i] & ~kCount)) {
+          run += (int)(w[i] & kCount);
+          ++moved;
+          done = (w[i] & kUpTo) != 0;
+        } else {
+          open = false;
+        }
       }
-      run[b] = acc;
+      p -= moved;
+      if (!done && moved == 0 && ++rounds > kLookRounds) {
+        s_lost = 1;
+        done = true;
+      }
     }
-    __syncthreads();
-    if (valid) {
-      const int pos = tile_off[d] + wcnt[warp][d] + rank;
-      key_out[pos] = k;
-      val_out[pos] = v;
+    slot[(int64_t)tile * kBuckets] = kUpTo | (unsigned)(run + count);
+  }
+  local[t] = b;
+  at[t] = a + run - b;
+  __syncthreads();
+  const int items = (int)min((int64_t)T, n - first);
+  if (s_lost) {  // (a later tile's counts are wrong too; its places are bounded below)
+    if (t == 0) atomicAdd(lost, (unsigned long long)items);
+    for (int i = t; i < items; i += kSortThreads) {
+      key_out[first + i] = key_in[first + i];
+      val_out[first + i] = use_iota ? (int)(first + i) : val_in[first + i];
     }
-    __syncthreads();
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < IT; ++r) {
+    if (base + r * 32 < n) {
+      const int d = (k[r] >> shift) & (kBuckets - 1);
+      const int q = local[d] + wcnt[warp][d] + rank[r];
+      s_key[q] = k[r];
+      s_val[q] = v[r];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < IT; ++r) {
+    const int i = t + r * kSortThreads;
+    if (i < items) {
+      const int key = s_key[i];
+      const int64_t q = (int64_t)at[(key >> shift) & (kBuckets - 1)] + i;
+      if (q >= 0 && q < n) {
+        key_out[q] = key;
+        val_out[q] = s_val[i];
+      }
+    }
+  }
+}
+
+// the passes of one sort on stream s; *kin / *vin: where the sorted keys and indices end up.  A
+// launch is counted and timed through ctx when it is given.
+void radix_launch(mic_ctx *ctx, cudaStream_t s, int **kin, int **kout, int **vin, int **vout, int64_t n, int passes,
+                  int *scratch, unsigned long long *lost) {
+  const int64_t tiles = tiles_for(n);
+  for (int p = 0; p < passes; ++p) {
+    unsigned *words = reinterpret_cast<unsigned *>(scratch + kOffTiles + (int64_t)p * tiles * kBuckets);
+    const int *counts = scratch + kOffCounts + p * kBuckets;
+    if (ctx) mic_prof_begin(ctx, "k_radix_pass", s);
+    if (items_for(n) == kItemsSmall)
+      k_radix_pass<kItemsSmall><<<(unsigned)tiles, kSortThreads, 0, s>>>(*kin, *vin, p == 0, *kout, *vout, n,
+                                                                         p * kRadixBits, counts, words,
+                                                                         scratch + kOffTicket + p, lost);
+    else
+      k_radix_pass<kItemsLarge><<<(unsigned)tiles, kSortThreads, 0, s>>>(*kin, *vin, p == 0, *kout, *vout, n,
+                                                                         p * kRadixBits, counts, words,
+                                                                         scratch + kOffTicket + p, lost);
+    if (ctx) mic_prof_end(ctx, s);
+    int *x = *kin;
+    *kin = *kout;
+    *kout = x;
+    x = *vin;
+    *vin = *vout;
+    *vout = x;
   }
 }
 
@@ -327,22 +493,13 @@ int scan_exclusive(mic_ctx *ctx, int *data, int64_t len, int *aux) {
   return cudaGetLastError() == cudaSuccess ? MIC_OK : MIC_ERR_CUDA;
 }
 
-int ensure_sort_scratch(mic_ctx *ctx, int ntiles) {
-  const int64_t need = (int64_t)kBuckets * ntiles;
-  if (ctx->hist_cap >= need) return MIC_OK;
-  cudaFree(ctx->hist);
-  cudaFree(ctx->scan_aux);
-  ctx->hist = nullptr;
-  ctx->scan_aux = nullptr;
-  ctx->hist_cap = 0;
-  if (cudaMalloc((void **)&ctx->hist, sizeof(int) * need) != cudaSuccess) return MIC_ERR_NOMEM;
-  int64_t aux = 0, l = need;
-  while (l > 1) {
-    l = (l + kScanBlock - 1) / kScanBlock;
-    aux += l + 1;
-  }
-  if (cudaMalloc((void **)&ctx->scan_aux, sizeof(int) * (aux + 16)) != cudaSuccess) return MIC_ERR_NOMEM;
-  ctx->hist_cap = (int)need;
+int ensure_sort_scratch(mic_ctx *ctx, int64_t need) {
+  if (ctx->sort_cap >= need) return MIC_OK;
+  cudaFree(ctx->sort_buf);
+  ctx->sort_buf = nullptr;
+  ctx->sort_cap = 0;
+  if (cudaMalloc((void **)&ctx->sort_buf, sizeof(int) * need) != cudaSuccess) return MIC_ERR_NOMEM;
+  ctx->sort_cap = need;
   return MIC_OK;
 }
 
@@ -351,7 +508,8 @@ int ensure_sort_scratch(mic_ctx *ctx, int ntiles) {
 // Bins every marker, sorts the columns by cell (stable) and rebuilds cell_start.
 int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
   const int64_t n = ctx->n;
-  cudaMemsetAsync(&ctx->d_status->n_out, 0, sizeof(unsigned long long), ctx->stream);
+  // n_out and bad_cell
+  MIC_CUDA_TRY(cudaMemsetAsync(&ctx->d_status->n_out, 0, 2 * sizeof(unsigned long long), ctx->stream));
   if (n == 0) {
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->cell_start, 0, sizeof(int) * ((size_t)ctx->ncells + 2), ctx->stream));
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->quad_start, 0, sizeof(int) * (4 * (size_t)ctx->ncells + 5), ctx->stream));
@@ -359,42 +517,23 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
     if (n_out) *n_out = 0;
     return MIC_OK;
   }
+  const int passes = passes_for(ctx->ncells);
+  const int64_t ints = sort_ints(tiles_for(n), passes);
+  int e = ensure_sort_scratch(ctx, ints);
+  if (e) return e;
+  MIC_CUDA_TRY(cudaMemsetAsync(ctx->sort_buf, 0, sizeof(int) * ints, ctx->stream));
   {
     MIC_KERNEL(ctx, "k_find_cells");
-    k_find_cells<<<grid_for(n, tuned_block(ctx, TU_FIND_CELLS)), tuned_block(ctx, TU_FIND_CELLS), 0, ctx->stream>>>(ctx->P, ctx->f64[C_X], ctx->f64[C_Y], ctx->i32[C_CELLX],
-                                                          ctx->i32[C_CELLY], ctx->i32[C_CPU], ctx->key, n,
-                                                          ctx->d_status);
+    const int block = tuned_block(ctx, TU_FIND_CELLS);
+    const unsigned full = grid_for(n, block), most = 2048 / block * sm_count(ctx);
+    k_find_cells<<<full < most ? full : most, block, 0, ctx->stream>>>(
+        ctx->P, ctx->f64[C_X], ctx->f64[C_Y], ctx->i32[C_CELLX], ctx->i32[C_CELLY], ctx->i32[C_CPU], ctx->key, n, passes,
+        ctx->sort_buf + kOffCounts, ctx->d_status);
   }
   MIC_CUDA_TRY(cudaGetLastError());
-  const int ntiles = (int)((n + kTile - 1) / kTile);
-  int e = ensure_sort_scratch(ctx, ntiles);
-  if (e) return e;
-  int bits = 1;
-  while ((1LL << bits) <= 4LL * ctx->ncells) ++bits;
-  const int passes = (bits + kRadixBits - 1) / kRadixBits;
   int *kin = ctx->key, *kout = ctx->key_alt, *vin = ctx->perm, *vout = ctx->perm_alt;
-  for (int p = 0; p < passes; ++p) {
-    const int shift = p * kRadixBits;
-    {
-      MIC_KERNEL(ctx, "k_radix_hist");
-      k_radix_hist<<<ntiles, kSortThreads, 0, ctx->stream>>>(kin, n, shift, ctx->hist, ntiles);
-    }
-    MIC_CUDA_TRY(cudaGetLastError());
-    e = scan_exclusive(ctx, ctx->hist, (int64_t)kBuckets * ntiles, ctx->scan_aux);
-    if (e) return e;
-    {
-      MIC_KERNEL(ctx, "k_radix_scatter");
-      k_radix_scatter<<<ntiles, kSortThreads, 0, ctx->stream>>>(kin, vin, p == 0, kout, vout, n, shift, ctx->hist,
-                                                                ntiles);
-    }
-    MIC_CUDA_TRY(cudaGetLastError());
-    int *t = kin;
-    kin = kout;
-    kout = t;
-    t = vin;
-    vin = vout;
-    vout = t;
-  }
+  radix_launch(ctx, ctx->stream, &kin, &kout, &vin, &vout, n, passes, ctx->sort_buf, &ctx->d_status->bad_cell);
+  MIC_CUDA_TRY(cudaGetLastError());
   // kin / vin now hold the sorted keys and the permutation
   {
     MIC_KERNEL(ctx, "k_cell_start");
@@ -434,6 +573,7 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
     MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
     MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     *n_out = (int64_t)ctx->h_status->n_out;
+    if (ctx->h_status->bad_cell) return MIC_ERR_CELL;
   }
   return MIC_OK;
 }
@@ -521,17 +661,19 @@ namespace {
 
 constexpr int64_t kNoallocMaxMarkers = MIC_NOALLOC_MAX_MARKERS;
 constexpr int64_t kNoallocMaxCells = MIC_NOALLOC_MAX_CELLS;
-constexpr int64_t kNoallocTiles = (kNoallocMaxMarkers + kTile - 1) / kTile;
-constexpr int64_t kNoallocHist = (int64_t)kBuckets * kNoallocTiles;
-// block totals of every scan level of the histogram matrix, with one spare entry per level
-constexpr int64_t kNoallocAux = (kNoallocHist + kScanBlock - 1) / kScanBlock + 64;
-// layout (in 4-byte words): key | key_alt | val_alt | hist | aux, then one 8-byte counter
+// the sort's own scratch at the largest tile count: tiles of the small sort up to kSmallSort
+// markers, of the large one beyond; the largest key has three digits
+constexpr int64_t kNoallocTiles = kSmallSort / (kSortThreads * kItemsSmall);
+static_assert(kNoallocTiles >= kNoallocMaxMarkers / (kSortThreads * kItemsLarge), "tiles of the largest sort");
+constexpr int kNoallocPasses = 3;
+static_assert(4 * kNoallocMaxCells < (1LL << (kNoallocPasses * kRadixBits)), "digits of the largest key");
+constexpr int64_t kNoallocSort = kOffTiles + kNoallocPasses * kNoallocTiles * kBuckets;
+// layout (in 4-byte words): key | key_alt | val_alt | sort, then two 8-byte counters
 constexpr int64_t kOffKey = 0;
 constexpr int64_t kOffKeyAlt = kOffKey + kNoallocMaxMarkers;
 constexpr int64_t kOffValAlt = kOffKeyAlt + kNoallocMaxMarkers;
-constexpr int64_t kOffHist = kOffValAlt + kNoallocMaxMarkers;
-constexpr int64_t kOffAux = kOffHist + kNoallocHist;
-constexpr int64_t kWords = (kOffAux + kNoallocAux + 63) / 64 * 64;
+constexpr int64_t kOffSort = kOffValAlt + kNoallocMaxMarkers;
+constexpr int64_t kWords = (kOffSort + kNoallocSort + 63) / 64 * 64;
 constexpr size_t kNoallocBytes = (size_t)kWords * 4 + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
@@ -575,15 +717,20 @@ unsigned long long current_context_id() {
 __global__ void k_find_cells_grid(const double *__restrict__ X, const double *__restrict__ Y,
                                   const double *__restrict__ xg, const double *__restrict__ yg, int NX, int NY,
                                   double LX, double LY, int *__restrict__ cellX, int *__restrict__ cellY,
-                                  int *__restrict__ key, int64_t n, unsigned long long *n_out) {
+                                  int *__restrict__ key, int64_t n, int passes, int *counts,
+                                  unsigned long long *n_out) {
   __shared__ unsigned long long s_out;
+  __shared__ int h[kMaxPasses][kBuckets];
   if (threadIdx.x == 0) s_out = 0;
+  clear_digits(h, passes);
   __syncthreads();
   const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  int k = 0;
   if (m < n) {
     const long long ux = nonneg_bits(X[m]), uy = nonneg_bits(Y[m]);
     const bool in = ux >= 0 && uy >= 0 && ux <= dbits(LX) && uy <= dbits(LY);
-    int cx = -1, cy = -1, k = 4 * (NX - 1) * (NY - 1);
+    int cx = -1, cy = -1;
+    k = 4 * (NX - 1) * (NY - 1);
     if (in) {
       int lo = 0, hi = NX - 1;
       while (hi - lo > 1) {
@@ -609,7 +756,9 @@ __global__ void k_find_cells_grid(const double *__restrict__ X, const double *__
     cellY[m] = cy;
     key[m] = k;
   }
+  count_digits(h, passes, m < n, k);
   __syncthreads();
+  add_digits(h, passes, counts);
   if (threadIdx.x == 0 && s_out) atomicAdd(n_out, s_out);
 }
 
@@ -659,42 +808,21 @@ extern "C" int mic_bin_sort_noalloc(const double *X, const double *Y, int64_t n,
   cudaStream_t s = (cudaStream_t)stream;
   int *words = reinterpret_cast<int *>(base);
   int *key = words + kOffKey, *key_alt = words + kOffKeyAlt, *val_alt = words + kOffValAlt;
-  int *hist = words + kOffHist, *aux = words + kOffAux;
-  unsigned long long *d_out = reinterpret_cast<unsigned long long *>(base + (size_t)kWords * 4);
-  // the counter keeps the previous call's value: clear it
-  if (cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), s) != cudaSuccess) return MIC_ERR_CUDA;
+  int *sort = words + kOffSort;
+  // markers outside the domain, and markers a sort that gave up has not placed
+  unsigned long long *d_out = reinterpret_cast<unsigned long long *>(base + (size_t)kWords * 4), *d_lost = d_out + 1;
+  // the counters keep the previous call's values: clear them
+  if (cudaMemsetAsync(d_out, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess) return MIC_ERR_CUDA;
   if (n > 0) {
-    k_find_cells_grid<<<grid_for(n), kBlock, 0, s>>>(X, Y, x, y, NX, NY, LX, LY, cellX, cellY, key, n, d_out);
+    const int passes = passes_for(ncells);
+    if (cudaMemsetAsync(sort, 0, sizeof(int) * sort_ints(tiles_for(n), passes), s) != cudaSuccess) return MIC_ERR_CUDA;
+    k_find_cells_grid<<<grid_for(n), kBlock, 0, s>>>(X, Y, x, y, NX, NY, LX, LY, cellX, cellY, key, n, passes,
+                                                     sort + kOffCounts, d_out);
     if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
-    const int ntiles = (int)((n + kTile - 1) / kTile);
-    int bits = 1;
-    while ((1LL << bits) <= 4 * ncells) ++bits;
-    const int passes = (bits + kRadixBits - 1) / kRadixBits;
-    // the last pass must write the caller's perm[]: pick the ping-pong order accordingly
-    int *vbuf[2] = {(passes & 1) ? perm : val_alt, (passes & 1) ? val_alt : perm};
-    int *kbuf[2] = {key_alt, key};
-    int *kin = key, *vin = nullptr;
-    for (int p = 0; p < passes; ++p) {
-      int *kout = kbuf[p & 1], *vout = vbuf[p & 1];
-      k_radix_hist<<<ntiles, kSortThreads, 0, s>>>(kin, n, p * kRadixBits, hist, ntiles);
-      if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
-      // every bucket of every tile is written by k_radix_hist, so nothing stale survives
-      const int64_t len = (int64_t)kBuckets * ntiles;
-      const int64_t nb = (len + kScanBlock - 1) / kScanBlock;
-      if (nb <= 1) {
-        k_scan_block<<<1, kScanThreads, 0, s>>>(hist, len, nullptr);
-      } else {
-        // two levels suffice: nb <= kScanBlock for the largest histogram matrix
-        k_scan_block<<<(unsigned)nb, kScanThreads, 0, s>>>(hist, len, aux);
-        k_scan_block<<<1, kScanThreads, 0, s>>>(aux, nb, nullptr);
-        k_scan_add<<<(unsigned)nb, kScanThreads, 0, s>>>(hist, len, aux);
-      }
-      k_radix_scatter<<<ntiles, kSortThreads, 0, s>>>(kin, vin, p == 0, kout, vout, n, p * kRadixBits, hist,
-                                                       ntiles);
-      if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
-      kin = kout;
-      vin = vout;
-    }
+    // the last pass must write the caller's perm[]: pick the buffers accordingly (the first reads none)
+    int *kin = key, *kout = key_alt, *vin = (passes & 1) ? val_alt : perm, *vout = (passes & 1) ? perm : val_alt;
+    radix_launch(nullptr, s, &kin, &kout, &vin, &vout, n, passes, sort, d_lost);
+    if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
     k_cell_start<<<grid_for(4LL * ncells + 5), kBlock, 0, s>>>(kin, n, (int)ncells, cell_start, nullptr);
   } else {
     if (cudaMemsetAsync(cell_start, 0, sizeof(int32_t) * (size_t)(ncells + 2), s) != cudaSuccess)
@@ -702,10 +830,11 @@ extern "C" int mic_bin_sort_noalloc(const double *X, const double *Y, int64_t n,
   }
   if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
   if (n_out) {
-    unsigned long long h = 0;
-    if (cudaMemcpyAsync(&h, d_out, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MIC_ERR_CUDA;
+    unsigned long long h[2] = {0, 0};
+    if (cudaMemcpyAsync(h, d_out, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MIC_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return MIC_ERR_CUDA;
-    *n_out = (int64_t)h;
+    *n_out = (int64_t)h[0];
+    if (h[1]) return MIC_ERR_CELL;
   }
   return MIC_OK;
 }

@@ -138,8 +138,7 @@ static void free_ctx(mic_ctx *ctx) {
   cudaFree(ctx->quad_start);
   cudaFree(ctx->part_b);
   cudaFree(ctx->part_c);
-  cudaFree(ctx->hist);
-  cudaFree(ctx->scan_aux);
+  cudaFree(ctx->sort_buf);
   for (int g = 0; g < 4; ++g) cudaFree(ctx->geo[g]);
   cudaFree(ctx->geo_flags);
   cudaFree(ctx->wgt[0]);
@@ -370,6 +369,8 @@ extern "C" int mic_create(mic_ctx **out, int device, void *stream, int NX, int N
   ALLOC(ctx->key_alt, sizeof(int) * cap);
   ALLOC(ctx->perm, sizeof(int) * cap);
   ALLOC(ctx->perm_alt, sizeof(int) * cap);
+  cudaMemset(ctx->perm, 0, sizeof(int) * cap);  // (an index in range, whatever happens to a sort)
+  cudaMemset(ctx->perm_alt, 0, sizeof(int) * cap);
   ALLOC(ctx->cell_start, sizeof(int) * (max_cells + 2));
   ALLOC(ctx->quad_start, sizeof(int) * (4 * max_cells + 5));
   ALLOC(ctx->part_b, sizeof(double) * 32 * max_cells);

@@ -38,11 +38,11 @@ enum I32Col { C_MAT = 0, C_CELLX, C_CELLY, C_CPU, C_ISYIELD, C_ID, C_I32_COUNT }
 
 // device status word (counts of events the reference aborts or prints on)
 struct Status {
-  unsigned long long bad_cell;      // impossible cell index (markers.c:74-77)
   unsigned long long nan_residual;  // NaN strain-rate residual (updateMarkerStrainPressure.c:302-306)
   unsigned long long nan_dsxy;      // NaN interpolated dsxy (updateMarkerStress.c:136-142)
   unsigned long long bad_law;       // unknown viscosity law (viscosity.c:60-62)
   unsigned long long n_out;         // out-of-domain markers after the last binning
+  unsigned long long bad_cell;      // impossible cell index (markers.c:74-77): markers not placed (cleared with n_out)
   int is_yielding;                  // any marker yielded in the last checkPlasticYielding
   int pad;
 };
@@ -147,9 +147,8 @@ struct mic_ctx {
   int *cell_start;     // ncells + 2 entries
   int *quad_start;     // 4*ncells + 5 entries: runs of each (cell, quadrant)
   double *part_b, *part_c;  // per-cell corner partial sums of the projections (product build)
-  int *hist;           // radix histograms (digit-major per tile)
-  int hist_cap;
-  int *scan_aux;
+  int *sort_buf;       // digit counts and tile words of the radix passes (grown on demand)
+  int64_t sort_cap;
   int sorted;          // columns are in cell order for the current positions
   // per-marker projection geometry for the current positions and order (see mic_project.cu)
   double *geo[4];      // mdx0, mdy0 (basic cell), mdx1, mdy1 (cell-centre stagger -1,-1)

@@ -1582,7 +1582,7 @@ YieldCols yield_cols(mic_ctx *ctx) {
 int read_status(mic_ctx *ctx) {
   MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
+  return ctx->h_status->bad_cell ? MIC_ERR_CELL : MIC_OK;  // markers the last binning could not place
 }
 
 int run_max(mic_ctx *ctx, int col, int absval, double *out) {
