@@ -514,6 +514,7 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->cell_start, 0, sizeof(int) * ((size_t)ctx->ncells + 2), ctx->stream));
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->quad_start, 0, sizeof(int) * (4 * (size_t)ctx->ncells + 5), ctx->stream));
     ctx->sorted = 1;
+    ctx->wn_valid = 0;
     if (n_out) *n_out = 0;
     return MIC_OK;
   }
@@ -569,6 +570,7 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
   }
   ctx->sorted = 1;
   ctx->geo_valid = 1;  // computed by the gather
+  ctx->wn_valid = 0;
   if (n_out) {
     MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
     MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));

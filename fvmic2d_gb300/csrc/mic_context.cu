@@ -136,6 +136,7 @@ static void free_ctx(mic_ctx *ctx) {
   cudaFree(ctx->perm_alt);
   cudaFree(ctx->cell_start);
   cudaFree(ctx->quad_start);
+  for (int g = 0; g < 2; ++g) cudaFree(ctx->wnode[g]);
   cudaFree(ctx->part_b);
   cudaFree(ctx->part_c);
   cudaFree(ctx->sort_buf);
@@ -380,6 +381,7 @@ extern "C" int mic_create(mic_ctx **out, int device, void *stream, int NX, int N
 #ifndef MIC_EXACT
   ALLOC(ctx->wgt[0], 4 * sizeof(double) * cap);
   ALLOC(ctx->wgt[1], 4 * sizeof(double) * cap);
+  for (int g = 0; g < 2; ++g) ALLOC(ctx->wnode[g], sizeof(double) * nn);
 #endif
   ALLOC(ctx->scr0, sizeof(double) * cap);
   ALLOC(ctx->scr1, sizeof(double) * cap);

@@ -156,6 +156,8 @@ struct mic_ctx {
   double *wgt[2];      // bilinear corner weights (product build), 4 per marker in corner order
                        // 00, 10, 01, 11: [0] of the basic cell, [1] of the cell-centre cell
   int geo_valid;
+  double *wnode[2];    // nodal weight sums of the binned markers (product build): basic nodes, cell centres
+  int wn_valid;        // bits 0, 1: wnode[0], wnode[1] hold this binning's
   // per-marker scratch
   double *scr0, *scr1, *scr2;
   double *node_scr[6];  // nodal scratch (NX*NY each)

@@ -38,6 +38,7 @@ __global__ void k_geometry(Params P, const double *__restrict__ X, const double 
 
 struct All2Out {
   double *rho, *rhodot, *etaN, *etaS, *muS, *muN, *k, *lastT, *Cp, *soxx, *soyy, *soxy;
+  double *w0, *w1;  // product build: the weight sums of the basic nodes and of the cell centres
 };
 
 struct MarkerView {
@@ -299,40 +300,52 @@ struct PartialView {
   const double *w0, *w1;  // stored corner weights of the basic and the cell-centre cell
 };
 
-// ALL2: rho, etaS, k, T, Cp, weight per corner (24) + nearest-node sxy, weight (8) = 32 sums.
-// !ALL2: scalar, weight per corner = 8 sums.  part[acc * ncells + cell].  VISC (with ALL2): only
-// the sums whose marker inputs yielding and the viscosity limit change (etaS per corner, the
-// nearest-node sxy and its weight); the other slots keep the previous ALL2 pass's sums.  FIRST
-// (with ALL2): only the others (rho, k, T, Cp and the weight per corner), for a projection whose
-// viscosity and stress fields a VISC pass replaces before they are read.
+// basic cells (ALL2): rho, etaS, k, T, Cp, weight per corner (24) + nearest-node sxy, weight (8) = 32
+// sums, part[acc * ncells + cell].  VISC: only the sums whose marker inputs yielding and the
+// viscosity limit change (etaS per corner, the nearest-node sxy and its weight); the other slots keep
+// the previous ALL2 pass's sums.  FIRST: only the others (rho, k, T, Cp and the weight per corner),
+// for a projection whose viscosity and stress fields a VISC pass replaces before they are read.
 //
-// One loop over the cell's markers (its four quadrant runs back to back, the same order as
-// quadrant by quadrant): a warp's lanes then wait for the longest cell of the warp once, not
-// for the longest run of each quadrant four times.  The nearest-node sums go to a per-thread
-// shared-memory slot picked by the marker's corner, so the loop has no corner branches.
-template <bool ALL2, bool VISC = false, bool FIRST = false>
+// Two forms with the same sums in the same order, bit for bit:
+//   a thread per cell (k_partials_*): one loop over the cell's markers (its four quadrant runs back
+//     to back, the same order as quadrant by quadrant): a warp's lanes then wait for the longest
+//     cell of the warp once, not for the longest run of each quadrant four times.  The nearest-node
+//     sums go to a per-thread shared-memory slot picked by the marker's corner, so the loop has no
+//     corner branches;
+//   a thread per cell and corner (k_corners_*): four lanes walk a cell's markers together, each with
+//     its own corner's weight, four markers' loads in flight.  A lane has a quarter of the FP64
+//     chain and the GPU four times the warps; but a marker's nearest-node sums keep one of its four
+//     lanes busy, so it issues more FP64 in all.
+// The second serves grids whose cells do not give every SM quarter a warp of the first, up to 32
+// cells per SM (4,864): there a pass is a chain of latencies (64 x 64 cells: 24 us for kFirst, 18 for
+// kVisc, 25 for the centres in the first form, 16, 14 and 14 in the second); and every single-field
+// projection, whose sums split evenly over the lanes (16.8 M markers: 298 us with a thread per cell
+// and weights, 147 with a thread per corner and the weights known).
+enum Sums { kFull, kVisc, kFirst };
+
+template <Sums WHAT>
 __global__ void __launch_bounds__(128) k_partials_basic(Params P, PartialView v, const int *__restrict__ qs,
                                                          mic_materials mat, double *__restrict__ part) {
-  __shared__ double sloc[(ALL2 && !FIRST) ? 8 : 1][128];
+  constexpr bool VISC = WHAT == kVisc, FIRST = WHAT == kFirst;
+  __shared__ double sloc[FIRST ? 1 : 8][128];
   const int ncells = P.NCX * (P.NY - 1);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncells) return;
-  constexpr int NA = ALL2 ? 6 : 2;
+  constexpr int NA = 6;
   const int t = threadIdx.x;
-  // ALL2: rho (0), k (2) and Cp (4) sums in double-float arithmetic (slot f of accd); etaS (1,
-  // whose own pass measured slower in double-float), T (3) and the weights (5), which later enter
-  // differences (T against marker T in the sub-grid temperature pass), and the scalar
-  // projections in FP64 (acc)
+  // rho (0), k (2) and Cp (4) sums in double-float arithmetic (slot f of accd); etaS (1, whose own
+  // pass measured slower in double-float), T (3) and the weights (5), which later enter
+  // differences (T against marker T in the sub-grid temperature pass), in FP64 (acc)
   double acc[4][NA];
-  df accd[4][ALL2 ? 5 : 1];
+  df accd[4][5];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
 #pragma unroll
     for (int f = 0; f < NA; ++f) acc[k][f] = 0.0;
 #pragma unroll
-    for (int f = 0; f < (ALL2 ? 5 : 1); ++f) accd[k][f] = df{0.0f, 0.0f};
+    for (int f = 0; f < 5; ++f) accd[k][f] = df{0.0f, 0.0f};
   }
-  if (ALL2 && !FIRST) {
+  if (!FIRST) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) sloc[k][t] = 0.0;
   }
@@ -340,11 +353,11 @@ __global__ void __launch_bounds__(128) k_partials_basic(Params P, PartialView v,
   for (int m = mb; m < me; ++m) {
     const W4 ww = load_w4(v.w0, m);
     const double w[4] = {ww.w00, ww.w10, ww.w01, ww.w11};
-    if (ALL2 && VISC) {
+    if (VISC) {
       const double e = v.eta[m];
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc[k][1] = fma(w[k], e, acc[k][1]);
-    } else if (ALL2) {
+    } else {
       const double tt = v.T[m];
       const df r = df_of(v.rho[m]);
       const double e = FIRST ? 0.0 : v.eta[m];
@@ -361,7 +374,7 @@ __global__ void __launch_bounds__(128) k_partials_basic(Params P, PartialView v,
         acc[k][5] += w[k];
       }
     }
-    if (ALL2 && !FIRST) {
+    if (!FIRST) {
       // nearest basic node (mdx0 >= .5, mdy0 >= .5): the weight of that corner, as w[corner]
       const int fl = v.flags[m];
       const int corner = ((fl >> 2) & 1) | (((fl >> 3) & 1) << 1);
@@ -369,13 +382,6 @@ __global__ void __launch_bounds__(128) k_partials_basic(Params P, PartialView v,
       double *L = &sloc[2 * corner][t];
       L[0] = fma(wc, v.sxy[m], L[0]);
       L[128] = __dadd_rn(L[128], wc);
-    } else if (!ALL2) {
-      const double sc = v.scalar[m];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        acc[k][0] = fma(w[k], sc, acc[k][0]);
-        acc[k][1] += w[k];
-      }
     }
   }
 #pragma unroll
@@ -383,87 +389,243 @@ __global__ void __launch_bounds__(128) k_partials_basic(Params P, PartialView v,
 #pragma unroll
     for (int f = 0; f < NA; ++f)
       if ((!VISC || f == 1) && (!FIRST || f != 1))
-        part[(size_t)(k * NA + f) * ncells + c] =
-            (ALL2 && (f == 0 || f == 2 || f == 4)) ? df_to_f64(accd[k][f]) : acc[k][f];
-    if (ALL2 && !FIRST) {
+        part[(size_t)(k * NA + f) * ncells + c] = (f == 0 || f == 2 || f == 4) ? df_to_f64(accd[k][f]) : acc[k][f];
+    if (!FIRST) {
       part[(size_t)(24 + 2 * k) * ncells + c] = sloc[2 * k][t];
       part[(size_t)(25 + 2 * k) * ncells + c] = sloc[2 * k + 1][t];
     }
   }
 }
 
+constexpr int kAhead = 4;  // markers whose loads a lane has in flight
+
+// the same sums, a thread per cell and corner
+template <Sums WHAT>
+__global__ void __launch_bounds__(128) k_corners_basic(Params P, PartialView v, const int *__restrict__ qs,
+                                                        mic_materials mat, double *__restrict__ part) {
+  constexpr bool VISC = WHAT == kVisc, FIRST = WHAT == kFirst;
+  const int ncells = P.NCX * (P.NY - 1);
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, c = idx >> 2, k = idx & 3;
+  if (c >= ncells) return;
+  double eta = 0.0, T = 0.0, wsum = 0.0, sxy = 0.0, wnear = 0.0;
+  df rho = {0.0f, 0.0f}, kth = rho, cp = rho;
+  const int mb = qs[4 * c], me = qs[4 * c + 4];
+  for (int m0 = mb; m0 < me; m0 += kAhead) {
+    double w[kAhead], e[kAhead], t[kAhead], r[kAhead], s[kAhead];
+    int mt[kAhead], fl[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int m = min(m0 + i, me - 1);
+      w[i] = __ldg(v.w0 + 4 * (size_t)m + k);
+      if (!FIRST) {
+        e[i] = v.eta[m];
+        s[i] = v.sxy[m];
+        fl[i] = v.flags[m];
+      }
+      if (!VISC) {
+        t[i] = v.T[m];
+        r[i] = v.rho[m];
+        mt[i] = v.mat[m];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      if (m0 + i >= me) break;
+      if (!FIRST) {
+        eta = fma(w[i], e[i], eta);
+        if ((((fl[i] >> 2) & 1) | (((fl[i] >> 3) & 1) << 1)) == k) {
+          sxy = fma(w[i], s[i], sxy);
+          wnear = __dadd_rn(wnear, w[i]);
+        }
+      }
+      if (!VISC) {
+        const df wk = df_of(w[i]);
+        rho = df_fma(wk, df_of(r[i]), rho);
+        kth = df_fma(wk, df_of(mat.materialkThermal[mt[i]]), kth);
+        cp = df_fma(wk, df_of(mat.materialCp[mt[i]]), cp);
+        T = fma(w[i], t[i], T);
+        wsum += w[i];
+      }
+    }
+  }
+  double *o = part + (size_t)(k * 6) * ncells + c;
+  if (!VISC) {
+    o[0] = df_to_f64(rho);
+    o[2 * (size_t)ncells] = df_to_f64(kth);
+    o[3 * (size_t)ncells] = T;
+    o[4 * (size_t)ncells] = df_to_f64(cp);
+    o[5 * (size_t)ncells] = wsum;
+  }
+  if (!FIRST) {
+    o[ncells] = eta;
+    part[(size_t)(24 + 2 * k) * ncells + c] = sxy;
+    part[(size_t)(25 + 2 * k) * ncells + c] = wnear;
+  }
+}
+
+// A single field on the basic cells, a thread per cell and corner: 2 k the corner's sum, and
+// (WEIGHT, when the nodes' weight sums are not known yet) 2 k + 1 its weight.
+template <bool WEIGHT>
+__global__ void __launch_bounds__(128) k_corners_basic_scalar(Params P, PartialView v, const int *__restrict__ qs,
+                                                               double *__restrict__ part) {
+  const int ncells = P.NCX * (P.NY - 1);
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, c = idx >> 2, k = idx & 3;
+  if (c >= ncells) return;
+  double a = 0.0, ws = 0.0;
+  const int mb = qs[4 * c], me = qs[4 * c + 4];
+  for (int m0 = mb; m0 < me; m0 += kAhead) {
+    double w[kAhead], x[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int m = min(m0 + i, me - 1);
+      w[i] = __ldg(v.w0 + 4 * (size_t)m + k);
+      x[i] = v.scalar[m];
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      if (m0 + i >= me) break;
+      a = fma(w[i], x[i], a);
+      if (WEIGHT) ws += w[i];
+    }
+  }
+  part[(size_t)(2 * k) * ncells + c] = a;
+  if (WEIGHT) part[(size_t)(2 * k + 1) * ncells + c] = ws;
+}
+
 // Staggered (cell-centre) cell s = (sx, sy), sx in [0, NCX]: its markers are quadrant 3 of
 // basic cell (sx-1, sy-1), quadrant 2 of (sx, sy-1), quadrant 1 of (sx-1, sy) and quadrant 0 of
-// (sx, sy).  ALL2: etaN, weight per corner (8) + nearest-node sxx, syy, weight (12) = 20 sums;
-// !ALL2: scalar, weight per corner = 8.  part[acc * (NX+1)*NY + s], s = sy (NX+1) + sx.
+// (sx, sy).  etaN, weight per corner (8) + nearest-node sxx, syy, weight (12) = 20 sums,
+// part[acc * (NX+1)*NY + s], s = sy (NX+1) + sx.
 //
 // The four runs are walked as one sequence (run 0's markers, then run 1's, ...) by one loop,
 // for the same reason as in k_partials_basic; the nearest-centre sums use per-thread shared
 // slots.
-template <bool ALL2>
+struct Runs {  // starts and ends (in the sequence) of a staggered cell's four runs
+  int rb[4], e1, e2, e3, total;
+  __device__ __forceinline__ int marker(int u) const {
+    return (u < e1) ? rb[0] + u : (u < e2) ? rb[1] + (u - e1) : (u < e3) ? rb[2] + (u - e2) : rb[3] + (u - e3);
+  }
+};
+// run r of staggered cell (sx, sy): basic cell (sx-1+dx, sy-1+dy)'s quadrant; empty outside the grid
+__device__ __forceinline__ void centre_run(const Params &P, const int *__restrict__ qs, int sx, int sy, int r, int &b,
+                                           int &n) {
+  const int dx = r & 1, dy = r >> 1;
+  const int cx = sx - 1 + dx, cy = sy - 1 + dy, q = (1 - dx) + 2 * (1 - dy);
+  b = 0;
+  n = 0;
+  if (cx >= 0 && cx < P.NCX && cy >= 0 && cy <= P.NY - 2) {
+    const int qq = 4 * (cy * P.NCX + cx) + q;
+    b = qs[qq];
+    n = qs[qq + 1] - b;
+  }
+}
+
 __global__ void __launch_bounds__(128) k_partials_centre(Params P, PartialView v, const int *__restrict__ qs,
                                                           double *__restrict__ part) {
-  __shared__ double sloc[ALL2 ? 12 : 1][128];
+  __shared__ double sloc[12][128];
   const int sx = blockIdx.x * blockDim.x + threadIdx.x;
   const int sy = blockIdx.y;
   if (sx > P.NCX || sy >= P.NY) return;
-  const int NC = P.NCX;
   const int t = threadIdx.x;
   const size_t ns = (size_t)(P.NX + 1) * P.NY, s = (size_t)sy * (P.NX + 1) + sx;
   double acc[4][2];
 #pragma unroll
   for (int k = 0; k < 4; ++k) acc[k][0] = acc[k][1] = 0.0;
-  if (ALL2) {
 #pragma unroll
-    for (int k = 0; k < 12; ++k) sloc[k][t] = 0.0;
-  }
-  int rb[4], rn[4];  // run starts and lengths; a run outside the grid is empty
+  for (int k = 0; k < 12; ++k) sloc[k][t] = 0.0;
+  Runs R;
+  int rn[4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int dx = r & 1, dy = r >> 1;         // basic cell (sx-1+dx, sy-1+dy) ...
-    const int cx = sx - 1 + dx, cy = sy - 1 + dy;
-    const int q = (1 - dx) + 2 * (1 - dy);      // ... contributes its quadrant q
-    rb[r] = 0;
-    rn[r] = 0;
-    if (cx >= 0 && cx < NC && cy >= 0 && cy <= P.NY - 2) {
-      const int qq = 4 * (cy * NC + cx) + q;
-      rb[r] = qs[qq];
-      rn[r] = qs[qq + 1] - qs[qq];
-    }
-  }
-  const int e1 = rn[0], e2 = e1 + rn[1], e3 = e2 + rn[2], total = e3 + rn[3];
-  for (int u = 0; u < total; ++u) {
-    const int m = (u < e1) ? rb[0] + u : (u < e2) ? rb[1] + (u - e1) : (u < e3) ? rb[2] + (u - e2) : rb[3] + (u - e3);
+  for (int r = 0; r < 4; ++r) centre_run(P, qs, sx, sy, r, R.rb[r], rn[r]);
+  R.e1 = rn[0];
+  R.e2 = R.e1 + rn[1];
+  R.e3 = R.e2 + rn[2];
+  R.total = R.e3 + rn[3];
+  for (int u = 0; u < R.total; ++u) {
+    const int m = R.marker(u);
     const W4 ww = load_w4(v.w1, m);
     const double w[4] = {ww.w00, ww.w10, ww.w01, ww.w11};
-    const double e = ALL2 ? v.eta[m] : v.scalar[m];
+    const double e = v.eta[m];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       acc[k][0] = fma(w[k], e, acc[k][0]);
       acc[k][1] += w[k];
     }
-    if (ALL2) {
-      // nearest cell centre (mdx1 >= .5, mdy1 >= .5), weight as w[corner]
-      const int fl = v.flags[m];
-      const int corner = ((fl >> 4) & 1) | (((fl >> 5) & 1) << 1);
-      const double wc = w4_at(ww, corner);
-      double *L = &sloc[3 * corner][t];
-      L[0] = fma(wc, v.sxx[m], L[0]);
-      L[128] = fma(wc, v.syy[m], L[128]);
-      L[256] = __dadd_rn(L[256], wc);
-    }
+    // nearest cell centre (mdx1 >= .5, mdy1 >= .5), weight as w[corner]
+    const int fl = v.flags[m];
+    const int corner = ((fl >> 4) & 1) | (((fl >> 5) & 1) << 1);
+    const double wc = w4_at(ww, corner);
+    double *L = &sloc[3 * corner][t];
+    L[0] = fma(wc, v.sxx[m], L[0]);
+    L[128] = fma(wc, v.syy[m], L[128]);
+    L[256] = __dadd_rn(L[256], wc);
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     part[(size_t)(2 * k) * ns + s] = acc[k][0];
     part[(size_t)(2 * k + 1) * ns + s] = acc[k][1];
-    if (ALL2) {
-      part[(size_t)(8 + 3 * k) * ns + s] = sloc[3 * k][t];
-      part[(size_t)(9 + 3 * k) * ns + s] = sloc[3 * k + 1][t];
-      part[(size_t)(10 + 3 * k) * ns + s] = sloc[3 * k + 2][t];
-    }
+    part[(size_t)(8 + 3 * k) * ns + s] = sloc[3 * k][t];
+    part[(size_t)(9 + 3 * k) * ns + s] = sloc[3 * k + 1][t];
+    part[(size_t)(10 + 3 * k) * ns + s] = sloc[3 * k + 2][t];
   }
 }
+
+// A thread per staggered cell and corner: the sums of k_partials_centre (ALL2), or a single field's
+// (2 k, and with WEIGHT its weight at 2 k + 1).  Lane r of a cell's four looks up run r.
+template <bool ALL2, bool WEIGHT>
+__global__ void __launch_bounds__(128) k_corners_centre(Params P, PartialView v, const int *__restrict__ qs,
+                                                         double *__restrict__ part) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, k = idx & 3;
+  const int sx = min(idx >> 2, P.NCX), sy = blockIdx.y;  // (lanes beyond the row stay for the exchange)
+  const size_t ns = (size_t)(P.NX + 1) * P.NY, s = (size_t)sy * (P.NX + 1) + sx;
+  int b, n;
+  centre_run(P, qs, sx, sy, k, b, n);
+  Runs R;
+  const int l0 = (threadIdx.x & 31) & ~3;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) R.rb[r] = __shfl_sync(0xffffffffu, b, l0 + r);
+  R.e1 = __shfl_sync(0xffffffffu, n, l0);
+  R.e2 = R.e1 + __shfl_sync(0xffffffffu, n, l0 + 1);
+  R.e3 = R.e2 + __shfl_sync(0xffffffffu, n, l0 + 2);
+  R.total = R.e3 + __shfl_sync(0xffffffffu, n, l0 + 3);
+  if ((idx >> 2) > P.NCX) return;
+  double a = 0.0, ws = 0.0, sxx = 0.0, syy = 0.0, wnear = 0.0;
+  for (int u0 = 0; u0 < R.total; u0 += kAhead) {
+    double w[kAhead], x[kAhead], xx[kAhead], yy[kAhead];
+    int fl[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int m = R.marker(min(u0 + i, R.total - 1));
+      w[i] = __ldg(v.w1 + 4 * (size_t)m + k);
+      x[i] = ALL2 ? v.eta[m] : v.scalar[m];
+      if (ALL2) {
+        xx[i] = v.sxx[m];
+        yy[i] = v.syy[m];
+        fl[i] = v.flags[m];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      if (u0 + i >= R.total) break;
+      a = fma(w[i], x[i], a);
+      if (WEIGHT) ws += w[i];
+      if (ALL2 && (((fl[i] >> 4) & 1) | (((fl[i] >> 5) & 1) << 1)) == k) {
+        sxx = fma(w[i], xx[i], sxx);
+        syy = fma(w[i], yy[i], syy);
+        wnear = __dadd_rn(wnear, w[i]);
+      }
+    }
+  }
+  part[(size_t)(2 * k) * ns + s] = a;
+  if (WEIGHT) part[(size_t)(2 * k + 1) * ns + s] = ws;
+  if (ALL2) {
+    part[(size_t)(8 + 3 * k) * ns + s] = sxx;
+    part[(size_t)(9 + 3 * k) * ns + s] = syy;
+    part[(size_t)(10 + 3 * k) * ns + s] = wnear;
+  }
+}
+inline dim3 corners_centre_grid(const Params &P) { return dim3((4 * (P.NCX + 1) + 127) / 128, P.NY); }
+inline bool few_cells(const mic_ctx *ctx) { return ctx->ncells <= 32 * sm_count(ctx); }
 
 // Node (i, j): basic sums from cells (i-1,j-1) corner 3, (i,j-1) corner 2, (i-1,j) corner 1,
 // (i,j) corner 0; centre sums from staggered cells with the same offsets.
@@ -521,8 +683,10 @@ __global__ void __launch_bounds__(128) k_combine_all2(Params P, const double *__
     o.etaN[q] = guarded(c[0], c[1]);
     o.soxx[q] = c[2] * r2;
     o.soyy[q] = c[3] * r2;
+    o.w1[q] = c[1];
   }
   if (!VISC) {
+    o.w0[q] = b[5];
     o.rho[q] = b[0] * r0;
     o.k[q] = b[2] * r0;
     o.lastT[q] = b[3] * r0;
@@ -533,15 +697,17 @@ __global__ void __launch_bounds__(128) k_combine_all2(Params P, const double *__
   }
 }
 
-template <int STAG>
+// KNOWN: the nodes' weight sums are in wk (k_combine_all2 of this binning: the same sums in the same
+// order); otherwise they are formed here from the partials'.
+template <int STAG, bool KNOWN>
 __global__ void __launch_bounds__(128) k_combine_scalar(Params P, const double *__restrict__ part,
-                                                         double *__restrict__ out) {
+                                                         const double *__restrict__ wk, double *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= P.NX || j >= P.NY) return;
   const int NC = P.NCX, ncells = NC * (P.NY - 1);
-  const size_t ns = (size_t)(P.NX + 1) * P.NY;
-  double a = 0.0, w = 0.0;
+  const size_t ns = (size_t)(P.NX + 1) * P.NY, q = (size_t)j * P.NX + i;
+  double a = 0.0, w = KNOWN ? wk[q] : 0.0;
   const int nL = (P.xper && i + P.NX <= NC + 1) ? 2 : 1;
   for (int l = 0; l < nL; ++l) {
     const int L = i + l * P.NX;
@@ -553,16 +719,16 @@ __global__ void __launch_bounds__(128) k_combine_scalar(Params P, const double *
         if (cx >= 0 && cx < NC && cy >= 0 && cy <= P.NY - 2) {
           const size_t cc = (size_t)cy * NC + cx;
           a += part[(size_t)(2 * k) * ncells + cc];
-          w += part[(size_t)(2 * k + 1) * ncells + cc];
+          if (!KNOWN) w += part[(size_t)(2 * k + 1) * ncells + cc];
         }
       } else if (cx >= 0 && cx <= NC && cy >= 0) {
         const size_t ss = (size_t)cy * (P.NX + 1) + cx;
         a += part[(size_t)(2 * k) * ns + ss];
-        w += part[(size_t)(2 * k + 1) * ns + ss];
+        if (!KNOWN) w += part[(size_t)(2 * k + 1) * ns + ss];
       }
     }
   }
-  out[(size_t)j * P.NX + i] = guarded(a, w);
+  out[q] = guarded(a, w);
 }
 #endif  // !MIC_EXACT
 
@@ -582,6 +748,7 @@ int mic_ensure_geometry(mic_ctx *ctx) {
     MIC_CUDA_TRY(cudaGetLastError());
   }
   ctx->geo_valid = 1;
+  ctx->wn_valid = 0;
   return MIC_OK;
 }
 
@@ -601,25 +768,35 @@ int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cud
     pv.flags = ctx->geo_flags;
     pv.w0 = ctx->wgt[0];
     pv.w1 = ctx->wgt[1];
+    const unsigned gb = grid_for(4LL * ctx->ncells, 128);
+    const dim3 gc = corners_centre_grid(ctx->P), gn = node_grid(ctx->P);
+    const bool known = (ctx->wn_valid >> (stag == 0 ? 0 : 1)) & 1;
     if (stag == 0) {
       {
         MIC_KERNEL_ON(ctx, "k_partials_basic<scalar>", s);
-        k_partials_basic<false><<<grid_for(ctx->ncells, 128), 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->mat,
-                                                                           ctx->part_b);
+        if (known)
+          k_corners_basic_scalar<false><<<gb, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_b);
+        else
+          k_corners_basic_scalar<true><<<gb, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_b);
       }
-      {
-        MIC_KERNEL_ON(ctx, "k_combine_scalar<0>", s);
-        k_combine_scalar<0><<<node_grid(ctx->P), 128, 0, s>>>(ctx->P, ctx->part_b, out);
-      }
+      MIC_KERNEL_ON(ctx, "k_combine_scalar<0>", s);
+      if (known)
+        k_combine_scalar<0, true><<<gn, 128, 0, s>>>(ctx->P, ctx->part_b, ctx->wnode[0], out);
+      else
+        k_combine_scalar<0, false><<<gn, 128, 0, s>>>(ctx->P, ctx->part_b, nullptr, out);
     } else {
       {
         MIC_KERNEL_ON(ctx, "k_partials_centre<scalar>", s);
-        k_partials_centre<false><<<centre_grid(ctx->P), 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
+        if (known)
+          k_corners_centre<false, false><<<gc, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
+        else
+          k_corners_centre<false, true><<<gc, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
       }
-      {
-        MIC_KERNEL_ON(ctx, "k_combine_scalar<-1>", s);
-        k_combine_scalar<-1><<<node_grid(ctx->P), 128, 0, s>>>(ctx->P, ctx->part_c, out);
-      }
+      MIC_KERNEL_ON(ctx, "k_combine_scalar<-1>", s);
+      if (known)
+        k_combine_scalar<-1, true><<<gn, 128, 0, s>>>(ctx->P, ctx->part_c, ctx->wnode[1], out);
+      else
+        k_combine_scalar<-1, false><<<gn, 128, 0, s>>>(ctx->P, ctx->part_c, nullptr, out);
     }
     MIC_CUDA_TRY(cudaGetLastError());
     return MIC_OK;
@@ -680,6 +857,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   o.soxx = ctx->nodal[MIC_NF_SOXX];
   o.soyy = ctx->nodal[MIC_NF_SOYY];
   o.soxy = ctx->nodal[MIC_NF_SOXY];
+  o.w0 = o.w1 = nullptr;
 #ifdef MIC_EXACT
   (void)visc;  // the exact build gathers every field in reference order each time
   (void)st;
@@ -703,18 +881,25 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   pv.flags = mv.flags;
   pv.w0 = ctx->wgt[0];
   pv.w1 = ctx->wgt[1];
+  o.w0 = ctx->wnode[0];
+  o.w1 = ctx->wnode[1];
+  const bool few = few_cells(ctx);
+  const unsigned g1 = grid_for(ctx->ncells, 128), g4 = grid_for(4LL * ctx->ncells, 128);
   if (mode == 2) {
     const cudaStream_t s = st ? st : ctx->stream;
     {
       MIC_KERNEL_ON(ctx, "k_partials_basic<first>", s);
-      k_partials_basic<true, false, true><<<grid_for(ctx->ncells, 128), 128, 0, s>>>(ctx->P, pv, ctx->quad_start,
-                                                                                     ctx->mat, ctx->part_b);
+      if (few)
+        k_corners_basic<kFirst><<<g4, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+      else
+        k_partials_basic<kFirst><<<g1, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
     }
     {
       MIC_KERNEL_ON(ctx, "k_combine_all2<first>", s);
       k_combine_all2<2><<<node_grid(ctx->P), 128, 0, s>>>(ctx->P, ctx->part_b, ctx->part_c, o);
     }
     MIC_CUDA_TRY(cudaGetLastError());
+    ctx->wn_valid |= 1;
     return MIC_OK;
   }
   // the cell-centre sums on the second stream, beside the basic-cell sums: both only read the
@@ -723,17 +908,25 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->aux_ev[0], 0));
   {
     MIC_KERNEL_ON(ctx, "k_partials_centre", ctx->aux);
-    k_partials_centre<true><<<centre_grid(ctx->P), 128, 0, ctx->aux>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
+    if (few)
+      k_corners_centre<true, true><<<corners_centre_grid(ctx->P), 128, 0, ctx->aux>>>(ctx->P, pv, ctx->quad_start,
+                                                                                       ctx->part_c);
+    else
+      k_partials_centre<<<centre_grid(ctx->P), 128, 0, ctx->aux>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
   }
   MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
   if (visc) {
     MIC_KERNEL(ctx, "k_partials_basic<visc>");
-    k_partials_basic<true, true><<<grid_for(ctx->ncells, 128), 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start,
-                                                                                      ctx->mat, ctx->part_b);
+    if (few)
+      k_corners_basic<kVisc><<<g4, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+    else
+      k_partials_basic<kVisc><<<g1, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
   } else {
     MIC_KERNEL(ctx, "k_partials_basic");
-    k_partials_basic<true><<<grid_for(ctx->ncells, 128), 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start,
-                                                                                ctx->mat, ctx->part_b);
+    if (few)
+      k_corners_basic<kFull><<<g4, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+    else
+      k_partials_basic<kFull><<<g1, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
   }
   MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->aux_ev[1], 0));  // the cell-centre sums
   if (visc) {
@@ -743,6 +936,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
     MIC_KERNEL(ctx, "k_combine_all2");
     k_combine_all2<0><<<node_grid(ctx->P), 128, 0, ctx->stream>>>(ctx->P, ctx->part_b, ctx->part_c, o);
   }
+  ctx->wn_valid |= visc ? 2 : 3;
 #endif
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
