@@ -3,8 +3,11 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
-
+#include <thread>
 #include <vector>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "mic_internal.cuh"
 
@@ -563,6 +566,56 @@ extern "C" int mic_markers_upload(mic_ctx *ctx, const mic_marker *host, int64_t 
   return MIC_OK;
 }
 
+// Gives a result buffer its pages before the device's copy fills it.  A host program that takes the
+// markers into a new array each step hands over memory without pages, and the copy then takes their
+// faults one after another.  Four threads ask for the pages, a quarter each, while the records are
+// still being packed: GB300 with a Grace host, 56.6 MB, the pages in 0.8 ms (1.8 by one thread, 1.1
+// by two, 1.6 by eight: they meet at the address space's lock) and the copy in 1.05 instead of 2.9
+// (0.31 into pages the device has seen before).  Only for buffers of which the system says that
+// kPopulateMin bytes have no pages -- below, the threads cost what they save, and the C library
+// reuses such memory anyway.  Where the system cannot say or give them, the copy does what it did.
+constexpr size_t kPopulateMin = 16u << 20;
+constexpr int kPopulateThreads = 4;
+
+static void populate_pages(void *host, size_t bytes) {
+#if defined(MADV_POPULATE_WRITE)
+  const long psz = sysconf(_SC_PAGESIZE);
+  if (bytes < kPopulateMin || psz <= 0) return;
+  const size_t page = (size_t)psz;
+  const size_t lo = ((size_t)host + page - 1) / page * page, hi = ((size_t)host + bytes) / page * page;
+  if (hi <= lo) return;
+  const size_t pages = (hi - lo) / page;
+  std::vector<unsigned char> in;
+  try {
+    in.resize(pages);
+  } catch (...) {
+    return;
+  }
+  if (mincore((void *)lo, hi - lo, in.data()) != 0) return;
+  size_t missing = 0;
+  for (size_t q = 0; q < pages; ++q) missing += !(in[q] & 1);
+  if (missing * page < kPopulateMin) return;
+  const auto ask = [=](int t) {
+    const size_t a = pages * t / kPopulateThreads, b = pages * (t + 1) / kPopulateThreads;
+    if (b > a) (void)madvise((void *)(lo + a * page), (b - a) * page, MADV_POPULATE_WRITE);
+  };
+  std::thread helper[kPopulateThreads - 1];
+  for (int t = 1; t < kPopulateThreads; ++t) {
+    try {
+      helper[t - 1] = std::thread(ask, t);
+    } catch (...) {  // no thread to be had
+      ask(t);
+    }
+  }
+  ask(0);
+  for (std::thread &h : helper)
+    if (h.joinable()) h.join();
+#else
+  (void)host;
+  (void)bytes;
+#endif
+}
+
 extern "C" int mic_markers_download(mic_ctx *ctx, mic_marker *host, int64_t n) {
   if (!ctx || (n > 0 && !host) || n != ctx->n) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
@@ -574,6 +627,7 @@ extern "C" int mic_markers_download(mic_ctx *ctx, mic_marker *host, int64_t n) {
     k_soa_to_aos<<<pack_grid(n), kPackRows, 0, ctx->stream>>>((pack_word *)ctx->stage_aos, cur_cols(ctx), n);
   }
   MIC_CUDA_TRY(cudaGetLastError());
+  populate_pages(host, (size_t)n * sizeof(mic_marker));
   MIC_CUDA_TRY(cudaMemcpyAsync(host, ctx->stage_aos, (size_t)n * sizeof(mic_marker), cudaMemcpyDeviceToHost,
                                ctx->stream));
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
