@@ -102,6 +102,7 @@ __device__ __forceinline__ void add_digits(int (*h)[kBuckets], int passes, int *
 __global__ void k_find_cells(Params P, const double *__restrict__ X, const double *__restrict__ Y,
                              int *__restrict__ cellX, int *__restrict__ cellY, int *__restrict__ cpu,
                              int *__restrict__ key, int64_t n, int passes, int *counts, Status *st) {
+  if (!after_previous()) return;
   __shared__ unsigned long long s_out;
   __shared__ int h[kMaxPasses][kBuckets];
   if (threadIdx.x == 0) s_out = 0;
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__res
                                                             int *__restrict__ val_out, int64_t n, int shift,
                                                             const int *__restrict__ counts, unsigned *tiles, int *ticket,
                                                             unsigned long long *lost) {
+  if (!after_previous()) return;
   constexpr int W = kSortThreads / 32, T = kSortThreads * IT;
   __shared__ int wcnt[W][kBuckets];        // per warp and digit: count, then offset in the tile's digit
   __shared__ int s_key[T], s_val[T];       // the tile in digit order
@@ -356,13 +358,11 @@ void radix_launch(mic_ctx *ctx, cudaStream_t s, int **kin, int **kout, int **vin
     const int *counts = scratch + kOffCounts + p * kBuckets;
     if (ctx) mic_prof_begin(ctx, "k_radix_pass", s);
     if (items_for(n) == kItemsSmall)
-      k_radix_pass<kItemsSmall><<<(unsigned)tiles, kSortThreads, 0, s>>>(*kin, *vin, p == 0, *kout, *vout, n,
-                                                                         p * kRadixBits, counts, words,
-                                                                         scratch + kOffTicket + p, lost);
+      launch_after(k_radix_pass<kItemsSmall>, (unsigned)tiles, kSortThreads, 0, s, *kin, *vin, p == 0, *kout, *vout,
+                   n, p * kRadixBits, counts, words, scratch + kOffTicket + p, lost);
     else
-      k_radix_pass<kItemsLarge><<<(unsigned)tiles, kSortThreads, 0, s>>>(*kin, *vin, p == 0, *kout, *vout, n,
-                                                                         p * kRadixBits, counts, words,
-                                                                         scratch + kOffTicket + p, lost);
+      launch_after(k_radix_pass<kItemsLarge>, (unsigned)tiles, kSortThreads, 0, s, *kin, *vin, p == 0, *kout, *vout,
+                   n, p * kRadixBits, counts, words, scratch + kOffTicket + p, lost);
     if (ctx) mic_prof_end(ctx, s);
     int *x = *kin;
     *kin = *kout;
@@ -377,6 +377,7 @@ void radix_launch(mic_ctx *ctx, cudaStream_t s, int **kin, int **kout, int **vin
 // q in [0, 4*ncells+4] (when qs is given) and cs[c] = qs[4c] for c in [0, ncells+1].
 __global__ void k_cell_start(const int *__restrict__ skey, int64_t n, int ncells, int *__restrict__ cs,
                              int *__restrict__ qs) {
+  if (!after_previous()) return;
   // one thread per (cell, quadrant) key q in [0, 4 ncells + 4]: the run of key q starts at the
   // first sorted position whose key is >= q (n when there is none), so empty stretches of cells
   // cost nothing extra.  cs[c] = qs[4c].  The search starts at the position q would have with
@@ -442,6 +443,7 @@ struct GatherCols {
 // The geometry's grid-line loads come before the stores for the same reason.
 template <bool GEO>
 __global__ void k_reorder(GatherCols g, const int *__restrict__ perm, int64_t n, Params P, GeoOut go) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int p = perm[k];
@@ -527,9 +529,9 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
     MIC_KERNEL(ctx, "k_find_cells");
     const int block = tuned_block(ctx, TU_FIND_CELLS);
     const unsigned full = grid_for(n, block), most = 2048 / block * sm_count(ctx);
-    k_find_cells<<<full < most ? full : most, block, 0, ctx->stream>>>(
-        ctx->P, ctx->f64[C_X], ctx->f64[C_Y], ctx->i32[C_CELLX], ctx->i32[C_CELLY], ctx->i32[C_CPU], ctx->key, n, passes,
-        ctx->sort_buf + kOffCounts, ctx->d_status);
+    launch_after(k_find_cells, full < most ? full : most, block, 0, ctx->stream, ctx->P, ctx->f64[C_X], ctx->f64[C_Y],
+                 ctx->i32[C_CELLX], ctx->i32[C_CELLY], ctx->i32[C_CPU], ctx->key, n, passes,
+                 ctx->sort_buf + kOffCounts, ctx->d_status);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   int *kin = ctx->key, *kout = ctx->key_alt, *vin = ctx->perm, *vout = ctx->perm_alt;
@@ -538,8 +540,8 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
   // kin / vin now hold the sorted keys and the permutation
   {
     MIC_KERNEL(ctx, "k_cell_start");
-    k_cell_start<<<grid_for(4LL * ctx->ncells + 5), kBlock, 0, ctx->stream>>>(kin, n, ctx->ncells,
-                                                                              ctx->cell_start, ctx->quad_start);
+    launch_after(k_cell_start, grid_for(4LL * ctx->ncells + 5), kBlock, 0, ctx->stream, kin, n, ctx->ncells,
+                 ctx->cell_start, ctx->quad_start);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   GatherCols g;
@@ -554,8 +556,8 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
   }
   {
     MIC_KERNEL(ctx, "k_reorder");
-    k_reorder<true><<<grid_for(n, tuned_block(ctx, TU_REORDER)), tuned_block(ctx, TU_REORDER), 0, ctx->stream>>>(
-        g, vin, n, ctx->P, geo_out(ctx));
+    launch_after(k_reorder<true>, grid_for(n, tuned_block(ctx, TU_REORDER)), tuned_block(ctx, TU_REORDER), 0,
+                 ctx->stream, g, vin, n, ctx->P, geo_out(ctx));
   }
   MIC_CUDA_TRY(cudaGetLastError());
   for (int c = 0; c < g.nf; ++c) {
@@ -613,7 +615,7 @@ int mic_restore_caller_order(mic_ctx *ctx) {
   }
   {
     MIC_KERNEL(ctx, "k_reorder");
-    k_reorder<false><<<grid_for(cap), kBlock, 0, ctx->stream>>>(g, ctx->perm, cap, ctx->P, GeoOut{});
+    launch_after(k_reorder<false>, grid_for(cap), kBlock, 0, ctx->stream, g, ctx->perm, cap, ctx->P, GeoOut{});
   }
   MIC_CUDA_TRY(cudaGetLastError());
   for (int c = 0; c < g.nf; ++c) {
@@ -825,7 +827,7 @@ extern "C" int mic_bin_sort_noalloc(const double *X, const double *Y, int64_t n,
     int *kin = key, *kout = key_alt, *vin = (passes & 1) ? val_alt : perm, *vout = (passes & 1) ? perm : val_alt;
     radix_launch(nullptr, s, &kin, &kout, &vin, &vout, n, passes, sort, d_lost);
     if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
-    k_cell_start<<<grid_for(4LL * ncells + 5), kBlock, 0, s>>>(kin, n, (int)ncells, cell_start, nullptr);
+    launch_after(k_cell_start, grid_for(4LL * ncells + 5), kBlock, 0, s, kin, n, (int)ncells, cell_start, nullptr);
   } else {
     if (cudaMemsetAsync(cell_start, 0, sizeof(int32_t) * (size_t)(ncells + 2), s) != cudaSuccess)
       return MIC_ERR_CUDA;

@@ -52,6 +52,7 @@ __device__ __forceinline__ void ve_update(double eta, double mu, double dt, doub
 // vorticity and shear strain rate at the basic node (wall ghosts from the boundary values),
 // and the stress updates of both
 __global__ void k_nss_pointwise(Params P, GridFields g, mic_bcinfo left, mic_bcinfo top, double dt) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (k >= (int64_t)NX * NY) return;
@@ -94,6 +95,7 @@ __global__ void k_nss_pointwise(Params P, GridFields g, mic_bcinfo left, mic_bci
 // shear heating and the second invariants at interior basic nodes (nodalStressStrain.c:
 // 330-370), from the four surrounding cell centres; zero elsewhere
 __global__ void k_nss_invariants(Params P, GridFields g) {
+  if (!after_previous()) return;
   const int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (a >= (int64_t)NX * NY) return;
@@ -133,6 +135,7 @@ __global__ void k_nss_invariants(Params P, GridFields g) {
 // never win, as the reference's `dt > dt1` test), and max |rhodot| over non-NaN entries
 __global__ void k_limit_dt(Params P, GridFields g, double factor, unsigned long long *mins, unsigned long long *maxr,
                            int *nonnan) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (k >= (int64_t)NX * NY) return;
@@ -167,6 +170,7 @@ __global__ void k_limit_dt(Params P, GridFields g, double factor, unsigned long 
 
 __global__ void k_retrieve(const double *__restrict__ S, int64_t nn, double Kcont, double *p, double *vx,
                            double *vy) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= nn) return;
   p[k] = M(S[3 * k + 2], Kcont);
@@ -176,6 +180,7 @@ __global__ void k_retrieve(const double *__restrict__ S, int64_t nn, double Kcon
 
 // dx-weighted mean pressure of row 1 in the reference's order (retrieveSolutions.c:52-62)
 __global__ void k_pressure_mean(Params P, const double *p, double *pm) {
+  if (!after_previous()) return;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double s = 0.0;
   for (int i = 1; i < P.NX; ++i) {
@@ -186,6 +191,7 @@ __global__ void k_pressure_mean(Params P, const double *p, double *pm) {
 }
 
 __global__ void k_pressure_shift(Params P, double *p, const double *pm) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= (int64_t)P.NX * P.NY) return;
   if (k % P.NX >= 1 && k / P.NX >= 1) p[k] = S(p[k], *pm);
@@ -202,12 +208,12 @@ extern "C" int mic_nodal_stress_strain(mic_ctx *ctx, double dt, double gy) {
   const GridFields g = grid_fields(ctx);
   {
     MIC_KERNEL(ctx, "k_nss_pointwise");
-    k_nss_pointwise<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, g, ctx->bcs.mechBCLeft, ctx->bcs.mechBCTop,
-                                                               dt);
+    launch_after(k_nss_pointwise, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, g, ctx->bcs.mechBCLeft,
+                 ctx->bcs.mechBCTop, dt);
   }
   {
     MIC_KERNEL(ctx, "k_nss_invariants");
-    k_nss_invariants<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, g);
+    launch_after(k_nss_invariants, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, g);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
@@ -223,8 +229,8 @@ extern "C" int mic_limit_displacement_timestep(mic_ctx *ctx, double factor, doub
   MIC_CUDA_TRY(cudaMemcpyAsync(d, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
   {
     MIC_KERNEL(ctx, "k_limit_dt");
-    k_limit_dt<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, grid_fields(ctx), factor, d, d + 1,
-                                                          reinterpret_cast<int *>(d + 2));
+    launch_after(k_limit_dt, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, grid_fields(ctx), factor, d, d + 1,
+                 reinterpret_cast<int *>(d + 2));
   }
   MIC_CUDA_TRY(cudaGetLastError());
   unsigned long long h[3];
@@ -262,16 +268,16 @@ extern "C" int mic_retrieve_solutions(mic_ctx *ctx, const double *S, double Kcon
   double *pm = ctx->red_buf + 28;
   {
     MIC_KERNEL(ctx, "k_retrieve");
-    k_retrieve<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->solution, nn, Kcont, ctx->nodal[MIC_NF_P],
-                                                          ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY]);
+    launch_after(k_retrieve, grid_for(nn), kBlock, 0, ctx->stream, ctx->solution, nn, Kcont, ctx->nodal[MIC_NF_P],
+                 ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY]);
   }
   {
     MIC_KERNEL(ctx, "k_pressure_mean");
-    k_pressure_mean<<<1, 32, 0, ctx->stream>>>(ctx->P, ctx->nodal[MIC_NF_P], pm);
+    launch_after(k_pressure_mean, 1, 32, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_P], pm);
   }
   {
     MIC_KERNEL(ctx, "k_pressure_shift");
-    k_pressure_shift<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, ctx->nodal[MIC_NF_P], pm);
+    launch_after(k_pressure_shift, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_P], pm);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // the caller may reuse S on return
@@ -286,6 +292,7 @@ namespace {
 // nusseltNumber (post.c:5-46): the surface heat flux integral, summed in the reference's order by
 // one thread (NX - 1 terms), every operation an IEEE intrinsic
 __global__ void k_nusselt(Params P, const double *__restrict__ T, double dTbc, double *out) {
+  if (!after_previous()) return;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const int NX = P.NX;
   const double dz = S(P.y[1], P.y[0]);
@@ -302,6 +309,7 @@ __global__ void k_nusselt(Params P, const double *__restrict__ T, double dTbc, d
 // cells in order; the two agree to rounding)
 __global__ void k_vrms_partial(Params P, const double *__restrict__ vx, const double *__restrict__ vy,
                                double *part) {
+  if (!after_previous()) return;
   __shared__ double sm[256];
   const int NX = P.NX, nc = (P.NX - 1) * (P.NY - 1);
   double acc = 0.0;
@@ -323,6 +331,7 @@ __global__ void k_vrms_partial(Params P, const double *__restrict__ vx, const do
 }
 
 __global__ void k_vrms_final(Params P, const double *__restrict__ part, int nparts, double *out) {
+  if (!after_previous()) return;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double s = 0.0;
   for (int b = 0; b < nparts; ++b) s = A(s, part[b]);
@@ -338,7 +347,7 @@ extern "C" int mic_nusselt_number(mic_ctx *ctx, double bottom_T, double top_T, d
   double *d = ctx->red_buf + 40;
   {
     MIC_KERNEL(ctx, "k_nusselt");
-    k_nusselt<<<1, 32, 0, ctx->stream>>>(ctx->P, ctx->nodal[MIC_NF_THIST], bottom_T - top_T, d);
+    launch_after(k_nusselt, 1, 32, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_THIST], bottom_T - top_T, d);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   MIC_CUDA_TRY(cudaMemcpyAsync(Nu, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -354,11 +363,12 @@ extern "C" int mic_rms_velocity(mic_ctx *ctx, double *vrms) {
   double *part = ctx->red_buf + 64, *d = ctx->red_buf + 41;
   {
     MIC_KERNEL(ctx, "k_vrms_partial");
-    k_vrms_partial<<<kParts, 256, 0, ctx->stream>>>(ctx->P, ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY], part);
+    launch_after(k_vrms_partial, kParts, 256, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY],
+                 part);
   }
   {
     MIC_KERNEL(ctx, "k_vrms_final");
-    k_vrms_final<<<1, 32, 0, ctx->stream>>>(ctx->P, part, kParts, d);
+    launch_after(k_vrms_final, 1, 32, 0, ctx->stream, ctx->P, part, kParts, d);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   MIC_CUDA_TRY(cudaMemcpyAsync(vrms, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

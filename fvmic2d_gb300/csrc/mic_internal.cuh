@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "mic_gb300.h"
 #include "mic_types.h"
 
@@ -193,6 +195,42 @@ struct ProfScope {  // brackets one kernel launch: counts it and, when enabled, 
 }  // namespace mic
 #define MIC_KERNEL(ctx, name) mic::ProfScope _mic_prof_scope(ctx, name, (ctx)->stream)
 #define MIC_KERNEL_ON(ctx, name, st) mic::ProfScope _mic_prof_scope(ctx, name, st)
+
+// ---- dependent launches ----------------------------------------------------------------
+//
+// A step is a chain of some 25 kernels, on small grids of 3 to 20 us each, and between two of them
+// the device spends as long again on ending one grid and starting the next.  launch_after starts a
+// kernel's blocks as soon as the last block of the kernel before it in the stream has ended, while
+// its end is still being reported; after_previous, the first statement of every kernel launched so,
+// waits until all of that kernel's writes (and, since it waited in turn, those of all kernels
+// before it) are visible.  GB300, a chain of 25 small kernels in a stream: 4.1 -> 2.4 us each.  No
+// kernel asks for its successor earlier than its end: blocks that wait take the places of those
+// that work (3.8 us each).
+//
+// after_previous gives true, but through the wait itself: no read of the kernel, not even one the
+// compiler takes for constant, can be moved in front of the branch on it.
+namespace mic {
+__device__ __forceinline__ bool after_previous() {
+  int stay;
+  asm volatile("griddepcontrol.wait;\n\tmov.b32 %0, 1;" : "=r"(stay)::"memory");
+  return stay != 0;
+}
+
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // errors: by cudaGetLastError, as for <<<>>>
+}
+}  // namespace mic
 
 // ---- helpers -------------------------------------------------------------------------
 

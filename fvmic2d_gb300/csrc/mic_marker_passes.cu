@@ -290,6 +290,7 @@ __device__ __forceinline__ bool yield_tc_round(tc::Block &B, const YieldCols &c,
 // updateViscosity (viscosity.c:77-88): rheology from the current marker stress
 __global__ void k_update_viscosity(YieldCols c, mic_materials M, mic_options O, CreepConfig cfg, int64_t n,
                                    Status *st) {
+  if (!after_previous()) return;
   const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (m >= n || c.cellX[m] == -1) return;
   double eta, mu;
@@ -306,6 +307,7 @@ __global__ void k_update_viscosity(YieldCols c, mic_materials M, mic_options O, 
 
 // limitViscosity (viscosity.c:90-104): every marker
 __global__ void k_limit_viscosity(double *eta, double etamin, double etamax, int64_t n) {
+  if (!after_previous()) return;
   const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (m >= n) return;
   const double e = eta[m];
@@ -478,6 +480,7 @@ __device__ __forceinline__ void strain_pressure_one(const Params &P, const Strai
 
 // area weighting of the projected residual (residual.c:23-38) and per-block partial sums
 __global__ void k_residual_weight(Params P, double *srr, double *partial) {
+  if (!after_previous()) return;
   __shared__ double sh[kBlock];
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double v = 0.0;
@@ -501,6 +504,7 @@ __global__ void k_residual_weight(Params P, double *srr, double *partial) {
 }
 
 __global__ void k_sum_partials(const double *partial, int np, double *out) {
+  if (!after_previous()) return;
   __shared__ double sh[1024];
   double v = 0.0;
   for (int k = threadIdx.x; k < np; k += blockDim.x) v += partial[k];
@@ -643,6 +647,7 @@ __global__ void __launch_bounds__(128) k_subgrid_stress_nodes(Params P, const in
                                                               const double *__restrict__ dyy,
                                                               const int *__restrict__ cs, double *dsxx, double *dsyy,
                                                               double *dsxy) {
+  if (!after_previous()) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= P.NX || j >= P.NY) return;
@@ -679,6 +684,7 @@ __global__ void __launch_bounds__(128) k_subgrid_partials(Params P, const double
                                                           const double *__restrict__ dxx,
                                                           const double *__restrict__ dyy,
                                                           const int *__restrict__ cs, double *__restrict__ part) {
+  if (!after_previous()) return;
   __shared__ double sloc[8][128];
   const int ncells = P.NCX * (P.NY - 1);
   const int t = threadIdx.x;
@@ -732,6 +738,7 @@ __global__ void __launch_bounds__(128) k_subgrid_partials(Params P, const double
 // subgridStressChanges.c:258-286.
 __global__ void __launch_bounds__(128) k_subgrid_combine(Params P, const double *__restrict__ part, double *dsxx,
                                                          double *dsyy, double *dsxy) {
+  if (!after_previous()) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= P.NX || j >= P.NY) return;
@@ -868,6 +875,7 @@ __device__ __forceinline__ void subgridT_markers_one(const Params &P, const SubT
 // nodal remainder thisT - lastT - projected subgrid change (VecAXPBYPCZ with alpha = 1)
 __global__ void k_subgridT_nodes(const double *thisT, const double *lastT, const double *proj, double *dT,
                                  int64_t nn) {
+  if (!after_previous()) return;
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (q >= nn) return;
   dT[q] = thisT[q] + -1.0 * lastT[q] + -1.0 * proj[q];
@@ -935,6 +943,7 @@ __device__ __forceinline__ df bil_eval_df(const BilDF *__restrict__ cells, size_
 __global__ void k_advect_coef(const double *__restrict__ vx, const double *__restrict__ vy,
                               const double *__restrict__ wz, mic_bcinfo top, mic_bcinfo left, int NX, int NY,
                               BilDF *cvx, BilDF *cvy, BilDF *cwz) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k < (int64_t)NY * (NX - 1)) {
     const int row = (int)(k / (NX - 1)), i = (int)(k % (NX - 1));
@@ -980,6 +989,7 @@ __global__ void k_advect_coef(const double *__restrict__ vx, const double *__res
 __global__ void k_advect_coef_periodic(const double *__restrict__ vx, const double *__restrict__ vy,
                                        const double *__restrict__ wz, mic_bcinfo top, int NX, int NY, Bil4 *cvx,
                                        Bil4 *cvy, Bil4 *cwz) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= (int64_t)NX * NY) return;
   const int row = (int)(k / NX), i = (int)(k % NX), i1 = next_col(i, NX);
@@ -1520,6 +1530,7 @@ __global__ void k_max(const int *cellX, const double *v, int absval, int64_t n, 
 // projectNodalFieldToMarkersS (markers.c:1670-1706)
 __global__ void k_nodal_to_markers(Params P, const int *cellX, const int *cellY, Geo g, const double *f,
                                    double *dst, int64_t n) {
+  if (!after_previous()) return;
   const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (m >= n) return;
   const int i = cellX[m], j = cellY[m];
@@ -1856,6 +1867,7 @@ __global__ void __maxnreg__(Op::kMaxRegs) k_batched(const typename Op::Job *__re
                                                          const int *__restrict__ ts, int njobs, int ntiles,
                                                          int tile_markers, int walk, unsigned int *ticket,
                                                          const __grid_constant__ typename Op::Job one) {
+  if (!after_previous()) return;
   using Job = typename Op::Job;
   __shared__ unsigned long long sj[sizeof(Job) / 8];
   const Job &J = *reinterpret_cast<const Job *>(sj);
@@ -1881,6 +1893,7 @@ __global__ void __launch_bounds__(512) k_yield_fp32_batched(const YieldJob *__re
                                                                     int ntiles, int tile_markers, int walk,
                                                                     unsigned int *ticket,
                                                                     const __grid_constant__ YieldJob one) {
+  if (!after_previous()) return;
   __shared__ float w2s[kH * kH];
   __shared__ unsigned long long sj[sizeof(YieldJob) / 8];
   const YieldJob &J = *reinterpret_cast<const YieldJob *>(sj);
@@ -1916,6 +1929,7 @@ __global__ void __launch_bounds__(tc::kTile, tc::kBlocksPerSM) k_yield_tc_batche
                                                                 const int *__restrict__ ts, int njobs, int ntiles,
                                                                 int tile_markers, int walk, unsigned int *ticket,
                                                                 const __grid_constant__ YieldJob one) {
+  if (!after_previous()) return;
   extern __shared__ unsigned char dyn[];
   __shared__ unsigned long long sj[sizeof(YieldJob) / 8];
   const YieldJob &J = *reinterpret_cast<const YieldJob *>(sj);
@@ -2016,8 +2030,8 @@ template <class Op>
 void launch_generic(unsigned grid, int block, cudaStream_t s, const unsigned char *jobs, const int *ts, int nj,
                     int ntiles, int tm, Walk wk, const void *one) {
   using Job = typename Op::Job;
-  k_batched<Op><<<grid, block, 0, s>>>(reinterpret_cast<const Job *>(jobs), ts, nj, ntiles, tm, wk.walk, wk.ticket,
-                                       job_arg<Job>(one));
+  launch_after(k_batched<Op>, grid, block, 0, s, reinterpret_cast<const Job *>(jobs), ts, nj, ntiles, tm, wk.walk,
+               wk.ticket, job_arg<Job>(one));
 }
 
 cudaError_t launch_pass(int pass, unsigned grid, int block, cudaStream_t s, const unsigned char *jobs, const int *ts,
@@ -2031,15 +2045,14 @@ cudaError_t launch_pass(int pass, unsigned grid, int block, cudaStream_t s, cons
     case BP_YIELD_PLAIN: launch_generic<YieldOp<2>>(grid, block, s, jobs, ts, nj, ntiles, tm, wk, one); break;
     case BP_YIELD_EXACT: launch_generic<YieldOp<0>>(grid, block, s, jobs, ts, nj, ntiles, tm, wk, one); break;
     case BP_YIELD_FP32:
-      k_yield_fp32_batched<<<grid, block, 0, s>>>(reinterpret_cast<const YieldJob *>(jobs), ts, nj, ntiles, tm,
-                                                   wk.walk, wk.ticket, job_arg<YieldJob>(one));
+      launch_after(k_yield_fp32_batched, grid, block, 0, s, reinterpret_cast<const YieldJob *>(jobs), ts, nj, ntiles,
+                   tm, wk.walk, wk.ticket, job_arg<YieldJob>(one));
       break;
     case BP_YIELD_TC: {
       const cudaError_t e = tc_kernel_attributes();
       if (e != cudaSuccess) return e;
-      k_yield_tc_batched<<<grid, tc::kTile, tc::kDynSmem, s>>>(reinterpret_cast<const YieldJob *>(jobs), ts, nj,
-                                                                ntiles, tm, wk.walk, wk.ticket,
-                                                                job_arg<YieldJob>(one));
+      launch_after(k_yield_tc_batched, grid, tc::kTile, tc::kDynSmem, s, reinterpret_cast<const YieldJob *>(jobs), ts,
+                   nj, ntiles, tm, wk.walk, wk.ticket, job_arg<YieldJob>(one));
       break;
     }
     case BP_STRAIN: launch_generic<StrainOp>(grid, block, s, jobs, ts, nj, ntiles, tm, wk, one); break;
@@ -2174,8 +2187,8 @@ extern "C" int mic_update_viscosity(mic_ctx *ctx) {
   if (ctx->n > 0) {
     {
       MIC_KERNEL(ctx, "k_update_viscosity");
-      k_update_viscosity<<<grid_for(ctx->n), kBlock, 0, ctx->stream>>>(yield_cols(ctx), ctx->mat, ctx->opt,
-                                                                       ctx->creep, ctx->n, ctx->d_status);
+      launch_after(k_update_viscosity, grid_for(ctx->n), kBlock, 0, ctx->stream, yield_cols(ctx), ctx->mat, ctx->opt,
+                   ctx->creep, ctx->n, ctx->d_status);
     }
     MIC_CUDA_TRY(cudaGetLastError());
   }
@@ -2188,8 +2201,8 @@ extern "C" int mic_limit_viscosity(mic_ctx *ctx) {
   if (ctx->n == 0) return MIC_OK;
   {
     MIC_KERNEL(ctx, "k_limit_viscosity");
-    k_limit_viscosity<<<grid_for(ctx->n), kBlock, 0, ctx->stream>>>(ctx->f64[C_ETA], ctx->opt.etamin,
-                                                                    ctx->opt.etamax, ctx->n);
+    launch_after(k_limit_viscosity, grid_for(ctx->n), kBlock, 0, ctx->stream, ctx->f64[C_ETA], ctx->opt.etamin,
+                 ctx->opt.etamax, ctx->n);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
@@ -2242,12 +2255,12 @@ static int residual_launch(mic_ctx *ctx, int iter, double *res_dev, cudaStream_t
   double *partial = ctx->node_scr[5];  // NX*NY >= number of blocks
   {
     MIC_KERNEL_ON(ctx, "k_residual_weight", s);
-    k_residual_weight<<<nb, kBlock, 0, s>>>(ctx->P, ctx->nodal[MIC_NF_SRR], partial);
+    launch_after(k_residual_weight, nb, kBlock, 0, s, ctx->P, ctx->nodal[MIC_NF_SRR], partial);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   {
     MIC_KERNEL_ON(ctx, "k_sum_partials", s);
-    k_sum_partials<<<1, 1024, 0, s>>>(partial, nb, res_dev);
+    launch_after(k_sum_partials, 1, 1024, 0, s, partial, nb, res_dev);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   (void)iter;
@@ -2333,26 +2346,24 @@ static int subgrid_nodes(mic_ctx *ctx) {
 #ifdef MIC_EXACT
   {
     MIC_KERNEL(ctx, "k_subgrid_stress_nodes");
-    k_subgrid_stress_nodes<<<grid, 128, 0, ctx->stream>>>(ctx->P, ctx->i32[C_CELLX], ctx->geo[0], ctx->geo[1],
-                                                          ctx->scr0, ctx->scr1, ctx->scr2, ctx->cell_start,
-                                                          ctx->nodal[MIC_NF_DSXX], ctx->nodal[MIC_NF_DSYY],
-                                                          ctx->nodal[MIC_NF_DSXY]);
+    launch_after(k_subgrid_stress_nodes, grid, 128, 0, ctx->stream, ctx->P, ctx->i32[C_CELLX], ctx->geo[0],
+                 ctx->geo[1], ctx->scr0, ctx->scr1, ctx->scr2, ctx->cell_start, ctx->nodal[MIC_NF_DSXX],
+                 ctx->nodal[MIC_NF_DSYY], ctx->nodal[MIC_NF_DSXY]);
   }
 #else
   if (ctx->n > 0) {
     MIC_KERNEL(ctx, "k_subgrid_partials");
     const int64_t full = grid_for(ctx->ncells, 128), cap = (int64_t)kSubgridBlocksPerSM * sm_count(ctx);
-    k_subgrid_partials<<<(unsigned)(full < cap ? full : cap), 128, 0, ctx->stream>>>(
-        ctx->P, ctx->geo[0], ctx->geo[1], ctx->wgt[0], ctx->scr0, ctx->scr1, ctx->scr2, ctx->cell_start,
-        ctx->part_b);
+    launch_after(k_subgrid_partials, (unsigned)(full < cap ? full : cap), 128, 0, ctx->stream, ctx->P, ctx->geo[0],
+                 ctx->geo[1], ctx->wgt[0], ctx->scr0, ctx->scr1, ctx->scr2, ctx->cell_start, ctx->part_b);
   } else {
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->part_b, 0, sizeof(double) * 11 * (size_t)ctx->ncells, ctx->stream));
   }
   MIC_CUDA_TRY(cudaGetLastError());
   {
     MIC_KERNEL(ctx, "k_subgrid_combine");
-    k_subgrid_combine<<<grid, 128, 0, ctx->stream>>>(ctx->P, ctx->part_b, ctx->nodal[MIC_NF_DSXX],
-                                                     ctx->nodal[MIC_NF_DSYY], ctx->nodal[MIC_NF_DSXY]);
+    launch_after(k_subgrid_combine, grid, 128, 0, ctx->stream, ctx->P, ctx->part_b, ctx->nodal[MIC_NF_DSXX],
+                 ctx->nodal[MIC_NF_DSYY], ctx->nodal[MIC_NF_DSXY]);
   }
 #endif
   MIC_CUDA_TRY(cudaGetLastError());
@@ -2426,8 +2437,8 @@ static int subt_nodes(mic_ctx *ctx) {
   const int64_t nn = (int64_t)ctx->P.NX * ctx->P.NY;
   {
     MIC_KERNEL(ctx, "k_subgridT_nodes");
-    k_subgridT_nodes<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->nodal[MIC_NF_THIST], ctx->nodal[MIC_NF_LASTT],
-                                                               ctx->node_scr[0], ctx->node_scr[1], nn);
+    launch_after(k_subgridT_nodes, grid_for(nn), kBlock, 0, ctx->stream, ctx->nodal[MIC_NF_THIST],
+                 ctx->nodal[MIC_NF_LASTT], ctx->node_scr[0], ctx->node_scr[1], nn);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
@@ -2486,13 +2497,13 @@ static int advect_launch(mic_ctx *ctx, double dt, bool wz_known, bool with_max =
       MIC_KERNEL(ctx, "k_advect_coef");
       if (ctx->P.xper) {
         Bil4 *cp = static_cast<Bil4 *>(ctx->adv_coef);
-        k_advect_coef_periodic<<<grid_for((int64_t)nn), kBlock, 0, ctx->stream>>>(
-            ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop, NX, NY, cp,
-            cp + nn, cp + 2 * nn);
+        launch_after(k_advect_coef_periodic, grid_for((int64_t)nn), kBlock, 0, ctx->stream, ctx->nodal[MIC_NF_VX],
+                     ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop, NX, NY, cp, cp + nn,
+                     cp + 2 * nn);
       } else {
-        k_advect_coef<<<grid_for((int64_t)nn), kBlock, 0, ctx->stream>>>(
-            ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop,
-            ctx->bcs.mechBCLeft, NX, NY, cb, cb + nn, cb + 2 * nn);
+        launch_after(k_advect_coef, grid_for((int64_t)nn), kBlock, 0, ctx->stream, ctx->nodal[MIC_NF_VX],
+                     ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop, ctx->bcs.mechBCLeft, NX, NY,
+                     cb, cb + nn, cb + 2 * nn);
       }
     }
     MIC_CUDA_TRY(cudaGetLastError());
@@ -2536,8 +2547,8 @@ extern "C" int mic_project_nodal_field_to_markers(mic_ctx *ctx, int f, int off) 
   if (ctx->n == 0) return MIC_OK;
   {
     MIC_KERNEL(ctx, "k_nodal_to_markers");
-    k_nodal_to_markers<<<grid_for(ctx->n), kBlock, 0, ctx->stream>>>(ctx->P, ctx->i32[C_CELLX], ctx->i32[C_CELLY],
-                                                                     geo_of(ctx), ctx->nodal[f], ctx->f64[col], ctx->n);
+    launch_after(k_nodal_to_markers, grid_for(ctx->n), kBlock, 0, ctx->stream, ctx->P, ctx->i32[C_CELLX],
+                 ctx->i32[C_CELLY], geo_of(ctx), ctx->nodal[f], ctx->f64[col], ctx->n);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;

@@ -31,6 +31,7 @@ namespace {
 
 __global__ void k_geometry(Params P, const double *__restrict__ X, const double *__restrict__ Y,
                            const int *__restrict__ cellX, const int *__restrict__ cellY, GeoOut o, int64_t n) {
+  if (!after_previous()) return;
   const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (m >= n) return;
   geometry_marker(P, X[m], Y[m], cellX[m], cellY[m], o, m);
@@ -106,6 +107,7 @@ __device__ __forceinline__ void all2_column(const Params &P, const MarkerView &m
 // x, nodes 0 and 1 add their seam image's sums (local columns NX, NX + 1) after their own.
 __global__ void __launch_bounds__(128) k_project_all2(Params P, MarkerView mv, const int *__restrict__ cs,
                                                        mic_materials mat, All2Out o) {
+  if (!after_previous()) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= P.NX || j >= P.NY) return;
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(128) k_project_geo_arith(Params P, const doubl
                                                             const double *__restrict__ gy,
                                                             const int *__restrict__ flags,
                                                             const int *__restrict__ cs, double *__restrict__ out) {
+  if (!after_previous()) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= P.NX || j >= P.NY) return;
@@ -326,6 +329,7 @@ enum Sums { kFull, kVisc, kFirst };
 template <Sums WHAT>
 __global__ void __launch_bounds__(128) k_partials_basic(Params P, PartialView v, const int *__restrict__ qs,
                                                          mic_materials mat, double *__restrict__ part) {
+  if (!after_previous()) return;
   constexpr bool VISC = WHAT == kVisc, FIRST = WHAT == kFirst;
   __shared__ double sloc[FIRST ? 1 : 8][128];
   const int ncells = P.NCX * (P.NY - 1);
@@ -403,6 +407,7 @@ constexpr int kAhead = 4;  // markers whose loads a lane has in flight
 template <Sums WHAT>
 __global__ void __launch_bounds__(128) k_corners_basic(Params P, PartialView v, const int *__restrict__ qs,
                                                         mic_materials mat, double *__restrict__ part) {
+  if (!after_previous()) return;
   constexpr bool VISC = WHAT == kVisc, FIRST = WHAT == kFirst;
   const int ncells = P.NCX * (P.NY - 1);
   const int idx = blockIdx.x * blockDim.x + threadIdx.x, c = idx >> 2, k = idx & 3;
@@ -468,6 +473,7 @@ __global__ void __launch_bounds__(128) k_corners_basic(Params P, PartialView v, 
 template <bool WEIGHT>
 __global__ void __launch_bounds__(128) k_corners_basic_scalar(Params P, PartialView v, const int *__restrict__ qs,
                                                                double *__restrict__ part) {
+  if (!after_previous()) return;
   const int ncells = P.NCX * (P.NY - 1);
   const int idx = blockIdx.x * blockDim.x + threadIdx.x, c = idx >> 2, k = idx & 3;
   if (c >= ncells) return;
@@ -522,6 +528,7 @@ __device__ __forceinline__ void centre_run(const Params &P, const int *__restric
 
 __global__ void __launch_bounds__(128) k_partials_centre(Params P, PartialView v, const int *__restrict__ qs,
                                                           double *__restrict__ part) {
+  if (!after_previous()) return;
   __shared__ double sloc[12][128];
   const int sx = blockIdx.x * blockDim.x + threadIdx.x;
   const int sy = blockIdx.y;
@@ -575,6 +582,7 @@ __global__ void __launch_bounds__(128) k_partials_centre(Params P, PartialView v
 template <bool ALL2, bool WEIGHT>
 __global__ void __launch_bounds__(128) k_corners_centre(Params P, PartialView v, const int *__restrict__ qs,
                                                          double *__restrict__ part) {
+  if (!after_previous()) return;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x, k = idx & 3;
   const int sx = min(idx >> 2, P.NCX), sy = blockIdx.y;  // (lanes beyond the row stay for the exchange)
   const size_t ns = (size_t)(P.NX + 1) * P.NY, s = (size_t)sy * (P.NX + 1) + sx;
@@ -639,6 +647,7 @@ __device__ __forceinline__ double guarded_rcp(double w) { return (w != 0.0) ? 1.
 template <int MODE>
 __global__ void __launch_bounds__(128) k_combine_all2(Params P, const double *__restrict__ pb,
                                                        const double *__restrict__ pc, All2Out o) {
+  if (!after_previous()) return;
   constexpr bool VISC = MODE == 1, FIRST = MODE == 2;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
@@ -702,6 +711,7 @@ __global__ void __launch_bounds__(128) k_combine_all2(Params P, const double *__
 template <int STAG, bool KNOWN>
 __global__ void __launch_bounds__(128) k_combine_scalar(Params P, const double *__restrict__ part,
                                                          const double *__restrict__ wk, double *__restrict__ out) {
+  if (!after_previous()) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= P.NX || j >= P.NY) return;
@@ -741,9 +751,8 @@ int mic_ensure_geometry(mic_ctx *ctx) {
   if (ctx->n > 0) {
     {
       MIC_KERNEL(ctx, "k_geometry");
-      k_geometry<<<grid_for(ctx->n), kBlock, 0, ctx->stream>>>(ctx->P, ctx->f64[C_X], ctx->f64[C_Y],
-                                                               ctx->i32[C_CELLX], ctx->i32[C_CELLY], geo_out(ctx),
-                                                               ctx->n);
+      launch_after(k_geometry, grid_for(ctx->n), kBlock, 0, ctx->stream, ctx->P, ctx->f64[C_X], ctx->f64[C_Y],
+                   ctx->i32[C_CELLX], ctx->i32[C_CELLY], geo_out(ctx), ctx->n);
     }
     MIC_CUDA_TRY(cudaGetLastError());
   }
@@ -775,28 +784,28 @@ int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cud
       {
         MIC_KERNEL_ON(ctx, "k_partials_basic<scalar>", s);
         if (known)
-          k_corners_basic_scalar<false><<<gb, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_b);
+          launch_after(k_corners_basic_scalar<false>, gb, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->part_b);
         else
-          k_corners_basic_scalar<true><<<gb, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_b);
+          launch_after(k_corners_basic_scalar<true>, gb, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->part_b);
       }
       MIC_KERNEL_ON(ctx, "k_combine_scalar<0>", s);
       if (known)
-        k_combine_scalar<0, true><<<gn, 128, 0, s>>>(ctx->P, ctx->part_b, ctx->wnode[0], out);
+        launch_after(k_combine_scalar<0, true>, gn, 128, 0, s, ctx->P, ctx->part_b, ctx->wnode[0], out);
       else
-        k_combine_scalar<0, false><<<gn, 128, 0, s>>>(ctx->P, ctx->part_b, nullptr, out);
+        launch_after(k_combine_scalar<0, false>, gn, 128, 0, s, ctx->P, ctx->part_b, nullptr, out);
     } else {
       {
         MIC_KERNEL_ON(ctx, "k_partials_centre<scalar>", s);
         if (known)
-          k_corners_centre<false, false><<<gc, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
+          launch_after(k_corners_centre<false, false>, gc, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->part_c);
         else
-          k_corners_centre<false, true><<<gc, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
+          launch_after(k_corners_centre<false, true>, gc, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->part_c);
       }
       MIC_KERNEL_ON(ctx, "k_combine_scalar<-1>", s);
       if (known)
-        k_combine_scalar<-1, true><<<gn, 128, 0, s>>>(ctx->P, ctx->part_c, ctx->wnode[1], out);
+        launch_after(k_combine_scalar<-1, true>, gn, 128, 0, s, ctx->P, ctx->part_c, ctx->wnode[1], out);
       else
-        k_combine_scalar<-1, false><<<gn, 128, 0, s>>>(ctx->P, ctx->part_c, nullptr, out);
+        launch_after(k_combine_scalar<-1, false>, gn, 128, 0, s, ctx->P, ctx->part_c, nullptr, out);
     }
     MIC_CUDA_TRY(cudaGetLastError());
     return MIC_OK;
@@ -807,14 +816,14 @@ int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cud
   if (stag == 0)
     {
       MIC_KERNEL(ctx, "k_project_geo_arith");
-      k_project_geo_arith<0><<<node_grid(ctx->P), 128, 0, ctx->stream>>>(
-          ctx->P, v, ctx->i32[C_CELLX], ctx->geo[0], ctx->geo[1], ctx->geo_flags, ctx->cell_start, out);
+      launch_after(k_project_geo_arith<0>, node_grid(ctx->P), 128, 0, ctx->stream, ctx->P, v, ctx->i32[C_CELLX],
+                   ctx->geo[0], ctx->geo[1], ctx->geo_flags, ctx->cell_start, out);
     }
   else
     {
       MIC_KERNEL(ctx, "k_project_geo_arith");
-      k_project_geo_arith<-1><<<node_grid(ctx->P), 128, 0, ctx->stream>>>(
-          ctx->P, v, ctx->i32[C_CELLX], ctx->geo[2], ctx->geo[3], ctx->geo_flags, ctx->cell_start, out);
+      launch_after(k_project_geo_arith<-1>, node_grid(ctx->P), 128, 0, ctx->stream, ctx->P, v, ctx->i32[C_CELLX],
+                   ctx->geo[2], ctx->geo[3], ctx->geo_flags, ctx->cell_start, out);
     }
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
@@ -863,7 +872,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   (void)st;
   {
     MIC_KERNEL(ctx, "k_project_all2");
-    k_project_all2<<<node_grid(ctx->P), 128, 0, ctx->stream>>>(ctx->P, mv, ctx->cell_start, ctx->mat, o);
+    launch_after(k_project_all2, node_grid(ctx->P), 128, 0, ctx->stream, ctx->P, mv, ctx->cell_start, ctx->mat, o);
   }
 #else
   PartialView pv = {};
@@ -890,13 +899,13 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
     {
       MIC_KERNEL_ON(ctx, "k_partials_basic<first>", s);
       if (few)
-        k_corners_basic<kFirst><<<g4, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+        launch_after(k_corners_basic<kFirst>, g4, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
       else
-        k_partials_basic<kFirst><<<g1, 128, 0, s>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+        launch_after(k_partials_basic<kFirst>, g1, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
     }
     {
       MIC_KERNEL_ON(ctx, "k_combine_all2<first>", s);
-      k_combine_all2<2><<<node_grid(ctx->P), 128, 0, s>>>(ctx->P, ctx->part_b, ctx->part_c, o);
+      launch_after(k_combine_all2<2>, node_grid(ctx->P), 128, 0, s, ctx->P, ctx->part_b, ctx->part_c, o);
     }
     MIC_CUDA_TRY(cudaGetLastError());
     ctx->wn_valid |= 1;
@@ -909,32 +918,37 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   {
     MIC_KERNEL_ON(ctx, "k_partials_centre", ctx->aux);
     if (few)
-      k_corners_centre<true, true><<<corners_centre_grid(ctx->P), 128, 0, ctx->aux>>>(ctx->P, pv, ctx->quad_start,
-                                                                                       ctx->part_c);
+      launch_after(k_corners_centre<true, true>, corners_centre_grid(ctx->P), 128, 0, ctx->aux, ctx->P, pv,
+                   ctx->quad_start, ctx->part_c);
     else
-      k_partials_centre<<<centre_grid(ctx->P), 128, 0, ctx->aux>>>(ctx->P, pv, ctx->quad_start, ctx->part_c);
+      launch_after(k_partials_centre, centre_grid(ctx->P), 128, 0, ctx->aux, ctx->P, pv, ctx->quad_start,
+                   ctx->part_c);
   }
   MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
   if (visc) {
     MIC_KERNEL(ctx, "k_partials_basic<visc>");
     if (few)
-      k_corners_basic<kVisc><<<g4, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+      launch_after(k_corners_basic<kVisc>, g4, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
+                   ctx->part_b);
     else
-      k_partials_basic<kVisc><<<g1, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+      launch_after(k_partials_basic<kVisc>, g1, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
+                   ctx->part_b);
   } else {
     MIC_KERNEL(ctx, "k_partials_basic");
     if (few)
-      k_corners_basic<kFull><<<g4, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+      launch_after(k_corners_basic<kFull>, g4, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
+                   ctx->part_b);
     else
-      k_partials_basic<kFull><<<g1, 128, 0, ctx->stream>>>(ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
+      launch_after(k_partials_basic<kFull>, g1, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
+                   ctx->part_b);
   }
   MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->aux_ev[1], 0));  // the cell-centre sums
   if (visc) {
     MIC_KERNEL(ctx, "k_combine_all2<visc>");
-    k_combine_all2<1><<<node_grid(ctx->P), 128, 0, ctx->stream>>>(ctx->P, ctx->part_b, ctx->part_c, o);
+    launch_after(k_combine_all2<1>, node_grid(ctx->P), 128, 0, ctx->stream, ctx->P, ctx->part_b, ctx->part_c, o);
   } else {
     MIC_KERNEL(ctx, "k_combine_all2");
-    k_combine_all2<0><<<node_grid(ctx->P), 128, 0, ctx->stream>>>(ctx->P, ctx->part_b, ctx->part_c, o);
+    launch_after(k_combine_all2<0>, node_grid(ctx->P), 128, 0, ctx->stream, ctx->P, ctx->part_b, ctx->part_c, o);
   }
   ctx->wn_valid |= visc ? 2 : 3;
 #endif

@@ -99,6 +99,7 @@ constexpr int kU = 0, kV = 1, kP = 2;  // DOF_U, DOF_V, DOF_P (fdcode.h:242-245)
 __global__ void k_vep_z(const double *__restrict__ etaN, const double *__restrict__ muN,
                         const double *__restrict__ etaS, const double *__restrict__ muS, int64_t nn, double dt,
                         double *etaNZ, double *etaSZ) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= nn) return;
   double den = A(etaN[k], M(dt, muN[k]));
@@ -111,6 +112,7 @@ __global__ void k_vep_z(const double *__restrict__ etaN, const double *__restric
 
 // VecMin (NaN entries skipped) of etaSZ, one block per slice, then one block over the slices
 __global__ void k_min_partial(const double *__restrict__ v, int64_t nn, double *part) {
+  if (!after_previous()) return;
   __shared__ double sm[256];
   double m = INFINITY;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x)
@@ -126,6 +128,7 @@ __global__ void k_min_partial(const double *__restrict__ v, int64_t nn, double *
 
 // Kbond = 4 etamin / (dx + dy)^2, Kcont = 2 etamin / (dx + dy) (vep_system.c:112-119)
 __global__ void k_vep_consts(Params P, const double *__restrict__ part, int nparts, double *K) {
+  if (!after_previous()) return;
   __shared__ double sm[256];
   double m = INFINITY;
   for (int k = threadIdx.x; k < nparts; k += blockDim.x)
@@ -150,6 +153,7 @@ __global__ void k_vep_consts(Params P, const double *__restrict__ part, int npar
 __global__ void k_vep_rows(Params P, Geo G, const double *__restrict__ etaNZ, const double *__restrict__ etaSZ,
                            const double *__restrict__ rho, const double *__restrict__ Kd, double gx, double gy,
                            Rows R) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (k >= (int64_t)NX * NY) return;
@@ -317,6 +321,7 @@ struct ThermalFields {
 // side) and 175-232 (boundary values inserted into the right-hand side)
 __global__ void k_thermal_rows(Params P, Geo G, ThermalFields F, double rho0, double dt, int doSteady, int topType,
                                double topValue, Rows R) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (k >= (int64_t)NX * NY) return;
@@ -381,6 +386,7 @@ __global__ void k_thermal_rows(Params P, Geo G, ThermalFields F, double rho0, do
 // enforceThermalBCs1 (enforceThermalBC.c:15-33): top value, then the left wall's slab inflow
 // temperature and the right wall's plate geotherm above the plate depth
 __global__ void k_enforce_thermal_bcs(Params P, Geo G, double topValue, double *lastT) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (k >= (int64_t)NX * NY) return;
@@ -598,22 +604,22 @@ extern "C" int mic_form_vep_system(mic_ctx *ctx, const mic_subduction_options *o
   double **f = ctx->nodal;
   {
     MIC_KERNEL(ctx, "k_vep_z");
-    k_vep_z<<<grid_for(nn), kBlock, 0, ctx->stream>>>(f[MIC_NF_ETAN], f[MIC_NF_MUN], f[MIC_NF_ETAS], f[MIC_NF_MUS],
-                                                      nn, dt, s.etaNZ, s.etaSZ);
+    launch_after(k_vep_z, grid_for(nn), kBlock, 0, ctx->stream, f[MIC_NF_ETAN], f[MIC_NF_MUN], f[MIC_NF_ETAS],
+                 f[MIC_NF_MUS], nn, dt, s.etaNZ, s.etaSZ);
   }
   const int parts = (int)std::min<int64_t>(kMinParts, (nn + kBlock - 1) / kBlock);
   {
     MIC_KERNEL(ctx, "k_min_partial");
-    k_min_partial<<<parts, 256, 0, ctx->stream>>>(s.etaSZ, nn, s.part);
+    launch_after(k_min_partial, parts, 256, 0, ctx->stream, s.etaSZ, nn, s.part);
   }
   {
     MIC_KERNEL(ctx, "k_vep_consts");
-    k_vep_consts<<<1, 256, 0, ctx->stream>>>(ctx->P, s.part, parts, s.K);
+    launch_after(k_vep_consts, 1, 256, 0, ctx->stream, ctx->P, s.part, parts, s.K);
   }
   {
     MIC_KERNEL(ctx, "k_vep_rows");
-    k_vep_rows<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, G, s.etaNZ, s.etaSZ, f[MIC_NF_RHO], s.K, o->gx,
-                                                         o->gy, rows_of(ctx->sys[0]));
+    launch_after(k_vep_rows, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, G, s.etaNZ, s.etaSZ, f[MIC_NF_RHO], s.K,
+                 o->gx, o->gy, rows_of(ctx->sys[0]));
   }
   MIC_CUDA_TRY(cudaGetLastError());
   double K[2];
@@ -637,8 +643,8 @@ extern "C" int mic_enforce_thermal_bcs(mic_ctx *ctx, const mic_subduction_option
   if (e) return e;
   const int64_t nn = (int64_t)ctx->P.NX * ctx->P.NY;
   MIC_KERNEL(ctx, "k_enforce_thermal_bcs");
-  k_enforce_thermal_bcs<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, G, o->thermalBCTopValue,
-                                                                   ctx->nodal[MIC_NF_LASTT]);
+  launch_after(k_enforce_thermal_bcs, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, G, o->thermalBCTopValue,
+               ctx->nodal[MIC_NF_LASTT]);
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
 }
@@ -657,9 +663,8 @@ extern "C" int mic_form_thermal_system(mic_ctx *ctx, const mic_subduction_option
   ThermalFields F{f[MIC_NF_KTHERMAL], f[MIC_NF_RHO], f[MIC_NF_CP], f[MIC_NF_LASTT], f[MIC_NF_VX], f[MIC_NF_HEATING]};
   {
     MIC_KERNEL(ctx, "k_thermal_rows");
-    k_thermal_rows<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->P, G, F, ctx->mat.materialRho[0], dt, doSteady,
-                                                             o->thermalBCTopType, o->thermalBCTopValue,
-                                                             rows_of(ctx->sys[1]));
+    launch_after(k_thermal_rows, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, G, F, ctx->mat.materialRho[0], dt,
+                 doSteady, o->thermalBCTopType, o->thermalBCTopValue, rows_of(ctx->sys[1]));
   }
   MIC_CUDA_TRY(cudaGetLastError());
   ctx->sys[1].factored = 0;

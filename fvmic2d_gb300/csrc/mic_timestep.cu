@@ -21,6 +21,7 @@ namespace {
 // VecNorm(thisT - lastT, NORM_INFINITY) (main:387-390), NaN entries skipped
 __global__ void k_temp_change(const double *__restrict__ thisT, const double *__restrict__ lastT, int64_t nn,
                               double *part) {
+  if (!after_previous()) return;
   __shared__ double sm[256];
   double m = 0.0;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x) {
@@ -53,6 +54,7 @@ __global__ void k_adiabatic_values(const int *__restrict__ cellX, const int *__r
 
 // VecAXPY(nodal_heating, 1.0, ha) (main_subduction.c:377)
 __global__ void k_add_heating(double *heat, const double *__restrict__ ha, int64_t nn) {
+  if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k < nn) heat[k] = heat[k] + 1.0 * ha[k];
 }
@@ -63,7 +65,8 @@ int max_temp_change(mic_ctx *ctx, double *out) {
   double *part = ctx->red_buf;  // reduction scratch of the context (at least 64 entries)
   {
     MIC_KERNEL(ctx, "k_temp_change");
-    k_temp_change<<<kParts, 256, 0, ctx->stream>>>(ctx->nodal[MIC_NF_THIST], ctx->nodal[MIC_NF_LASTT], nn, part);
+    launch_after(k_temp_change, kParts, 256, 0, ctx->stream, ctx->nodal[MIC_NF_THIST], ctx->nodal[MIC_NF_LASTT], nn,
+                 part);
   }
   double h[kParts];
   MIC_CUDA_TRY(cudaMemcpyAsync(h, part, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
@@ -102,7 +105,8 @@ extern "C" int mic_adiabatic_heating(mic_ctx *ctx, double gy) {
   if ((e = mic_project_scalar(ctx, ctx->scr1, 0, ctx->node_scr[5]))) return e;
   {
     MIC_KERNEL(ctx, "k_add_heating");
-    k_add_heating<<<grid_for(nn), kBlock, 0, ctx->stream>>>(ctx->nodal[MIC_NF_HEATING], ctx->node_scr[5], nn);
+    launch_after(k_add_heating, grid_for(nn), kBlock, 0, ctx->stream, ctx->nodal[MIC_NF_HEATING], ctx->node_scr[5],
+                 nn);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   return MIC_OK;
