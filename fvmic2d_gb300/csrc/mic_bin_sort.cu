@@ -508,10 +508,17 @@ int ensure_sort_scratch(mic_ctx *ctx, int64_t need) {
 }  // namespace
 
 // Bins every marker, sorts the columns by cell (stable) and rebuilds cell_start.
-int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
+int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out, bool step) {
   const int64_t n = ctx->n;
-  // n_out and bad_cell
-  MIC_CUDA_TRY(cudaMemsetAsync(&ctx->d_status->n_out, 0, 2 * sizeof(unsigned long long), ctx->stream));
+  const int passes = passes_for(ctx->ncells);
+  const int64_t ints = n > 0 ? sort_ints(tiles_for(n), passes) : 0;
+  int e = n > 0 ? ensure_sort_scratch(ctx, ints) : MIC_OK;
+  if (e) return e;
+  mic_clear_list clear;
+  clear.add(&ctx->d_status->n_out, 2 * sizeof(unsigned long long));  // and bad_cell
+  if (n > 0) clear.add(ctx->sort_buf, sizeof(int) * ints);
+  if (step) mic_clear_yield(ctx, clear, true);
+  if ((e = mic_clear(ctx, clear))) return e;
   if (n == 0) {
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->cell_start, 0, sizeof(int) * ((size_t)ctx->ncells + 2), ctx->stream));
     MIC_CUDA_TRY(cudaMemsetAsync(ctx->quad_start, 0, sizeof(int) * (4 * (size_t)ctx->ncells + 5), ctx->stream));
@@ -520,11 +527,6 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
     if (n_out) *n_out = 0;
     return MIC_OK;
   }
-  const int passes = passes_for(ctx->ncells);
-  const int64_t ints = sort_ints(tiles_for(n), passes);
-  int e = ensure_sort_scratch(ctx, ints);
-  if (e) return e;
-  MIC_CUDA_TRY(cudaMemsetAsync(ctx->sort_buf, 0, sizeof(int) * ints, ctx->stream));
   {
     MIC_KERNEL(ctx, "k_find_cells");
     const int block = tuned_block(ctx, TU_FIND_CELLS);
@@ -574,8 +576,7 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out) {
   ctx->geo_valid = 1;  // computed by the gather
   ctx->wn_valid = 0;
   if (n_out) {
-    MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
-    MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if ((e = mic_fetch_status(ctx))) return e;
     *n_out = (int64_t)ctx->h_status->n_out;
     if (ctx->h_status->bad_cell) return MIC_ERR_CELL;
   }

@@ -755,11 +755,50 @@ extern "C" int mic_get_stream(mic_ctx *ctx, void **stream) {
   return MIC_OK;
 }
 
+namespace {
+__global__ void __launch_bounds__(256) k_clear(const mic_clear_list l) {
+  if (!after_previous()) return;
+  for (int r = 0; r < l.n; ++r)
+    for (int64_t q = blockIdx.x * 256LL + threadIdx.x; q < l.words[r]; q += gridDim.x * 256LL) l.p[r][q] = 0;
+}
+
+// The status goes to the host by a kernel's own stores into the pinned mirror: a copy would wait for
+// the copy engine to take over from the kernels.
+__global__ void __launch_bounds__(32) k_status_out(const unsigned int *d, volatile unsigned int *h) {
+  if (!after_previous()) return;
+  static_assert(sizeof(Status) % 4 == 0 && sizeof(Status) / 4 <= 32, "one word a lane");
+  if (threadIdx.x < sizeof(Status) / 4) h[threadIdx.x] = d[threadIdx.x];
+}
+}  // namespace
+
+int mic_clear(mic_ctx *ctx, const mic_clear_list &l) {
+  if (l.n > mic_clear_list::kMost) return MIC_ERR_ARG;
+  int64_t most = 1;
+  for (int r = 0; r < l.n; ++r) most = l.words[r] > most ? l.words[r] : most;
+  const int64_t full = (most + 1023) / 1024, cap = 4 * (int64_t)sm_count(ctx);
+  {
+    MIC_KERNEL(ctx, "k_clear");
+    launch_after(k_clear, (unsigned)(full < cap ? full : cap), 256, 0, ctx->stream, l);
+  }
+  MIC_CUDA_TRY(cudaGetLastError());
+  return MIC_OK;
+}
+
+int mic_fetch_status(mic_ctx *ctx) {
+  {
+    MIC_KERNEL(ctx, "k_status_out");
+    launch_after(k_status_out, 1, 32, 0, ctx->stream, reinterpret_cast<const unsigned int *>(ctx->d_status),
+                 reinterpret_cast<volatile unsigned int *>(ctx->h_status));
+  }
+  MIC_CUDA_TRY(cudaGetLastError());
+  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return MIC_OK;
+}
+
 extern "C" int mic_get_status(mic_ctx *ctx, mic_status *st) {
   if (!ctx || !st) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
-  MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (const int e = mic_fetch_status(ctx)) return e;
   st->bad_cell = ctx->h_status->bad_cell;
   st->nan_residual = ctx->h_status->nan_residual;
   st->nan_dsxy = ctx->h_status->nan_dsxy;

@@ -42,11 +42,13 @@ enum I32Col { C_MAT = 0, C_CELLX, C_CELLY, C_CPU, C_ISYIELD, C_ID, C_I32_COUNT }
 struct Status {
   unsigned long long nan_residual;  // NaN strain-rate residual (updateMarkerStrainPressure.c:302-306)
   unsigned long long nan_dsxy;      // NaN interpolated dsxy (updateMarkerStress.c:136-142)
-  unsigned long long bad_law;       // unknown viscosity law (viscosity.c:60-62)
   unsigned long long n_out;         // out-of-domain markers after the last binning
   unsigned long long bad_cell;      // impossible cell index (markers.c:74-77): markers not placed (cleared with n_out)
-  int is_yielding;                  // any marker yielded in the last checkPlasticYielding
+  unsigned long long bad_law;       // unknown viscosity law (viscosity.c:60-62)
+  int is_yielding;                  // any marker yielded in the last checkPlasticYielding (cleared with bad_law)
   int pad;
+  unsigned long long max_bits;      // a step's maximum (marker temperature, then |sxx|): its bits
+  double residual;                  // the strain-rate residual's sum over the area
 };
 
 // Composite creep (law 7) settings and per-pass counters
@@ -247,7 +249,29 @@ int mic_ensure_sorted(mic_ctx *ctx);  // bins + sorts if positions changed since
 int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cudaStream_t s = nullptr);
 void mic_invalidate_sort(mic_ctx *ctx);
 void mic_front_plan_free(mic_front_plan *plan);  // (mic_front_lu.cu)
-int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out);
+// step: also clears what the first pieces of a step add to (max_bits, the yield pass's results)
+int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out, bool step = false);
+int mic_fetch_status(mic_ctx *ctx);  // *d_status into *h_status; waits for the stream
+
+// Memory to be zeroed by one launch: a step's flags, maxima and digit counts lie apart, and a memset
+// each would also keep the kernels around it from overlapping (launch_after).  GB300: a step's nine
+// memsets as two such launches, and its results by one kernel's stores instead of four copies, took
+// the cycle of the 64 x 64 box from 254 to 212 us.
+struct mic_clear_list {
+  static constexpr int kMost = 4;
+  unsigned int *p[kMost];
+  int64_t words[kMost];
+  int n = 0;  // above kMost: too many were added (mic_clear refuses)
+  void add(void *mem, size_t bytes) {
+    if (n < kMost) {
+      p[n] = static_cast<unsigned int *>(mem);
+      words[n] = (int64_t)(bytes / sizeof(unsigned int));
+    }
+    ++n;
+  }
+};
+int mic_clear(mic_ctx *ctx, const mic_clear_list &l);
+void mic_clear_yield(mic_ctx *ctx, mic_clear_list &l, bool step = false);  // what the yield pass adds to
 int mic_ensure_geometry(mic_ctx *ctx);  // sorted columns + projection geometry
 // projectMarkersNodesAll2 again after a full pass on unchanged positions, densities, temperatures
 // and materials (only viscosities and stresses changed): the product build re-forms only those

@@ -942,9 +942,10 @@ __device__ __forceinline__ df bil_eval_df(const BilDF *__restrict__ cells, size_
 // the left boundary condition, rows 0 .. NY-2) and basic cells of the vorticity.
 __global__ void k_advect_coef(const double *__restrict__ vx, const double *__restrict__ vy,
                               const double *__restrict__ wz, mic_bcinfo top, mic_bcinfo left, int NX, int NY,
-                              BilDF *cvx, BilDF *cvy, BilDF *cwz) {
+                              BilDF *cvx, BilDF *cvy, BilDF *cwz, unsigned long long *clear) {
   if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k == 0 && clear) *clear = 0;  // the maximum that the advection adds to
   if (k < (int64_t)NY * (NX - 1)) {
     const int row = (int)(k / (NX - 1)), i = (int)(k % (NX - 1));
     const size_t r1 = (size_t)row * NX;
@@ -988,9 +989,10 @@ __global__ void k_advect_coef(const double *__restrict__ vx, const double *__res
 // one's right column wrapping to column 0, and no ghost column at the left wall.
 __global__ void k_advect_coef_periodic(const double *__restrict__ vx, const double *__restrict__ vy,
                                        const double *__restrict__ wz, mic_bcinfo top, int NX, int NY, Bil4 *cvx,
-                                       Bil4 *cvy, Bil4 *cwz) {
+                                       Bil4 *cvy, Bil4 *cwz, unsigned long long *clear) {
   if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k == 0 && clear) *clear = 0;
   if (k >= (int64_t)NX * NY) return;
   const int row = (int)(k / NX), i = (int)(k % NX), i1 = next_col(i, NX);
   const size_t r0 = (size_t)row * NX;
@@ -1591,13 +1593,12 @@ YieldCols yield_cols(mic_ctx *ctx) {
 }
 
 int read_status(mic_ctx *ctx) {
-  MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (const int e = mic_fetch_status(ctx)) return e;
   return ctx->h_status->bad_cell ? MIC_ERR_CELL : MIC_OK;  // markers the last binning could not place
 }
 
 int run_max(mic_ctx *ctx, int col, int absval, double *out) {
-  unsigned long long *d = reinterpret_cast<unsigned long long *>(ctx->red_buf + 8);
+  unsigned long long *d = &ctx->d_status->max_bits;
   MIC_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream));
   if (ctx->n > 0) {
     {
@@ -1607,12 +1608,8 @@ int run_max(mic_ctx *ctx, int col, int absval, double *out) {
     MIC_CUDA_TRY(cudaGetLastError());
   }
   if (out) {
-    unsigned long long h = 0;
-    MIC_CUDA_TRY(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    double v;
-    memcpy(&v, &h, sizeof(v));
-    *out = v;
+    if (const int e = mic_fetch_status(ctx)) return e;
+    memcpy(out, &ctx->h_status->max_bits, sizeof(double));
   }
   return MIC_OK;
 }
@@ -2112,12 +2109,11 @@ struct mic_batch {
   }
 };
 
-// with_max: the step's maximum marker temperature into the reduction slot as well (run_max's)
+// with_max: the step's maximum marker temperature into the status as well, cleared by the binning
 static int update_rho(mic_ctx *ctx, bool with_max, mic_batch *b = nullptr) {
   int e = mic_ensure_sorted(ctx);
   if (e) return e;
-  unsigned long long *d = reinterpret_cast<unsigned long long *>(ctx->red_buf + 8);
-  if (with_max) MIC_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream));
+  unsigned long long *d = &ctx->d_status->max_bits;
   if (ctx->n == 0) return MIC_OK;
   RhoJob J = {ctx->i32[C_CELLX], ctx->i32[C_MAT], ctx->f64[C_T], ctx->f64[C_RHO], ctx->f64[C_RHODOT], {}, {},
               ctx->n, with_max ? d : nullptr};
@@ -2146,13 +2142,25 @@ extern "C" int mic_max_abs_sxx(mic_ctx *ctx, double *v) {
   return run_max(ctx, C_SXX, 1, v);
 }
 
+// bad_law and is_yielding, with step also the max_bits behind them, and the creep counters
+void mic_clear_yield(mic_ctx *ctx, mic_clear_list &l, bool step) {
+  static_assert(offsetof(Status, is_yielding) == offsetof(Status, bad_law) + 8 &&
+                    offsetof(Status, max_bits) == offsetof(Status, bad_law) + 16,
+                "cleared together");
+  l.add(&ctx->d_status->bad_law, step ? 24 : 12);
+  l.add(ctx->d_creep, sizeof(CreepCounters));
+}
+
 // limit: limitViscosity (viscosity.c:90-104) fused into the pass, for callers that run it next
-static int yield_launch(mic_ctx *ctx, double dt, bool limit = false, mic_batch *b = nullptr) {
+// cleared: the step's binning has cleared the pass's results
+static int yield_launch(mic_ctx *ctx, double dt, bool limit = false, bool cleared = false, mic_batch *b = nullptr) {
   int e = mic_ensure_sorted(ctx);
   if (e) return e;
-  MIC_CUDA_TRY(cudaMemsetAsync(&ctx->d_status->is_yielding, 0, sizeof(int), ctx->stream));
-  MIC_CUDA_TRY(cudaMemsetAsync(&ctx->d_status->bad_law, 0, sizeof(unsigned long long), ctx->stream));
-  MIC_CUDA_TRY(cudaMemsetAsync(ctx->d_creep, 0, sizeof(CreepCounters), ctx->stream));
+  if (!cleared) {
+    mic_clear_list l;
+    mic_clear_yield(ctx, l);
+    if ((e = mic_clear(ctx, l))) return e;
+  }
   if (ctx->n == 0) return MIC_OK;
   const int mode = ctx->creep.mlp ? ctx->creep.mode : 0;
   bool law7 = false;
@@ -2209,10 +2217,14 @@ extern "C" int mic_limit_viscosity(mic_ctx *ctx) {
 }
 
 // keep: store the interpolated old stresses for a sub-grid stress pass that follows in this step
-static int strain_launch(mic_ctx *ctx, double dt, bool keep = false, mic_batch *b = nullptr) {
+// step: clears the flag of the step's stress pass as well
+static int strain_launch(mic_ctx *ctx, double dt, bool keep = false, bool step = false, mic_batch *b = nullptr) {
   int e = mic_ensure_geometry(ctx);
   if (e) return e;
-  MIC_CUDA_TRY(cudaMemsetAsync(&ctx->d_status->nan_residual, 0, sizeof(unsigned long long), ctx->stream));
+  mic_clear_list l;
+  l.add(&ctx->d_status->nan_residual, sizeof(unsigned long long));
+  if (step) l.add(&ctx->d_status->nan_dsxy, sizeof(unsigned long long));
+  if ((e = mic_clear(ctx, l))) return e;
   if (ctx->n == 0) return MIC_OK;
   StrainCols c;
   c.cellX = ctx->i32[C_CELLX];
@@ -2270,13 +2282,9 @@ static int residual_launch(mic_ctx *ctx, int iter, double *res_dev, cudaStream_t
 extern "C" int mic_update_global_strain_rate_residual(mic_ctx *ctx, int iter, double *residual) {
   CHECK_CTX();
   if (iter < 0) return MIC_ERR_ARG;
-  double *d = ctx->red_buf + 16;
-  int e = residual_launch(ctx, iter, d);
-  if (e) return e;
-  double s = 0.0;
-  MIC_CUDA_TRY(cudaMemcpyAsync(&s, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  s /= (ctx->P.LX * ctx->P.LY);
+  int e = residual_launch(ctx, iter, &ctx->d_status->residual);
+  if (e || (e = mic_fetch_status(ctx))) return e;
+  const double s = ctx->h_status->residual / (ctx->P.LX * ctx->P.LY);
   ctx->residuals[iter % 100] = s;
   if (residual) *residual = s;
   return MIC_OK;
@@ -2376,10 +2384,15 @@ extern "C" int mic_subgrid_stress_changes(mic_ctx *ctx, double dt, double D) {
   return e ? e : subgrid_nodes(ctx);
 }
 
-static int stress_launch(mic_ctx *ctx, mic_batch *b = nullptr) {
+// cleared: the step's strain-rate pass has cleared the flag
+static int stress_launch(mic_ctx *ctx, bool cleared = false, mic_batch *b = nullptr) {
   int e = mic_ensure_geometry(ctx);
   if (e) return e;
-  MIC_CUDA_TRY(cudaMemsetAsync(&ctx->d_status->nan_dsxy, 0, sizeof(unsigned long long), ctx->stream));
+  if (!cleared) {
+    mic_clear_list l;
+    l.add(&ctx->d_status->nan_dsxy, sizeof(unsigned long long));
+    if ((e = mic_clear(ctx, l))) return e;
+  }
   if (ctx->n == 0) return MIC_OK;
   StressCols c;
   c.cellX = ctx->i32[C_CELLX];
@@ -2464,8 +2477,17 @@ extern "C" int mic_subgrid_temperature_changes(mic_ctx *ctx, double dt) {
 static int advect_launch(mic_ctx *ctx, double dt, bool wz_known, bool with_max = false, mic_batch *b = nullptr) {
   int e = mic_ensure_geometry(ctx);
   if (e) return e;
-  unsigned long long *d = reinterpret_cast<unsigned long long *>(ctx->red_buf + 8);
-  if (with_max) MIC_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream));
+  unsigned long long *d = &ctx->d_status->max_bits;
+#ifdef MIC_EXACT
+  const bool in_coef = false;
+#else
+  const bool in_coef = ctx->n > 0;  // the coefficients' kernel clears the slot
+#endif
+  if (with_max && !in_coef) {
+    mic_clear_list l;
+    l.add(d, sizeof(unsigned long long));
+    if ((e = mic_clear(ctx, l))) return e;
+  }
   if (ctx->n > 0) {
     AdvectCols c;
     c.cellX = ctx->i32[C_CELLX];
@@ -2499,11 +2521,11 @@ static int advect_launch(mic_ctx *ctx, double dt, bool wz_known, bool with_max =
         Bil4 *cp = static_cast<Bil4 *>(ctx->adv_coef);
         launch_after(k_advect_coef_periodic, grid_for((int64_t)nn), kBlock, 0, ctx->stream, ctx->nodal[MIC_NF_VX],
                      ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop, NX, NY, cp, cp + nn,
-                     cp + 2 * nn);
+                     cp + 2 * nn, with_max ? d : nullptr);
       } else {
         launch_after(k_advect_coef, grid_for((int64_t)nn), kBlock, 0, ctx->stream, ctx->nodal[MIC_NF_VX],
                      ctx->nodal[MIC_NF_VY], ctx->nodal[MIC_NF_WXY], ctx->bcs.mechBCTop, ctx->bcs.mechBCLeft, NX, NY,
-                     cb, cb + nn, cb + 2 * nn);
+                     cb, cb + nn, cb + 2 * nn, with_max ? d : nullptr);
       }
     }
     MIC_CUDA_TRY(cudaGetLastError());
@@ -2576,12 +2598,12 @@ int mic_step_segment(mic_ctx *ctx, int seg, double dt_disp, double dt_thermal, i
       // one rank without density control, so one binning gives all three results.  The density
       // update also finds the maximum temperature (main:271-281; the projection between changes no
       // marker temperature).
-      if ((e = mic_bin_and_sort(ctx, nullptr))) return e;
+      if ((e = mic_bin_and_sort(ctx, nullptr, true))) return e;
       return update_rho(ctx, true, b);
     case 1:
 #ifdef MIC_EXACT
       if ((e = mic_project_markers_nodes_all2(ctx))) return e;
-      return yield_launch(ctx, dt_disp, false, b);
+      return yield_launch(ctx, dt_disp, false, true, b);
 #else
       // The first projection (main:268) and the yield pass touch disjoint marker columns (rho, T,
       // materials against viscosity, modulus and stresses), and the first projection's viscosity
@@ -2593,7 +2615,7 @@ int mic_step_segment(mic_ctx *ctx, int seg, double dt_disp, double dt_thermal, i
       MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->aux_ev[0], 0));
       if ((e = mic_project_all2_first(ctx, ctx->aux))) return e;
       MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
-      return yield_launch(ctx, dt_disp, /*limit=*/true, b);  // limitViscosity fused in
+      return yield_launch(ctx, dt_disp, /*limit=*/true, true, b);  // limitViscosity fused in
 #endif
     case 2:
 #ifdef MIC_EXACT
@@ -2604,23 +2626,23 @@ int mic_step_segment(mic_ctx *ctx, int seg, double dt_disp, double dt_thermal, i
       // the second projection: yielding and the limit changed viscosities and stresses only
       return mic_project_all2_viscous(ctx);
     case 3:
-      return strain_launch(ctx, dt_disp, keep, b);
+      return strain_launch(ctx, dt_disp, keep, true, b);
     case 4:
 #ifdef MIC_EXACT
-      if ((e = residual_launch(ctx, 0, ctx->red_buf + 16))) return e;
+      if ((e = residual_launch(ctx, 0, &ctx->d_status->residual))) return e;
 #else
       // the residual (a cell-centre projection of srr and its area-weighted sum) shares no buffer
       // with the sub-grid stress and stress-update passes: it runs on the second stream beside them
       if ((e = mic_ensure_geometry(ctx))) return e;
       MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[0], ctx->stream));
       MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->aux_ev[0], 0));
-      if ((e = residual_launch(ctx, 0, ctx->red_buf + 16, ctx->aux))) return e;  // leaves the scratch columns alone
+      if ((e = residual_launch(ctx, 0, &ctx->d_status->residual, ctx->aux))) return e;  // (no scratch column)
       MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
 #endif
       return sub ? subgrid_markers(ctx, dt_disp, ctx->opt.subgridStressDiffusivity, keep, b) : MIC_OK;
     case 5:
       if (sub && (e = subgrid_nodes(ctx))) return e;
-      return stress_launch(ctx, b);
+      return stress_launch(ctx, true, b);
     case 6:
 #ifndef MIC_EXACT
       MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->aux_ev[1], 0));
@@ -2647,13 +2669,6 @@ static int run_segments(mic_ctx *ctx, int s0, int s1, double dt_disp, double dt_
   return MIC_OK;
 }
 
-static int read_max_slot(mic_ctx *ctx, double *out) {
-  unsigned long long h = 0;
-  MIC_CUDA_TRY(cudaMemcpyAsync(&h, ctx->red_buf + 8, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  memcpy(out, &h, sizeof(double));
-  return MIC_OK;
-}
 
 extern "C" int mic_step_pre_stokes(mic_ctx *ctx, double dt_disp, int *is_yielding, double *max_T) {
   CHECK_CTX();
@@ -2662,18 +2677,14 @@ extern "C" int mic_step_pre_stokes(mic_ctx *ctx, double dt_disp, int *is_yieldin
   if (is_yielding || max_T) {
     if ((e = read_status(ctx))) return e;
     if (is_yielding) *is_yielding = ctx->h_status->is_yielding;
-    if (max_T && (e = read_max_slot(ctx, max_T))) return e;
+    if (max_T) memcpy(max_T, &ctx->h_status->max_bits, sizeof(double));
   }
   return MIC_OK;
 }
 
 static int read_residual(mic_ctx *ctx, double *residual) {
-  double s = 0.0;
-  MIC_CUDA_TRY(cudaMemcpyAsync(&s, ctx->red_buf + 16, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  s /= (ctx->P.LX * ctx->P.LY);
-  ctx->residuals[0] = s;
-  *residual = s;
+  if (const int e = mic_fetch_status(ctx)) return e;
+  *residual = ctx->residuals[0] = ctx->h_status->residual / (ctx->P.LX * ctx->P.LY);
   return MIC_OK;
 }
 
@@ -2689,7 +2700,10 @@ extern "C" int mic_step_post_thermal(mic_ctx *ctx, double dt_thermal, double *ma
   int e;
   // the marker vorticity may be stale here: a caller between the calls may replace nodal fields
   if ((e = run_segments(ctx, 7, kStepSegments, 0.0, dt_thermal, 0, 0))) return e;
-  return max_abs_sxx ? read_max_slot(ctx, max_abs_sxx) : MIC_OK;
+  if (!max_abs_sxx) return MIC_OK;
+  if ((e = mic_fetch_status(ctx))) return e;
+  memcpy(max_abs_sxx, &ctx->h_status->max_bits, sizeof(double));
+  return MIC_OK;
 }
 
 extern "C" int mic_step(mic_ctx *ctx, double dt_disp, double dt_thermal, int subgrid_stress, double *residual) {
