@@ -916,19 +916,27 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     }
     // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
-    // Ahead only where the update leaves SMs idle: once its multiply-adds alone take longer than a
-    // panel (about 25 us at 2 per SM and clock), both wait for the same FP64 pipes and the split
-    // costs (513 x 129 Stokes: 54.3 ms with every update split, 51.6 with none; 129 x 33: 2.46 and 2.79)
+    // The rest of an update runs beside the next panel, in one of two orders.  Light (its
+    // multiply-adds under 75 us at 2 per SM and clock, or a panel that fits beside its blocks in
+    // an SM's shared memory): it starts with the update of the next panel's columns.  Heavy: only
+    // after that one, so that the panel, which may need an SM's whole shared memory, finds free SMs;
+    // behind a heavy update it would start when that ends (513 x 129 Stokes: 54.3 ms with every
+    // update light, 46.9 with the heavy ones whole before the next panel, 41.8 so; 129 x 33: 2.35
+    // with every update of 25 us and more before the next panel, 2.40 with all heavy, 2.21 so).
     const double us = (double)cols * below * NB * L.count / (2.0 * 1.9e3 * sm_count(ctx));
-    const bool ahead = k0 + NB < L.maxP && cols > NB && us < 25.0;
+    const bool ahead = k0 + NB < L.maxP && cols > NB, light = us < 75.0 || rows < 400;
     const int near = ahead ? NB : 0, rest = cols - near;
     cudaStream_t st = ahead ? main : chain;
-    if (ahead) {
+    if (ahead && light) {
       MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], chain));
       MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
     }
     if (far) MIC_CUDA_TRY(cudaStreamWaitEvent(chain, ctx->lu_ev[1], 0));
     if (ahead) update<NB, 64, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+    if (ahead && !light) {
+      MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], chain));
+      MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
+    }
     // the tile whose blocks, padding and triangular solves included, take the least time on the
     // fullest SM (multiply-adds, 2 per clock; 600 clocks a block to start and end)
     const double nsm = sm_count(ctx);
