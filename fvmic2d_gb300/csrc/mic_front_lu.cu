@@ -621,13 +621,14 @@ __global__ void __launch_bounds__(256) k_front_border(const Front *__restrict__ 
   if (lane == 0) u[q.C - 1] -= s;
 }
 
-// U11 x = y, 32 rows at a time from the bottom, one block per front: a warp per row for the part
-// from solved unknowns (border: those of the border too), one warp for the 32 x 32 triangle with
-// all reciprocals formed at once
-__global__ void __launch_bounds__(1024) k_front_back(const Front *__restrict__ fr, int first,
-                                                    const int *__restrict__ tab, const double *__restrict__ U,
-                                                    double *x, int border) {
-  extern __shared__ double xs[];  // the front's unknowns: pivots, then (border) the border's
+// U11 x = y for fronts of at most 32 pivots, one block per front: a warp per row for the part from
+// the border's unknowns, one warp for the triangle with all reciprocals formed at once.  The lowest
+// levels have thousands of such fronts, of 10 to 20 pivots: little shared memory, so that many
+// share an SM (16,384 fronts of 12 pivots: 47 us; 115 in the form for many rows below).
+__global__ void __launch_bounds__(256) k_front_back_small(const Front *__restrict__ fr, int first,
+                                                          const int *__restrict__ tab, const double *__restrict__ U,
+                                                          double *x, int border) {
+  extern __shared__ double xs[];  // the border's unknowns, behind the pivots' places
   __shared__ double acc[32];
   __shared__ double Ud[32][33];
   const Front q = fr[first + blockIdx.x];
@@ -637,32 +638,110 @@ __global__ void __launch_bounds__(1024) k_front_back(const Front *__restrict__ f
   const int top = border ? q.C - 1 : q.P;
   for (int c = q.P + tid; c < top; c += blockDim.x) xs[c] = x[col[c]];
   __syncthreads();
-  for (int j1 = q.P; j1 > 0; j1 -= 32) {
-    const int j0 = max(j1 - 32, 0), nr = j1 - j0;
-    for (int w = warp; w < nr; w += nw) {
-      const double *u = U + q.u + (int64_t)(j0 + w) * q.C;
-      double s = 0.0;
+  for (int w = warp; w < q.P; w += nw) {
+    const double *u = U + q.u + (int64_t)w * q.C;
+    double s = 0.0;
 #pragma unroll 4
-      for (int c = j1 + lane; c < top; c += 32) s += u[c] * xs[c];
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0) acc[w] = u[q.C - 1] - s;
-      Ud[w][lane] = (lane >= w && lane < nr) ? u[j0 + lane] : 0.0;
+    for (int c = q.P + lane; c < top; c += 32) s += u[c] * xs[c];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) acc[w] = u[q.C - 1] - s;
+    Ud[w][lane] = (lane >= w && lane < q.P) ? u[lane] : 0.0;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  double a = lane < q.P ? acc[lane] : 0.0;
+  const double rd = 1.0 / (lane < q.P ? Ud[lane][lane] : 1.0);
+  for (int t = q.P - 1; t >= 0; --t) {
+    const double xt = __shfl_sync(0xffffffffu, a * rd, t);
+    if (lane < t) a -= Ud[lane][t] * xt;
+    if (lane == t) a = xt;
+  }
+  if (lane < q.P) x[col[lane]] = a;
+}
+
+// U11 x = y, one block per front, 32 rows at a time from the bottom (border: the part from the
+// border's unknowns too).  Bound by the chain of the unknowns and by the FP64 pipe, on which a
+// warp's instruction takes its quarter of the SM for 64 cycles whatever it computes:
+//   - a step of a triangle's solve is one shuffle and one multiply-add of warp 0, the rows having
+//     been divided by their diagonals before;
+//   - meanwhile the other warps fetch the next 32 rows and bring them up to date with the unknowns
+//     known before: a lane a row, the columns shared out between the warps, so that a row's sum
+//     needs no tree of additions;
+//   - between two triangles four warps form the part from the 32 new unknowns and add up the warps'
+//     sums, the others divide the next triangle.
+// GB300: 165 pivots 26 us, 645 121 (a warp a row with a tree a row, one phase after the other: 42, 184).
+__global__ void __launch_bounds__(1024) k_front_back(const Front *__restrict__ fr, int first,
+                                                    const int *__restrict__ tab, const double *__restrict__ U,
+                                                    double *x, int border) {
+  extern __shared__ double xs[];  // the front's unknowns: pivots, then (border) the border's
+  __shared__ double Ud[2][32][33], Un[32][33];  // triangles; the next rows' part on the unknowns being solved
+  __shared__ double part[32][32], comb[4][32], rhs[2][32], rd[2][32];
+  const Front q = fr[first + blockIdx.x];
+  if (q.P == 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int *col = tab + q.col;
+  const int top = border ? q.C - 1 : q.P;
+  for (int c = q.P + tid; c < top; c += blockDim.x) xs[c] = x[col[c]];
+  __syncthreads();
+  // rows j0 .. j1 - 1, by the warps from w0 on; the unknowns from `known` on are known
+  const auto prepare = [&](int j0, int j1, int known, int buf, int w0) {
+    const int n = j1 - j0, nv = nw - w0, me = warp - w0;
+    const double *u0 = U + q.u + (int64_t)j0 * q.C;
+    for (int w = me; w < n; w += nv) {
+      const double *u = u0 + (int64_t)w * q.C;
+      Ud[buf][w][lane] = lane >= w && lane < n ? u[j0 + lane] : 0.0;
+      Un[w][lane] = j1 + lane < known ? u[j1 + lane] : 0.0;
+      if (lane == 0) rhs[buf][w] = u[q.C - 1];
     }
+    const double *u = u0 + (int64_t)min(lane, n - 1) * q.C;
+    if (me == nv - 1) rd[buf][lane] = 1.0 / u[j0 + min(lane, n - 1)];
+    const int share = (top - known + nv - 1) / nv, c1 = min(known + (me + 1) * share, top);
+    double s = 0.0;
+#pragma unroll 8
+    for (int c = known + me * share; c < c1; ++c) s += u[c] * xs[c];
+    part[me][lane] = s;
+  };
+  int j1 = q.P, j0 = max(j1 - 32, 0), buf = 0, nv = nw, before = 0;  // before: unknowns of the last triangle
+  prepare(j0, j1, j1, 0, 0);
+  for (;;) {
+    __syncthreads();
+    const int n = j1 - j0, n0 = max(j0 - 32, 0);
+    if (warp < 4) {
+      double s = 0.0;
+#pragma unroll
+      for (int t = 0; t < 8; ++t)
+        if (8 * warp + t < before) s += Un[lane][8 * warp + t] * xs[j1 + 8 * warp + t];
+#pragma unroll 8
+      for (int w = warp; w < nv; w += 4) s += part[w][lane];
+      comb[warp][lane] = s;
+    }
+    if (warp >= 4 || nw == 4)
+      for (int w = warp - (nw > 4 ? 4 : 0); w < n; w += nw > 4 ? nw - 4 : nw) Ud[buf][w][lane] *= rd[buf][w];
     __syncthreads();
     if (warp == 0) {
-      double a = lane < nr ? acc[lane] : 0.0;
-      const double rd = 1.0 / (lane < nr ? Ud[lane][lane] : 1.0);
-      for (int t = nr - 1; t >= 0; --t) {
-        const double xt = __shfl_sync(0xffffffffu, a * rd, t);
-        if (lane < t) a -= Ud[lane][t] * xt;
-        if (lane == t) a = xt;
+      double a = 0.0;
+      if (lane < n) {
+        const double known = (comb[0][lane] + comb[1][lane]) + (comb[2][lane] + comb[3][lane]);
+        a = (rhs[buf][lane] - known) * rd[buf][lane];
       }
-      if (lane < nr) {
+#pragma unroll 4
+      for (int t = n - 1; t > 0; --t) {
+        const double xt = __shfl_sync(0xffffffffu, a, t), d = a - Ud[buf][lane][t] * xt;
+        a = lane < t ? d : a;
+      }
+      if (lane < n) {
         xs[j0 + lane] = a;
         x[col[j0 + lane]] = a;
       }
+    } else if (j0 > 0) {
+      prepare(n0, j0, j1, buf ^ 1, 1);
     }
-    __syncthreads();
+    if (j0 == 0) return;
+    before = n;
+    nv = nw - 1;
+    j1 = j0;
+    j0 = n0;
+    buf ^= 1;
   }
 }
 
@@ -1003,15 +1082,19 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
   for (int l = 0; l < nl; ++l) {
     const Level &L = pl.levels[l];
     // border part apart once a front's P x B block is more than one SM should read
-    const bool apart = L.maxC > L.maxP + 1 && ((int64_t)L.maxP * (L.maxC - L.maxP) > 8192 || L.maxC > 4096);
+    const bool apart = L.maxC > L.maxP + 1 && ((int64_t)L.maxP * (L.maxC - L.maxP) > 8192 || L.maxC > 1024);
     if (apart) {
       MIC_KERNEL(ctx, "k_front_border");
       k_front_border<<<dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x);
     }
     MIC_KERNEL(ctx, "k_front_back");
-    const int threads = L.maxP <= 16 ? 128 : L.maxP <= 64 ? 256 : 1024;
-    k_front_back<<<L.count, threads, sizeof(double) * (apart ? L.maxP : L.maxC), ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x,
-                                                                            apart ? 0 : 1);
+    const size_t smem = sizeof(double) * (apart ? L.maxP : L.maxC);
+    if (L.maxP <= 32)
+      k_front_back_small<<<L.count, L.maxP <= 16 ? 128 : 256, smem, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U,
+                                                                                  x, apart ? 0 : 1);
+    else
+      k_front_back<<<L.count, L.maxP <= 64 ? 256 : 1024, smem, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x,
+                                                                             apart ? 0 : 1);
   }
   return MIC_OK;
 }
@@ -1026,6 +1109,8 @@ cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
     e = cudaFuncSetAttribute(k_front_panel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_panel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_back, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
   return e;
 }
 
