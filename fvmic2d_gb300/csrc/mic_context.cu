@@ -202,6 +202,7 @@ static void free_ctx(mic_ctx *ctx) {
     if (ctx->aux_ev[k]) cudaEventDestroy(ctx->aux_ev[k]);
   cudaFree(ctx->stage_aos);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
+  if (ctx->h_words) cudaFreeHost(ctx->h_words);
   if (ctx->owns_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   free(ctx->h_x);
   delete ctx;
@@ -426,6 +427,10 @@ extern "C" int mic_create(mic_ctx **out, int device, void *stream, int NX, int N
     return MIC_ERR_NOMEM;
   }
   memset(ctx->h_status, 0, sizeof(Status));
+  if (cudaHostAlloc((void **)&ctx->h_words, kWordsOut, cudaHostAllocDefault) != cudaSuccess) {
+    free_ctx(ctx);
+    return MIC_ERR_NOMEM;
+  }
   cudaMemcpyToSymbol(c_f64_off, h_f64_off, sizeof(h_f64_off));
   cudaMemcpyToSymbol(c_i32_off, h_i32_off, sizeof(h_i32_off));
   for (int b = 0; b < 4; ++b) {
@@ -762,12 +767,22 @@ __global__ void __launch_bounds__(256) k_clear(const mic_clear_list l) {
     for (int64_t q = blockIdx.x * 256LL + threadIdx.x; q < l.words[r]; q += gridDim.x * 256LL) l.p[r][q] = 0;
 }
 
-// The status goes to the host by a kernel's own stores into the pinned mirror: a copy would wait for
+// Small results go to the host by a kernel's own stores into a pinned mirror: a copy would wait for
 // the copy engine to take over from the kernels.
-__global__ void __launch_bounds__(32) k_status_out(const unsigned int *d, volatile unsigned int *h) {
+__global__ void __launch_bounds__(kWordsOut / 4) k_words_out(const unsigned int *d, volatile unsigned int *h, int n) {
   if (!after_previous()) return;
-  static_assert(sizeof(Status) % 4 == 0 && sizeof(Status) / 4 <= 32, "one word a lane");
-  if (threadIdx.x < sizeof(Status) / 4) h[threadIdx.x] = d[threadIdx.x];
+  if ((int)threadIdx.x < n) h[threadIdx.x] = d[threadIdx.x];
+}
+
+int words_out(mic_ctx *ctx, const void *dev, void *host, size_t bytes) {
+  if (bytes % 4 || bytes > kWordsOut) return MIC_ERR_ARG;
+  {
+    MIC_KERNEL(ctx, "k_words_out");
+    launch_after(k_words_out, 1, (unsigned)(kWordsOut / 4), 0, ctx->stream, static_cast<const unsigned int *>(dev),
+                 static_cast<volatile unsigned int *>(host), (int)(bytes / 4));
+  }
+  MIC_CUDA_TRY(cudaGetLastError());
+  return MIC_OK;
 }
 }  // namespace
 
@@ -784,13 +799,10 @@ int mic_clear(mic_ctx *ctx, const mic_clear_list &l) {
   return MIC_OK;
 }
 
+int mic_words_out(mic_ctx *ctx, const void *dev, size_t bytes) { return words_out(ctx, dev, ctx->h_words, bytes); }
+
 int mic_fetch_status(mic_ctx *ctx) {
-  {
-    MIC_KERNEL(ctx, "k_status_out");
-    launch_after(k_status_out, 1, 32, 0, ctx->stream, reinterpret_cast<const unsigned int *>(ctx->d_status),
-                 reinterpret_cast<volatile unsigned int *>(ctx->h_status));
-  }
-  MIC_CUDA_TRY(cudaGetLastError());
+  if (const int e = words_out(ctx, ctx->d_status, ctx->h_status, sizeof(Status))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return MIC_OK;
 }

@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <iterator>
 #include <new>
 #include <vector>
@@ -1249,9 +1250,10 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
     if ((e = solve_launches(ctx, pl, B, sys, out))) return e;
   }
   MIC_CUDA_TRY(cudaGetLastError());
-  int h[kInfo];
-  MIC_CUDA_TRY(cudaMemcpyAsync(h, B.info, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+  if ((e = mic_words_out(ctx, B.info, sizeof(int) * kInfo))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  int h[kInfo];
+  memcpy(h, ctx->h_words, sizeof(h));
   S.factored = 1;
   S.kl = h[2];
   S.ku = h[3];

@@ -133,68 +133,96 @@ __global__ void k_nss_invariants(Params P, GridFields g) {
 
 // limitDisplacementTimestep candidates: min over nodes (order-preserving bits; NaN candidates
 // never win, as the reference's `dt > dt1` test), and max |rhodot| over non-NaN entries
+__global__ void __launch_bounds__(32) k_limit_start(unsigned long long *d) {
+  if (!after_previous()) return;
+  if (threadIdx.x < 3) d[threadIdx.x] = threadIdx.x == 0 ? 0x7FFFFFFFFFFFFFFFULL : 0ULL;
+}
+
 __global__ void k_limit_dt(Params P, GridFields g, double factor, unsigned long long *mins, unsigned long long *maxr,
                            int *nonnan) {
   if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
-  if (k >= (int64_t)NX * NY) return;
-  const int ix = (int)(k % NX), jy = (int)(k / NX);
-  long long best = LLONG_MAX;
+  long long best = LLONG_MAX, mr = -1;  // mr: no non-NaN |rhodot|
   auto take = [&](double c) {
     if (!nan_bits(dbits(c))) best = min(best, ordered_bits(c));
   };
-  double dx, dy;
-  if (ix == 0) dx = P.x[1] - P.x[0];
-  else if (ix == NX - 1) dx = P.x[NX - 1] - P.x[NX - 2];
-  else {
-    const double dx1 = P.x[ix + 1] - P.x[ix], dx2 = P.x[ix] - P.x[ix - 1];
-    dx = (dx1 <= dx2) ? dx1 : dx2;
+  if (k < (int64_t)NX * NY) {
+    const int ix = (int)(k % NX), jy = (int)(k / NX);
+    double dx, dy;
+    if (ix == 0) dx = P.x[1] - P.x[0];
+    else if (ix == NX - 1) dx = P.x[NX - 1] - P.x[NX - 2];
+    else {
+      const double dx1 = P.x[ix + 1] - P.x[ix], dx2 = P.x[ix] - P.x[ix - 1];
+      dx = (dx1 <= dx2) ? dx1 : dx2;
+    }
+    if (g.vx[k] != 0.0) take(M(D(dx, fabs(g.vx[k])), factor));
+    if (jy == 0) dy = P.y[1] - P.y[0];
+    else if (jy == NY - 1) dy = P.y[NY - 1] - P.y[NY - 2];
+    else {
+      const double dy1 = P.y[jy + 1] - P.y[jy], dy2 = P.y[jy] - P.y[jy - 1];
+      dy = (dy1 <= dy2) ? dy1 : dy2;
+    }
+    if (g.vy[k] != 0.0) take(M(D(dy, fabs(g.vy[k])), factor));
+    const double rd = g.rhodot[k];
+    if (rd != 0.0) take(fabs(D(M(0.01, g.rho[k]), rd)));
+    if (!nan_bits(dbits(rd))) mr = nonneg_bits(fabs(rd));
   }
-  if (g.vx[k] != 0.0) take(M(D(dx, fabs(g.vx[k])), factor));
-  if (jy == 0) dy = P.y[1] - P.y[0];
-  else if (jy == NY - 1) dy = P.y[NY - 1] - P.y[NY - 2];
-  else {
-    const double dy1 = P.y[jy + 1] - P.y[jy], dy2 = P.y[jy] - P.y[jy - 1];
-    dy = (dy1 <= dy2) ? dy1 : dy2;
+  for (int o = 16; o > 0; o >>= 1) {
+    best = min(best, __shfl_down_sync(0xffffffffu, best, o));
+    mr = max(mr, __shfl_down_sync(0xffffffffu, mr, o));
   }
-  if (g.vy[k] != 0.0) take(M(D(dy, fabs(g.vy[k])), factor));
-  const double rd = g.rhodot[k];
-  if (rd != 0.0) take(fabs(D(M(0.01, g.rho[k]), rd)));
+  if ((threadIdx.x & 31) != 0) return;
   if (best != LLONG_MAX) atomicMin(reinterpret_cast<long long *>(mins), best);
-  if (!nan_bits(dbits(rd))) {
-    atomicMax(maxr, (unsigned long long)nonneg_bits(fabs(rd)));
+  if (mr >= 0) {
+    atomicMax(maxr, (unsigned long long)mr);
     *nonnan = 1;
   }
 }
 
-__global__ void k_retrieve(const double *__restrict__ S, int64_t nn, double Kcont, double *p, double *vx,
-                           double *vy) {
-  if (!after_previous()) return;
-  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= nn) return;
-  p[k] = M(S[3 * k + 2], Kcont);
-  vx[k] = S[3 * k + 0];
-  vy[k] = S[3 * k + 1];
-}
-
-// dx-weighted mean pressure of row 1 in the reference's order (retrieveSolutions.c:52-62)
-__global__ void k_pressure_mean(Params P, const double *p, double *pm) {
-  if (!after_previous()) return;
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// term(0) + .. + term(n - 1) in this order, on thread 0.  The sums of retrieveSolutions and
+// nusseltNumber are bound by their chain of additions; the terms, a division each, are formed by
+// all threads of the block before it (129 columns: 115 us with one thread forming and adding).
+template <class F>
+__device__ __forceinline__ double ordered_sum(int n, F term) {
+  __shared__ double t[256];
   double s = 0.0;
-  for (int i = 1; i < P.NX; ++i) {
-    const double dx = S(P.x[i], P.x[i - 1]);
-    s = A(s, D(M(p[P.NX + i], dx), P.LX));
+  for (int c0 = 0; c0 < n; c0 += blockDim.x) {
+    const int m = min((int)blockDim.x, n - c0);
+    if ((int)threadIdx.x < m) t[threadIdx.x] = term(c0 + (int)threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int q = 0; q < m; ++q) s = A(s, t[q]);
+    }
+    __syncthreads();
   }
-  *pm = s;
+  return s;
 }
 
-__global__ void k_pressure_shift(Params P, double *p, const double *pm) {
+// retrieveSolutions: pressures scaled, less the dx-weighted mean pressure of row 1 in the
+// reference's order (retrieveSolutions.c:52-62) off the first row and column.  Every block forms the
+// mean for itself (one wave of blocks), which saves two launches and a second pass.  GB300, 129 x 33
+// nodes: 13 us for what were three kernels of 129.
+__global__ void __launch_bounds__(256) k_retrieve(Params P, const double *__restrict__ sol, double Kcont,
+                                                  double *__restrict__ p, double *__restrict__ vx,
+                                                  double *__restrict__ vy) {
   if (!after_previous()) return;
-  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= (int64_t)P.NX * P.NY) return;
-  if (k % P.NX >= 1 && k / P.NX >= 1) p[k] = S(p[k], *pm);
+  __shared__ double mean;
+  const double s = ordered_sum(P.NX - 1, [&](int q) {
+    const double dx = S(P.x[q + 1], P.x[q]);
+    return D(M(M(sol[3 * (int64_t)(P.NX + q + 1) + 2], Kcont), dx), P.LX);
+  });
+  if (threadIdx.x == 0) mean = s;
+  __syncthreads();
+  const int64_t nn = (int64_t)P.NX * P.NY;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x) {
+    double v = M(sol[3 * k + 2], Kcont);
+    if (k % P.NX >= 1 && k >= P.NX) v = S(v, mean);
+    p[k] = v;
+    vx[k] = sol[3 * k + 0];
+    vy[k] = sol[3 * k + 1];
+  }
 }
 
 }  // namespace
@@ -219,23 +247,23 @@ extern "C" int mic_nodal_stress_strain(mic_ctx *ctx, double dt, double gy) {
   return MIC_OK;
 }
 
-extern "C" int mic_limit_displacement_timestep(mic_ctx *ctx, double factor, double *dt) {
-  if (ctx && ctx->P.xper) return MIC_ERR_BC;  // grids periodic in x: the marker path only
-  if (!ctx || !dt) return MIC_ERR_ARG;
-  cudaSetDevice(ctx->device);
-  const int64_t nn = (int64_t)ctx->P.NX * ctx->P.NY;
+int mic_limit_launch(mic_ctx *ctx, double factor) {
   unsigned long long *d = reinterpret_cast<unsigned long long *>(ctx->red_buf + 24);  // min, max |rhodot|, flag
-  const unsigned long long init[3] = {0x7FFFFFFFFFFFFFFFULL, 0ULL, 0ULL};
-  MIC_CUDA_TRY(cudaMemcpyAsync(d, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
+  {
+    MIC_KERNEL(ctx, "k_limit_start");
+    launch_after(k_limit_start, 1, 32, 0, ctx->stream, d);
+  }
   {
     MIC_KERNEL(ctx, "k_limit_dt");
-    launch_after(k_limit_dt, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, grid_fields(ctx), factor, d, d + 1,
-                 reinterpret_cast<int *>(d + 2));
+    launch_after(k_limit_dt, grid_for((int64_t)ctx->P.NX * ctx->P.NY), kBlock, 0, ctx->stream, ctx->P,
+                 grid_fields(ctx), factor, d, d + 1, reinterpret_cast<int *>(d + 2));
   }
-  MIC_CUDA_TRY(cudaGetLastError());
+  return mic_words_out(ctx, d, 3 * sizeof(unsigned long long));
+}
+
+void mic_limit_result(const mic_ctx *ctx, double *dt) {
   unsigned long long h[3];
-  MIC_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  memcpy(h, ctx->h_words, sizeof(h));
   double t = *dt;
   if (h[0] != 0x7FFFFFFFFFFFFFFFULL) {  // smallest candidate, back from its ordered image
     long long b = (long long)h[0];
@@ -245,12 +273,21 @@ extern "C" int mic_limit_displacement_timestep(mic_ctx *ctx, double factor, doub
     if (t > c) t = c;
   }
   double mx;
-  if (*reinterpret_cast<int *>(&h[2]))
+  if ((int)h[2])
     memcpy(&mx, &h[1], sizeof(mx));
   else
     mx = INFINITY;  // no non-NaN rhodot: VecMax / VecMin give -inf / inf
   if (mx * t > 0.01) t = 0.01 / mx;
   *dt = t;
+}
+
+extern "C" int mic_limit_displacement_timestep(mic_ctx *ctx, double factor, double *dt) {
+  if (ctx && ctx->P.xper) return MIC_ERR_BC;  // grids periodic in x: the marker path only
+  if (!ctx || !dt) return MIC_ERR_ARG;
+  cudaSetDevice(ctx->device);
+  if (const int e = mic_limit_launch(ctx, factor)) return e;
+  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  mic_limit_result(ctx, dt);
   return MIC_OK;
 }
 
@@ -265,22 +302,14 @@ extern "C" int mic_retrieve_solutions(mic_ctx *ctx, const double *S, double Kcon
   // S = NULL: the solution mic_linear_solve left on the device
   if (S)
     MIC_CUDA_TRY(cudaMemcpyAsync(ctx->solution, S, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, ctx->stream));
-  double *pm = ctx->red_buf + 28;
   {
     MIC_KERNEL(ctx, "k_retrieve");
-    launch_after(k_retrieve, grid_for(nn), kBlock, 0, ctx->stream, ctx->solution, nn, Kcont, ctx->nodal[MIC_NF_P],
-                 ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY]);
-  }
-  {
-    MIC_KERNEL(ctx, "k_pressure_mean");
-    launch_after(k_pressure_mean, 1, 32, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_P], pm);
-  }
-  {
-    MIC_KERNEL(ctx, "k_pressure_shift");
-    launch_after(k_pressure_shift, grid_for(nn), kBlock, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_P], pm);
+    const int64_t full = grid_for(nn, 256), wave = 2 * (int64_t)sm_count(ctx);
+    launch_after(k_retrieve, (unsigned)(full < wave ? full : wave), 256, 0, ctx->stream, ctx->P, ctx->solution, Kcont,
+                 ctx->nodal[MIC_NF_P], ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY]);
   }
   MIC_CUDA_TRY(cudaGetLastError());
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // the caller may reuse S on return
+  if (S) MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // the caller may reuse S on return
   if (foundnan) *foundnan = 0;  // the reference checks for NaN only in its TEXTURE build
   return MIC_OK;
 }
@@ -290,19 +319,16 @@ extern "C" int mic_retrieve_solutions(mic_ctx *ctx, const double *S, double Kcon
 namespace {
 
 // nusseltNumber (post.c:5-46): the surface heat flux integral, summed in the reference's order by
-// one thread (NX - 1 terms), every operation an IEEE intrinsic
-__global__ void k_nusselt(Params P, const double *__restrict__ T, double dTbc, double *out) {
+// one block (NX - 1 terms), every operation an IEEE intrinsic
+__global__ void __launch_bounds__(256) k_nusselt(Params P, const double *__restrict__ T, double dTbc, double *out) {
   if (!after_previous()) return;
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const int NX = P.NX;
   const double dz = S(P.y[1], P.y[0]);
-  double integrand = 0.0;
-  for (int ix = 0; ix < NX - 1; ++ix) {
+  const double integrand = ordered_sum(NX - 1, [&](int ix) {
     const double dT = D(S(A(S(T[NX + ix], T[ix]), T[NX + ix + 1]), T[ix + 1]), 2.0);
-    const double dx = S(P.x[ix + 1], P.x[ix]);
-    integrand = A(integrand, M(D(dT, dz), dx));
-  }
-  out[0] = M(D(D(P.LY, P.LX), dTbc), integrand);
+    return M(D(dT, dz), S(P.x[ix + 1], P.x[ix]));
+  });
+  if (threadIdx.x == 0) out[0] = M(D(D(P.LY, P.LX), dTbc), integrand);
 }
 
 // rmsVelocity (post.c:49-92): one term per cell, summed by a fixed tree (the reference sums the
@@ -340,18 +366,33 @@ __global__ void k_vrms_final(Params P, const double *__restrict__ part, int npar
 
 }  // namespace
 
+int mic_diagnostics_launch(mic_ctx *ctx, double dTbc, bool nusselt, bool vrms) {
+  double *d = ctx->red_buf + 40;  // Nusselt number, rms velocity
+  if (nusselt) {
+    MIC_KERNEL(ctx, "k_nusselt");
+    launch_after(k_nusselt, 1, 256, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_THIST], dTbc, d);
+  }
+  if (vrms) {
+    constexpr int kParts = 64;
+    double *part = ctx->red_buf + 64;
+    {
+      MIC_KERNEL(ctx, "k_vrms_partial");
+      launch_after(k_vrms_partial, kParts, 256, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY],
+                   part);
+    }
+    MIC_KERNEL(ctx, "k_vrms_final");
+    launch_after(k_vrms_final, 1, 32, 0, ctx->stream, ctx->P, part, kParts, d + 1);
+  }
+  return mic_words_out(ctx, d, 2 * sizeof(double));
+}
+
 extern "C" int mic_nusselt_number(mic_ctx *ctx, double bottom_T, double top_T, double *Nu) {
   if (ctx && ctx->P.xper) return MIC_ERR_BC;  // grids periodic in x: the marker path only
   if (!ctx || !Nu) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
-  double *d = ctx->red_buf + 40;
-  {
-    MIC_KERNEL(ctx, "k_nusselt");
-    launch_after(k_nusselt, 1, 32, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_THIST], bottom_T - top_T, d);
-  }
-  MIC_CUDA_TRY(cudaGetLastError());
-  MIC_CUDA_TRY(cudaMemcpyAsync(Nu, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  if (const int e = mic_diagnostics_launch(ctx, bottom_T - top_T, true, false)) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  *Nu = ctx->h_words[0];
   return MIC_OK;
 }
 
@@ -359,19 +400,8 @@ extern "C" int mic_rms_velocity(mic_ctx *ctx, double *vrms) {
   if (ctx && ctx->P.xper) return MIC_ERR_BC;  // grids periodic in x: the marker path only
   if (!ctx || !vrms) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
-  constexpr int kParts = 64;
-  double *part = ctx->red_buf + 64, *d = ctx->red_buf + 41;
-  {
-    MIC_KERNEL(ctx, "k_vrms_partial");
-    launch_after(k_vrms_partial, kParts, 256, 0, ctx->stream, ctx->P, ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY],
-                 part);
-  }
-  {
-    MIC_KERNEL(ctx, "k_vrms_final");
-    launch_after(k_vrms_final, 1, 32, 0, ctx->stream, ctx->P, part, kParts, d);
-  }
-  MIC_CUDA_TRY(cudaGetLastError());
-  MIC_CUDA_TRY(cudaMemcpyAsync(vrms, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  if (const int e = mic_diagnostics_launch(ctx, 0.0, false, true)) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  *vrms = ctx->h_words[1];
   return MIC_OK;
 }

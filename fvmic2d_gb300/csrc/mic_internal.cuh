@@ -51,6 +51,8 @@ struct Status {
   double residual;                  // the strain-rate residual's sum over the area
 };
 
+constexpr size_t kWordsOut = 512;  // bytes of a context's pinned buffer for small results
+
 // Composite creep (law 7) settings and per-pass counters
 struct CreepConfig {
   int mode;             // 0: exact Newton; 1: surrogate guess + polish + exact fallback
@@ -132,6 +134,8 @@ struct mic_ctx {
   mic_system_store sys[2];    // assembled systems: 0 Stokes (vep_system.c), 1 thermal
   void *sys_scratch;          // assembly scratch: geometry tables, scaled viscosities
   size_t sys_scratch_bytes;
+  int sys_held;               // a time step's call holds the geometry tables of its options
+  double sys_scalars[3];      // the tables' plate depth at LX and slab velocity
   void *lu_buf;               // the direct solver's storage (grown on demand)
   size_t lu_bytes;
   cudaStream_t lu_chain;      // the solver's chain of panels (high priority); its hand-offs with
@@ -171,6 +175,7 @@ struct mic_ctx {
   int red_cap;
   mic::Status *d_status;
   mic::Status *h_status;  // pinned mirror
+  double *h_words;        // pinned: small results on their way to the host (kWordsOut bytes)
   unsigned char *stage_aos;  // device staging for AoS transfers
   int64_t stage_cap;
   double residuals[100];
@@ -252,6 +257,17 @@ void mic_front_plan_free(mic_front_plan *plan);  // (mic_front_lu.cu)
 // step: also clears what the first pieces of a step add to (max_bits, the yield pass's results)
 int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out, bool step = false);
 int mic_fetch_status(mic_ctx *ctx);  // *d_status into *h_status; waits for the stream
+// up to kWordsOut bytes into h_words, without waiting
+int mic_words_out(mic_ctx *ctx, const void *dev, size_t bytes);
+// the pieces of a time step's calls whose results are read together: launches without a wait
+int mic_strain_launch(mic_ctx *ctx, double dt);
+int mic_residual_launch(mic_ctx *ctx);                     // into the status
+void mic_residual_store(mic_ctx *ctx, int iter, double *residual);  // from the mirror
+int mic_limit_launch(mic_ctx *ctx, double factor);         // into h_words
+void mic_limit_result(const mic_ctx *ctx, double *dt);
+int mic_diagnostics_launch(mic_ctx *ctx, double dTbc, bool nusselt, bool vrms);  // into h_words[0], [1]
+int mic_max_abs_sxx_launch(mic_ctx *ctx);                  // into the status
+int mic_prepare_system(mic_ctx *ctx, const mic_subduction_options *o);  // boundary tables, kept until released
 
 // Memory to be zeroed by one launch: a step's flags, maxima and digit counts lie apart, and a memset
 // each would also keep the kernels around it from overlapping (launch_after).  GB300: a step's nine

@@ -2137,6 +2137,8 @@ extern "C" int mic_max_marker_T(mic_ctx *ctx, double *maxT) {
   return run_max(ctx, C_T, 0, maxT);
 }
 
+int mic_max_abs_sxx_launch(mic_ctx *ctx) { return run_max(ctx, C_SXX, 1, nullptr); }
+
 extern "C" int mic_max_abs_sxx(mic_ctx *ctx, double *v) {
   CHECK_CTX();
   return run_max(ctx, C_SXX, 1, v);
@@ -2247,6 +2249,8 @@ static int strain_launch(mic_ctx *ctx, double dt, bool keep = false, bool step =
   return solo_pass(ctx, BP_STRAIN, J, tuned_block(ctx, TU_STRAIN), "k_strain_pressure");
 }
 
+int mic_strain_launch(mic_ctx *ctx, double dt) { return strain_launch(ctx, dt); }
+
 extern "C" int mic_update_marker_strain_pressure(mic_ctx *ctx, double dt) {
   CHECK_CTX();
   int e = strain_launch(ctx, dt);
@@ -2279,14 +2283,20 @@ static int residual_launch(mic_ctx *ctx, int iter, double *res_dev, cudaStream_t
   return MIC_OK;
 }
 
+int mic_residual_launch(mic_ctx *ctx) { return residual_launch(ctx, 0, &ctx->d_status->residual); }
+
+void mic_residual_store(mic_ctx *ctx, int iter, double *residual) {
+  const double s = ctx->h_status->residual / (ctx->P.LX * ctx->P.LY);
+  ctx->residuals[iter % 100] = s;
+  if (residual) *residual = s;
+}
+
 extern "C" int mic_update_global_strain_rate_residual(mic_ctx *ctx, int iter, double *residual) {
   CHECK_CTX();
   if (iter < 0) return MIC_ERR_ARG;
   int e = residual_launch(ctx, iter, &ctx->d_status->residual);
   if (e || (e = mic_fetch_status(ctx))) return e;
-  const double s = ctx->h_status->residual / (ctx->P.LX * ctx->P.LY);
-  ctx->residuals[iter % 100] = s;
-  if (residual) *residual = s;
+  mic_residual_store(ctx, iter, residual);
   return MIC_OK;
 }
 

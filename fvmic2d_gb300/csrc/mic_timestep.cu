@@ -3,12 +3,13 @@
 // Stokes solve, the sub-grid stress and stress updates, the thermal solve (repeated with a
 // shorter step when the temperature changes too much) and the marker advection.  Every stage is
 // the library's own entry point for the reference routine of the same name; the linear systems
-// are assembled and solved on the device (mic_systems.cu, mic_band_lu.cu).  Nodal fields and
+// are assembled and solved on the device (mic_systems.cu, mic_front_lu.cu).  Nodal fields and
 // markers stay on the device; only scalars (time steps, flags, maxima) come back to the host,
 // where main_subduction's control flow runs.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <thread>
 #include <vector>
 
@@ -68,12 +69,11 @@ int max_temp_change(mic_ctx *ctx, double *out) {
     launch_after(k_temp_change, kParts, 256, 0, ctx->stream, ctx->nodal[MIC_NF_THIST], ctx->nodal[MIC_NF_LASTT], nn,
                  part);
   }
-  double h[kParts];
-  MIC_CUDA_TRY(cudaMemcpyAsync(h, part, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+  if (const int e = mic_words_out(ctx, part, sizeof(double) * kParts)) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   double m = 0.0;
-  for (double v : h)
-    if (v > m) m = v;
+  for (int k = 0; k < kParts; ++k)
+    if (ctx->h_words[k] > m) m = ctx->h_words[k];
   *out = m;
   return MIC_OK;
 }
@@ -142,6 +142,12 @@ extern "C" int mic_subduction_timestep(mic_ctx *ctx, const mic_timestep_options 
     return MIC_OK;
   }
   // main:292-362: plasticity iterations
+  struct Hold {  // the boundary tables of this step's options, until the call ends
+    mic_ctx *c;
+    ~Hold() { c->sys_held = 0; }
+  } hold{ctx};
+  MIC_TRY(mic_prepare_system(ctx, &o->sub));
+  ctx->sys_held = 1;
   double displacementdt = o->dtMax;
   int isYielding = 1, converged = 0, iPlastic = 0;
   const double gy = o->sub.gy;
@@ -162,11 +168,17 @@ extern "C" int mic_subduction_timestep(mic_ctx *ctx, const mic_timestep_options 
     MIC_TRY(mic_retrieve_solutions(ctx, nullptr, rep->Kcont, &fn));
     if (fn) return MIC_ERR_NAN;
     MIC_TRY(mic_nodal_stress_strain(ctx, displacementdt, gy));
-    MIC_TRY(mic_update_marker_strain_pressure(ctx, displacementdt));
-    MIC_TRY(mic_update_global_strain_rate_residual(ctx, iPlastic, &rep->residual));
+    // (updateMarkerStrainPressure, the residual and the step limit: one wait for all three)
+    MIC_TRY(mic_strain_launch(ctx, displacementdt));
+    MIC_TRY(mic_residual_launch(ctx));
+    MIC_TRY(mic_limit_launch(ctx, o->displacementStepLimit));
+    MIC_TRY(mic_fetch_status(ctx));
+    if (ctx->h_status->bad_cell) return MIC_ERR_CELL;
+    if (ctx->h_status->nan_residual) return MIC_ERR_NAN;
+    mic_residual_store(ctx, iPlastic, &rep->residual);
     MIC_TRY(mic_check_convergence(ctx, 1e-16, 1e-1, iPlastic, &converged));
     const double lastdt = displacementdt;
-    MIC_TRY(mic_limit_displacement_timestep(ctx, o->displacementStepLimit, &displacementdt));
+    mic_limit_result(ctx, &displacementdt);
     if (displacementdt != lastdt) converged = 0;
     ++iPlastic;
   }
@@ -198,11 +210,13 @@ extern "C" int mic_subduction_timestep(mic_ctx *ctx, const mic_timestep_options 
   // main:409, 435: sub-grid temperature changes with the new temperature, the diagnostics,
   // advection
   MIC_TRY(mic_subgrid_temperature_changes(ctx, dt));
-  MIC_TRY(mic_nusselt_number(ctx, o->thermalBCBottomValue, o->sub.thermalBCTopValue, &rep->nusselt));
-  MIC_TRY(mic_rms_velocity(ctx, &rep->vrms));
+  MIC_TRY(mic_diagnostics_launch(ctx, o->thermalBCBottomValue - o->sub.thermalBCTopValue, true, true));
   MIC_TRY(mic_advect_markers_rk(ctx, dt));
-  MIC_TRY(mic_max_abs_sxx(ctx, &rep->max_abs_sxx));
-  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  MIC_TRY(mic_max_abs_sxx_launch(ctx));
+  MIC_TRY(mic_fetch_status(ctx));
+  rep->nusselt = ctx->h_words[0];
+  rep->vrms = ctx->h_words[1];
+  memcpy(&rep->max_abs_sxx, &ctx->h_status->max_bits, sizeof(double));
   return MIC_OK;
 }
 
