@@ -66,12 +66,10 @@ struct Front {
 // info[2], info[3]: lower and upper band widths of the matrix in grid order (mic_system_band)
 constexpr int kInfo = 4;
 
-__device__ __forceinline__ int64_t bmap(int64_t r, int dof, int NX, int NY, int transpose) {
-  if (!transpose) return r;
-  const int64_t node = r / dof;
-  const int d = (int)(r % dof);
-  const int ix = (int)(node % NX), jy = (int)(node / NX);
-  return ((int64_t)ix * NY + jy) * dof + d;
+__device__ __forceinline__ int bmap(unsigned r, unsigned dof, unsigned NX, unsigned NY, int transpose) {
+  if (!transpose) return (int)r;
+  const unsigned node = r / dof, d = r - node * dof, jy = node / NX, ix = node - jy * NX;
+  return (int)((ix * NY + jy) * dof + d);
 }
 
 // band widths with the nodes numbered along the shorter grid side (reported, and the size limit)
@@ -80,11 +78,12 @@ __global__ void k_band_width(const int *__restrict__ cnt, const int *__restrict_
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int lo = 0, up = 0;
   if (r < n) {
-    const int64_t bi = bmap(r, dof, NX, NY, transpose);
-    for (int k = 0; k < cnt[r]; ++k) {
-      const int64_t bj = bmap(col[r * width + k], dof, NX, NY, transpose);
-      lo = max(lo, (int)(bi - bj));
-      up = max(up, (int)(bj - bi));
+    const int bi = bmap((unsigned)r, dof, NX, NY, transpose), count = cnt[r];
+#pragma unroll 4
+    for (int k = 0; k < count; ++k) {
+      const int bj = bmap((unsigned)col[r * width + k], dof, NX, NY, transpose);
+      lo = max(lo, bi - bj);
+      up = max(up, bj - bi);
     }
   }
   lo = __reduce_max_sync(0xffffffffu, lo);
@@ -171,6 +170,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
                                                               const int *__restrict__ act, SystemRows sys,
                                                               const double *__restrict__ Fin, double *F, double *U,
                                                               int *info) {
+  if (!after_previous()) return;
   constexpr int kSmallWarps = kSmallThreads / 32;
   extern __shared__ double A[];
   __shared__ int2 red[32];
@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
 __global__ void __launch_bounds__(256) k_front_gather(const Front *__restrict__ fr, int first,
                                                      const int *__restrict__ tab, int *act,
                                                      const double *__restrict__ Fin, double *F) {
+  if (!after_previous()) return;
   const Front q = fr[first + blockIdx.x];
   const int r = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= q.R) return;
@@ -317,6 +318,7 @@ template <int NB>
 __global__ void __launch_bounds__(kPanelThreads, 2)
     k_front_panel(const Front *__restrict__ fr, int first, int k0, int turn, const double *__restrict__ F, double *U,
                   double *Lb, int *act, const int *__restrict__ tab, int *info) {
+  if (!after_previous()) return;
   extern __shared__ double S[];
   __shared__ int2 red[32];
   __shared__ double s_rcp;
@@ -486,6 +488,7 @@ template <int NB>
 __global__ void __launch_bounds__(256) k_front_solve(const Front *__restrict__ fr, int first, int k0, int turn,
                                                     const double *__restrict__ F, double *U,
                                                     const double *__restrict__ Lb, const int *__restrict__ act) {
+  if (!after_previous()) return;
   constexpr int TC = 64;
   __shared__ double Us[NB][TC + 1];
   __shared__ double L11[NB][NB + 1];
@@ -519,6 +522,7 @@ template <int NB, int TR, int TC, bool SOLVE>
 __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
     k_front_update(const Front *__restrict__ fr, int first, int k0, int turn, int coff, int clen, double *F, double *U,
                    const double *__restrict__ Lb, const int *__restrict__ act) {
+  if (!after_previous()) return;
   constexpr int RT = TR / 16, CT = TC / 16;  // a thread's rows and columns
   __shared__ double Us[NB][TC + 1];
   __shared__ double Ls[TR][NB + 1];
@@ -611,6 +615,7 @@ __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
 __global__ void __launch_bounds__(256) k_front_border(const Front *__restrict__ fr, int first,
                                                      const int *__restrict__ tab, double *U,
                                                      const double *__restrict__ x) {
+  if (!after_previous()) return;
   const Front q = fr[first + blockIdx.x];
   const int r = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= q.P) return;
@@ -629,6 +634,7 @@ __global__ void __launch_bounds__(256) k_front_border(const Front *__restrict__ 
 __global__ void __launch_bounds__(256) k_front_back_small(const Front *__restrict__ fr, int first,
                                                           const int *__restrict__ tab, const double *__restrict__ U,
                                                           double *x, int border) {
+  if (!after_previous()) return;
   extern __shared__ double xs[];  // the border's unknowns, behind the pivots' places
   __shared__ double acc[32];
   __shared__ double Ud[32][33];
@@ -674,6 +680,7 @@ __global__ void __launch_bounds__(256) k_front_back_small(const Front *__restric
 __global__ void __launch_bounds__(1024) k_front_back(const Front *__restrict__ fr, int first,
                                                     const int *__restrict__ tab, const double *__restrict__ U,
                                                     double *x, int border) {
+  if (!after_previous()) return;
   extern __shared__ double xs[];  // the front's unknowns: pivots, then (border) the border's
   __shared__ double Ud[2][32][33], Un[32][33];  // triangles; the next rows' part on the unknowns being solved
   __shared__ double part[32][32], comb[4][32], rhs[2][32], rd[2][32];
@@ -971,9 +978,8 @@ template <int NB, int TR, int TC, bool SOLVE>
 void update(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, double *F, int k0, int turn,
             int rows, int coff, int cols, cudaStream_t st) {
   MIC_KERNEL_ON(ctx, "k_front_update", st);
-  k_front_update<NB, TR, TC, SOLVE>
-      <<<dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC), kUpdateBlocks, 0, st>>>(
-          pl.d_fronts, L.first, k0, turn, coff, cols, F, B.U, B.Lb + turn * pl.nL, B.act);
+  launch_after(k_front_update<NB, TR, TC, SOLVE>, dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC),
+               kUpdateBlocks, 0, st, pl.d_fronts, L.first, k0, turn, coff, cols, F, B.U, B.Lb + turn * pl.nL, B.act);
 }
 
 // One level in panels.  The chain (panel, then its update of the next panel's columns) runs on the
@@ -991,8 +997,8 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     const int threads = rows <= 256 ? 256 : kPanelThreads;
     {
       MIC_KERNEL_ON(ctx, "k_front_panel", chain);
-      k_front_panel<NB><<<L.count, threads, (size_t)rows * ((NB + 1) * sizeof(double) + kPanelBytes), chain>>>(
-          pl.d_fronts, L.first, k0, turn, F, B.U, B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
+      launch_after(k_front_panel<NB>, L.count, threads, (size_t)rows * ((NB + 1) * sizeof(double) + kPanelBytes),
+                   chain, pl.d_fronts, L.first, k0, turn, F, B.U, B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
     }
     // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
@@ -1030,8 +1036,8 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     if (best == c64 || best == c128) {
       {
         MIC_KERNEL_ON(ctx, "k_front_solve", st);
-        k_front_solve<NB><<<dim3(L.count, (cols + 63) / 64), 256, 0, st>>>(pl.d_fronts, L.first, k0, turn, F, B.U,
-                                                                         B.Lb + turn * pl.nL, B.act);
+        launch_after(k_front_solve<NB>, dim3(L.count, (cols + 63) / 64), 256, 0, st, pl.d_fronts, L.first, k0, turn,
+                     F, B.U, B.Lb + turn * pl.nL, B.act);
       }
       if (best == c64)
         update<NB, 64, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
@@ -1050,9 +1056,22 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
   return MIC_OK;
 }
 
-// every launch of one solve, on the context's stream
+void band_width(mic_ctx *ctx, const SystemRows &sys, int64_t n, int *bw, cudaStream_t st) {
+  MIC_KERNEL_ON(ctx, "k_band_width", st);
+  k_band_width<<<grid_for(n), kBlock, 0, st>>>(sys.cnt, sys.col, sys.width, n, sys.dof, sys.NX, sys.NY,
+                                               sys.NX > sys.NY ? 1 : 0, bw);
+}
+
+// every launch of one solve, on the context's stream; the band widths, which only the caller asks
+// for, beside the lowest levels
 int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, const SystemRows &sys, double *x) {
   const int nl = (int)pl.levels.size();
+  MIC_CUDA_TRY(cudaMemsetAsync(B.info, 0x7f, sizeof(int), ctx->stream));
+  MIC_CUDA_TRY(cudaMemsetAsync(B.info + 1, 0, sizeof(int) * (kInfo - 1), ctx->stream));
+  MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], ctx->stream));
+  MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->lu_chain, ctx->lu_ev[0], 0));
+  band_width(ctx, sys, (int64_t)sys.dof * sys.NX * sys.NY, B.info + 2, ctx->lu_chain);
+  MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[1], ctx->lu_chain));
   for (int l = nl - 1; l >= 0; --l) {
     const Level &L = pl.levels[l];
     const double *Fin = B.F[(l + 1) & 1];
@@ -1060,17 +1079,17 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
       MIC_KERNEL(ctx, "k_front_small");
       // (more warps where one front fills an SM's shared memory)
       if (L.smem_small > kMaxSmem / 2)
-        k_front_small<512><<<L.count, 512, L.smem_small, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act, sys,
-                                                                        Fin, B.F[l & 1], B.U, B.info);
+        launch_after(k_front_small<512>, L.count, 512, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
+                     B.act, sys, Fin, B.F[l & 1], B.U, B.info);
       else
-        k_front_small<256><<<L.count, 256, L.smem_small, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act, sys,
-                                                                        Fin, B.F[l & 1], B.U, B.info);
+        launch_after(k_front_small<256>, L.count, 256, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
+                     B.act, sys, Fin, B.F[l & 1], B.U, B.info);
       continue;
     }
     {
       MIC_KERNEL(ctx, "k_front_gather");
-      k_front_gather<<<dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.act,
-                                                                              Fin, B.F[l & 1]);
+      launch_after(k_front_gather, dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first,
+                   pl.d_tab, B.act, Fin, B.F[l & 1]);
     }
     int e = MIC_OK;
     switch (panel_columns(L.maxR)) {
@@ -1086,17 +1105,20 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     const bool apart = L.maxC > L.maxP + 1 && ((int64_t)L.maxP * (L.maxC - L.maxP) > 8192 || L.maxC > 1024);
     if (apart) {
       MIC_KERNEL(ctx, "k_front_border");
-      k_front_border<<<dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x);
+      launch_after(k_front_border, dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first,
+                   pl.d_tab, B.U, x);
     }
     MIC_KERNEL(ctx, "k_front_back");
     const size_t smem = sizeof(double) * (apart ? L.maxP : L.maxC);
     if (L.maxP <= 32)
-      k_front_back_small<<<L.count, L.maxP <= 16 ? 128 : 256, smem, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U,
-                                                                                  x, apart ? 0 : 1);
+      launch_after(k_front_back_small, L.count,
+                   L.maxP <= 16 ? 128 : 256, smem, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.U, x, apart ? 0 : 1);
     else
-      k_front_back<<<L.count, L.maxP <= 64 ? 256 : 1024, smem, ctx->stream>>>(pl.d_fronts, L.first, pl.d_tab, B.U, x,
-                                                                             apart ? 0 : 1);
+      launch_after(k_front_back, L.count,
+                   L.maxP <= 64 ? 256 : 1024, smem, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.U, x, apart ? 0 : 1);
   }
+  // (the band widths where no level used the second stream; else an event of this stream by now)
+  MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->lu_ev[1], 0));
   return MIC_OK;
 }
 
@@ -1169,12 +1191,8 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
   const int NX = ctx->P.NX, NY = ctx->P.NY;
   const int dof = which == 0 ? 3 : 1;
   const int64_t n = S.n;
-  const int transpose = NX > NY ? 1 : 0;
   int e;
-  auto band_width = [&](int *bw) {
-    MIC_KERNEL(ctx, "k_band_width");
-    k_band_width<<<grid_for(n), kBlock, 0, ctx->stream>>>(S.cnt, S.col, S.width, n, dof, NX, NY, transpose, bw);
-  };
+  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY};
   // the solver's size limit, a band of 1,016 below the diagonal: only a grid whose shorter side
   // could reach it has its band measured first
   constexpr int kMaxBand = 1016;
@@ -1182,7 +1200,7 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
     if ((e = ensure_lu(ctx, 4096))) return e;
     int *bw = static_cast<int *>(ctx->lu_buf), h[2];
     MIC_CUDA_TRY(cudaMemsetAsync(bw, 0, 2 * sizeof(int), ctx->stream));
-    band_width(bw);
+    band_width(ctx, sys, n, bw, ctx->stream);
     MIC_CUDA_TRY(cudaMemcpyAsync(h, bw, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     if (h[0] > kMaxBand) return MIC_ERR_SOLVE;
@@ -1214,10 +1232,6 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
   B.U = carve<double>(p, pl.nU);
   B.Lb = carve<double>(p, 2 * pl.nL);
   B.act = carve<int>(p, pl.nAct);
-  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY};
-  MIC_CUDA_TRY(cudaMemsetAsync(B.info, 0x7f, sizeof(int), ctx->stream));
-  MIC_CUDA_TRY(cudaMemsetAsync(B.info + 1, 0, sizeof(int) * (kInfo - 1), ctx->stream));
-  band_width(B.info + 2);
   // The launches are the same for every solve of a system: captured once as a graph and replayed,
   // so host launch cost stays off the chain of levels.  Not while launches are being timed one by
   // one.
