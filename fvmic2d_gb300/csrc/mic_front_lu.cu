@@ -27,10 +27,10 @@
 //
 // Two forms of a level, chosen by estimated time (plan_level):
 //   small  the front in shared memory, one block per front, unblocked (k_front_small);
-//   large  the front in global memory, panels of NB columns: one block per front factors a panel
-//          in shared memory (k_front_panel), then the trailing tiles of every front are updated,
-//          each block forming its own piece of U12 (k_front_update): the next panel's columns
-//          first, the rest beside the next panel's factorisation.
+//   large  the front in global memory, panels of 16 columns: a block per front, or a cluster of
+//          blocks, factors a panel in shared memory (k_front_panel, k_front_panel_cluster), then
+//          the trailing tiles of every front are updated, each block forming its own piece of U12
+//          (k_front_update): the next panel's columns first, the rest beside the next panel.
 // FP64 multiply-adds bound the updates (2 per SM and clock); the panels and the small fronts are
 // bound by the latency of their column steps.  One CUDA graph holds all launches of a solve.
 #include <algorithm>
@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(256) k_front_gather(const Front *__restrict__ 
 // compiler cannot tell a row from the pivot row).
 constexpr int kPanelThreads = 512;
 constexpr int kPanelBytes = 8;  // per row besides its values: its number, whether it is a pivot
+
 template <int NB>
 __global__ void __launch_bounds__(kPanelThreads, 2)
     k_front_panel(const Front *__restrict__ fr, int first, int k0, int turn, const double *__restrict__ F, double *U,
@@ -480,6 +481,256 @@ __device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB
     Us[k][c] = u[i];
     if (store && k < nb && c < cols) u_out[(int64_t)k * ldu + c] = u[i];
   }
+}
+
+// The same panel on a cluster of CL blocks, the rows shared out between them in runs: the FP64 pipes
+// of CL SMs update it.  Each block finds the best of its own rows; one warp brings that row up to
+// date and sends it to every block, whose barrier in shared memory counts the bytes; all blocks then
+// choose the same winner, form its reciprocal for themselves and have its row at hand.  One such
+// exchange a column (some 500 clocks; a barrier of the whole cluster around the stores takes 670),
+// beside which the other warps update the later columns.  Four places for the offers: a block may
+// be sent the second exchange of a column (no row of any block has a value that counts: each then
+// looks for its exact largest) and the first of the next while its warps still read the row before.
+// GB300, us a panel on one SM and on a cluster: 27 and 22 of 330 rows, 33 and 22 of 645, 70 and 33
+// of 1,290.
+constexpr int kOffers = 4;
+constexpr int kExchangeTries = 1 << 20;  // a wait of some 1 s at the very least
+struct PanelOffer {
+  double v[16];
+  long long row;  // number in the front's list; -1: the block has no row left
+};
+__device__ __forceinline__ unsigned shared_address(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned peer_address(unsigned mine, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(mine), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send_async(unsigned to, long long bits, unsigned bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to), "l"(bits),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool offers_here(unsigned bar, unsigned parity) {
+  unsigned ok = 0;
+  for (int n = 0; !ok && n < kExchangeTries; ++n)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  return ok != 0;
+}
+
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
+    k_front_panel_cluster(const Front *__restrict__ fr, int first, int k0, int turn, const double *__restrict__ F,
+                          double *U, double *Lb, int *act, const int *__restrict__ tab, int *info) {
+  if (!after_previous()) return;
+  constexpr int NB = 16;
+  extern __shared__ double S[];
+  __shared__ PanelOffer ex[kOffers][CL];
+  __shared__ __align__(8) unsigned long long bars[kOffers];
+  __shared__ int2 red[32];
+  __shared__ double s_rcp;
+  __shared__ int s_win, s_place;  // the last winner and the place of its offer
+  __shared__ int s_rare;          // the column's exchange is to be done again
+  __shared__ int piv[NB];         // the pivots so far, numbers in the list
+  const Front q = fr[first + blockIdx.x / CL];
+  if (k0 >= q.P) return;  // (the whole cluster)
+  constexpr int LD = NB + 1, RW = 32 / NB, BATCH = 8;
+  const unsigned rank = blockIdx.x % CL;
+  const int nb = min(NB, q.P - k0), all = q.R - k0, share = (all + CL - 1) / CL;
+  const int base = min((int)rank * share, all), m = min(share, all - base);
+  int *id = reinterpret_cast<int *>(S + (int64_t)share * LD), *used = id + share;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int *list = act + q.act + (int64_t)turn * q.R + k0 + base;
+  int *out = act + q.act + (int64_t)(1 - turn) * q.R + k0;
+  {
+    const int lc = lane % NB;
+    for (int r0 = warp * RW + lane / NB; r0 < m; r0 += nw * RW * BATCH) {
+      int k[BATCH];
+      double v[BATCH];
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) k[i] = r0 + i * nw * RW < m ? list[r0 + i * nw * RW] : -1;
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) v[i] = (k[i] >= 0 && lc < nb) ? F[q.f + (int64_t)k[i] * q.C + k0 + lc] : 0.0;
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i)
+        if (k[i] >= 0) {
+          S[(r0 + i * nw * RW) * LD + lc] = v[i];
+          if (lc == 0) {
+            id[r0 + i * nw * RW] = k[i];
+            used[r0 + i * nw * RW] = 0;
+          }
+        }
+    }
+  }
+  if (tid < kOffers)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&bars[tid])) : "memory");
+  for (int e = tid; e < kOffers * CL; e += nt) ex[e / CL][e % CL] = PanelOffer{};
+  if (tid == 0) s_win = s_place = s_rare = 0;
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  // every block of the cluster has come this far before one sends to another
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  int key = -1, who = -1;
+  for (int r = tid; r < m; r += nt) {
+    const int k = pivot_key(S[r * LD]);
+    if (who < 0 || k > key) {
+      key = k;
+      who = r;
+    }
+  }
+  const int G = (m + 31) / 32, workers = nw - 1, CS = max(1, workers / max(G, 1));
+  unsigned mine = 0;  // which of this thread's rows are pivots
+  int sent = 0;       // exchanges so far (the sending warp)
+  bool lost = false;  // one did not arrive in time: no more waits, the solve fails
+  // column c: row p of this block (-1: none), its values from column c on in the lanes, to every
+  // block; the winner's place, reciprocal and number.  Rare: no value that counts in any block
+  const auto exchange = [&](int c, int p, double v) {
+    const int place = sent % kOffers;
+    const unsigned bar = shared_address(&bars[place]);
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                   "r"(CL * (int)sizeof(PanelOffer))
+                   : "memory");
+    __syncwarp();
+    const PanelOffer *slot = &ex[place][rank];
+    const unsigned from = shared_address(lane < NB ? (const void *)&slot->v[lane] : (const void *)&slot->row);
+    const long long bits = lane < NB ? dbits(v) : (long long)(p >= 0 ? base + p : -1);
+#pragma unroll
+    for (unsigned d = 0; d < CL; ++d)
+      if (lane <= NB) send_async(peer_address(from, d), bits, peer_address(bar, d));
+    if (!lost && !offers_here(bar, (sent / kOffers) & 1)) lost = true;
+    ++sent;
+    // the same choice in every block: the largest |value|, the first block's where they agree
+    long long top = -3;
+    int win = 0;
+#pragma unroll
+    for (int d = 0; d < CL; ++d) {
+      long long b = dbits(ex[place][d].v[c]) & 0x7fffffffffffffffLL;
+      if (b > 0x7ff0000000000000LL) b = -1;
+      if (ex[place][d].row < 0) b = -2;
+      if (b > top) {
+        top = b;
+        win = d;
+      }
+    }
+    if (lane == 0) {
+      const double w = ex[place][win].v[c];
+      s_rcp = pivot_rcp(w);
+      s_win = win;
+      s_place = place;
+      s_rare = (top >> 32) <= 0 && !s_rare;
+      piv[c] = (int)ex[place][win].row;
+      if (lost || (rank == 0 && !s_rare && (dbits(w) << 1) == 0)) atomicMin(&info[0], tab[q.col + k0 + c]);
+    }
+  };
+  for (int j = -1; j < nb; ++j) {
+    const double *pr = ex[s_place][s_win].v;  // the pivot row of column j
+    // phase 1 of step j (none before the first): multipliers, column j + 1
+    if (j >= 0) {
+      const double rcp = s_rcp;
+      const int p = piv[j] - base;
+      const bool more = j + 1 < nb;
+      key = -1;
+      who = -1;
+      const double pn = more ? pr[j + 1] : 0.0;
+      unsigned bit = 1;
+      for (int r = tid; r < m; r += nt, bit <<= 1) {
+        if (r == p) {
+          mine |= bit;
+          used[r] = 1;
+        }
+        if (mine & bit) continue;
+        double *row = S + r * LD;
+        const double aj = row[j], an = more ? row[j + 1] : 0.0, l = aj * rcp;
+        row[j] = l;
+        if (more) {
+          const double v = an - l * pn;
+          row[j + 1] = v;
+          const int k = pivot_key(v);
+          if (who < 0 || k > key) {
+            key = k;
+            who = r;
+          }
+        }
+      }
+    }
+    if (j + 1 == nb) break;
+    const int2 offer = warp_best(key, who);
+    if (lane == 0) red[warp] = offer;
+    __syncthreads();
+    // phase 2: the pivot of column j + 1 and its reciprocal; the columns after it
+    if (warp == nw - 1) {
+      const int2 e = lane < nw ? red[lane] : make_int2(-1, -1);
+      const int p = warp_best(e.x, e.y).y;
+      double v = 0.0;
+      if (p >= 0 && lane > j && lane < nb) {
+        v = S[p * LD + lane];
+        if (j >= 0 && lane > j + 1) v -= S[p * LD + j] * pr[lane];
+      }
+      asm volatile("bar.arrive 1, %0;" ::"r"(nt) : "memory");  // the row is read: the others may update it
+      exchange(j + 1, p, v);
+    } else {
+      asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+      if (j >= 0) {
+        for (int t = warp; t < G * CS; t += workers) {
+          const int r = (t % G) * 32 + lane;
+          if (r >= m || used[r]) continue;
+          double *row = S + r * LD;
+          const double l = row[j];
+          for (int c = j + 2 + t / G; c < nb; c += 4 * CS) {
+            double v[4], u[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int ci = c + i * CS;
+              v[i] = ci < nb ? row[ci] : 0.0;
+              u[i] = ci < nb ? pr[ci] : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (c + i * CS < nb) row[c + i * CS] = v[i] - l * u[i];
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (s_rare) {  // (the same in every block)
+      if (warp == nw - 1) {
+        int p = m > 0 ? pivot_rare(S + j + 1, LD, m, used) : -1;
+        if (p >= 0 && used[p]) p = -1;
+        exchange(j + 1, p, p >= 0 && lane > j && lane < nb ? S[p * LD + lane] : 0.0);
+      }
+      __syncthreads();
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < nb * NB; e += nt) {  // the block's pivots in order: U11 and the multipliers before it
+    const int k = e / NB, c = e % NB, r = piv[k] - base;
+    if (r < 0 || r >= m) continue;
+    const double v = c < nb ? S[r * LD + c] : 0.0;
+    if (c >= k && c < nb) U[q.u + (int64_t)(k0 + k) * q.C + k0 + c] = v;
+    Lb[q.lb + e] = c < k ? v : 0.0;
+    if (c == 0) out[k] = id[r];
+  }
+  {  // its other rows in their order behind all pivots
+    const int lc = lane % NB;
+    for (int r = warp * RW + lane / NB; r < m; r += nw * RW) {
+      if (used[r]) continue;
+      int pos = nb + base + r;
+#pragma unroll
+      for (int k = 0; k < NB; ++k) pos -= k < nb && piv[k] < base + r;
+      if (pos >= all) continue;  // (after a lost exchange)
+      Lb[q.lb + (int64_t)pos * NB + lc] = lc < nb ? S[r * LD + lc] : 0.0;
+      if (lc == 0) out[pos] = id[r];
+    }
+  }
+  // (no block leaves while another could still send to it)
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // U12 of a panel apart, for updates so large that every tile forming its own piece would cost more
@@ -786,10 +1037,16 @@ struct Level {
 constexpr size_t kMaxSmem = 227 * 1024 - 1024;  // dynamic shared memory (static parts stay below 1 KB)
 constexpr int kUpdateBlocks = 256;
 
-int panel_columns(int maxR) {  // panel width: the widest whose panel fits shared memory
-  for (int nb : {16, 8, 4})
-    if ((size_t)maxR * ((nb + 1) * sizeof(double) + kPanelBytes) <= kMaxSmem) return nb;
-  return 0;
+// Blocks a panel's rows are shared out between: as many as bring them to 112 a block while the fronts
+// do not fill the SMs, and as many as shared memory asks for (a level's rows end at 4,056: the
+// solver's size limit).  GB300, solves of 129 x 33, 257 x 65 and 513 x 129 Stokes and of 513 x 129
+// temperatures, ms: one block always 2.11, 8.27, 41.3, 5.19; 64 rows 2.04, 7.62, 39.8, 4.87; 96 rows
+// 2.02, 7.60, 39.8, 4.86; 128 rows 2.04, 7.63, 39.8, 4.84; 256 rows 2.09, 8.00, 40.1, 5.16.
+constexpr int kPanelCols = 16, kPanelRows = 1500;
+int cluster_blocks(int fronts, int rows, int nsm) {
+  int cl = 1;
+  while (cl < 8 && (rows > kPanelRows * cl || (rows > 112 * cl && fronts * cl * 2 <= nsm))) cl *= 2;
+  return cl;
 }
 
 }  // namespace
@@ -927,7 +1184,7 @@ int build_plan(mic_front_plan &pl, int dof, int NX, int NY, int nsm) {
       L.minP = std::min(L.minP, q.P);
     }
     plan_level(L, pl.fronts, nsm);
-    if (!L.small && panel_columns(L.maxR) == 0) return MIC_ERR_SOLVE;
+    if (!L.small && L.maxR > 8 * kPanelRows) return MIC_ERR_SOLVE;
     for (int i = L.first; i < L.first + L.count; ++i) {
       Front &q = pl.fronts[i];
       q.full = L.small ? 0 : 1;
@@ -938,7 +1195,7 @@ int build_plan(mic_front_plan &pl, int dof, int NX, int NY, int nsm) {
       if (q.full) {
         q.lb = L.nL;
         L.nL += (int64_t)q.R * 16;
-        const int nb = panel_columns(L.maxR), panels = (q.P + nb - 1) / nb;
+        const int panels = (q.P + kPanelCols - 1) / kPanelCols;
         q.act = pl.nAct;
         q.left = q.act + (panels & 1 ? q.R : 0) + q.P;
         pl.nAct += 2 * q.R;
@@ -994,11 +1251,23 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
   bool far = false;
   for (int k0 = 0, turn = 0; k0 < L.maxP; k0 += NB, turn ^= 1) {
     const int rows = L.maxR - k0;
-    const int threads = rows <= 256 ? 256 : kPanelThreads;
+    const int cl = cluster_blocks(L.count, rows, sm_count(ctx));
+    const int share = (rows + cl - 1) / cl, threads = share <= 256 ? 256 : kPanelThreads;
+    const size_t smem = (size_t)share * ((NB + 1) * sizeof(double) + kPanelBytes);
     {
       MIC_KERNEL_ON(ctx, "k_front_panel", chain);
-      launch_after(k_front_panel<NB>, L.count, threads, (size_t)rows * ((NB + 1) * sizeof(double) + kPanelBytes),
-                   chain, pl.d_fronts, L.first, k0, turn, F, B.U, B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
+      const auto launch = [&](auto *kernel) {
+        launch_after(kernel, L.count * cl, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U,
+                     B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
+      };
+      if (cl == 8)
+        launch(k_front_panel_cluster<8>);
+      else if (cl == 4)
+        launch(k_front_panel_cluster<4>);
+      else if (cl == 2)
+        launch(k_front_panel_cluster<2>);
+      else
+        launch(k_front_panel<NB>);
     }
     // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
@@ -1091,12 +1360,7 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
       launch_after(k_front_gather, dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first,
                    pl.d_tab, B.act, Fin, B.F[l & 1]);
     }
-    int e = MIC_OK;
-    switch (panel_columns(L.maxR)) {
-      case 16: e = large_level<16>(ctx, pl, L, B, B.F[l & 1]); break;
-      case 8: e = large_level<8>(ctx, pl, L, B, B.F[l & 1]); break;
-      default: e = large_level<4>(ctx, pl, L, B, B.F[l & 1]); break;
-    }
+    const int e = large_level<kPanelCols>(ctx, pl, L, B, B.F[l & 1]);
     if (e) return e;
   }
   for (int l = 0; l < nl; ++l) {
@@ -1122,16 +1386,20 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
   return MIC_OK;
 }
 
+constexpr int kPanelSmem = kPanelRows * ((kPanelCols + 1) * (int)sizeof(double) + kPanelBytes);
+
 cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
   cudaError_t e = cudaFuncSetAttribute(k_front_small<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_small<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    e = cudaFuncSetAttribute(k_front_panel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    e = cudaFuncSetAttribute(k_front_panel_cluster<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    e = cudaFuncSetAttribute(k_front_panel_cluster<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_panel_cluster<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_back, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
   return e;

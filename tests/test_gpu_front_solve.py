@@ -81,10 +81,10 @@ def test_zero_column_is_refused_and_the_context_stays_usable():
 
 @pytest.mark.parametrize("nx,ny", [(260, 90), (430, 430), (770, 760)])
 def test_tall_fronts_residual(nx, ny):
-    """Temperatures on grids whose top fronts need panels of 16, 8 and 4 columns to fit a block's
-    shared memory, and whose updates take every tile size: the residual stays at rounding level
-    (a diagonally dominant matrix, no growth: n eps at most, 2e-10 at the largest, in practice a few
-    eps; bound 1e-12)."""
+    """Temperatures on grids whose panels are factored by one, two, four and eight blocks (180, 860
+    and 1,520 rows at the top), and whose updates take every tile size: the residual stays at
+    rounding level (a diagonally dominant matrix, no growth: n eps at most, 2e-10 at the largest, in
+    practice a few eps; bound 1e-12)."""
     P, so = _problem(nx, ny)
     P.enforceThermalBCs1(so)
     P.formThermalSystem(so, 3.0e11)
@@ -95,4 +95,40 @@ def test_tall_fronts_residual(nx, ny):
     r = np.add.reduceat(v * x[c], rp[:-1]) - b
     a = np.add.reduceat(np.abs(v), rp[:-1])
     assert np.max(np.abs(r)) <= 1e-12 * np.max(a) * np.max(np.abs(x))
+    P.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(61, 61), (129, 33), (220, 64)])
+def test_tall_stokes_fronts_residual(nx, ny):
+    """Stokes systems with panels on clusters of blocks, whose pivots wander between the blocks:
+    the residual within n eps of the matrix and the solution."""
+    P, so = _problem(nx, ny)
+    P.formVEPSystem(so, 3.0e11)
+    P.linear_solve(P.STOKES)
+    x = P.solution(P.STOKES)
+    rp, c, v, b = P.system(P.STOKES)
+    assert np.all(np.isfinite(x))
+    r = np.add.reduceat(v * x[c], rp[:-1]) - b
+    a = np.add.reduceat(np.abs(v), rp[:-1])
+    assert np.max(np.abs(r)) <= len(b) * np.finfo(float).eps * np.max(a) * np.max(np.abs(x))
+    P.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(260, 90), (300, 300)])
+def test_zero_columns_in_tall_fronts(nx, ny):
+    """empty rows on a grid whose top panels are factored by clusters: no block has a pivot, the
+    solve reports it, and a proper system is solved after it"""
+    P, so = _problem(nx, ny, top_type=2)
+    P.enforceThermalBCs1(so)
+    P.formThermalSystem(so, 3.0e11)
+    with pytest.raises(gpu.MicError) as e:
+        P.linear_solve(P.THERMAL)
+    assert e.value.code == 12  # MIC_ERR_SOLVE
+    so.thermalBCTopType = 0
+    P.formThermalSystem(so, 3.0e11)
+    P.linear_solve(P.THERMAL)
+    x = P.solution(P.THERMAL)
+    rp, c, v, b = P.system(P.THERMAL)
+    r = np.add.reduceat(v * x[c], rp[:-1]) - b
+    assert np.max(np.abs(r)) <= len(b) * np.finfo(float).eps * np.max(np.add.reduceat(np.abs(v), rp[:-1])) * np.max(np.abs(x))
     P.close()
