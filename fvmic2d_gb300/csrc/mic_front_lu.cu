@@ -100,15 +100,22 @@ struct SystemRows {  // the assembled rows (mic_systems.cu)
   int width, dof, NX, NY;
 };
 
-// Largest |a| in a column by its high word (sign, exponent, 20 bits of mantissa): an integer key,
-// so the search costs no FP64 slot and one warp instruction per warp.  Rows whose keys agree
-// differ by less than 2^-20 relatively, as good a pivot.  -1 for a NaN.
-__device__ __forceinline__ int pivot_key(double a) {
-  const int h = (int)((unsigned long long)dbits(a) >> 32) & 0x7fffffff;
-  return h <= 0x7ff00000 ? h : -1;
+// What a row offers as pivot of a column: the leading 21 bits of |a| (exponent, 10 of mantissa) above
+// the row's number in one integer, so that the search costs no FP64 slot and one reduction of a warp
+// finds value and row (a reduction of the high word, a ballot and a shuffle for the row took 90
+// clocks more, twice a column).  Rows whose keys agree differ by less than 2^-10 relatively: the
+// multipliers stay below 1 + 2^-10, as good as 1 for the growth of the sums.  A NaN counts as 0.
+// 0 is no offer.
+constexpr int kOfferRow = 11, kOfferRows = 1 << kOfferRow;
+__device__ __forceinline__ unsigned pivot_offer(double a, int row) {
+  const unsigned h = (unsigned)((unsigned long long)dbits(a) >> 32) & 0x7fffffffu;
+  return ((h <= 0x7ff00000u ? h >> 10 : 0u) + 1) << kOfferRow | (unsigned)row;
 }
+__device__ __forceinline__ unsigned warp_best(unsigned offer) { return __reduce_max_sync(0xffffffffu, offer); }
+__device__ __forceinline__ int offer_row(unsigned offer) { return (int)(offer % kOfferRows); }
+__device__ __forceinline__ bool offer_counts(unsigned offer) { return offer >= 2 * kOfferRows; }
 
-// a column whose best key is 0 or none (every |a| below 2^-1042, or NaN): the exact largest |a| of
+// a column in which no offer counts (every |a| below 2^-1032, or NaN): the exact largest |a| of
 // the rows not used, the first of them when there is no other
 __device__ int pivot_rare(const double *col, int stride, int rows, const int *used) {
   long long best = -2;
@@ -142,13 +149,6 @@ __device__ __forceinline__ double pivot_rcp(double p) {
   return __longlong_as_double(rb | (long long)(b & 0x8000000000000000ULL));
 }
 
-// (key, row) of the warp's best lane, in every lane
-__device__ __forceinline__ int2 warp_best(int key, int row) {
-  const int m = __reduce_max_sync(0xffffffffu, key);
-  const unsigned b = __ballot_sync(0xffffffffu, key == m);
-  return make_int2(m, __shfl_sync(0xffffffffu, row, __ffs(b) - 1));
-}
-
 // value of column c (of q's columns) in left-over row i of child k: where the child keeps it
 __device__ __forceinline__ const double *child_row(const Front &k, int i, const double *F, const int *act) {
   return k.full ? F + k.f + (int64_t)act[k.left + i] * k.C + k.P : F + k.f + (int64_t)i * (k.C - k.P);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   if (!after_previous()) return;
   constexpr int kSmallWarps = kSmallThreads / 32;
   extern __shared__ double A[];
-  __shared__ int2 red[32];
+  __shared__ unsigned red[32];
   __shared__ double s_rcp;
   const Front q = fr[first + blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -215,15 +215,14 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   int G = (R + 31) / 32;  // candidate entries waiting in red
   for (int g = warp; g < G; g += kSmallWarps) {
     const int r = g * 32 + lane;
-    const int2 best = warp_best(r < R ? pivot_key(A[r * ld]) : -1, r);
+    const unsigned best = warp_best(r < R ? pivot_offer(A[r * ld], r) : 0u);
     if (lane == 0) red[g] = best;
   }
   __syncthreads();
   for (int j = 0; j < P; ++j) {
-    const int2 e = lane < G ? red[lane] : make_int2(-1, j);
-    const int2 best = warp_best(e.x, e.y);
-    int p = best.y;
-    if (best.x <= 0) {
+    const unsigned best = warp_best(lane < G ? red[lane] : 0u);
+    int p = offer_row(best);
+    if (!offer_counts(best)) {
       p = j + pivot_rare(A + j * ld + j, ld, R - j, nullptr);
       __syncthreads();  // every thread has read the column before rows move
     }
@@ -253,7 +252,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
           v = row[c] - l * piv[c];
           row[c] = v;
         }
-        const int2 b = warp_best(r < R ? pivot_key(v) : -1, r);
+        const unsigned b = warp_best(r < R ? pivot_offer(v, r) : 0u);
         if (lane == 0) red[g] = b;
         c += SL;
       }
@@ -321,7 +320,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
                   double *Lb, int *act, const int *__restrict__ tab, int *info) {
   if (!after_previous()) return;
   extern __shared__ double S[];
-  __shared__ int2 red[32];
+  __shared__ unsigned red[32];
   __shared__ double s_rcp;
   __shared__ int piv[NB];  // rows of the pivots so far
   const Front q = fr[first + blockIdx.x];
@@ -353,14 +352,8 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
     }
   }
   __syncthreads();
-  int key = -1, who = 0;
-  for (int r = tid; r < na; r += nt) {
-    const int k = pivot_key(S[r * LD]);
-    if (k > key) {
-      key = k;
-      who = r;
-    }
-  }
+  unsigned offer = 0;
+  for (int r = tid; r < na; r += nt) offer = max(offer, pivot_offer(S[r * LD], r));
   // row groups and column shares of phase 2; the reciprocal's warp takes part only where there is
   // more work than the others can share evenly
   const int G = (na + 31) / 32, workers = G >= nw ? nw : nw - 1, CS = max(1, workers / G);
@@ -371,8 +364,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
       const double rcp = s_rcp;
       const int p = piv[j];
       const bool more = j + 1 < nb;
-      key = -1;
-      who = 0;
+      offer = 0;
       const double pn = more ? S[p * LD + j + 1] : 0.0;
       unsigned bit = 1;
       for (int r = tid; r < na; r += nt, bit <<= 1) {
@@ -387,24 +379,19 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
         if (more) {
           const double v = an - l * pn;
           row[j + 1] = v;
-          const int k = pivot_key(v);
-          if (k > key) {
-            key = k;
-            who = r;
-          }
+          offer = max(offer, pivot_offer(v, r));
         }
       }
     }
     if (j + 1 == nb) break;
-    const int2 offer = warp_best(key, who);
+    offer = warp_best(offer);
     if (lane == 0) red[warp] = offer;
     __syncthreads();
     // phase 2: the pivot of column j + 1 and its reciprocal; the columns after it
     if (warp == nw - 1) {
-      const int2 e = lane < nw ? red[lane] : make_int2(-1, 0);
-      const int2 best = warp_best(e.x, e.y);
-      int p = best.y;
-      if (best.x <= 0) p = pivot_rare(S + j + 1, LD, na, used);
+      const unsigned best = warp_best(lane < nw ? red[lane] : 0u);
+      int p = offer_row(best);
+      if (!offer_counts(best)) p = pivot_rare(S + j + 1, LD, na, used);
       if (lane == 0) {
         const double v = S[p * LD + j + 1];
         s_rcp = pivot_rcp(v);
@@ -532,7 +519,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   extern __shared__ double S[];
   __shared__ PanelOffer ex[kOffers][CL];
   __shared__ __align__(8) unsigned long long bars[kOffers];
-  __shared__ int2 red[32];
+  __shared__ unsigned red[32];
   __shared__ double s_rcp;
   __shared__ int s_win, s_place;  // the last winner and the place of its offer
   __shared__ int s_rare;          // the column's exchange is to be done again
@@ -575,14 +562,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   __syncthreads();
   // every block of the cluster has come this far before one sends to another
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  int key = -1, who = -1;
-  for (int r = tid; r < m; r += nt) {
-    const int k = pivot_key(S[r * LD]);
-    if (who < 0 || k > key) {
-      key = k;
-      who = r;
-    }
-  }
+  unsigned offer = 0;
+  for (int r = tid; r < m; r += nt) offer = max(offer, pivot_offer(S[r * LD], r));
   const int G = (m + 31) / 32, workers = nw - 1, CS = max(1, workers / max(G, 1));
   unsigned mine = 0;  // which of this thread's rows are pivots
   int sent = 0;       // exchanges so far (the sending warp)
@@ -635,8 +616,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       const double rcp = s_rcp;
       const int p = piv[j] - base;
       const bool more = j + 1 < nb;
-      key = -1;
-      who = -1;
+      offer = 0;
       const double pn = more ? pr[j + 1] : 0.0;
       unsigned bit = 1;
       for (int r = tid; r < m; r += nt, bit <<= 1) {
@@ -651,22 +631,18 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
         if (more) {
           const double v = an - l * pn;
           row[j + 1] = v;
-          const int k = pivot_key(v);
-          if (who < 0 || k > key) {
-            key = k;
-            who = r;
-          }
+          offer = max(offer, pivot_offer(v, r));
         }
       }
     }
     if (j + 1 == nb) break;
-    const int2 offer = warp_best(key, who);
+    offer = warp_best(offer);
     if (lane == 0) red[warp] = offer;
     __syncthreads();
     // phase 2: the pivot of column j + 1 and its reciprocal; the columns after it
     if (warp == nw - 1) {
-      const int2 e = lane < nw ? red[lane] : make_int2(-1, -1);
-      const int p = warp_best(e.x, e.y).y;
+      const unsigned best = warp_best(lane < nw ? red[lane] : 0u);
+      const int p = best ? offer_row(best) : -1;
       double v = 0.0;
       if (p >= 0 && lane > j && lane < nb) {
         v = S[p * LD + lane];
