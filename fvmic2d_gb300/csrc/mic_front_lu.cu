@@ -570,7 +570,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   bool lost = false;  // one did not arrive in time: no more waits, the solve fails
   // column c: row p of this block (-1: none), its values from column c on in the lanes, to every
   // block; the winner's place, reciprocal and number.  Rare: no value that counts in any block
-  const auto exchange = [&](int c, int p, double v) {
+  const auto exchange = [&](int c, int p, double v, bool again) {
     const int place = sent % kOffers;
     const unsigned bar = shared_address(&bars[place]);
     if (lane == 0)
@@ -586,27 +586,18 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       if (lane <= NB) send_async(peer_address(from, d), bits, peer_address(bar, d));
     if (!lost && !offers_here(bar, (sent / kOffers) & 1)) lost = true;
     ++sent;
-    // the same choice in every block: the largest |value|, the first block's where they agree
-    long long top = -3;
-    int win = 0;
-#pragma unroll
-    for (int d = 0; d < CL; ++d) {
-      long long b = dbits(ex[place][d].v[c]) & 0x7fffffffffffffffLL;
-      if (b > 0x7ff0000000000000LL) b = -1;
-      if (ex[place][d].row < 0) b = -2;
-      if (b > top) {
-        top = b;
-        win = d;
-      }
-    }
-    if (lane == 0) {
-      const double w = ex[place][win].v[c];
-      s_rcp = pivot_rcp(w);
-      s_win = win;
+    // the same choice in every block; the lanes form all offers' reciprocals beside it
+    const int d = min(lane, CL - 1), row = (int)ex[place][d].row;
+    const double w = ex[place][d].v[c];
+    const unsigned mine = row < 0 ? 0u : pivot_offer(w, CL - 1 - d), top = warp_best(lane < CL ? mine : 0u);
+    const double rcp = pivot_rcp(offer_counts(mine) ? w : 1.0);
+    if (lane < CL && mine == top) {
+      s_rcp = offer_counts(mine) ? rcp : pivot_rcp(w);
+      s_win = d;
       s_place = place;
-      s_rare = (top >> 32) <= 0 && !s_rare;
-      piv[c] = (int)ex[place][win].row;
-      if (lost || (rank == 0 && !s_rare && (dbits(w) << 1) == 0)) atomicMin(&info[0], tab[q.col + k0 + c]);
+      s_rare = !again && !offer_counts(top);
+      piv[c] = row;
+      if (lost || (again && rank == 0 && (dbits(w) << 1) == 0)) atomicMin(&info[0], tab[q.col + k0 + c]);
     }
   };
   for (int j = -1; j < nb; ++j) {
@@ -649,7 +640,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
         if (j >= 0 && lane > j + 1) v -= S[p * LD + j] * pr[lane];
       }
       asm volatile("bar.arrive 1, %0;" ::"r"(nt) : "memory");  // the row is read: the others may update it
-      exchange(j + 1, p, v);
+      exchange(j + 1, p, v, false);
     } else {
       asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
       if (j >= 0) {
@@ -678,7 +669,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       if (warp == nw - 1) {
         int p = m > 0 ? pivot_rare(S + j + 1, LD, m, used) : -1;
         if (p >= 0 && used[p]) p = -1;
-        exchange(j + 1, p, p >= 0 && lane > j && lane < nb ? S[p * LD + lane] : 0.0);
+        exchange(j + 1, p, p >= 0 && lane > j && lane < nb ? S[p * LD + lane] : 0.0, true);
       }
       __syncthreads();
     }
