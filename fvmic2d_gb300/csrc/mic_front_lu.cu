@@ -443,28 +443,29 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
   }
 }
 
-// U12 = L11^-1 A12 of TC columns in shared memory, NB rows: four lanes a column, each every fourth
-// row, so that all warps take part (a warp's FP64 instruction holds a quarter of the SM for 64
-// cycles, whatever its lanes).  Threads from 4 TC on return; store: also to U.
+// U12 = L11^-1 A12 of TC columns in shared memory, NB rows: four lanes a column (eight where there
+// are few columns), each every fourth (eighth) row, so that all quarters of the SM take part (a
+// warp's FP64 instruction holds its quarter for 64 cycles, whatever its lanes).  Other threads
+// return at once; store: also to U.
 template <int NB, int TC>
 __device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB + 1], int tid, double *u_out, int ldu,
                                           int nb, int cols, bool store) {
-  if (tid >= 4 * TC) return;  // whole warps
-  constexpr int PER = NB / 4;
-  const int part = tid & 3, c = tid >> 2;
+  constexpr int LC = TC <= 16 ? 8 : 4, PER = NB / LC;
+  if (tid >= LC * TC) return;  // whole warps
+  const int part = tid % LC, c = tid / LC;
   double u[PER];
 #pragma unroll
-  for (int i = 0; i < PER; ++i) u[i] = Us[4 * i + part][c];
+  for (int i = 0; i < PER; ++i) u[i] = Us[LC * i + part][c];
 #pragma unroll
   for (int j = 0; j < NB - 1; ++j) {
-    const double uj = __shfl_sync(0xffffffffu, u[j / 4], (tid & 28) | (j & 3));
+    const double uj = __shfl_sync(0xffffffffu, u[j / LC], (tid & (32 - LC)) | (j % LC));
 #pragma unroll
-    for (int i = j / 4; i < PER; ++i)
-      if (4 * i + part > j) u[i] -= L11[4 * i + part][j] * uj;
+    for (int i = j / LC; i < PER; ++i)
+      if (LC * i + part > j) u[i] -= L11[LC * i + part][j] * uj;
   }
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    const int k = 4 * i + part;
+    const int k = LC * i + part;
     Us[k][c] = u[i];
     if (store && k < nb && c < cols) u_out[(int64_t)k * ldu + c] = u[i];
   }
@@ -1254,7 +1255,18 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
       MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
     }
     if (far) MIC_CUDA_TRY(cudaStreamWaitEvent(chain, ctx->lu_ev[1], 0));
-    if (ahead) update<NB, 64, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+    if (ahead) {
+      // on the chain: tiles as small as still get an SM each.  GB300: 64 rows always 1.97 ms for 129 x
+      // 33 Stokes, 7.48 for 257 x 65, 4.75 for 513 x 129 temperatures; up to one tile an SM 1.84, 7.45,
+      // 4.65; up to four 1.84, 7.62, 4.74
+      const int at_once = sm_count(ctx);
+      if (L.count * ((below + 15) / 16) <= at_once)
+        update<NB, 16, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+      else if (L.count * ((below + 31) / 32) <= at_once)
+        update<NB, 32, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+      else
+        update<NB, 64, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+    }
     if (ahead && !light) {
       MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], chain));
       MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
