@@ -27,8 +27,8 @@
 //
 // Two forms of a level, chosen by estimated time (plan_level):
 //   small  the front in shared memory, one block per front, unblocked (k_front_small);
-//   large  the front in global memory, panels of 16 columns: a block per front, or a cluster of
-//          blocks, factors a panel in shared memory (k_front_panel, k_front_panel_cluster), then
+//   large  the front in global memory, panels of 16 or 32 columns: a block per front, or a cluster
+//          of blocks, factors a panel in shared memory (k_front_panel, k_front_panel_cluster), then
 //          the trailing tiles of every front are updated, each block forming its own piece of U12
 //          (k_front_update): the next panel's columns first, the rest beside the next panel.
 // FP64 multiply-adds bound the updates (2 per SM and clock); the panels and the small fronts are
@@ -443,14 +443,15 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
   }
 }
 
-// U12 = L11^-1 A12 of TC columns in shared memory, NB rows: four lanes a column (eight where there
-// are few columns), each every fourth (eighth) row, so that all quarters of the SM take part (a
-// warp's FP64 instruction holds its quarter for 64 cycles, whatever its lanes).  Other threads
-// return at once; store: also to U.
+// U12 = L11^-1 A12 of TC columns in shared memory, NB rows, by up to 256 threads: LC lanes a column,
+// each every LC-th row, so that all quarters of the SM take part and no more warps than that need
+// (a warp's FP64 instruction holds its quarter for 64 cycles, whatever its lanes).  Threads without a
+// column return at once; store: also to U.
 template <int NB, int TC>
 __device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB + 1], int tid, double *u_out, int ldu,
                                           int nb, int cols, bool store) {
-  constexpr int LC = TC <= 16 ? 8 : 4, PER = NB / LC;
+  constexpr int LC = NB == 16 ? (TC <= 16 ? 8 : 4) : 256 / TC, PER = NB / LC;
+  static_assert(LC <= 32 && PER >= 1 && LC * PER == NB, "whole groups of lanes");
   if (tid >= LC * TC) return;  // whole warps
   const int part = tid % LC, c = tid / LC;
   double u[PER];
@@ -483,8 +484,9 @@ __device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB
 // of 1,290.
 constexpr int kOffers = 4;
 constexpr int kExchangeTries = 1 << 20;  // a wait of some 1 s at the very least
+template <int NB>
 struct PanelOffer {
-  double v[16];
+  double v[NB];
   long long row;  // number in the front's list; -1: the block has no row left
 };
 __device__ __forceinline__ unsigned shared_address(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -511,14 +513,13 @@ __device__ __forceinline__ bool offers_here(unsigned bar, unsigned parity) {
   return ok != 0;
 }
 
-template <int CL>
+template <int NB, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
     k_front_panel_cluster(const Front *__restrict__ fr, int first, int k0, int turn, const double *__restrict__ F,
                           double *U, double *Lb, int *act, const int *__restrict__ tab, int *info) {
   if (!after_previous()) return;
-  constexpr int NB = 16;
   extern __shared__ double S[];
-  __shared__ PanelOffer ex[kOffers][CL];
+  __shared__ PanelOffer<NB> ex[kOffers][CL];
   __shared__ __align__(8) unsigned long long bars[kOffers];
   __shared__ unsigned red[32];
   __shared__ double s_rcp;
@@ -557,7 +558,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   }
   if (tid < kOffers)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&bars[tid])) : "memory");
-  for (int e = tid; e < kOffers * CL; e += nt) ex[e / CL][e % CL] = PanelOffer{};
+  for (int e = tid; e < kOffers * CL; e += nt) ex[e / CL][e % CL] = PanelOffer<NB>{};
   if (tid == 0) s_win = s_place = s_rare = 0;
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
@@ -576,15 +577,16 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
     const unsigned bar = shared_address(&bars[place]);
     if (lane == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                   "r"(CL * (int)sizeof(PanelOffer))
+                   "r"(CL * (int)sizeof(PanelOffer<NB>))
                    : "memory");
     __syncwarp();
-    const PanelOffer *slot = &ex[place][rank];
-    const unsigned from = shared_address(lane < NB ? (const void *)&slot->v[lane] : (const void *)&slot->row);
-    const long long bits = lane < NB ? dbits(v) : (long long)(p >= 0 ? base + p : -1);
+    const unsigned to = shared_address(&ex[place][rank].v[lane % NB]), row_to = shared_address(&ex[place][rank].row);
 #pragma unroll
-    for (unsigned d = 0; d < CL; ++d)
-      if (lane <= NB) send_async(peer_address(from, d), bits, peer_address(bar, d));
+    for (unsigned d = 0; d < CL; ++d) {
+      const unsigned peer_bar = peer_address(bar, d);
+      if (lane < NB) send_async(peer_address(to, d), dbits(v), peer_bar);
+      if (lane == 31) send_async(peer_address(row_to, d), (long long)(p >= 0 ? base + p : -1), peer_bar);
+    }
     if (!lost && !offers_here(bar, (sent / kOffers) & 1)) lost = true;
     ++sent;
     // the same choice in every block; the lanes form all offers' reciprocals beside it
@@ -705,47 +707,52 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
 // than a launch
 template <int NB>
 __global__ void __launch_bounds__(256) k_front_solve(const Front *__restrict__ fr, int first, int k0, int turn,
-                                                    const double *__restrict__ F, double *U,
+                                                    int coff, const double *__restrict__ F, double *U,
                                                     const double *__restrict__ Lb, const int *__restrict__ act) {
   if (!after_previous()) return;
-  constexpr int TC = 64;
+  constexpr int TC = 32, NU = NB * TC / 256, N1 = NB * NB / 256;
   __shared__ double Us[NB][TC + 1];
   __shared__ double L11[NB][NB + 1];
   const Front q = fr[first + blockIdx.x];
   if (k0 >= q.P) return;
-  const int nb = min(NB, q.P - k0), c0 = k0 + nb + blockIdx.y * TC, tid = threadIdx.x;
+  const int nb = min(NB, q.P - k0), c0 = k0 + nb + coff + blockIdx.y * TC, tid = threadIdx.x;
   if (c0 >= q.C) return;
   const int *list = act + q.act + (int64_t)(1 - turn) * q.R + k0;
-  double u[NB * TC / 256], l1 = 0.0;
+  double u[NU], l1[N1];
 #pragma unroll
-  for (int i = 0; i < NB * TC / 256; ++i) {
+  for (int i = 0; i < NU; ++i) {
     const int e = tid + 256 * i, k = e / TC, c = c0 + e % TC;
     u[i] = (k < nb && c < q.C) ? F[q.f + (int64_t)list[k] * q.C + c] : 0.0;
   }
-  if (tid < NB * NB && tid / NB < nb) l1 = Lb[q.lb + tid];
 #pragma unroll
-  for (int i = 0; i < NB * TC / 256; ++i) Us[(tid + 256 * i) / TC][(tid + 256 * i) % TC] = u[i];
-  if (tid < NB * NB) L11[tid / NB][tid % NB] = l1;
+  for (int i = 0; i < N1; ++i) l1[i] = (tid + 256 * i) / NB < nb ? Lb[q.lb + tid + 256 * i] : 0.0;
+#pragma unroll
+  for (int i = 0; i < NU; ++i) Us[(tid + 256 * i) / TC][(tid + 256 * i) % TC] = u[i];
+#pragma unroll
+  for (int i = 0; i < N1; ++i) L11[(tid + 256 * i) / NB][(tid + 256 * i) % NB] = l1[i];
   __syncthreads();
   solve_u12<NB, TC>(Us, L11, tid, U + q.u + (int64_t)k0 * q.C + c0, q.C, nb, q.C - c0, true);
 }
 
-// A22 -= L21 U12 for columns right of the panel, TR x TC tiles.  SOLVE: each block forms U12 of its
-// own columns (NB^2 / 2 multiply-adds a column against NB TR for the tile: 25% more work at
-// TR = 32, for one launch and one wait less per panel), and the first row of tiles stores it;
-// otherwise U12 is in U.  The FP64 pipe is the bound: small tiles where there are too few large
-// ones to fill the SMs evenly.  Columns coff .. coff + clen - 1 of those right of the panel: the
-// next panel's columns go first, on the chain of panels, the others beside the next panel's
-// factorisation.
+// A22 -= L21 U12 for columns right of the panel, TR x TC tiles.  The FP64 pipe is the bound: small
+// tiles where there are too few large ones to fill the SMs evenly.  SOLVE (the next panel's columns, on
+// the chain of panels): each block forms U12 of its own columns, and the first row of tiles stores
+// it, for one launch and one wait less; otherwise U12 is in U.  Columns coff .. coff + clen - 1 of
+// those right of the panel.
+template <int NB, int TR, int TC, bool SOLVE>
+constexpr int update_smem() {
+  return (int)sizeof(double) * (NB * (TC + 1) + TR * (NB + 1) + (SOLVE ? NB * (NB + 1) : 0));
+}
 template <int NB, int TR, int TC, bool SOLVE>
 __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
     k_front_update(const Front *__restrict__ fr, int first, int k0, int turn, int coff, int clen, double *F, double *U,
                    const double *__restrict__ Lb, const int *__restrict__ act) {
   if (!after_previous()) return;
   constexpr int RT = TR / 16, CT = TC / 16;  // a thread's rows and columns
-  __shared__ double Us[NB][TC + 1];
-  __shared__ double Ls[TR][NB + 1];
-  __shared__ double L11[SOLVE ? NB : 1][NB + 1];
+  extern __shared__ double tile[];
+  double(*Us)[TC + 1] = reinterpret_cast<double(*)[TC + 1]>(tile);
+  double(*Ls)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(tile + NB * (TC + 1));
+  double(*L11)[NB + 1] = Ls + TR;  // (SOLVE)
   const Front q = fr[first + blockIdx.x];
   if (k0 >= q.P) return;
   const int nb = min(NB, q.P - k0);
@@ -772,33 +779,34 @@ __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
       v[a][b] = (at[a] >= 0 && c < cend) ? base[at[a] + c] : 0.0;
     }
   {
-    constexpr int NU = (NB * TC + 255) / 256, NL = (TR * NB + 255) / 256;
-    double u[NU], l[NL], l1 = 0.0;
+    constexpr int NU = NB * TC / 256, NL = TR * NB / 256, N1 = SOLVE ? NB * NB / 256 : 0, HALF = NL > 8 ? NL / 2 : NL;
+    double u[NU], l[HALF], l1[N1 + 1];
 #pragma unroll
     for (int i = 0; i < NU; ++i) {
       const int e = tid + 256 * i, k = e / TC, c = c0 + e % TC;
-      const bool in = e < NB * TC && k < nb && c < cend;
+      const bool in = k < nb && c < cend;
       if (SOLVE)
         u[i] = in ? base[(int64_t)list[k] * q.C + c] : 0.0;
       else
         u[i] = in ? U[q.u + (int64_t)(k0 + k) * q.C + c] : 0.0;
     }
-    if (SOLVE && tid < NB * NB && tid / NB < nb) l1 = L[tid];
 #pragma unroll
-    for (int i = 0; i < NL; ++i) {
-      const int e = tid + 256 * i, r = r0 + e / NB;
-      l[i] = (e < TR * NB && r < na) ? L[(int64_t)r * NB + e % NB] : 0.0;
-    }
+    for (int i = 0; i < N1; ++i) l1[i] = (tid + 256 * i) / NB < nb ? L[tid + 256 * i] : 0.0;
 #pragma unroll
-    for (int i = 0; i < NU; ++i) {
-      const int e = tid + 256 * i;
-      if (e < NB * TC) Us[e / TC][e % TC] = u[i];
-    }
-    if (SOLVE && tid < NB * NB) L11[tid / NB][tid % NB] = l1;
+    for (int h = 0; h < NL; h += HALF) {
 #pragma unroll
-    for (int i = 0; i < NL; ++i) {
-      const int e = tid + 256 * i;
-      if (e < TR * NB) Ls[e / NB][e % NB] = l[i];
+      for (int i = 0; i < HALF; ++i) {
+        const int e = tid + 256 * (h + i), r = r0 + e / NB;
+        l[i] = r < na ? L[(int64_t)r * NB + e % NB] : 0.0;
+      }
+      if (h == 0) {
+#pragma unroll
+        for (int i = 0; i < NU; ++i) Us[(tid + 256 * i) / TC][(tid + 256 * i) % TC] = u[i];
+#pragma unroll
+        for (int i = 0; i < N1; ++i) L11[(tid + 256 * i) / NB][(tid + 256 * i) % NB] = l1[i];
+      }
+#pragma unroll
+      for (int i = 0; i < HALF; ++i) Ls[(tid + 256 * (h + i)) / NB][(tid + 256 * (h + i)) % NB] = l[i];
     }
   }
   __syncthreads();
@@ -806,8 +814,9 @@ __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
     solve_u12<NB, TC>(Us, L11, tid, U + q.u + (int64_t)k0 * q.C + c0, q.C, nb, cend - c0, blockIdx.y == 0);
     __syncthreads();
   }
+  const int steps = (nb + 3) & ~3;  // (zeros behind nb)
 #pragma unroll 4
-  for (int k = 0; k < NB; ++k) {
+  for (int k = 0; k < steps; ++k) {
     double l[RT], u[CT];
 #pragma unroll
     for (int a = 0; a < RT; ++a) l[a] = Ls[ti + 16 * a][k];
@@ -998,19 +1007,20 @@ struct Level {
   int first, count;          // fronts
   int maxR, maxP, maxC, minP;
   bool small;
+  int nb;                    // columns of a panel: 16 or 32
   int64_t nF, nL;            // doubles of row storage and of panel buffer
   size_t smem_small;
 };
 
 constexpr size_t kMaxSmem = 227 * 1024 - 1024;  // dynamic shared memory (static parts stay below 1 KB)
-constexpr int kUpdateBlocks = 256;
+constexpr int kUpdateThreads = 256;
 
 // Blocks a panel's rows are shared out between: as many as bring them to 112 a block while the fronts
 // do not fill the SMs, and as many as shared memory asks for (a level's rows end at 4,056: the
 // solver's size limit).  GB300, solves of 129 x 33, 257 x 65 and 513 x 129 Stokes and of 513 x 129
 // temperatures, ms: one block always 2.11, 8.27, 41.3, 5.19; 64 rows 2.04, 7.62, 39.8, 4.87; 96 rows
 // 2.02, 7.60, 39.8, 4.86; 128 rows 2.04, 7.63, 39.8, 4.84; 256 rows 2.09, 8.00, 40.1, 5.16.
-constexpr int kPanelCols = 16, kPanelRows = 1500;
+constexpr int kPanelRows = 800;
 int cluster_blocks(int fronts, int rows, int nsm) {
   int cl = 1;
   while (cl < 8 && (rows > kPanelRows * cl || (rows > 112 * cl && fronts * cl * 2 <= nsm))) cl *= 2;
@@ -1031,12 +1041,19 @@ struct mic_front_plan {
 
 namespace {
 
-// The level's form, by estimated time (us).  Small: a front's multiply-adds on one SM (2 per
-// clock), 1.5 us a column step, 8 us to load and store.  Large: per panel of 16 columns, 28 us for
-// its factorisation and the launches, and the update's 32 x 32 tiles (padding included) over all
-// SMs at 5.4 us a tile; 9 us for the gather.  Measured on the levels of five systems: the lines
-// cross near 60 fronts of 100 x 170 (241 us small, 230 large); 256 fronts of 52 x 90 take 81 us
-// small and 280 large, 16 of 80 x 133 take 134 us small and 98 large.
+// The level's form, by estimated time (us).  Small: a front's multiply-adds on one SM (2 per clock),
+// 1.1 us a column step, 6 us to load and store.  Large: per panel of 16 columns, 28 us for its
+// factorisation and the launches, and the update's 32 x 32 tiles (padding included) over all SMs at
+// 5.4 us a tile; 9 us for the gather.  Measured on the levels of five systems: the lines cross near
+// 60 fronts of 100 x 170 (241 us small, 230 large); 256 fronts of 52 x 90 take 81 us small and 280
+// large, 16 of 80 x 133 take 134 us small and 98 large.  With the small estimate a third higher 513 x
+// 129 Stokes take 37.5 ms instead of 36.9, with it a third lower 129 x 33 take 1.93 instead of 1.85.
+//
+// Columns of a panel: 16 where the chain of panels bounds the level, 32 where the updates do (twice
+// the multiply-adds for each value of the trailing rows read and written; the panels' own work and
+// the solve of U12 double).  By the level's first update at 2 multiply-adds per SM and clock, 16
+// columns deep: from 15 us 129 x 33 Stokes take 2.10 ms, from 40 us 1.85, with 16 always 1.84; 257 x
+// 65 6.87, 6.87 and 7.44; 513 x 129 37.6, 37.6 and 39.3, from 80 us 37.9.
 void plan_level(Level &L, const std::vector<Front> &fr, int nsm) {
   double total = 0, most = 0, large = 9.0;
   for (int i = L.first; i < L.first + L.count; ++i) {
@@ -1049,7 +1066,9 @@ void plan_level(Level &L, const std::vector<Front> &fr, int nsm) {
   }
   large += 28.0 * ((L.maxP + 15) / 16);
   const double waves = (L.count + nsm - 1) / nsm, clk = 1.9e3;
-  const double small = std::max(waves * most, total / nsm) / 2 / clk * 1.3 + 1.5 * L.maxP + 8.0;
+  const double first = 16.0 * L.maxR * (L.maxC - std::min(16, L.maxP)) * L.count / (2.0 * clk * nsm);
+  L.nb = first > 40.0 ? 32 : 16;
+  const double small = std::max(waves * most, total / nsm) / 2 / clk + 1.1 * L.maxP + 6.0;
   L.smem_small = (size_t)L.maxR * (L.maxC | 1) * sizeof(double);
   L.small = L.smem_small <= kMaxSmem && L.maxR <= 1024 && (fr[L.first].child < 0 || small <= large);
 }
@@ -1162,8 +1181,8 @@ int build_plan(mic_front_plan &pl, int dof, int NX, int NY, int nsm) {
       pl.nU += (int64_t)q.P * q.C;
       if (q.full) {
         q.lb = L.nL;
-        L.nL += (int64_t)q.R * 16;
-        const int panels = (q.P + kPanelCols - 1) / kPanelCols;
+        L.nL += (int64_t)q.R * L.nb;
+        const int panels = (q.P + L.nb - 1) / L.nb;
         q.act = pl.nAct;
         q.left = q.act + (panels & 1 ? q.R : 0) + q.P;
         pl.nAct += 2 * q.R;
@@ -1204,7 +1223,8 @@ void update(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffer
             int rows, int coff, int cols, cudaStream_t st) {
   MIC_KERNEL_ON(ctx, "k_front_update", st);
   launch_after(k_front_update<NB, TR, TC, SOLVE>, dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC),
-               kUpdateBlocks, 0, st, pl.d_fronts, L.first, k0, turn, coff, cols, F, B.U, B.Lb + turn * pl.nL, B.act);
+               kUpdateThreads, update_smem<NB, TR, TC, SOLVE>(), st, pl.d_fronts, L.first, k0, turn, coff, cols, F,
+               B.U, B.Lb + turn * pl.nL, B.act);
 }
 
 // One level in panels.  The chain (panel, then its update of the next panel's columns) runs on the
@@ -1229,25 +1249,25 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
                      B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
       };
       if (cl == 8)
-        launch(k_front_panel_cluster<8>);
+        launch(k_front_panel_cluster<NB, 8>);
       else if (cl == 4)
-        launch(k_front_panel_cluster<4>);
+        launch(k_front_panel_cluster<NB, 4>);
       else if (cl == 2)
-        launch(k_front_panel_cluster<2>);
+        launch(k_front_panel_cluster<NB, 2>);
       else
         launch(k_front_panel<NB>);
     }
     // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
     // The rest of an update runs beside the next panel, in one of two orders.  Light (its
-    // multiply-adds under 75 us at 2 per SM and clock, or a panel that fits beside its blocks in
-    // an SM's shared memory): it starts with the update of the next panel's columns.  Heavy: only
-    // after that one, so that the panel, which may need an SM's whole shared memory, finds free SMs;
-    // behind a heavy update it would start when that ends (513 x 129 Stokes: 54.3 ms with every
-    // update light, 46.9 with the heavy ones whole before the next panel, 41.8 so; 129 x 33: 2.35
-    // with every update of 25 us and more before the next panel, 2.40 with all heavy, 2.21 so).
+    // multiply-adds under 50 us at 2 per SM and clock, or a panel that fits beside its blocks in an
+    // SM's shared memory): it starts with the update of the next panel's columns.  Heavy: only after
+    // that one, so that the panel, which may need an SM's whole shared memory, finds free SMs; behind
+    // a heavy update it would start when that ends (513 x 129 Stokes: 54.3 ms with every update
+    // light, 46.9 with the heavy ones whole before the next panel, 41.8 so; 513 x 129 temperatures
+    // with the line at 50 us and 200 rows 4.48, at 75 us and 400 rows 4.57).
     const double us = (double)cols * below * NB * L.count / (2.0 * 1.9e3 * sm_count(ctx));
-    const bool ahead = k0 + NB < L.maxP && cols > NB, light = us < 75.0 || rows < 400;
+    const bool ahead = k0 + NB < L.maxP && cols > NB, light = us < 50.0 || rows < 200;
     const int near = ahead ? NB : 0, rest = cols - near;
     cudaStream_t st = ahead ? main : chain;
     if (ahead && light) {
@@ -1272,29 +1292,31 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
       MIC_CUDA_TRY(cudaStreamWaitEvent(main, ctx->lu_ev[0], 0));
     }
     // the tile whose blocks, padding and triangular solves included, take the least time on the
-    // fullest SM (multiply-adds, 2 per clock; 600 clocks a block to start and end)
+    // fullest SM (multiply-adds, 2 per clock; 600 clocks a block to start and end).  16 columns: small
+    // tiles form U12 themselves (25% more work at 32 rows, for a launch less); with 32 the solve is
+    // half a small tile's work
     const double nsm = sm_count(ctx);
-    auto cost = [&](int tr, int tc, bool solve) {
+    const auto cost = [&](int tr, int tc, bool solve) {
       const double n = (double)((rest + tc - 1) / tc) * ((below + tr - 1) / tr) * L.count;
-      return std::ceil(n / nsm) * (0.5 * tc * NB * (tr + (solve ? NB / 2 : 0)) + 600.0);
+      return std::ceil(n / nsm) * (0.5 * tc * NB * (tr + (solve ? NB / 2 : 0)) + 600.0) + (solve ? 0.0 : 8000.0);
     };
-    const double c32 = cost(32, 32, true), c6432 = cost(64, 32, true), c64 = cost(64, 64, false) + 8000.0,
-                 c128 = cost(128, 64, false) + 8000.0;  // (8,000 clocks: U12's launch and solve)
+    const double c32 = cost(32, 32, NB == 16), c6432 = cost(64, 32, NB == 16), c64 = cost(64, 64, false),
+                 c128 = cost(128, 64, false);  // (8,000 clocks: U12's launch and solve)
     const double best = std::min(std::min(c32, c6432), std::min(c64, c128));
-    if (best == c64 || best == c128) {
-      {
+    if (rest > 0) {
+      if (NB == 32 || best == c64 || best == c128) {
         MIC_KERNEL_ON(ctx, "k_front_solve", st);
-        launch_after(k_front_solve<NB>, dim3(L.count, (cols + 63) / 64), 256, 0, st, pl.d_fronts, L.first, k0, turn,
-                     F, B.U, B.Lb + turn * pl.nL, B.act);
+        launch_after(k_front_solve<NB>, dim3(L.count, (rest + 31) / 32), 256, 0, st, pl.d_fronts, L.first, k0, turn,
+                     near, F, B.U, B.Lb + turn * pl.nL, B.act);
       }
-      if (best == c64)
-        update<NB, 64, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
-      else
+      if (best == c128)
         update<NB, 128, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
-    } else if (best == c6432) {
-      update<NB, 64, 32, true>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
-    } else {
-      update<NB, 32, 32, true>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+      else if (best == c64)
+        update<NB, 64, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+      else if (best == c6432)
+        update<NB, 64, 32, NB == 16>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+      else
+        update<NB, 32, 32, NB == 16>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
     }
     far = ahead;
     if (ahead) MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[1], main));
@@ -1339,7 +1361,7 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
       launch_after(k_front_gather, dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first,
                    pl.d_tab, B.act, Fin, B.F[l & 1]);
     }
-    const int e = large_level<kPanelCols>(ctx, pl, L, B, B.F[l & 1]);
+    const int e = L.nb == 32 ? large_level<32>(ctx, pl, L, B, B.F[l & 1]) : large_level<16>(ctx, pl, L, B, B.F[l & 1]);
     if (e) return e;
   }
   for (int l = 0; l < nl; ++l) {
@@ -1365,22 +1387,27 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
   return MIC_OK;
 }
 
-constexpr int kPanelSmem = kPanelRows * ((kPanelCols + 1) * (int)sizeof(double) + kPanelBytes);
+template <class K>
+cudaError_t allow(K *kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+template <int NB>
+cudaError_t allow_panels() {
+  constexpr size_t bytes = (size_t)kPanelRows * ((NB + 1) * sizeof(double) + kPanelBytes);
+  cudaError_t e = allow(k_front_panel<NB>, bytes);
+  if (e == cudaSuccess) e = allow(k_front_panel_cluster<NB, 2>, bytes);
+  if (e == cudaSuccess) e = allow(k_front_panel_cluster<NB, 4>, bytes);
+  if (e == cudaSuccess) e = allow(k_front_panel_cluster<NB, 8>, bytes);
+  return e;
+}
 
 cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
-  cudaError_t e = cudaFuncSetAttribute(k_front_small<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel_cluster<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel_cluster<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_panel_cluster<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_back, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  cudaError_t e = allow(k_front_small<256>, kMaxSmem);
+  if (e == cudaSuccess) e = allow(k_front_small<512>, kMaxSmem);
+  if (e == cudaSuccess) e = allow_panels<16>();
+  if (e == cudaSuccess) e = allow_panels<32>();
+  if (e == cudaSuccess) e = allow(k_front_update<32, 128, 64, false>, update_smem<32, 128, 64, false>());
+  if (e == cudaSuccess) e = allow(k_front_back, 64 * 1024);
   return e;
 }
 
