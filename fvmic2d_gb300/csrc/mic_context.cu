@@ -346,7 +346,12 @@ extern "C" int mic_create(mic_ctx **out, int device, void *stream, int NX, int N
     }
     ctx->owns_stream = 1;
   }
-  if (cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess ||
+  // The second stream's work is short and waited for (projections beside longer passes): its blocks go
+  // first.  GB300, cycles with and without: 1024 x 256 box 3,157 and 3,321 us, periodic 509 x 127 1,625
+  // and 1,741, 333 x 517 ice 2,090 and 2,157.
+  int least = 0, most = 0;
+  if (cudaDeviceGetStreamPriorityRange(&least, &most) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&ctx->aux, cudaStreamNonBlocking, most) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->aux_ev[0], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->aux_ev[1], cudaEventDisableTiming) != cudaSuccess) {
     free_ctx(ctx);

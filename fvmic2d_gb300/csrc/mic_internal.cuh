@@ -405,6 +405,9 @@ inline int sm_count(const mic_ctx *ctx) {
   return n;
 }
 
+// a grid whose cells, a thread each, would leave most of the SMs' quarters without a warp
+inline bool few_cells(const mic_ctx *ctx) { return ctx->ncells <= 32 * sm_count(ctx); }
+
 // Bit pattern of a non-negative double, canonicalising -0.0 to +0.0, so that for
 // non-negative finite values a >= b  <=>  bits(a) >= bits(b) as signed integers.
 // Bilinear weights (1-mdx)(1-mdy), mdx(1-mdy), (1-mdx)mdy, mdx mdy, formed as the reference's

@@ -2153,6 +2153,13 @@ void mic_clear_yield(mic_ctx *ctx, mic_clear_list &l, bool step) {
   l.add(ctx->d_creep, sizeof(CreepCounters));
 }
 
+static int yield_pass(const mic_ctx *ctx) {
+  const int mode = ctx->creep.mlp ? ctx->creep.mode : 0;
+  bool law7 = false;
+  for (int k = 0; k < MIC_MAXMAT; ++k) law7 = law7 || ctx->mat.hasEtaT[k] == 7;
+  return !law7 ? BP_YIELD_PLAIN : mode == 0 ? BP_YIELD_EXACT : mode == 1 ? BP_YIELD_FP32 : BP_YIELD_TC;
+}
+
 // limit: limitViscosity (viscosity.c:90-104) fused into the pass, for callers that run it next
 // cleared: the step's binning has cleared the pass's results
 static int yield_launch(mic_ctx *ctx, double dt, bool limit = false, bool cleared = false, mic_batch *b = nullptr) {
@@ -2164,12 +2171,9 @@ static int yield_launch(mic_ctx *ctx, double dt, bool limit = false, bool cleare
     if ((e = mic_clear(ctx, l))) return e;
   }
   if (ctx->n == 0) return MIC_OK;
-  const int mode = ctx->creep.mlp ? ctx->creep.mode : 0;
-  bool law7 = false;
-  for (int k = 0; k < MIC_MAXMAT; ++k) law7 = law7 || ctx->mat.hasEtaT[k] == 7;
   YieldJob J = {yield_cols(ctx), ctx->mat,    ctx->opt,     ctx->creep,   dt,
                 ctx->n,          ctx->d_status, ctx->d_creep, limit ? 1 : 0};
-  const int pass = !law7 ? BP_YIELD_PLAIN : mode == 0 ? BP_YIELD_EXACT : mode == 1 ? BP_YIELD_FP32 : BP_YIELD_TC;
+  const int pass = yield_pass(ctx);
   if (b) {
     if (pass == BP_YIELD_FP32 || pass == BP_YIELD_TC) J.cfg.mlp = b->shared_net(ctx->mlp_key, J.cfg.mlp);
     return b->add(pass, J, ctx->n);
@@ -2602,6 +2606,17 @@ int mic_step_segment(mic_ctx *ctx, int seg, double dt_disp, double dt_thermal, i
   // from the strain-rate pass, subgridStressChanges.c:91-92, 186-187)
   const bool keep = sub && ctx->n > 0 && !ctx->P.xper;
 #endif
+#ifndef MIC_EXACT
+  // The first projection of a step beside its yield pass (segment 1), or before it where the yield
+  // pass is the surrogate's: its blocks stay for the whole pass, and those that come beside the
+  // projection's find less room than they would keep to the end, or leave it too little.  Before it
+  // also on small grids, where the second stream's events cost more than the overlap gains.  GB300,
+  // us a cycle beside and before: 1024 x 1024 ice with the surrogate 14,290 and 13,410; 333 x 517 ice
+  // 2,096 and 2,112; 1024 x 256 two-material box 3,176 and 3,185; periodic 509 x 127 1,632 and 1,651;
+  // 64 x 64 box 210 and 204.
+  const int yp = yield_pass(ctx);
+  const bool first_beside = b || !(yp == BP_YIELD_TC || yp == BP_YIELD_FP32 || few_cells(ctx));
+#endif
   switch (seg) {
     case 0:
       // findMarkerCells (main:243, 247, 252): positions do not change between the three calls on
@@ -2621,17 +2636,21 @@ int mic_step_segment(mic_ctx *ctx, int seg, double dt_disp, double dt_thermal, i
       // forms only rho, k, T and Cp, on the second stream, beside the yield pass (which applies
       // the viscosity limit of main:297 to every marker as it stores the viscosities).
       if ((e = mic_ensure_geometry(ctx))) return e;
-      MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[0], ctx->stream));
-      MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->aux_ev[0], 0));
-      if ((e = mic_project_all2_first(ctx, ctx->aux))) return e;
-      MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
+      if (first_beside) {
+        MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[0], ctx->stream));
+        MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->aux_ev[0], 0));
+        if ((e = mic_project_all2_first(ctx, ctx->aux))) return e;
+        MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
+      } else if ((e = mic_project_all2_first(ctx, ctx->stream))) {
+        return e;
+      }
       return yield_launch(ctx, dt_disp, /*limit=*/true, true, b);  // limitViscosity fused in
 #endif
     case 2:
 #ifdef MIC_EXACT
       if ((e = mic_limit_viscosity(ctx))) return e;
 #else
-      MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->aux_ev[1], 0));
+      if (first_beside) MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->aux_ev[1], 0));
 #endif
       // the second projection: yielding and the limit changed viscosities and stresses only
       return mic_project_all2_viscous(ctx);

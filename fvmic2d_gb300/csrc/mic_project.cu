@@ -633,7 +633,6 @@ __global__ void __launch_bounds__(128) k_corners_centre(Params P, PartialView v,
   }
 }
 inline dim3 corners_centre_grid(const Params &P) { return dim3((4 * (P.NCX + 1) + 127) / 128, P.NY); }
-inline bool few_cells(const mic_ctx *ctx) { return ctx->ncells <= 32 * sm_count(ctx); }
 
 // Node (i, j): basic sums from cells (i-1,j-1) corner 3, (i,j-1) corner 2, (i-1,j) corner 1,
 // (i,j) corner 0; centre sums from staggered cells with the same offsets.
