@@ -210,9 +210,10 @@ struct ProfScope {  // brackets one kernel launch: counts it and, when enabled, 
 // kernel's blocks as soon as the last block of the kernel before it in the stream has ended, while
 // its end is still being reported; after_previous, the first statement of every kernel launched so,
 // waits until all of that kernel's writes (and, since it waited in turn, those of all kernels
-// before it) are visible.  GB300, a chain of 25 small kernels in a stream: 4.1 -> 2.4 us each.  No
-// kernel asks for its successor earlier than its end: blocks that wait take the places of those
-// that work (3.8 us each).
+// before it) are visible.  GB300, a chain of 25 small kernels in a stream: 4.1 -> 2.4 us each.
+// next_may_start lets the successor's blocks come as soon as all of this kernel's have started.
+// They wait in after_previous all the same, but take places of blocks that work (in that chain 3.8
+// us each): only for kernels of a few blocks on a chain (the direct solver's panels).
 //
 // after_previous gives true, but through the wait itself: no read of the kernel, not even one the
 // compiler takes for constant, can be moved in front of the branch on it.
@@ -222,6 +223,8 @@ __device__ __forceinline__ bool after_previous() {
   asm volatile("griddepcontrol.wait;\n\tmov.b32 %0, 1;" : "=r"(stay)::"memory");
   return stay != 0;
 }
+
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
 void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
