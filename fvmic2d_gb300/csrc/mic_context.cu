@@ -191,6 +191,7 @@ static void free_ctx(mic_ctx *ctx) {
     cudaFree(ctx->sys[w].col);
     cudaFree(ctx->sys[w].val);
     cudaFree(ctx->sys[w].rhs);
+    cudaFree(ctx->sys[w].free_cell);
   }
   cudaFree(ctx->sys_scratch);
   cudaFree(ctx->lu_buf);

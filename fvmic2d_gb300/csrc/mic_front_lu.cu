@@ -62,7 +62,8 @@ struct Front {
   int64_t left; // the left-over rows in the list its last panel wrote
 };
 
-// info[0]: smallest unknown with a zero pivot; info[1]: entries outside the assumed stencils;
+// info[0]: smallest unknown with a zero pivot; info[1]: entries outside the assumed stencils, and
+// exchanges of a cluster's panel that did not arrive;
 // info[2], info[3]: lower and upper band widths of the matrix in grid order (mic_system_band)
 constexpr int kInfo = 4;
 
@@ -98,6 +99,7 @@ struct SystemRows {  // the assembled rows (mic_systems.cu)
   const int *cnt, *col;
   const double *val, *rhs;
   int width, dof, NX, NY;
+  const unsigned char *free_cell;  // per node: cells whose pressure no equation holds (null: none)
 };
 
 // What a row offers as pivot of a column: the leading 21 bits of |a| (exponent, 10 of mantissa) above
@@ -198,6 +200,12 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
           atomicAdd(&info[1], 1);
       }
       A[r * ld + C - 1] = sys.rhs[g];
+      if (sys.free_cell && d == 2 && sys.free_cell[g / 3]) {  // its pressure is free: pinned (mic_systems.cu)
+        double most = 0.0;
+        for (int k = 0; k < n; ++k) most = fmax(most, fabs(sys.val[g * sys.width + k]));
+        const int cx = q.x0 + node % w - tx, cy = q.y0 + node / w - ty;
+        A[r * ld + tab[q.map + (cy * tw + cx) * sys.dof + 2]] = most;
+      }
     }
   } else {
     const Front a = fr[q.child], b = fr[q.child + 1];
@@ -602,7 +610,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       s_place = place;
       s_rare = !again && !offer_counts(top);
       piv[c] = row;
-      if (lost || (again && rank == 0 && (dbits(w) << 1) == 0)) atomicMin(&info[0], tab[q.col + k0 + c]);
+      if (lost) atomicAdd(&info[1], 1);
+      if (again && rank == 0 && (dbits(w) << 1) == 0) atomicMin(&info[0], tab[q.col + k0 + c]);
     }
   };
   for (int j = -1; j < nb; ++j) {
@@ -1471,7 +1480,7 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
   const int dof = which == 0 ? 3 : 1;
   const int64_t n = S.n;
   int e;
-  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY};
+  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY, S.free_cell};
   // the solver's size limit, a band of 1,016 below the diagonal: only a grid whose shorter side
   // could reach it has its band measured first
   constexpr int kMaxBand = 1016;

@@ -95,6 +95,7 @@ struct mic_system_store {
   int width;
   int *cnt, *col;
   double *val, *rhs;
+  unsigned char *free_cell;  // Stokes: per node, a cell whose pressure no equation holds
   double Kbond, Kcont;
   int factored;
   int kl, ku;       // band widths of the matrix in grid order

@@ -504,6 +504,102 @@ int prepare(mic_ctx *ctx, const mic_subduction_options &o, Scratch &s, Geo &G) {
   return MIC_OK;
 }
 
+// Pressure cells cut off from the rest.  Where the slab meets the plate on a coarse grid, a few
+// pressure cells, usually two, can lie between imposed velocities on all sides: their common
+// pressure is in no equation and the matrix is singular.  An elimination in grid order meets a pivot
+// of rounding there and goes on, to pressures of 1e26; in the solver's order the pivot is often
+// exactly zero.  Such a group is found from the equations (a momentum equation that holds two
+// pressures links their cells), and in the solve its first cell's continuity equation has an entry at
+// its own pressure, of the size of its others: the free pressure comes out near zero, all else as
+// it is.  No other matrix is touched, and the assembled rows (mic_system_get) stay as they are.
+constexpr int kGroup = 8;  // cells of a group at most
+struct Links {
+  int to[8], n;
+  bool held;  // an equation holds this pressure alone
+};
+// which of two columns a row holds (bits 0 and 1); its twelve places read at once
+__device__ __forceinline__ int holds(const Rows &s, int row, int c0, int c1) {
+  static_assert(kMaxEnt == 12, "three groups of four");
+  const int4 *q = reinterpret_cast<const int4 *>(s.col + (int64_t)row * kMaxEnt);
+  const int n = s.cnt[row];
+  int hit = 0;
+#pragma unroll
+  for (int g = 0; g < 3; ++g) {
+    const int4 v = q[g];
+    const int c[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) hit |= (4 * g + k < n) * ((c[k] == c0) | (c[k] == c1) << 1);
+  }
+  return hit;
+}
+// the momentum equations around a cell: f(neighbour) for a link, f(-1) for one that holds it alone
+template <class F>
+__device__ __forceinline__ void cell_faces(const Rows &s, int NX, int NY, int cell, F f) {
+  const int x = cell % NX, y = cell / NX;
+  const int eq[4] = {3 * (cell - NX), 3 * (cell - NX - 1), 3 * (cell - 1) + 1, 3 * (cell - NX - 1) + 1};
+  const int to[4] = {x + 1 < NX ? cell + 1 : -1, cell - 1, y + 1 < NY ? cell + NX : -1, cell - NX};
+  const bool there[4] = {y > 0, y > 0 && x > 0, x > 0, y > 0 && x > 0};
+  int hit[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    hit[k] = there[k] ? holds(s, eq[k], 3 * cell + 2, to[k] >= 0 ? 3 * to[k] + 2 : -1) : 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (hit[k] & 1) f(hit[k] & 2 ? to[k] : -1);
+}
+__device__ Links cell_links(const Rows &s, int NX, int NY, int cell) {
+  Links l;
+  l.n = 0;
+  l.held = false;
+  cell_faces(s, NX, NY, cell, [&](int to) {
+    if (to >= 0)
+      l.to[l.n++] = to;
+    else
+      l.held = true;
+  });
+  // the cell's own equation, where it is one for pressures (boundaries, solids)
+  const int own = 3 * cell + 2, n = s.cnt[own];
+  if (holds(s, own, own, own)) {
+    if (n == 1) l.held = true;
+    for (int k = 0; k < n && l.n < 8; ++k) {
+      const int c = s.col[(int64_t)own * kMaxEnt + k];
+      if (c != own && c % 3 == 2) l.to[l.n++] = c / 3;
+    }
+  }
+  return l;
+}
+// Is this the first cell, of those with at most two links, of a group that nothing holds?
+__device__ __noinline__ bool cut_off_first(const Rows &s, int NX, int NY, int cell) {
+  int group[kGroup], n = 1;
+  group[0] = cell;
+  for (int i = 0; i < n; ++i) {
+    const Links l = cell_links(s, NX, NY, group[i]);
+    const int own = 3 * group[i] + 2;
+    if (l.held) return false;
+    if (l.n <= 2 && group[i] < cell && !holds(s, own, own, own)) return false;
+    for (int k = 0; k < l.n; ++k) {
+      bool seen = false;
+      for (int j = 0; j < n; ++j) seen = seen || group[j] == l.to[k];
+      if (seen) continue;
+      if (n == kGroup) return false;
+      group[n++] = l.to[k];
+    }
+  }
+  return true;
+}
+__global__ void __launch_bounds__(64) k_free_cells(Rows s, int NX, int NY, unsigned char *free_cell) {
+  if (!after_previous()) return;
+  const int cell = blockIdx.x * 64 + threadIdx.x;
+  if (cell >= NX * NY) return;
+  int links = 0;
+  bool held = holds(s, 3 * cell + 2, 3 * cell + 2, 3 * cell + 2) != 0;
+  cell_faces(s, NX, NY, cell, [&](int to) {
+    links += to >= 0;
+    held |= to < 0;
+  });
+  free_cell[cell] = !held && links >= 1 && links <= 2 && cut_off_first(s, NX, NY, cell);
+}
+
 int ensure_system(mic_ctx *ctx, int which, int64_t n) {
   mic_system_store &S = ctx->sys[which];
   if (S.n == n && S.cnt) return MIC_OK;
@@ -511,12 +607,14 @@ int ensure_system(mic_ctx *ctx, int which, int64_t n) {
   cudaFree(S.col);
   cudaFree(S.val);
   cudaFree(S.rhs);
+  cudaFree(S.free_cell);
   if (S.lu_exec) cudaGraphExecDestroy(S.lu_exec);
   mic_front_plan_free(S.plan);
   S = mic_system_store{};
   if (cudaMalloc(&S.cnt, sizeof(int) * n) != cudaSuccess || cudaMalloc(&S.col, sizeof(int) * n * kMaxEnt) != cudaSuccess ||
       cudaMalloc(&S.val, sizeof(double) * n * kMaxEnt) != cudaSuccess ||
-      cudaMalloc(&S.rhs, sizeof(double) * n) != cudaSuccess)
+      cudaMalloc(&S.rhs, sizeof(double) * n) != cudaSuccess ||
+      (which == 0 && cudaMalloc(&S.free_cell, (size_t)n / 3) != cudaSuccess))
     return MIC_ERR_NOMEM;
   S.n = n;
   S.width = kMaxEnt;
@@ -646,6 +744,12 @@ extern "C" int mic_form_vep_system(mic_ctx *ctx, const mic_subduction_options *o
   if ((e = mic_words_out(ctx, s.K, 2 * sizeof(double)))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   const double K[2] = {ctx->h_words[0], ctx->h_words[1]};
+  {  // (after the wait: it runs while the host goes on)
+    MIC_KERNEL(ctx, "k_free_cells");
+    launch_after(k_free_cells, (unsigned)((nn + 63) / 64), 64, 0, ctx->stream, rows_of(ctx->sys[0]), NX, NY,
+                 ctx->sys[0].free_cell);
+  }
+  MIC_CUDA_TRY(cudaGetLastError());
   ctx->sys[0].Kbond = K[0];
   ctx->sys[0].Kcont = K[1];
   ctx->sys[0].factored = 0;

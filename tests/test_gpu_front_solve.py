@@ -132,3 +132,22 @@ def test_zero_columns_in_tall_fronts(nx, ny):
     r = np.add.reduceat(v * x[c], rp[:-1]) - b
     assert np.max(np.abs(r)) <= len(b) * np.finfo(float).eps * np.max(np.add.reduceat(np.abs(v), rp[:-1])) * np.max(np.abs(x))
     P.close()
+
+
+@pytest.mark.parametrize("k", [4, 6])
+def test_cut_off_pressure_cells_do_not_refuse_the_solve(k):
+    """A pair of pressure cells cut off between slab and plate: the matrix is singular, with no empty
+    row or column.  The solve goes on with the free pressure at zero: every equation but the one
+    that was dropped for it holds to rounding (n eps of the matrix and the solution)."""
+    wl, topt = W.subduction_box(nx_cells=128, ny_cells=32, nm=4, seed=10 + k)
+    topt.sub.slabAngle = 0.6 + 0.02 * k
+    P = gpu.MicProblem(wl)
+    P.subductionTimestep(topt, 0.0)
+    x = P.solution(P.STOKES)
+    rp, c, v, b = P.system(P.STOKES)
+    assert np.all(np.isfinite(x))
+    r = np.abs(np.add.reduceat(v * x[c], rp[:-1]) - b)
+    bound = len(b) * np.finfo(float).eps * np.max(np.add.reduceat(np.abs(v), rp[:-1])) * np.max(np.abs(x))
+    assert 0 < np.count_nonzero(r > bound) <= 1 or np.max(r) <= bound
+    assert np.all(np.isfinite(P.markers["p"]))
+    P.close()
