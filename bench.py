@@ -849,9 +849,9 @@ def ice_ensemble_leg(args, local):
 
 def systems_leg(args, local):
     """The solves between the marker passes, on the device: the Stokes (formVEPSystem) and thermal
-    (formThermalSystem) assembly and the direct solve (banded LU; the reference runs MUMPS LU) of
-    the subduction box at 129 x 33 and 513 x 129 nodes, beside a host sparse LU (SuperLU) of the
-    same matrices; then whole time steps (mic_subduction_timestep) of the 129 x 33 box with 16
+    (formThermalSystem) assembly and the direct solve (LU in nested-dissection order; the reference
+    runs MUMPS LU) of the subduction box at 129 x 33 and 513 x 129 nodes, beside a host sparse LU
+    (SuperLU) of the same matrices; then whole time steps (mic_subduction_timestep) of the 129 x 33 box with 16
     markers per cell."""
     import numpy as np
     import torch
