@@ -197,21 +197,23 @@ __global__ void k_scan_add(int *__restrict__ data, int64_t len, const int *__res
 // One pass of the sort.  Tiles are taken in order from a ticket, so the tiles a block waits for are
 // running or done.  A tile publishes per digit its own count, then (after looking back) the count of
 // all tiles up to it; a later tile adds counts backwards until it meets one of the latter, eight
-// tiles' words in flight at a time.  The wait is bounded: a block that gives up counts its tile's
-// markers in bad_cell (the binning then reports MIC_ERR_CELL) and leaves its items where they are.
+// tiles' words in flight at a time.  The wait is bounded (limit: rounds that find nothing new): a
+// block that gives up leaves its items where they are, adds to *lost, and sets
+// *flag, a word in the host's memory that stays set until the markers are uploaded or reset; every
+// call that waits for the device reads it there and returns MIC_ERR_CELL.  What the pass then leaves
+// is no order, so k_cell_start puts the identity in its place: the markers stay as they were.
 // Bound by the ranking (a chain of warp matches and shared-memory counts: half the issue slots, 15%
 // of HBM's rate); matching by eight ballots instead took 159 against 129 us, eight items a thread
 // 150.  The five launches of a pass (digit counts, three of their scan, scatter) became one: 16.8 M
 // markers 224 -> 129 us a pass, 65,536 markers 42 -> 10.
 constexpr unsigned kHas = 1u << 30, kUpTo = 2u << 30, kCount = kHas - 1;  // (2^30 markers of 440 B fit no GPU)
-constexpr int kLookRounds = 1 << 22;
 
 template <int IT>
 __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__restrict__ key_in, const int *__restrict__ val_in,
                                                             int use_iota, int *__restrict__ key_out,
                                                             int *__restrict__ val_out, int64_t n, int shift,
                                                             const int *__restrict__ counts, unsigned *tiles, int *ticket,
-                                                            unsigned long long *lost) {
+                                                            int limit, unsigned long long *lost, int *flag) {
   if (!after_previous()) return;
   constexpr int W = kSortThreads / 32, T = kSortThreads * IT;
   __shared__ int wcnt[W][kBuckets];        // per warp and digit: count, then offset in the tile's digit
@@ -289,6 +291,10 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__res
     int p = tile - 1, rounds = 0;
     bool done = false;
     while (!done) {
+      if (rounds >= limit) {
+        s_lost = 1;
+        break;
+      }
       unsigned w[LB];
 #pragma unroll
       for (int i = 0; i < LB; ++i) w[i] = p - i >= 0 ? (unsigned)slot[(int64_t)(p - i) * kBuckets] : (2u << 30);
@@ -305,10 +311,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__res
         }
       }
       p -= moved;
-      if (!done && moved == 0 && ++rounds > kLookRounds) {
-        s_lost = 1;
-        done = true;
-      }
+      rounds += moved == 0;
     }
     slot[(int64_t)tile * kBuckets] = kUpTo | (unsigned)(run + count);
   }
@@ -317,7 +320,10 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__res
   __syncthreads();
   const int items = (int)min((int64_t)T, n - first);
   if (s_lost) {  // (a later tile's counts are wrong too; its places are bounded below)
-    if (t == 0) atomicAdd(lost, (unsigned long long)items);
+    if (t == 0) {
+      atomicAdd(lost, (unsigned long long)items);
+      if (flag) *static_cast<volatile int *>(flag) = 1;
+    }
     for (int i = t; i < items; i += kSortThreads) {
       key_out[first + i] = key_in[first + i];
       val_out[first + i] = use_iota ? (int)(first + i) : val_in[first + i];
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_radix_pass(const int *__res
 // the passes of one sort on stream s; *kin / *vin: where the sorted keys and indices end up.  A
 // launch is counted and timed through ctx when it is given.
 void radix_launch(mic_ctx *ctx, cudaStream_t s, int **kin, int **kout, int **vin, int **vout, int64_t n, int passes,
-                  int *scratch, unsigned long long *lost) {
+                  int *scratch, int limit, unsigned long long *lost, int *flag) {
   const int64_t tiles = tiles_for(n);
   for (int p = 0; p < passes; ++p) {
     unsigned *words = reinterpret_cast<unsigned *>(scratch + kOffTiles + (int64_t)p * tiles * kBuckets);
@@ -359,10 +365,10 @@ void radix_launch(mic_ctx *ctx, cudaStream_t s, int **kin, int **kout, int **vin
     if (ctx) mic_prof_begin(ctx, "k_radix_pass", s);
     if (items_for(n) == kItemsSmall)
       launch_after(k_radix_pass<kItemsSmall>, (unsigned)tiles, kSortThreads, 0, s, *kin, *vin, p == 0, *kout, *vout,
-                   n, p * kRadixBits, counts, words, scratch + kOffTicket + p, lost);
+                   n, p * kRadixBits, counts, words, scratch + kOffTicket + p, limit, lost, flag);
     else
       launch_after(k_radix_pass<kItemsLarge>, (unsigned)tiles, kSortThreads, 0, s, *kin, *vin, p == 0, *kout, *vout,
-                   n, p * kRadixBits, counts, words, scratch + kOffTicket + p, lost);
+                   n, p * kRadixBits, counts, words, scratch + kOffTicket + p, limit, lost, flag);
     if (ctx) mic_prof_end(ctx, s);
     int *x = *kin;
     *kin = *kout;
@@ -374,9 +380,10 @@ void radix_launch(mic_ctx *ctx, cudaStream_t s, int **kin, int **kout, int **vin
 }
 
 // From the sorted (cell, quadrant) keys: qs[q] = first sorted position with key >= q for
-// q in [0, 4*ncells+4] (when qs is given) and cs[c] = qs[4c] for c in [0, ncells+1].
+// q in [0, 4*ncells+4] (when qs is given) and cs[c] = qs[4c] for c in [0, ncells+1].  After a sort
+// that gave up: the identity as the order, no marker in any cell, and *lost all markers.
 __global__ void k_cell_start(const int *__restrict__ skey, int64_t n, int ncells, int *__restrict__ cs,
-                             int *__restrict__ qs) {
+                             int *__restrict__ qs, unsigned long long *lost, int *perm) {
   if (!after_previous()) return;
   // one thread per (cell, quadrant) key q in [0, 4 ncells + 4]: the run of key q starts at the
   // first sorted position whose key is >= q (n when there is none), so empty stretches of cells
@@ -389,7 +396,11 @@ __global__ void k_cell_start(const int *__restrict__ skey, int64_t n, int ncells
   const int64_t qmax = 4LL * ncells + 4;
   if (q > qmax) return;
   int64_t lo = 0, hi = n;
-  if (n > 0) {
+  if (*lost) {
+    if (q == 0) *lost = (unsigned long long)n;
+    for (int64_t k = q; k < n; k += qmax + 1) perm[k] = (int)k;
+    hi = 0;
+  } else if (n > 0) {
     const int64_t g = q * n / (qmax + 1);  // in [0, n)
     if (skey[g] < q) {
       lo = g + 1;
@@ -537,13 +548,14 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out, bool step) {
   }
   MIC_CUDA_TRY(cudaGetLastError());
   int *kin = ctx->key, *kout = ctx->key_alt, *vin = ctx->perm, *vout = ctx->perm_alt;
-  radix_launch(ctx, ctx->stream, &kin, &kout, &vin, &vout, n, passes, ctx->sort_buf, &ctx->d_status->bad_cell);
+  radix_launch(ctx, ctx->stream, &kin, &kout, &vin, &vout, n, passes, ctx->sort_buf, ctx->sort_limit,
+               &ctx->d_status->bad_cell, ctx->h_lost);
   MIC_CUDA_TRY(cudaGetLastError());
   // kin / vin now hold the sorted keys and the permutation
   {
     MIC_KERNEL(ctx, "k_cell_start");
     launch_after(k_cell_start, grid_for(4LL * ctx->ncells + 5), kBlock, 0, ctx->stream, kin, n, ctx->ncells,
-                 ctx->cell_start, ctx->quad_start);
+                 ctx->cell_start, ctx->quad_start, &ctx->d_status->bad_cell, vin);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   GatherCols g;
@@ -576,9 +588,9 @@ int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out, bool step) {
   ctx->geo_valid = 1;  // computed by the gather
   ctx->wn_valid = 0;
   if (n_out) {
-    if ((e = mic_fetch_status(ctx))) return e;
+    e = mic_fetch_status(ctx);
     *n_out = (int64_t)ctx->h_status->n_out;
-    if (ctx->h_status->bad_cell) return MIC_ERR_CELL;
+    if (e) return e;
   }
   return MIC_OK;
 }
@@ -826,9 +838,10 @@ extern "C" int mic_bin_sort_noalloc(const double *X, const double *Y, int64_t n,
     if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
     // the last pass must write the caller's perm[]: pick the buffers accordingly (the first reads none)
     int *kin = key, *kout = key_alt, *vin = (passes & 1) ? val_alt : perm, *vout = (passes & 1) ? perm : val_alt;
-    radix_launch(nullptr, s, &kin, &kout, &vin, &vout, n, passes, sort, d_lost);
+    radix_launch(nullptr, s, &kin, &kout, &vin, &vout, n, passes, sort, kLookRounds, d_lost, nullptr);
     if (cudaGetLastError() != cudaSuccess) return MIC_ERR_CUDA;
-    launch_after(k_cell_start, grid_for(4LL * ncells + 5), kBlock, 0, s, kin, n, (int)ncells, cell_start, nullptr);
+    launch_after(k_cell_start, grid_for(4LL * ncells + 5), kBlock, 0, s, kin, n, (int)ncells, cell_start, nullptr,
+                 d_lost, vin);
   } else {
     if (cudaMemsetAsync(cell_start, 0, sizeof(int32_t) * (size_t)(ncells + 2), s) != cudaSuccess)
       return MIC_ERR_CUDA;

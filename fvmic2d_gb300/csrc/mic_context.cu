@@ -433,10 +433,13 @@ extern "C" int mic_create(mic_ctx **out, int device, void *stream, int NX, int N
     return MIC_ERR_NOMEM;
   }
   memset(ctx->h_status, 0, sizeof(Status));
-  if (cudaHostAlloc((void **)&ctx->h_words, kWordsOut, cudaHostAllocDefault) != cudaSuccess) {
+  if (cudaHostAlloc((void **)&ctx->h_words, kWordsOut + sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
     free_ctx(ctx);
     return MIC_ERR_NOMEM;
   }
+  ctx->h_lost = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(ctx->h_words) + kWordsOut);
+  *ctx->h_lost = 0;
+  ctx->sort_limit = kLookRounds;
   cudaMemcpyToSymbol(c_f64_off, h_f64_off, sizeof(h_f64_off));
   cudaMemcpyToSymbol(c_i32_off, h_i32_off, sizeof(h_i32_off));
   for (int b = 0; b < 4; ++b) {
@@ -574,6 +577,7 @@ extern "C" int mic_markers_upload(mic_ctx *ctx, const mic_marker *host, int64_t 
   ctx->has_grain = 0;  // grain column back to its uniform default
   mic_invalidate_sort(ctx);
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  *ctx->h_lost = 0;  // (every binning of the markers before has ended)
   return MIC_OK;
 }
 
@@ -642,7 +646,7 @@ extern "C" int mic_markers_download(mic_ctx *ctx, mic_marker *host, int64_t n) {
   MIC_CUDA_TRY(cudaMemcpyAsync(host, ctx->stage_aos, (size_t)n * sizeof(mic_marker), cudaMemcpyDeviceToHost,
                                ctx->stream));
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
+  return mic_sort_error(ctx);
 }
 
 extern "C" int mic_markers_count(mic_ctx *ctx, int64_t *n) {
@@ -666,7 +670,7 @@ extern "C" int mic_nodal_download(mic_ctx *ctx, int f, double *host) {
   MIC_CUDA_TRY(cudaMemcpyAsync(host, ctx->nodal[f], sizeof(double) * (size_t)ctx->P.NX * ctx->P.NY,
                                cudaMemcpyDeviceToHost, ctx->stream));
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
+  return mic_sort_error(ctx);
 }
 
 // ---- batched nodal transfers --------------------------------------------------------
@@ -734,7 +738,7 @@ int nodal_batch(mic_ctx *ctx, const int *fields, const double *const *host_in, d
   }
   MIC_CUDA_TRY(cudaGetLastError());
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
+  return host_in ? MIC_OK : mic_sort_error(ctx);
 }
 
 }  // namespace
@@ -757,6 +761,13 @@ extern "C" int mic_synchronize(mic_ctx *ctx) {
   if (!ctx) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return mic_sort_error(ctx);
+}
+
+extern "C" int mic_debug_set_wait_limit(mic_ctx *ctx, int which, int limit) {
+  if (!ctx || which != MIC_WAIT_SORT || limit < 0) return MIC_ERR_ARG;
+  ctx->sort_limit = limit;
+  ctx->gen++;  // (captured steps hold the limit)
   return MIC_OK;
 }
 
@@ -807,16 +818,21 @@ int mic_clear(mic_ctx *ctx, const mic_clear_list &l) {
 
 int mic_words_out(mic_ctx *ctx, const void *dev, size_t bytes) { return words_out(ctx, dev, ctx->h_words, bytes); }
 
-int mic_fetch_status(mic_ctx *ctx) {
+static int status_to_host(mic_ctx *ctx) {
   if (const int e = words_out(ctx, ctx->d_status, ctx->h_status, sizeof(Status))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return MIC_OK;
 }
 
+int mic_fetch_status(mic_ctx *ctx) {
+  const int e = status_to_host(ctx);
+  return e ? e : mic_sort_error(ctx);
+}
+
 extern "C" int mic_get_status(mic_ctx *ctx, mic_status *st) {
   if (!ctx || !st) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
-  if (const int e = mic_fetch_status(ctx)) return e;
+  if (const int e = status_to_host(ctx)) return e;  // (the record itself: whatever it holds)
   st->bad_cell = ctx->h_status->bad_cell;
   st->nan_residual = ctx->h_status->nan_residual;
   st->nan_dsxy = ctx->h_status->nan_dsxy;
@@ -1099,6 +1115,7 @@ extern "C" int mic_reset_markers(mic_ctx *ctx) {
   ctx->has_grain = 0;
   ctx->gen++;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  *ctx->h_lost = 0;
   return MIC_OK;
 }
 

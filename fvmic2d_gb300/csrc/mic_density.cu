@@ -713,6 +713,7 @@ extern "C" int mic_check_marker_density(mic_ctx *ctx, const mic_density_options 
   MIC_CUDA_TRY(cudaMemcpyAsync(&h, tot, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
   MIC_CUDA_TRY(cudaMemcpyAsync(herr, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if ((e = mic_sort_error(ctx))) return e;
   if (herr[0]) return MIC_ERR_DENSITY;
   // ---- removal ----
   const unsigned long long s0 = ctx->rng48;

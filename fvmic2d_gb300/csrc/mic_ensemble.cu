@@ -420,7 +420,10 @@ extern "C" int mic_ensemble_synchronize(mic_ensemble *E) {
   if (!E) return MIC_ERR_ARG;
   cudaSetDevice(E->device);
   cudaError_t ce = cudaStreamSynchronize(E->stream);
-  return ce == cudaSuccess ? MIC_OK : fail(ce);
+  if (ce != cudaSuccess) return fail(ce);
+  for (const mic_ctx *c : E->m)
+    if (const int e = mic_sort_error(c)) return e;
+  return MIC_OK;
 }
 
 extern "C" int mic_ensemble_launch_count(mic_ensemble *E, int64_t *launches, int64_t *graph_kernels) {

@@ -43,7 +43,7 @@ struct Status {
   unsigned long long nan_residual;  // NaN strain-rate residual (updateMarkerStrainPressure.c:302-306)
   unsigned long long nan_dsxy;      // NaN interpolated dsxy (updateMarkerStress.c:136-142)
   unsigned long long n_out;         // out-of-domain markers after the last binning
-  unsigned long long bad_cell;      // impossible cell index (markers.c:74-77): markers not placed (cleared with n_out)
+  unsigned long long bad_cell;      // markers the last binning could not place (cleared with n_out)
   unsigned long long bad_law;       // unknown viscosity law (viscosity.c:60-62)
   int is_yielding;                  // any marker yielded in the last checkPlasticYielding (cleared with bad_law)
   int pad;
@@ -52,6 +52,8 @@ struct Status {
 };
 
 constexpr size_t kWordsOut = 512;  // bytes of a context's pinned buffer for small results
+
+constexpr int kLookRounds = 1 << 22;  // a radix pass's look-back: seconds, where it takes microseconds
 
 // Composite creep (law 7) settings and per-pass counters
 struct CreepConfig {
@@ -177,6 +179,8 @@ struct mic_ctx {
   mic::Status *d_status;
   mic::Status *h_status;  // pinned mirror
   double *h_words;        // pinned: small results on their way to the host (kWordsOut bytes)
+  int *h_lost;            // pinned, behind them: a sort has given up since the markers were last replaced
+  int sort_limit;         // rounds a radix pass looks back for (kLookRounds)
   unsigned char *stage_aos;  // device staging for AoS transfers
   int64_t stage_cap;
   double residuals[100];
@@ -260,7 +264,12 @@ void mic_invalidate_sort(mic_ctx *ctx);
 void mic_front_plan_free(mic_front_plan *plan);  // (mic_front_lu.cu)
 // step: also clears what the first pieces of a step add to (max_bits, the yield pass's results)
 int mic_bin_and_sort(mic_ctx *ctx, int64_t *n_out, bool step = false);
-int mic_fetch_status(mic_ctx *ctx);  // *d_status into *h_status; waits for the stream
+// *d_status into *h_status; waits for the stream; MIC_ERR_CELL when a sort has given up
+int mic_fetch_status(mic_ctx *ctx);
+// after a wait for the device: MIC_ERR_CELL when a sort has given up since the markers were replaced
+inline int mic_sort_error(const mic_ctx *ctx) {
+  return *static_cast<const volatile int *>(ctx->h_lost) ? MIC_ERR_CELL : MIC_OK;
+}
 // up to kWordsOut bytes into h_words, without waiting
 int mic_words_out(mic_ctx *ctx, const void *dev, size_t bytes);
 // the pieces of a time step's calls whose results are read together: launches without a wait

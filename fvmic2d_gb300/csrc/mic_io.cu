@@ -103,6 +103,7 @@ extern "C" int mic_save_markers_binary(mic_ctx *ctx, const char *path, double el
     if ((e = mic_scan_exclusive(ctx, pos, n + 1, aux))) return e;
     MIC_CUDA_TRY(cudaMemcpyAsync(&count, pos + n, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if ((e = mic_sort_error(ctx))) return e;
   }
   PackPtrs pp;
   size_t off[kNFields], bytes[kNFields], at = 0;
@@ -181,5 +182,5 @@ extern "C" int mic_restart_from_markers(mic_ctx *ctx, const char *path, double *
   if ((e = mic_bin_and_sort(ctx, nullptr))) return e;  // findMarkerCells (restart.c:114)
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (elapsed_time) *elapsed_time = t;
-  return MIC_OK;
+  return mic_sort_error(ctx);
 }

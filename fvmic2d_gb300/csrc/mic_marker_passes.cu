@@ -1592,11 +1592,6 @@ YieldCols yield_cols(mic_ctx *ctx) {
   return c;
 }
 
-int read_status(mic_ctx *ctx) {
-  if (const int e = mic_fetch_status(ctx)) return e;
-  return ctx->h_status->bad_cell ? MIC_ERR_CELL : MIC_OK;  // markers the last binning could not place
-}
-
 int run_max(mic_ctx *ctx, int col, int absval, double *out) {
   unsigned long long *d = &ctx->d_status->max_bits;
   MIC_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream));
@@ -2188,7 +2183,7 @@ extern "C" int mic_check_plastic_yielding(mic_ctx *ctx, double dt, int *is_yield
   (void)elapsed_time;  // only read by the SANDBOX build of the reference
   int e = yield_launch(ctx, dt);
   if (e) return e;
-  if ((e = read_status(ctx))) return e;
+  if ((e = mic_fetch_status(ctx))) return e;
   if (is_yielding) *is_yielding = ctx->h_status->is_yielding;
   return ctx->h_status->bad_law ? MIC_ERR_LAW : MIC_OK;
 }
@@ -2206,7 +2201,7 @@ extern "C" int mic_update_viscosity(mic_ctx *ctx) {
     }
     MIC_CUDA_TRY(cudaGetLastError());
   }
-  if ((e = read_status(ctx))) return e;
+  if ((e = mic_fetch_status(ctx))) return e;
   return ctx->h_status->bad_law ? MIC_ERR_LAW : MIC_OK;
 }
 
@@ -2259,7 +2254,7 @@ extern "C" int mic_update_marker_strain_pressure(mic_ctx *ctx, double dt) {
   CHECK_CTX();
   int e = strain_launch(ctx, dt);
   if (e) return e;
-  if ((e = read_status(ctx))) return e;
+  if ((e = mic_fetch_status(ctx))) return e;
   return ctx->h_status->nan_residual ? MIC_ERR_NAN : MIC_OK;
 }
 
@@ -2704,7 +2699,7 @@ extern "C" int mic_step_pre_stokes(mic_ctx *ctx, double dt_disp, int *is_yieldin
   int e;
   if ((e = run_segments(ctx, 0, 3, dt_disp, 0.0, 0, 0))) return e;
   if (is_yielding || max_T) {
-    if ((e = read_status(ctx))) return e;
+    if ((e = mic_fetch_status(ctx))) return e;
     if (is_yielding) *is_yielding = ctx->h_status->is_yielding;
     if (max_T) memcpy(max_T, &ctx->h_status->max_bits, sizeof(double));
   }

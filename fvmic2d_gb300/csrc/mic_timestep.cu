@@ -173,7 +173,6 @@ extern "C" int mic_subduction_timestep(mic_ctx *ctx, const mic_timestep_options 
     MIC_TRY(mic_residual_launch(ctx));
     MIC_TRY(mic_limit_launch(ctx, o->displacementStepLimit));
     MIC_TRY(mic_fetch_status(ctx));
-    if (ctx->h_status->bad_cell) return MIC_ERR_CELL;
     if (ctx->h_status->nan_residual) return MIC_ERR_NAN;
     mic_residual_store(ctx, iPlastic, &rep->residual);
     MIC_TRY(mic_check_convergence(ctx, 1e-16, 1e-1, iPlastic, &converged));

@@ -68,6 +68,7 @@ SIGNATURES = {
     "mic_get_status": (_I, [_P, _P]),
     "mic_debug_sorted_ids": (_I, [_P, _P]),
     "mic_debug_cell_start": (_I, [_P, _P]),
+    "mic_debug_set_wait_limit": (_I, [_P, _I, _I]),
     "mic_debug_div_sp": (_I, [_P, _P, _P, _I64, _P]),
     "mic_markers_reset_host": (_I, [_P, _I64]),
     "mic_get_strain_rate_residual": (_I, [_P, _I, _DP]),
@@ -211,6 +212,11 @@ class MicProblem:
     def _check(self, code, what):
         if code != 0:
             raise MicError(code, what)
+
+    WAIT_SORT = 0
+
+    def debug_set_wait_limit(self, which, limit):
+        self._check(self.L.mic_debug_set_wait_limit(self.h, which, limit), "mic_debug_set_wait_limit")
 
     def set_stress_rotation(self, rotation):
         """MIC_ROTATION_EXACT (markers.c:2158-2164) or MIC_ROTATION_JAUMANN (2147-2156)"""

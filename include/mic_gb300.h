@@ -32,7 +32,10 @@ enum {
   MIC_ERR_ARG = 1,        /* invalid argument (bad field id, stagger, method, size) */
   MIC_ERR_CUDA = 2,       /* CUDA runtime error (context left usable where CUDA allows) */
   MIC_ERR_NOMEM = 3,      /* device or host allocation failed */
-  MIC_ERR_CELL = 4,       /* impossible cell index; markers.c:74-77 aborts */
+  MIC_ERR_CELL = 4,       /* impossible cell index (markers.c:74-77 aborts): a binning that gave up waiting for
+                             its sort.  The markers keep their order and no cell holds any, so what a step
+                             computes after it is not valid; every call that waits for the device returns this
+                             code until the markers are uploaded or reset */
   MIC_ERR_NAN = 5,        /* NaN strain-rate residual; updateMarkerStrainPressure.c:302-306 aborts */
   MIC_ERR_LAW = 6,        /* undefined viscosity law; viscosity.c:60-62 aborts */
   MIC_ERR_BC = 7,         /* unsupported boundary type, or a routine outside the marker path on a grid
@@ -47,7 +50,7 @@ enum {
 };
 
 typedef struct {
-  uint64_t bad_cell;      /* markers with an impossible cell index in the last binning */
+  uint64_t bad_cell;      /* markers the last binning could not place */
   uint64_t nan_residual;  /* markers with a NaN strain-rate residual */
   uint64_t nan_dsxy;      /* markers whose interpolated dsxy was NaN (the reference only prints) */
   uint64_t bad_law;       /* markers whose material has an undefined viscosity law */
@@ -224,6 +227,11 @@ int mic_get_status(mic_ctx *ctx, mic_status *status);
  * ((NX-1)*(NY-1)+2 entries; the last two bracket the out-of-domain markers) */
 int mic_debug_sorted_ids(mic_ctx *ctx, int32_t *ids);
 int mic_debug_cell_start(mic_ctx *ctx, int32_t *cell_start);
+/* the library's bounded waits between blocks, for tests of what happens when one runs out: rounds
+ * before it does (0: it gives up at once).  MIC_WAIT_SORT: a radix pass's look-back (default 2^22,
+ * seconds; MIC_ERR_CELL) */
+enum { MIC_WAIT_SORT = 0 };
+int mic_debug_set_wait_limit(mic_ctx *ctx, int which, int limit);
 /* num[k] / den[k] (host arrays) computed the way the kernels divide by a grid spacing: the
  * correctly rounded reciprocal and one residual correction (the FMA-free build divides) */
 int mic_debug_div_sp(mic_ctx *ctx, const double *num, const double *den, int64_t n, double *quot);
@@ -457,7 +465,8 @@ int mic_ensemble_get_stream(mic_ensemble *ens, void **stream);
  *   cell_start [(NX-1)*(NY-1)+2]  out: first sorted position of each cell; the last two
  *                     entries bracket the out-of-domain markers
  *   stream            cudaStream_t to run on (NULL: the legacy default stream)
- *   n_out             optional host pointer: markers outside the domain (synchronises stream)
+ *   n_out             optional host pointer: markers outside the domain (synchronises stream;
+ *                     MIC_ERR_CELL after a sort that gave up: perm is the identity, cell_start 0)
  * Limits: n <= MIC_NOALLOC_MAX_MARKERS and (NX-1)*(NY-1) <= MIC_NOALLOC_MAX_CELLS, else
  * MIC_ERR_CAPACITY.  The first call in a CUDA context (on each device, and again after a
  * cudaDeviceReset) looks up the array's device address, so make that first call before
