@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "mic_internal.cuh"
+#include "mic_pivot.cuh"
 
 using namespace mic;
 
@@ -102,55 +103,6 @@ struct SystemRows {  // the assembled rows (mic_systems.cu)
   const unsigned char *free_cell;  // per node: cells whose pressure no equation holds (null: none)
 };
 
-// What a row offers as pivot of a column: the leading 21 bits of |a| (exponent, 10 of mantissa) above
-// the row's number in one integer, so that the search costs no FP64 slot and one reduction of a warp
-// finds value and row (a reduction of the high word, a ballot and a shuffle for the row took 90
-// clocks more, twice a column).  Rows whose keys agree differ by less than 2^-10 relatively: the
-// multipliers stay below 1 + 2^-10, as good as 1 for the growth of the sums.  A NaN counts as 0.
-// 0 is no offer.
-constexpr int kOfferRow = 11, kOfferRows = 1 << kOfferRow;
-__device__ __forceinline__ unsigned pivot_offer(double a, int row) {
-  const unsigned h = (unsigned)((unsigned long long)dbits(a) >> 32) & 0x7fffffffu;
-  return ((h <= 0x7ff00000u ? h >> 10 : 0u) + 1) << kOfferRow | (unsigned)row;
-}
-__device__ __forceinline__ unsigned warp_best(unsigned offer) { return __reduce_max_sync(0xffffffffu, offer); }
-__device__ __forceinline__ int offer_row(unsigned offer) { return (int)(offer % kOfferRows); }
-__device__ __forceinline__ bool offer_counts(unsigned offer) { return offer >= 2 * kOfferRows; }
-
-// a column in which no offer counts (every |a| below 2^-1032, or NaN): the exact largest |a| of
-// the rows not used, the first of them when there is no other
-__device__ int pivot_rare(const double *col, int stride, int rows, const int *used) {
-  long long best = -2;
-  int p = 0;
-  for (int r = 0; r < rows; ++r) {
-    if (used && used[r]) continue;
-    const long long b = dbits(col[(int64_t)r * stride]) & 0x7fffffffffffffffLL;
-    const long long k = b <= 0x7ff0000000000000LL ? b : -1;
-    if (k > best) {
-      best = k;
-      p = r;
-    }
-  }
-  return p;
-}
-
-// 1 / p by Newton's iteration of third order from an FP32 reciprocal of p's mantissa: with
-// e = 1 - m r, |e| < 2^-22, r (1 + e + e^2) is 1 / m to e^3 < 2^-66, so to rounding, in three
-// dependent FP64 operations (a pivot's reciprocal is on the chain of every column step).  Pivots
-// whose reciprocal leaves the normal range are divided.
-__device__ __forceinline__ double pivot_rcp(double p) {
-  const unsigned long long b = (unsigned long long)dbits(p);
-  const int ex = (int)(b >> 52) & 0x7ff;
-  if (ex < 8 || ex > 2038) return p != 0.0 ? 1.0 / p : 0.0;
-  const double m = __longlong_as_double((long long)((b & 0xfffffffffffffULL) | 0x3ff0000000000000ULL));
-  const float f = __uint_as_float(0x3f800000u | ((unsigned)(b >> 29) & 0x7fffffu));
-  const double r0 = f64_of(__frcp_rn(f));
-  const double e = fma(-m, r0, 1.0);
-  const double r = fma(r0, fma(e, e, e), r0);  // in (1/2, 1]
-  const long long rb = dbits(r) - ((long long)(ex - 1023) << 52);
-  return __longlong_as_double(rb | (long long)(b & 0x8000000000000000ULL));
-}
-
 // value of column c (of q's columns) in left-over row i of child k: where the child keeps it
 __device__ __forceinline__ const double *child_row(const Front &k, int i, const double *F, const int *act) {
   return k.full ? F + k.f + (int64_t)act[k.left + i] * k.C + k.P : F + k.f + (int64_t)i * (k.C - k.P);
@@ -175,7 +127,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   if (!after_previous()) return;
   constexpr int kSmallWarps = kSmallThreads / 32;
   extern __shared__ double A[];
-  __shared__ unsigned red[32];
+  __shared__ Offer red[32];
   __shared__ double s_rcp;
   const Front q = fr[first + blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -223,14 +175,14 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   int G = (R + 31) / 32;  // candidate entries waiting in red
   for (int g = warp; g < G; g += kSmallWarps) {
     const int r = g * 32 + lane;
-    const unsigned best = warp_best(r < R ? pivot_offer(A[r * ld], r) : 0u);
-    if (lane == 0) red[g] = best;
+    const long long key = r < R ? pivot_key(A[r * ld]) : -2;
+    if (lane == warp_best(key)) red[g] = Offer{key, r};
   }
   __syncthreads();
   for (int j = 0; j < P; ++j) {
-    const unsigned best = warp_best(lane < G ? red[lane] : 0u);
-    int p = offer_row(best);
-    if (!offer_counts(best)) {
+    const Offer best = red[warp_best(lane < G ? red[lane].key : -2)];
+    int p = best.row;
+    if (best.key <= 0) {
       p = j + pivot_rare(A + j * ld + j, ld, R - j, nullptr);
       __syncthreads();  // every thread has read the column before rows move
     }
@@ -260,8 +212,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
           v = row[c] - l * piv[c];
           row[c] = v;
         }
-        const unsigned b = warp_best(r < R ? pivot_offer(v, r) : 0u);
-        if (lane == 0) red[g] = b;
+        const long long key = r < R ? pivot_key(v) : -2;
+        if (lane == warp_best(key)) red[g] = Offer{key, r};
         c += SL;
       }
       if (r < R) {
@@ -329,7 +281,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
   if (NB == 16) next_may_start();
   if (!after_previous()) return;
   extern __shared__ double S[];
-  __shared__ unsigned red[32];
+  __shared__ Offer red[32];
   __shared__ double s_rcp;
   __shared__ int piv[NB];  // rows of the pivots so far
   const Front q = fr[first + blockIdx.x];
@@ -361,8 +313,8 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
     }
   }
   __syncthreads();
-  unsigned offer = 0;
-  for (int r = tid; r < na; r += nt) offer = max(offer, pivot_offer(S[r * LD], r));
+  Offer offer = {-2, 0};
+  for (int r = tid; r < na; r += nt) take_better(offer, S[r * LD], r);
   // row groups and column shares of phase 2; the reciprocal's warp takes part only where there is
   // more work than the others can share evenly
   const int G = (na + 31) / 32, workers = G >= nw ? nw : nw - 1, CS = max(1, workers / G);
@@ -373,7 +325,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
       const double rcp = s_rcp;
       const int p = piv[j];
       const bool more = j + 1 < nb;
-      offer = 0;
+      offer = Offer{-2, 0};
       const double pn = more ? S[p * LD + j + 1] : 0.0;
       unsigned bit = 1;
       for (int r = tid; r < na; r += nt, bit <<= 1) {
@@ -388,19 +340,18 @@ __global__ void __launch_bounds__(kPanelThreads, 2)
         if (more) {
           const double v = an - l * pn;
           row[j + 1] = v;
-          offer = max(offer, pivot_offer(v, r));
+          take_better(offer, v, r);
         }
       }
     }
     if (j + 1 == nb) break;
-    offer = warp_best(offer);
-    if (lane == 0) red[warp] = offer;
+    if (lane == warp_best(offer.key)) red[warp] = offer;
     __syncthreads();
     // phase 2: the pivot of column j + 1 and its reciprocal; the columns after it
     if (warp == nw - 1) {
-      const unsigned best = warp_best(lane < nw ? red[lane] : 0u);
-      int p = offer_row(best);
-      if (!offer_counts(best)) p = pivot_rare(S + j + 1, LD, na, used);
+      const Offer best = red[warp_best(lane < nw ? red[lane].key : -2)];
+      int p = best.row;
+      if (best.key <= 0) p = pivot_rare(S + j + 1, LD, na, used);
       if (lane == 0) {
         const double v = S[p * LD + j + 1];
         s_rcp = pivot_rcp(v);
@@ -531,7 +482,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   extern __shared__ double S[];
   __shared__ PanelOffer<NB> ex[kOffers][CL];
   __shared__ __align__(8) unsigned long long bars[kOffers];
-  __shared__ unsigned red[32];
+  __shared__ Offer red[32];
   __shared__ double s_rcp;
   __shared__ int s_win, s_place;  // the last winner and the place of its offer
   __shared__ int s_rare;          // the column's exchange is to be done again
@@ -574,8 +525,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   __syncthreads();
   // every block of the cluster has come this far before one sends to another
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  unsigned offer = 0;
-  for (int r = tid; r < m; r += nt) offer = max(offer, pivot_offer(S[r * LD], r));
+  Offer offer = {-2, -1};
+  for (int r = tid; r < m; r += nt) take_better(offer, S[r * LD], r);
   const int G = (m + 31) / 32, workers = nw - 1, CS = max(1, workers / max(G, 1));
   unsigned mine = 0;  // which of this thread's rows are pivots
   int sent = 0;       // exchanges so far (the sending warp)
@@ -602,13 +553,14 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
     // the same choice in every block; the lanes form all offers' reciprocals beside it
     const int d = min(lane, CL - 1), row = (int)ex[place][d].row;
     const double w = ex[place][d].v[c];
-    const unsigned mine = row < 0 ? 0u : pivot_offer(w, CL - 1 - d), top = warp_best(lane < CL ? mine : 0u);
-    const double rcp = pivot_rcp(offer_counts(mine) ? w : 1.0);
-    if (lane < CL && mine == top) {
-      s_rcp = offer_counts(mine) ? rcp : pivot_rcp(w);
+    const long long key = lane < CL && row >= 0 ? pivot_key(w) : -2;
+    const int win = warp_best(key);
+    const double rcp = pivot_rcp(key > 0 ? w : 1.0);
+    if (lane == win) {
+      s_rcp = key > 0 ? rcp : pivot_rcp(w);
       s_win = d;
       s_place = place;
-      s_rare = !again && !offer_counts(top);
+      s_rare = !again && key <= 0;
       piv[c] = row;
       if (lost) atomicAdd(&info[1], 1);
       if (again && rank == 0 && (dbits(w) << 1) == 0) atomicMin(&info[0], tab[q.col + k0 + c]);
@@ -621,7 +573,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       const double rcp = s_rcp;
       const int p = piv[j] - base;
       const bool more = j + 1 < nb;
-      offer = 0;
+      offer = Offer{-2, -1};
       const double pn = more ? pr[j + 1] : 0.0;
       unsigned bit = 1;
       for (int r = tid; r < m; r += nt, bit <<= 1) {
@@ -636,18 +588,16 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
         if (more) {
           const double v = an - l * pn;
           row[j + 1] = v;
-          offer = max(offer, pivot_offer(v, r));
+          take_better(offer, v, r);
         }
       }
     }
     if (j + 1 == nb) break;
-    offer = warp_best(offer);
-    if (lane == 0) red[warp] = offer;
+    if (lane == warp_best(offer.key)) red[warp] = offer;
     __syncthreads();
     // phase 2: the pivot of column j + 1 and its reciprocal; the columns after it
     if (warp == nw - 1) {
-      const unsigned best = warp_best(lane < nw ? red[lane] : 0u);
-      const int p = best ? offer_row(best) : -1;
+      const int p = red[warp_best(lane < nw ? red[lane].key : -2)].row;
       double v = 0.0;
       if (p >= 0 && lane > j && lane < nb) {
         v = S[p * LD + lane];
