@@ -727,21 +727,27 @@ __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
   const int *list = act + q.act + (int64_t)(1 - turn) * q.R + k0;
   double *base = F + q.f;
   const double *L = Lb + q.lb;
-  // every load in flight before the first is stored or used
-  double v[RT][CT];
-  int64_t at[RT];
+  // every load in flight before the first is stored or used; a large tile's own values come last, a
+  // few rows at a time: its multiply-adds take 17 us and more, and its SM has another block
+  constexpr bool LATE = RT * CT >= 16;
+  constexpr int RV = LATE ? (RT * CT >= 32 ? 2 : 4) : RT;  // rows of a thread loaded together
+  double v[RV][CT];
+  int64_t at[RV];
+  const auto load = [&](int a0) {
 #pragma unroll
-  for (int a = 0; a < RT; ++a) {
-    const int r = r0 + ti + 16 * a;
-    at[a] = r < na ? (int64_t)list[r] * q.C : -1;
-  }
-#pragma unroll
-  for (int a = 0; a < RT; ++a)
-#pragma unroll
-    for (int b = 0; b < CT; ++b) {
-      const int c = c0 + tj + 16 * b;
-      v[a][b] = (at[a] >= 0 && c < cend) ? base[at[a] + c] : 0.0;
+    for (int a = 0; a < RV; ++a) {
+      const int r = r0 + ti + 16 * (a0 + a);
+      at[a] = r < na ? (int64_t)list[r] * q.C : -1;
     }
+#pragma unroll
+    for (int a = 0; a < RV; ++a)
+#pragma unroll
+      for (int b = 0; b < CT; ++b) {
+        const int c = c0 + tj + 16 * b;
+        v[a][b] = (at[a] >= 0 && c < cend) ? base[at[a] + c] : 0.0;
+      }
+  };
+  if (!LATE) load(0);
   {
     constexpr int NU = NB * TC / 256, NL = TR * NB / 256, N1 = SOLVE ? NB * NB / 256 : 0, HALF = NL > 8 ? NL / 2 : NL;
     double u[NU], l[HALF], l1[N1 + 1];
@@ -779,6 +785,11 @@ __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
     __syncthreads();
   }
   const int steps = (nb + 3) & ~3;  // (zeros behind nb)
+  double w[RT][CT];  // the products' sum: one rounding at the values' size a panel, not one a product
+#pragma unroll
+  for (int a = 0; a < RT; ++a)
+#pragma unroll
+    for (int b = 0; b < CT; ++b) w[a][b] = 0.0;
 #pragma unroll 4
   for (int k = 0; k < steps; ++k) {
     double l[RT], u[CT];
@@ -789,15 +800,19 @@ __global__ void __launch_bounds__(256, TR >= 128 ? 2 : 3)
 #pragma unroll
     for (int a = 0; a < RT; ++a)
 #pragma unroll
-      for (int b = 0; b < CT; ++b) v[a][b] -= l[a] * u[b];
+      for (int b = 0; b < CT; ++b) w[a][b] += l[a] * u[b];
   }
 #pragma unroll
-  for (int a = 0; a < RT; ++a)
+  for (int a0 = 0; a0 < RT; a0 += RV) {
+    if (LATE) load(a0);
 #pragma unroll
-    for (int b = 0; b < CT; ++b) {
-      const int c = c0 + tj + 16 * b;
-      if (at[a] >= 0 && c < cend) base[at[a] + c] = v[a][b];
-    }
+    for (int a = 0; a < RV; ++a)
+#pragma unroll
+      for (int b = 0; b < CT; ++b) {
+        const int c = c0 + tj + 16 * b;
+        if (at[a] >= 0 && c < cend) base[at[a] + c] = v[a][b] - w[a0 + a][b];
+      }
+  }
 }
 
 // ---- back substitution ------------------------------------------------------------------
