@@ -115,9 +115,15 @@ __device__ __forceinline__ const double *child_row(const Front &k, int i, const 
 // once, then a lane takes a row (its multiplier in a register) and the warps share out rows and
 // columns; the warps that update column j + 1 also find its candidates.  Two barriers a step.
 // The step is bound by this chain (about 1 us) until a front exceeds some 50,000 multiply-adds,
-// then by the FP64 pipe.  A row's values are read four at a time before any is written: the
-// compiler cannot tell the row from the pivot row, so a load written after a store would wait
-// for it.
+// then by the FP64 pipe.
+// Pivots are taken in groups of four columns.  A step updates the group's columns and, of the
+// others, row j alone; the rest follow once a group, each value's products summed before they are
+// subtracted, which leaves a quarter of the roundings at the value's size.  Error against a refined
+// solution of 513 x 129 temperatures (largest, of the largest value): 1.27e-15; 1.65e-15 without
+// groups, 1.24e-15 in an elimination of the band.  GB300, solves of 129 x 33 and 513 x 129 Stokes and
+// of 513 x 129 temperatures with groups of 1, 2, 4, 8 and 16, ms: 1.94, 2.01, 1.98, 2.01, 2.09; 38.0,
+// 39.2, 38.7, 38.9, 40.1; 4.60, 4.98, 4.78, 4.81, 5.09.
+constexpr int kGroupCols = 4;
 template <int kSmallThreads>
 __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__restrict__ fr, int first,
                                                               const int *__restrict__ tab,
@@ -128,7 +134,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   constexpr int kSmallWarps = kSmallThreads / 32;
   extern __shared__ double A[];
   __shared__ Offer red[32];
-  __shared__ double s_rcp;
+  __shared__ double s_rcp[kGroupCols];
   const Front q = fr[first + blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int R = q.R, P = q.P, C = q.C, ld = C | 1;
@@ -179,37 +185,92 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
     if (lane == warp_best(key)) red[g] = Offer{key, r};
   }
   __syncthreads();
-  for (int j = 0; j < P; ++j) {
-    const Offer best = red[warp_best(lane < G ? red[lane].key : -2)];
-    int p = best.row;
-    if (best.key <= 0) {
-      p = j + pivot_rare(A + j * ld + j, ld, R - j, nullptr);
-      __syncthreads();  // every thread has read the column before rows move
-    }
-    for (int c = j + tid; c < C; c += kSmallThreads) {
-      const double up = A[p * ld + c], dn = A[j * ld + c];
-      A[j * ld + c] = up;
-      A[p * ld + c] = dn;
-      if (c == j) {
-        s_rcp = pivot_rcp(up);
-        if (up == 0.0) atomicMin(&info[0], tab[q.col + j]);
+  for (int j0 = 0; j0 < P; j0 += kGroupCols) {
+    const int je = min(j0 + kGroupCols, P);  // the group's end
+    for (int j = j0; j < je; ++j) {
+      const Offer best = red[warp_best(lane < G ? red[lane].key : -2)];
+      int p = best.row;
+      if (best.key <= 0) {
+        p = j + pivot_rare(A + j * ld + j, ld, R - j, nullptr);
+        __syncthreads();  // every thread has read the column before rows move
       }
+      for (int c = j0 + tid; c < C; c += kSmallThreads) {
+        const double up = A[p * ld + c], dn = A[j * ld + c];
+        A[j * ld + c] = up;
+        A[p * ld + c] = dn;
+        if (c == j) {
+          s_rcp[j - j0] = pivot_rcp(up);
+          if (up == 0.0) atomicMin(&info[0], tab[q.col + j]);
+        }
+      }
+      __syncthreads();
+      const double rcp = s_rcp[j - j0];
+      const int n = R - j - 1, m = je - j - 1;  // rows below, columns of the group after j
+      G = (n + 31) / 32;
+      const int SL = max(1, min(m, kSmallWarps / max(G, 1))), T1 = m > 0 ? G * SL : 0;
+      const int T2 = j > j0 ? (C - je + 31) / 32 : 0;
+      const double *piv = A + j * ld;
+      for (int t = warp; t < T1 + T2; t += kSmallWarps) {
+        if (t < T1) {  // rows below in the group's columns, the next column first, with its candidates
+          const int g = t % G, s = t / G, r = j + 1 + g * 32 + lane;
+          double *row = A + r * ld;
+          const double l = r < R ? row[j] * rcp : 0.0;
+          int c = j + 1 + s;
+          if (s == 0) {
+            double v = 0.0;
+            if (r < R) {
+              v = row[c] - l * piv[c];
+              row[c] = v;
+            }
+            const long long key = r < R ? pivot_key(v) : -2;
+            if (lane == warp_best(key)) red[g] = Offer{key, r};
+            c += SL;
+          }
+          if (r < R)
+            for (; c < je; c += SL) row[c] -= l * piv[c];
+        } else {  // row j, a row of U, behind the group
+          const int c = je + (t - T1) * 32 + lane;
+          const double l = j0 + lane < j ? piv[j0 + lane] * s_rcp[lane] : 0.0;
+          double sum = 0.0;
+          for (int k = 0; k < j - j0; ++k) {
+            const double lk = __shfl_sync(0xffffffffu, l, k);
+            if (c < C) sum += lk * A[(j0 + k) * ld + c];
+          }
+          if (c < C) A[j * ld + c] -= sum;
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    const double rcp = s_rcp;
-    const int n = R - j - 1;
+    // the columns behind the group, the next one first, with its candidates
+    const int n = R - je, kk = je - j0;
     G = (n + 31) / 32;
     const int SL = max(1, kSmallWarps / max(G, 1));
     for (int t = warp; t < G * SL; t += kSmallWarps) {
-      const int g = t % G, s = t / G, r = j + 1 + g * 32 + lane;
+      const int g = t % G, s = t / G, r = je + g * 32 + lane;
       double *row = A + r * ld;
-      const double *piv = A + j * ld;
-      const double l = r < R ? row[j] * rcp : 0.0;
-      int c = j + 1 + s;
-      if (s == 0 && j + 1 < P) {  // the next column first, with its candidates
+      const double *u = A + j0 * ld;
+      double l[kGroupCols];
+#pragma unroll
+      for (int k = 0; k < kGroupCols; ++k) {
+        l[k] = k < kk && r < R ? row[j0 + k] * s_rcp[k] : 0.0;
+      }
+      const auto sum = [&](int c) {
+        double a = 0.0;
+        if (kk == kGroupCols) {
+#pragma unroll
+          for (int k = 0; k < kGroupCols; ++k) a += l[k] * u[k * ld + c];
+        } else {
+#pragma unroll
+          for (int k = 0; k < kGroupCols - 1; ++k)
+            if (k < kk) a += l[k] * u[k * ld + c];
+        }
+        return a;
+      };
+      int c = je + s;
+      if (s == 0 && je < P) {
         double v = 0.0;
         if (r < R) {
-          v = row[c] - l * piv[c];
+          v = row[c] - sum(c);
           row[c] = v;
         }
         const long long key = r < R ? pivot_key(v) : -2;
@@ -217,17 +278,12 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
         c += SL;
       }
       if (r < R) {
-        for (; c + 3 * SL < C; c += 4 * SL) {
-          double v[4], u[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            v[i] = row[c + i * SL];
-            u[i] = piv[c + i * SL];
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) row[c + i * SL] = v[i] - l * u[i];
+        for (; c + SL < C; c += 2 * SL) {
+          const double v0 = row[c], v1 = row[c + SL], a0 = sum(c), a1 = sum(c + SL);
+          row[c] = v0 - a0;
+          row[c + SL] = v1 - a1;
         }
-        for (; c < C; c += SL) row[c] -= l * piv[c];
+        for (; c < C; c += SL) row[c] -= sum(c);
       }
     }
     __syncthreads();
