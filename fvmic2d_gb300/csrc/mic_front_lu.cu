@@ -1247,6 +1247,13 @@ T *carve(unsigned char *&p, size_t count) {
 }
 size_t room(size_t bytes) { return ((bytes + 255) / 256) * 256; }
 
+// A launch that was refused ends the solve there: what follows would read what it was to write, and a
+// graph without it must not be kept.
+#define LU_LAUNCH(...)                                                                        \
+  do {                                                                                        \
+    if (launch_after(__VA_ARGS__) != cudaSuccess) return mic_fail_cuda(ctx, cudaGetLastError()); \
+  } while (0)
+
 struct Buffers {
   int *info;
   double *F[2], *U, *Lb;
@@ -1254,12 +1261,14 @@ struct Buffers {
 };
 
 template <int NB, int TR, int TC, bool SOLVE>
-void update(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, double *F, int k0, int turn,
-            int rows, int coff, int cols, cudaStream_t st) {
+int update(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, double *F, int k0, int turn,
+           int rows, int coff, int cols, cudaStream_t st) {
   MIC_KERNEL_ON(ctx, "k_front_update", st);
-  launch_after(k_front_update<NB, TR, TC, SOLVE>, dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC),
-               kUpdateThreads, update_smem<NB, TR, TC, SOLVE>(), st, pl.d_fronts, L.first, k0, turn, coff, cols, F,
-               B.U, B.Lb + turn * pl.nL, B.act);
+  constexpr auto kernel = k_front_update<NB, TR, TC, SOLVE>;
+  LU_LAUNCH(kernel, dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC), kUpdateThreads,
+            (update_smem<NB, TR, TC, SOLVE>()), st, pl.d_fronts, L.first, k0, turn, coff, cols, F, B.U,
+            B.Lb + turn * pl.nL, B.act);
+  return MIC_OK;
 }
 
 // One level in panels.  The chain (panel, then its update of the next panel's columns) runs on the
@@ -1279,18 +1288,12 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     const size_t smem = (size_t)share * ((NB + 1) * sizeof(double) + kPanelBytes);
     {
       MIC_KERNEL_ON(ctx, "k_front_panel", chain);
-      const auto launch = [&](auto *kernel) {
-        launch_after(kernel, L.count * cl, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U,
-                     B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
-      };
-      if (cl == 8)
-        launch(k_front_panel_cluster<NB, 8>);
-      else if (cl == 4)
-        launch(k_front_panel_cluster<NB, 4>);
-      else if (cl == 2)
-        launch(k_front_panel_cluster<NB, 2>);
-      else
-        launch(k_front_panel<NB>);
+      const auto kernel = cl == 8   ? k_front_panel_cluster<NB, 8>
+                          : cl == 4 ? k_front_panel_cluster<NB, 4>
+                          : cl == 2 ? k_front_panel_cluster<NB, 2>
+                                    : k_front_panel<NB>;
+      LU_LAUNCH(kernel, L.count * cl, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U,
+                B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
     }
     // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);
@@ -1315,12 +1318,10 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
       // 33 Stokes, 7.48 for 257 x 65, 4.75 for 513 x 129 temperatures; up to one tile an SM 1.84, 7.45,
       // 4.65; up to four 1.84, 7.62, 4.74
       const int at_once = sm_count(ctx);
-      if (L.count * ((below + 15) / 16) <= at_once)
-        update<NB, 16, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
-      else if (L.count * ((below + 31) / 32) <= at_once)
-        update<NB, 32, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
-      else
-        update<NB, 64, 16, true>(ctx, pl, L, B, F, k0, turn, below, 0, near, chain);
+      const auto tile = L.count * ((below + 15) / 16) <= at_once   ? update<NB, 16, 16, true>
+                        : L.count * ((below + 31) / 32) <= at_once ? update<NB, 32, 16, true>
+                                                                   : update<NB, 64, 16, true>;
+      if (const int e = tile(ctx, pl, L, B, F, k0, turn, below, 0, near, chain)) return e;
     }
     if (ahead && !light) {
       MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], chain));
@@ -1341,17 +1342,14 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     if (rest > 0) {
       if (NB == 32 || best == c64 || best == c128) {
         MIC_KERNEL_ON(ctx, "k_front_solve", st);
-        launch_after(k_front_solve<NB>, dim3(L.count, (rest + 31) / 32), 256, 0, st, pl.d_fronts, L.first, k0, turn,
-                     near, F, B.U, B.Lb + turn * pl.nL, B.act);
+        LU_LAUNCH(k_front_solve<NB>, dim3(L.count, (rest + 31) / 32), 256, 0, st, pl.d_fronts, L.first, k0, turn, near,
+                  F, B.U, B.Lb + turn * pl.nL, B.act);
       }
-      if (best == c128)
-        update<NB, 128, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
-      else if (best == c64)
-        update<NB, 64, 64, false>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
-      else if (best == c6432)
-        update<NB, 64, 32, NB == 16>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
-      else
-        update<NB, 32, 32, NB == 16>(ctx, pl, L, B, F, k0, turn, below, near, rest, st);
+      const auto tile = best == c128    ? update<NB, 128, 64, false>
+                        : best == c64   ? update<NB, 64, 64, false>
+                        : best == c6432 ? update<NB, 64, 32, NB == 16>
+                                        : update<NB, 32, 32, NB == 16>;
+      if (const int e = tile(ctx, pl, L, B, F, k0, turn, below, near, rest, st)) return e;
     }
     far = ahead;
     if (ahead) MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[1], main));
@@ -1361,10 +1359,12 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
   return MIC_OK;
 }
 
-void band_width(mic_ctx *ctx, const SystemRows &sys, int64_t n, int *bw, cudaStream_t st) {
+int band_width(mic_ctx *ctx, const SystemRows &sys, int64_t n, int *bw, cudaStream_t st) {
   MIC_KERNEL_ON(ctx, "k_band_width", st);
   k_band_width<<<grid_for(n), kBlock, 0, st>>>(sys.cnt, sys.col, sys.width, n, sys.dof, sys.NX, sys.NY,
                                                sys.NX > sys.NY ? 1 : 0, bw);
+  MIC_CUDA_TRY(cudaGetLastError());
+  return MIC_OK;
 }
 
 // every launch of one solve, on the context's stream; the band widths, which only the caller asks
@@ -1375,7 +1375,7 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
   MIC_CUDA_TRY(cudaMemsetAsync(B.info + 1, 0, sizeof(int) * (kInfo - 1), ctx->stream));
   MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[0], ctx->stream));
   MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->lu_chain, ctx->lu_ev[0], 0));
-  band_width(ctx, sys, (int64_t)sys.dof * sys.NX * sys.NY, B.info + 2, ctx->lu_chain);
+  if (const int e = band_width(ctx, sys, (int64_t)sys.dof * sys.NX * sys.NY, B.info + 2, ctx->lu_chain)) return e;
   MIC_CUDA_TRY(cudaEventRecord(ctx->lu_ev[1], ctx->lu_chain));
   for (int l = nl - 1; l >= 0; --l) {
     const Level &L = pl.levels[l];
@@ -1383,18 +1383,16 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     if (L.small) {
       MIC_KERNEL(ctx, "k_front_small");
       // (more warps where one front fills an SM's shared memory)
-      if (L.smem_small > kMaxSmem / 2)
-        launch_after(k_front_small<512>, L.count, 512, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
-                     B.act, sys, Fin, B.F[l & 1], B.U, B.info);
-      else
-        launch_after(k_front_small<256>, L.count, 256, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
-                     B.act, sys, Fin, B.F[l & 1], B.U, B.info);
+      const bool wide = L.smem_small > kMaxSmem / 2;
+      const auto kernel = wide ? k_front_small<512> : k_front_small<256>;
+      LU_LAUNCH(kernel, L.count, wide ? 512 : 256, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.act,
+                sys, Fin, B.F[l & 1], B.U, B.info);
       continue;
     }
     {
       MIC_KERNEL(ctx, "k_front_gather");
-      launch_after(k_front_gather, dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first,
-                   pl.d_tab, B.act, Fin, B.F[l & 1]);
+      LU_LAUNCH(k_front_gather, dim3(L.count, (L.maxR + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
+                B.act, Fin, B.F[l & 1]);
     }
     const int e = L.nb == 32 ? large_level<32>(ctx, pl, L, B, B.F[l & 1]) : large_level<16>(ctx, pl, L, B, B.F[l & 1]);
     if (e) return e;
@@ -1405,17 +1403,15 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     const bool apart = L.maxC > L.maxP + 1 && ((int64_t)L.maxP * (L.maxC - L.maxP) > 8192 || L.maxC > 1024);
     if (apart) {
       MIC_KERNEL(ctx, "k_front_border");
-      launch_after(k_front_border, dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first,
-                   pl.d_tab, B.U, x);
+      LU_LAUNCH(k_front_border, dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
+                B.U, x);
     }
     MIC_KERNEL(ctx, "k_front_back");
     const size_t smem = sizeof(double) * (apart ? L.maxP : L.maxC);
-    if (L.maxP <= 32)
-      launch_after(k_front_back_small, L.count,
-                   L.maxP <= 16 ? 128 : 256, smem, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.U, x, apart ? 0 : 1);
-    else
-      launch_after(k_front_back, L.count,
-                   L.maxP <= 64 ? 256 : 1024, smem, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.U, x, apart ? 0 : 1);
+    const bool few = L.maxP <= 32;
+    const int threads = few ? (L.maxP <= 16 ? 128 : 256) : (L.maxP <= 64 ? 256 : 1024);
+    const auto kernel = few ? k_front_back_small : k_front_back;
+    LU_LAUNCH(kernel, L.count, threads, smem, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.U, x, apart ? 0 : 1);
   }
   // (the band widths where no level used the second stream; else an event of this stream by now)
   MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->lu_ev[1], 0));
@@ -1509,7 +1505,7 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
     if ((e = ensure_lu(ctx, 4096))) return e;
     int *bw = static_cast<int *>(ctx->lu_buf), h[2];
     MIC_CUDA_TRY(cudaMemsetAsync(bw, 0, 2 * sizeof(int), ctx->stream));
-    band_width(ctx, sys, n, bw, ctx->stream);
+    if ((e = band_width(ctx, sys, n, bw, ctx->stream))) return e;
     MIC_CUDA_TRY(cudaMemcpyAsync(h, bw, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     if (h[0] > kMaxBand) return MIC_ERR_SOLVE;
@@ -1550,11 +1546,15 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
     ctx->launches += S.lu_nodes;
   } else if (graphable && cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
     const long long l0 = ctx->launches;
-    e = solve_launches(ctx, pl, B, sys, out);
+    if ((e = solve_launches(ctx, pl, B, sys, out))) {  // (the second stream leaves the capture too)
+      cudaEventRecord(ctx->lu_ev[0], ctx->lu_chain);
+      cudaStreamWaitEvent(ctx->stream, ctx->lu_ev[0], 0);
+    }
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
     if (e || ce != cudaSuccess) {
       if (g) cudaGraphDestroy(g);
+      cudaGetLastError();
       return e ? e : mic_fail_cuda(ctx, ce);
     }
     if (S.lu_exec) cudaGraphExecDestroy(S.lu_exec);

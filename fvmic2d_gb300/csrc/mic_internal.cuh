@@ -232,7 +232,7 @@ __device__ __forceinline__ bool after_previous() {
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
-void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -243,7 +243,7 @@ void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // errors: by cudaGetLastError, as for <<<>>>
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // (errors also by cudaGetLastError, as for <<<>>>)
 }
 }  // namespace mic
 
