@@ -440,6 +440,7 @@ extern "C" int mic_create(mic_ctx **out, int device, void *stream, int NX, int N
   ctx->h_lost = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(ctx->h_words) + kWordsOut);
   *ctx->h_lost = 0;
   ctx->sort_limit = kLookRounds;
+  ctx->solve_limit = kExchangePolls;
   cudaMemcpyToSymbol(c_f64_off, h_f64_off, sizeof(h_f64_off));
   cudaMemcpyToSymbol(c_i32_off, h_i32_off, sizeof(h_i32_off));
   for (int b = 0; b < 4; ++b) {
@@ -765,9 +766,14 @@ extern "C" int mic_synchronize(mic_ctx *ctx) {
 }
 
 extern "C" int mic_debug_set_wait_limit(mic_ctx *ctx, int which, int limit) {
-  if (!ctx || which != MIC_WAIT_SORT || limit < 0) return MIC_ERR_ARG;
-  ctx->sort_limit = limit;
-  ctx->gen++;  // (captured steps hold the limit)
+  if (!ctx || (which != MIC_WAIT_SORT && which != MIC_WAIT_SOLVE) || limit < 0) return MIC_ERR_ARG;
+  if (which == MIC_WAIT_SORT) {
+    ctx->sort_limit = limit;
+    ctx->gen++;  // (captured steps hold the limit)
+  } else {
+    ctx->solve_limit = limit;
+    for (mic_system_store &S : ctx->sys) S.lu_key_buf = nullptr;  // (so do captured solves)
+  }
   return MIC_OK;
 }
 

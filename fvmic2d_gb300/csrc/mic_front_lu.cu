@@ -64,7 +64,7 @@ struct Front {
 };
 
 // info[0]: smallest unknown with a zero pivot; info[1]: entries outside the assumed stencils, and
-// exchanges of a cluster's panel that did not arrive;
+// blocks of a cluster's panel whose exchange did not arrive;
 // info[2], info[3]: lower and upper band widths of the matrix in grid order (mic_system_band)
 constexpr int kInfo = 4;
 
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(256) k_front_gather(const Front *__restrict__ 
   const Front q = fr[first + blockIdx.x];
   const int r = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= q.R) return;
-  if (lane == 0) act[q.act + r] = r;
+  if (lane == 0) act[q.act + r] = act[q.act + q.R + r] = r;  // (both lists: row numbers whatever a panel writes)
   const bool fa = r < q.nA;
   const Front k = fr[q.child + (fa ? 0 : 1)];
   const double *src = child_row(k, fa ? r : r - q.nA, Fin, act);
@@ -496,10 +496,14 @@ __device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB
 // beside which the other warps update the later columns.  Four places for the offers: a block may
 // be sent the second exchange of a column (no row of any block has a value that counts: each then
 // looks for its exact largest) and the first of the next while its warps still read the row before.
+// The wait for an exchange is bounded.  A block whose wait runs out takes no further part: it sends and
+// awaits nothing more (so the others' waits run out too), writes nothing of the panel, and counts
+// itself in info[1], which fails the solve.  What follows reads row lists that hold row numbers all
+// the same.  It stays until what the others have sent it has arrived.
 // GB300, us a panel on one SM and on a cluster: 27 and 22 of 330 rows, 33 and 22 of 645, 70 and 33
 // of 1,290.
 constexpr int kOffers = 4;
-constexpr int kExchangeTries = 1 << 20;  // tens of milliseconds at the very least; an exchange takes 0.3 us
+constexpr int kDrainPolls = 1 << 16;  // a millisecond for what is on its way already
 template <int NB>
 struct PanelOffer {
   double v[NB];
@@ -516,23 +520,28 @@ __device__ __forceinline__ void send_async(unsigned to, long long bits, unsigned
                "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ bool offers_here(unsigned bar, unsigned parity) {
+// polls: how often the barrier is asked (none: not at all).  test_wait returns at once, so the polls
+// bound the time.
+__device__ __forceinline__ bool offers_here(unsigned bar, unsigned parity, int polls) {
   unsigned ok = 0;
-  for (int n = 0; !ok && n < kExchangeTries; ++n)
+  for (int n = 0; !ok && n < polls; ++n)
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ void await_offers(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 
 template <int NB, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
     k_front_panel_cluster(const Front *__restrict__ fr, int first, int k0, int turn, const double *__restrict__ F,
-                          double *U, double *Lb, int *act, const int *__restrict__ tab, int *info) {
+                          double *U, double *Lb, int *act, const int *__restrict__ tab, int *info, int polls) {
   if (NB == 16) next_may_start();
   if (!after_previous()) return;
   extern __shared__ double S[];
@@ -542,6 +551,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   __shared__ double s_rcp;
   __shared__ int s_win, s_place;  // the last winner and the place of its offer
   __shared__ int s_rare;          // the column's exchange is to be done again
+  __shared__ int s_lost;          // an exchange did not arrive: the block takes no further part
   __shared__ int piv[NB];         // the pivots so far, numbers in the list
   const Front q = fr[first + blockIdx.x / CL];
   if (k0 >= q.P) return;  // (the whole cluster)
@@ -576,7 +586,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   if (tid < kOffers)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&bars[tid])) : "memory");
   for (int e = tid; e < kOffers * CL; e += nt) ex[e / CL][e % CL] = PanelOffer<NB>{};
-  if (tid == 0) s_win = s_place = s_rare = 0;
+  if (tid == 0) s_win = s_place = s_rare = s_lost = 0;
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   // every block of the cluster has come this far before one sends to another
@@ -585,17 +595,13 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
   for (int r = tid; r < m; r += nt) take_better(offer, S[r * LD], r);
   const int G = (m + 31) / 32, workers = nw - 1, CS = max(1, workers / max(G, 1));
   unsigned mine = 0;  // which of this thread's rows are pivots
-  int sent = 0;       // exchanges so far (the sending warp)
-  bool lost = false;  // one did not arrive in time: no more waits, the solve fails
+  int sent = 0;       // exchanges that have arrived (the sending warp)
   // column c: row p of this block (-1: none), its values from column c on in the lanes, to every
   // block; the winner's place, reciprocal and number.  Rare: no value that counts in any block
   const auto exchange = [&](int c, int p, double v, bool again) {
     const int place = sent % kOffers;
     const unsigned bar = shared_address(&bars[place]);
-    if (lane == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                   "r"(CL * (int)sizeof(PanelOffer<NB>))
-                   : "memory");
+    if (lane == 0) await_offers(bar, CL * sizeof(PanelOffer<NB>));
     __syncwarp();
     const unsigned to = shared_address(&ex[place][rank].v[lane % NB]), row_to = shared_address(&ex[place][rank].row);
 #pragma unroll
@@ -604,7 +610,10 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       if (lane < NB) send_async(peer_address(to, d), dbits(v), peer_bar);
       if (lane == 31) send_async(peer_address(row_to, d), (long long)(p >= 0 ? base + p : -1), peer_bar);
     }
-    if (!lost && !offers_here(bar, (sent / kOffers) & 1)) lost = true;
+    if (!__all_sync(0xffffffffu, offers_here(bar, (sent / kOffers) & 1, polls))) {
+      if (lane == 0) s_lost = 1;
+      return;
+    }
     ++sent;
     // the same choice in every block; the lanes form all offers' reciprocals beside it
     const int d = min(lane, CL - 1), row = (int)ex[place][d].row;
@@ -618,7 +627,6 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       s_place = place;
       s_rare = !again && key <= 0;
       piv[c] = row;
-      if (lost) atomicAdd(&info[1], 1);
       if (again && rank == 0 && (dbits(w) << 1) == 0) atomicMin(&info[0], tab[q.col + k0 + c]);
     }
   };
@@ -685,6 +693,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       }
     }
     __syncthreads();
+    if (s_lost) break;
     if (s_rare) {  // (the same in every block)
       if (warp == nw - 1) {
         int p = m > 0 ? pivot_rare(S + j + 1, LD, m, used) : -1;
@@ -692,9 +701,24 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
         exchange(j + 1, p, p >= 0 && lane > j && lane < nb ? S[p * LD + lane] : 0.0, true);
       }
       __syncthreads();
+      if (s_lost) break;
     }
   }
   __syncthreads();
+  if (s_lost) {
+    if (tid == 0) atomicAdd(&info[1], 1);
+    // no block sends once all are here; what is on its way then is exchange `sent`, which this block
+    // awaited in vain, and the next one of blocks that had it complete
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (warp == nw - 1) {
+      offers_here(shared_address(&bars[sent % kOffers]), (sent / kOffers) & 1, kDrainPolls);
+      const int next = sent + 1;
+      if (lane == 0) await_offers(shared_address(&bars[next % kOffers]), CL * sizeof(PanelOffer<NB>));
+      __syncwarp();
+      offers_here(shared_address(&bars[next % kOffers]), (next / kOffers) & 1, kDrainPolls);
+    }
+    return;
+  }
   for (int e = tid; e < nb * NB; e += nt) {  // the block's pivots in order: U11 and the multipliers before it
     const int k = e / NB, c = e % NB, r = piv[k] - base;
     if (r < 0 || r >= m) continue;
@@ -710,12 +734,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kPanelThreads, 2)
       int pos = nb + base + r;
 #pragma unroll
       for (int k = 0; k < NB; ++k) pos -= k < nb && piv[k] < base + r;
-      if (pos >= all) continue;  // (after a lost exchange)
       Lb[q.lb + (int64_t)pos * NB + lc] = lc < nb ? S[r * LD + lc] : 0.0;
       if (lc == 0) out[pos] = id[r];
     }
   }
-  // (no block leaves while another could still send to it)
+  // (a block that lost an exchange waits here for all)
   __syncthreads();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
@@ -1288,12 +1311,17 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     const size_t smem = (size_t)share * ((NB + 1) * sizeof(double) + kPanelBytes);
     {
       MIC_KERNEL_ON(ctx, "k_front_panel", chain);
-      const auto kernel = cl == 8   ? k_front_panel_cluster<NB, 8>
-                          : cl == 4 ? k_front_panel_cluster<NB, 4>
-                          : cl == 2 ? k_front_panel_cluster<NB, 2>
-                                    : k_front_panel<NB>;
-      LU_LAUNCH(kernel, L.count * cl, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U,
-                B.Lb + turn * pl.nL, B.act, pl.d_tab, B.info);
+      double *const Lb = B.Lb + turn * pl.nL;
+      if (cl == 1) {
+        LU_LAUNCH(k_front_panel<NB>, L.count, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U, Lb, B.act,
+                  pl.d_tab, B.info);
+      } else {
+        const auto kernel = cl == 8   ? k_front_panel_cluster<NB, 8>
+                            : cl == 4 ? k_front_panel_cluster<NB, 4>
+                                      : k_front_panel_cluster<NB, 2>;
+        LU_LAUNCH(kernel, L.count * cl, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U, Lb, B.act,
+                  pl.d_tab, B.info, ctx->solve_limit);
+      }
     }
     // trailing columns: the most any front has (its panel may be narrower than NB)
     const int cols = L.maxC - std::min(k0 + NB, std::max(L.minP, k0 + 1)), below = std::max(rows - 1, 1);

@@ -54,6 +54,7 @@ struct Status {
 constexpr size_t kWordsOut = 512;  // bytes of a context's pinned buffer for small results
 
 constexpr int kLookRounds = 1 << 22;  // a radix pass's look-back: seconds, where it takes microseconds
+constexpr int kExchangePolls = 1 << 22;  // a panel exchange's barrier: tens of milliseconds, where it takes 0.3 us
 
 // Composite creep (law 7) settings and per-pass counters
 struct CreepConfig {
@@ -181,6 +182,7 @@ struct mic_ctx {
   double *h_words;        // pinned: small results on their way to the host (kWordsOut bytes)
   int *h_lost;            // pinned, behind them: a sort has given up since the markers were last replaced
   int sort_limit;         // rounds a radix pass looks back for (kLookRounds)
+  int solve_limit;        // polls of a panel exchange's barrier (kExchangePolls)
   unsigned char *stage_aos;  // device staging for AoS transfers
   int64_t stage_cap;
   double residuals[100];

@@ -213,7 +213,7 @@ class MicProblem:
         if code != 0:
             raise MicError(code, what)
 
-    WAIT_SORT = 0
+    WAIT_SORT, WAIT_SOLVE = 0, 1
 
     def debug_set_wait_limit(self, which, limit):
         self._check(self.L.mic_debug_set_wait_limit(self.h, which, limit), "mic_debug_set_wait_limit")

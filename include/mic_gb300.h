@@ -229,8 +229,9 @@ int mic_debug_sorted_ids(mic_ctx *ctx, int32_t *ids);
 int mic_debug_cell_start(mic_ctx *ctx, int32_t *cell_start);
 /* the library's bounded waits between blocks, for tests of what happens when one runs out: rounds
  * before it does (0: it gives up at once).  MIC_WAIT_SORT: a radix pass's look-back (default 2^22,
- * seconds; MIC_ERR_CELL) */
-enum { MIC_WAIT_SORT = 0 };
+ * seconds; MIC_ERR_CELL).  MIC_WAIT_SOLVE: an exchange of the direct solver's cluster panels (default
+ * 2^22, tens of milliseconds; MIC_ERR_SOLVE, and the next solve starts afresh) */
+enum { MIC_WAIT_SORT = 0, MIC_WAIT_SOLVE = 1 };
 int mic_debug_set_wait_limit(mic_ctx *ctx, int which, int limit);
 /* num[k] / den[k] (host arrays) computed the way the kernels divide by a grid spacing: the
  * correctly rounded reciprocal and one residual correction (the FMA-free build divides) */

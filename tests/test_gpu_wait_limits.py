@@ -7,11 +7,12 @@ import pytest
 
 from fvmic2d_gb300 import gpu
 from fvmic2d_gb300 import workloads as W
+from tests.test_gpu_front_solve import _problem
 
 pytestmark = pytest.mark.gpu
 
-ERR_CELL = 4
-LOOK_BACK = 1 << 22  # the default
+ERR_CELL, ERR_SOLVE = 4, 12
+LOOK_BACK = POLLS = 1 << 22  # the defaults
 
 
 def _refused(f, *a):
@@ -85,3 +86,28 @@ def test_ensemble_reports_a_member_whose_sort_gave_up(graph):
     _refused(E.synchronize)
     assert Ps[0].L.mic_synchronize(Ps[0].h) == 0
     assert Ps[1].L.mic_synchronize(Ps[1].h) == ERR_CELL
+
+
+@pytest.mark.parametrize("nx,ny,which", [(260, 90, 1), (61, 61, 0), (129, 33, 0), (300, 300, 1)])
+@pytest.mark.parametrize("polls", [0, 3])
+def test_panel_exchange_that_gives_up_fails_the_solve(nx, ny, which, polls):
+    """Panels on clusters of two to eight blocks; no poll (every block gives up at its first exchange) and
+    a few (some exchanges arrive): the solve fails or is right, and the next one is the undisturbed one's
+    equal, bit for bit."""
+    P, so = _problem(nx, ny)
+    if which == P.STOKES:
+        P.formVEPSystem(so, 3.0e11)
+    else:
+        P.enforceThermalBCs1(so)
+        P.formThermalSystem(so, 3.0e11)
+    P.linear_solve(which)
+    x = P.solution(which)
+    P.debug_set_wait_limit(P.WAIT_SOLVE, polls)
+    for _ in range(2):  # the launches as they are captured, and the captured graph
+        code = P.L.mic_linear_solve(P.h, which)
+        assert code == ERR_SOLVE if polls == 0 else code in (0, ERR_SOLVE)
+        assert code == ERR_SOLVE or np.array_equal(P.solution(which), x)
+    P.debug_set_wait_limit(P.WAIT_SOLVE, POLLS)
+    P.linear_solve(which)
+    assert np.array_equal(P.solution(which), x)
+    P.close()
