@@ -21,7 +21,7 @@ extern "C" const char *mic_error_string(int code) {
     case MIC_ERR_ARG: return "invalid argument";
     case MIC_ERR_CUDA: return "CUDA runtime error";
     case MIC_ERR_NOMEM: return "out of memory";
-    case MIC_ERR_CELL: return "impossible marker cell index";
+    case MIC_ERR_CELL: return "impossible marker cell index (a binning gave up waiting for its sort)";
     case MIC_ERR_NAN: return "NaN strain-rate residual";
     case MIC_ERR_LAW: return "undefined viscosity law";
     case MIC_ERR_BC: return "unsupported boundary condition";
@@ -29,7 +29,7 @@ extern "C" const char *mic_error_string(int code) {
     case MIC_ERR_NO_DEVICE: return "no CUDA device";
     case MIC_ERR_DENSITY: return "marker density control cannot proceed";
     case MIC_ERR_IO: return "checkpoint file could not be read or written";
-    case MIC_ERR_SOLVE: return "direct solve failed (zero pivot, or a band too wide)";
+    case MIC_ERR_SOLVE: return "direct solve failed (zero pivot, band too wide, or a wait between blocks that ran out)";
     default: return "unknown error";
   }
 }
@@ -191,7 +191,7 @@ static void free_ctx(mic_ctx *ctx) {
     cudaFree(ctx->sys[w].col);
     cudaFree(ctx->sys[w].val);
     cudaFree(ctx->sys[w].rhs);
-    cudaFree(ctx->sys[w].free_cell);
+    cudaFree(ctx->sys[w].group);
   }
   cudaFree(ctx->sys_scratch);
   cudaFree(ctx->lu_buf);

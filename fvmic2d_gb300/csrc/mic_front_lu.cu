@@ -100,7 +100,7 @@ struct SystemRows {  // the assembled rows (mic_systems.cu)
   const int *cnt, *col;
   const double *val, *rhs;
   int width, dof, NX, NY;
-  const unsigned char *free_cell;  // per node: cells whose pressure no equation holds (null: none)
+  const int *group, *first;  // Stokes: a cell whose pressure no equation holds is first[group[cell]]
 };
 
 // value of column c (of q's columns) in left-over row i of child k: where the child keeps it
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
           atomicAdd(&info[1], 1);
       }
       A[r * ld + C - 1] = sys.rhs[g];
-      if (sys.free_cell && d == 2 && sys.free_cell[g / 3]) {  // its pressure is free: pinned (mic_systems.cu)
+      if (d == 2 && sys.first[sys.group[g / 3]] == g / 3) {  // its pressure is free: pinned (mic_systems.cu)
         double most = 0.0;
         for (int k = 0; k < n; ++k) most = fmax(most, fabs(sys.val[g * sys.width + k]));
         const int cx = q.x0 + node % w - tx, cy = q.y0 + node / w - ty;
@@ -1525,7 +1525,7 @@ extern "C" int mic_linear_solve(mic_ctx *ctx, int which) {
   const int dof = which == 0 ? 3 : 1;
   const int64_t n = S.n;
   int e;
-  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY, S.free_cell};
+  const SystemRows sys = {S.cnt, S.col, S.val, S.rhs, S.width, dof, NX, NY, S.group, S.group + n / 3};
   // the solver's size limit, a band of 1,016 below the diagonal: only a grid whose shorter side
   // could reach it has its band measured first
   constexpr int kMaxBand = 1016;

@@ -98,7 +98,8 @@ struct mic_system_store {
   int width;
   int *cnt, *col;
   double *val, *rhs;
-  unsigned char *free_cell;  // Stokes: per node, a cell whose pressure no equation holds
+  int *group;  // Stokes: the groups of pressure cells (mic_systems.cu): per node a cell of its group, then per
+               // root the cell to pin (INT_MAX: none), then whether it is held (bytes)
   double Kbond, Kcont;
   int factored;
   int kl, ku;       // band widths of the matrix in grid order

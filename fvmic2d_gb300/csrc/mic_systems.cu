@@ -148,6 +148,12 @@ __global__ void k_vep_consts(Params P, const double *__restrict__ part, int npar
   }
 }
 
+// the pressure cells' groups (k_group_links)
+struct Groups {
+  int *parent, *first;  // first: at the root of a group that nothing holds, the cell to pin
+  unsigned char *held;
+};
+
 // the three rows of node (ix, jy): continuity (vep_system.c:243-284), x-momentum (288-395) and
 // y-momentum (398-512); the ADD_VALUES pass after them (517-571) is disabled in the reference
 // Bound by the latency of a row's divisions (some 15 in a row of the stencil, 440 clocks each) as
@@ -157,12 +163,17 @@ constexpr int kRowBlock = 64;
 __global__ void __launch_bounds__(kRowBlock) k_vep_rows(Params P, Geo G, const double *__restrict__ etaNZ,
                                                         const double *__restrict__ etaSZ,
                                                         const double *__restrict__ rho, const double *__restrict__ Kd,
-                                                        double gx, double gy, Rows R) {
+                                                        double gx, double gy, Rows R, Groups cells) {
   if (!after_previous()) return;
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int NX = P.NX, NY = P.NY;
   if (k >= (int64_t)NX * NY) return;
   const int ix = (int)(k % NX), jy = (int)(k / NX);
+  if (blockIdx.y == 0) {  // (for k_group_links)
+    cells.parent[k] = (int)k;
+    cells.first[k] = INT_MAX;
+    cells.held[k] = 0;
+  }
   const double Kbond = Kd[0], Kcont = Kd[1];
   const double *x = P.x, *y = P.y, *xc = P.xc, *yc = P.yc;
   Row r;
@@ -505,18 +516,39 @@ int prepare(mic_ctx *ctx, const mic_subduction_options &o, Scratch &s, Geo &G) {
 }
 
 // Pressure cells cut off from the rest.  Where the slab meets the plate on a coarse grid, a few
-// pressure cells, usually two, can lie between imposed velocities on all sides: their common
-// pressure is in no equation and the matrix is singular.  An elimination in grid order meets a pivot
-// of rounding there and goes on, to pressures of 1e26; in the solver's order the pivot is often
-// exactly zero.  Such a group is found from the equations (a momentum equation that holds two
-// pressures links their cells), and in the solve its first cell's continuity equation has an entry at
-// its own pressure, of the size of its others: the free pressure comes out near zero, all else as
-// it is.  No other matrix is touched, and the assembled rows (mic_system_get) stay as they are.
-constexpr int kGroup = 8;  // cells of a group at most
-struct Links {
-  int to[8], n;
-  bool held;  // an equation holds this pressure alone
-};
+// pressure cells, usually two, can lie between imposed velocities on all sides (a thick plate root
+// encloses hundreds): their common pressure is in no equation and the matrix is singular.  An
+// elimination in grid order meets a pivot of rounding there and goes on, to pressures of 1e26; in the
+// solver's order the pivot is often exactly zero.  Such a group is found from the equations: one that
+// holds two pressures links their cells, one that holds a pressure alone holds its group.  In the solve
+// a cell's continuity equation has an entry at its own pressure, of the size of its others: the free
+// pressure comes out near zero, all else as it is.  No other matrix is touched, and the assembled rows
+// (mic_system_get) stay as they are.
+//
+// Groups are trees of cells (parent: a cell of a smaller number, or the cell itself, the root), joined
+// root to root.  GB300, each kernel alone: 24, 7 and 6 us at 129 x 33 nodes, 55, 7 and 8 at 513 x 129 (a
+// walk from each cell that knew groups of eight cells at most: 18 and 19).
+__device__ __forceinline__ int group_root(int *parent, int c) {
+  volatile int *p = parent;
+  for (int a = p[c]; a != c;) {
+    const int b = p[a];
+    if (b != a) p[c] = b;  // (an ancestor whatever others write: c is no root any more)
+    c = a;
+    a = b;
+  }
+  return c;
+}
+__device__ __forceinline__ void group_join(int *parent, int a, int b) {
+  for (;;) {
+    a = group_root(parent, a);
+    b = group_root(parent, b);
+    if (a == b) return;
+    const int lo = min(a, b), hi = max(a, b);
+    if (atomicCAS(parent + hi, hi, lo) == hi) return;  // else hi has got a smaller parent: nearer the end
+    a = lo;
+    b = hi;
+  }
+}
 // which of two columns a row holds (bits 0 and 1); its twelve places read at once
 __device__ __forceinline__ int holds(const Rows &s, int row, int c0, int c1) {
   static_assert(kMaxEnt == 12, "three groups of four");
@@ -547,57 +579,52 @@ __device__ __forceinline__ void cell_faces(const Rows &s, int NX, int NY, int ce
   for (int k = 0; k < 4; ++k)
     if (hit[k] & 1) f(hit[k] & 2 ? to[k] : -1);
 }
-__device__ Links cell_links(const Rows &s, int NX, int NY, int cell) {
-  Links l;
-  l.n = 0;
-  l.held = false;
-  cell_faces(s, NX, NY, cell, [&](int to) {
-    if (to >= 0)
-      l.to[l.n++] = to;
-    else
-      l.held = true;
-  });
-  // the cell's own equation, where it is one for pressures (boundaries, solids)
-  const int own = 3 * cell + 2, n = s.cnt[own];
-  if (holds(s, own, own, own)) {
-    if (n == 1) l.held = true;
-    for (int k = 0; k < n && l.n < 8; ++k) {
-      const int c = s.col[(int64_t)own * kMaxEnt + k];
-      if (c != own && c % 3 == 2) l.to[l.n++] = c / 3;
-    }
-  }
-  return l;
-}
-// Is this the first cell, of those with at most two links, of a group that nothing holds?
-__device__ __noinline__ bool cut_off_first(const Rows &s, int NX, int NY, int cell) {
-  int group[kGroup], n = 1;
-  group[0] = cell;
-  for (int i = 0; i < n; ++i) {
-    const Links l = cell_links(s, NX, NY, group[i]);
-    const int own = 3 * group[i] + 2;
-    if (l.held) return false;
-    if (l.n <= 2 && group[i] < cell && !holds(s, own, own, own)) return false;
-    for (int k = 0; k < l.n; ++k) {
-      bool seen = false;
-      for (int j = 0; j < n; ++j) seen = seen || group[j] == l.to[k];
-      if (seen) continue;
-      if (n == kGroup) return false;
-      group[n++] = l.to[k];
-    }
-  }
-  return true;
-}
-__global__ void __launch_bounds__(64) k_free_cells(Rows s, int NX, int NY, unsigned char *free_cell) {
+// links of a cell's own equation and of the momentum equations behind it (to the next cell in x and in
+// y), and which cells an equation holds alone
+__global__ void __launch_bounds__(64) k_group_links(Rows s, int NX, int NY, Groups g) {
   if (!after_previous()) return;
   const int cell = blockIdx.x * 64 + threadIdx.x;
   if (cell >= NX * NY) return;
+  const int x = cell % NX, y = cell / NX, own = 3 * cell + 2;
+  const int eq[2] = {3 * (cell - NX), 3 * (cell - 1) + 1};
+  const int to[2] = {x + 1 < NX ? cell + 1 : -1, y + 1 < NY ? cell + NX : -1};
+  const bool there[2] = {y > 0, x > 0};
+  int hit[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) hit[k] = there[k] ? holds(s, eq[k], own, to[k] >= 0 ? 3 * to[k] + 2 : -1) : 0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (hit[k] == 3) group_join(g.parent, cell, to[k]);
+    if (hit[k] == 1) g.held[cell] = 1;
+    if (hit[k] == 2) g.held[to[k]] = 1;
+  }
+  if (holds(s, own, own, own)) {  // an equation for pressures (boundaries, solids)
+    const int n = s.cnt[own];
+    if (n == 1) g.held[cell] = 1;
+    for (int k = 0; k < n; ++k) {
+      const int c = s.col[(int64_t)own * kMaxEnt + k];
+      if (c != own && c % 3 == 2) group_join(g.parent, cell, c / 3);
+    }
+  }
+}
+// a root is held when a cell of its group is
+__global__ void __launch_bounds__(64) k_group_held(int cells, Groups g) {
+  if (!after_previous()) return;
+  const int cell = blockIdx.x * 64 + threadIdx.x;
+  if (cell < cells && g.held[cell]) g.held[group_root(g.parent, cell)] = 1;
+}
+// of a group that nothing holds, the first cell whose own equation is free for the entry (a lone cell
+// is in no equation at all: an empty column, refused as it is)
+__global__ void __launch_bounds__(64) k_group_free(Rows s, int NX, int NY, Groups g) {
+  if (!after_previous()) return;
+  const int cell = blockIdx.x * 64 + threadIdx.x;
+  if (cell >= NX * NY || g.held[cell]) return;
+  const int root = group_root(g.parent, cell), own = 3 * cell + 2;
+  if (g.held[root]) return;
+  g.parent[cell] = root;
   int links = 0;
-  bool held = holds(s, 3 * cell + 2, 3 * cell + 2, 3 * cell + 2) != 0;
-  cell_faces(s, NX, NY, cell, [&](int to) {
-    links += to >= 0;
-    held |= to < 0;
-  });
-  free_cell[cell] = !held && links >= 1 && links <= 2 && cut_off_first(s, NX, NY, cell);
+  cell_faces(s, NX, NY, cell, [&](int to) { links += to >= 0; });
+  if (links > 0 && !holds(s, own, own, own)) atomicMin(g.first + root, cell);
 }
 
 int ensure_system(mic_ctx *ctx, int which, int64_t n) {
@@ -607,14 +634,14 @@ int ensure_system(mic_ctx *ctx, int which, int64_t n) {
   cudaFree(S.col);
   cudaFree(S.val);
   cudaFree(S.rhs);
-  cudaFree(S.free_cell);
+  cudaFree(S.group);
   if (S.lu_exec) cudaGraphExecDestroy(S.lu_exec);
   mic_front_plan_free(S.plan);
   S = mic_system_store{};
   if (cudaMalloc(&S.cnt, sizeof(int) * n) != cudaSuccess || cudaMalloc(&S.col, sizeof(int) * n * kMaxEnt) != cudaSuccess ||
       cudaMalloc(&S.val, sizeof(double) * n * kMaxEnt) != cudaSuccess ||
       cudaMalloc(&S.rhs, sizeof(double) * n) != cudaSuccess ||
-      (which == 0 && cudaMalloc(&S.free_cell, (size_t)n / 3) != cudaSuccess))
+      (which == 0 && cudaMalloc(&S.group, (2 * sizeof(int) + 1) * (size_t)n / 3) != cudaSuccess))
     return MIC_ERR_NOMEM;
   S.n = n;
   S.width = kMaxEnt;
@@ -622,6 +649,9 @@ int ensure_system(mic_ctx *ctx, int which, int64_t n) {
 }
 
 Rows rows_of(const mic_system_store &S) { return Rows{S.cnt, S.col, S.val, S.rhs}; }
+Groups groups_of(const mic_system_store &S) {
+  return Groups{S.group, S.group + S.n / 3, reinterpret_cast<unsigned char *>(S.group + 2 * (S.n / 3))};
+}
 
 // initialConditionsVanKeken (benchmarkInitialConditions.c:8-33) for one marker: temperature by
 // region (slab: the half-space cooling profile; overriding plate: the linear geotherm; wedge:
@@ -738,16 +768,26 @@ extern "C" int mic_form_vep_system(mic_ctx *ctx, const mic_subduction_options *o
   {
     MIC_KERNEL(ctx, "k_vep_rows");
     launch_after(k_vep_rows, dim3(grid_for(nn, kRowBlock), 3), kRowBlock, 0, ctx->stream, ctx->P, G, s.etaNZ, s.etaSZ,
-                 f[MIC_NF_RHO], s.K, o->gx, o->gy, rows_of(ctx->sys[0]));
+                 f[MIC_NF_RHO], s.K, o->gx, o->gy, rows_of(ctx->sys[0]), groups_of(ctx->sys[0]));
   }
   MIC_CUDA_TRY(cudaGetLastError());
   if ((e = mic_words_out(ctx, s.K, 2 * sizeof(double)))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   const double K[2] = {ctx->h_words[0], ctx->h_words[1]};
-  {  // (after the wait: it runs while the host goes on)
-    MIC_KERNEL(ctx, "k_free_cells");
-    launch_after(k_free_cells, (unsigned)((nn + 63) / 64), 64, 0, ctx->stream, rows_of(ctx->sys[0]), NX, NY,
-                 ctx->sys[0].free_cell);
+  {  // (after the wait: they run while the host goes on)
+    const unsigned grid = (unsigned)((nn + 63) / 64);
+    const Rows R = rows_of(ctx->sys[0]);
+    const Groups cells = groups_of(ctx->sys[0]);
+    {
+      MIC_KERNEL(ctx, "k_group_links");
+      launch_after(k_group_links, grid, 64, 0, ctx->stream, R, NX, NY, cells);
+    }
+    {
+      MIC_KERNEL(ctx, "k_group_held");
+      launch_after(k_group_held, grid, 64, 0, ctx->stream, (int)nn, cells);
+    }
+    MIC_KERNEL(ctx, "k_group_free");
+    launch_after(k_group_free, grid, 64, 0, ctx->stream, R, NX, NY, cells);
   }
   MIC_CUDA_TRY(cudaGetLastError());
   ctx->sys[0].Kbond = K[0];

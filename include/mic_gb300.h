@@ -46,7 +46,8 @@ enum {
                            * markers (markers.c:590-593 aborts), an overfull quarter cell with no
                            * marker inside its bounds, or more than 2048 markers in one */
   MIC_ERR_IO = 11,        /* checkpoint file could not be opened, read or written */
-  MIC_ERR_SOLVE = 12      /* direct solve: zero pivot (singular matrix) or a band too wide */
+  MIC_ERR_SOLVE = 12      /* direct solve: a zero pivot (singular matrix), a band too wide, or a panel whose
+                             blocks gave up waiting for one another */
 };
 
 typedef struct {
@@ -360,7 +361,10 @@ int mic_system_get(mic_ctx *ctx, int which, int32_t *rowptr, int32_t *cols, doub
 /* kspLinearSolve (kspLinearSolve.c:13) as the reference's option files run it (preonly + LU,
  * option_files/run_mumps.petscopt): a direct solve on the device, LU with partial pivoting in
  * nested-dissection order.  The Stokes solution stays on the device for mic_retrieve_solutions(ctx, NULL, ...);
- * the temperature goes to MIC_NF_THIST.  MIC_ERR_SOLVE for a zero pivot. */
+ * the temperature goes to MIC_NF_THIST.  MIC_ERR_SOLVE for a zero pivot.  Pressure cells that imposed
+ * velocities cut off from the rest (a pair where slab and plate meet, a pocket below a thick root:
+ * groups of two cells and more, of any size) leave the Stokes matrix singular by their common
+ * pressure; the solve goes on with that pressure near zero. */
 int mic_linear_solve(mic_ctx *ctx, int which);
 int mic_solution_get(mic_ctx *ctx, int which, double *out);
 /* band widths (lower, upper) of the matrix the last solve of a system factorised, nodes numbered
