@@ -291,6 +291,17 @@ extern "C" int mic_limit_displacement_timestep(mic_ctx *ctx, double factor, doub
   return MIC_OK;
 }
 
+int mic_retrieve_launch(mic_ctx *ctx, double Kcont) {
+  {
+    MIC_KERNEL(ctx, "k_retrieve");
+    const int64_t full = grid_for((int64_t)ctx->P.NX * ctx->P.NY, 256), wave = 2 * (int64_t)sm_count(ctx);
+    launch_after(k_retrieve, (unsigned)(full < wave ? full : wave), 256, 0, ctx->stream, ctx->P, ctx->solution, Kcont,
+                 ctx->nodal[MIC_NF_P], ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY]);
+  }
+  MIC_CUDA_TRY(cudaGetLastError());
+  return MIC_OK;
+}
+
 extern "C" int mic_retrieve_solutions(mic_ctx *ctx, const double *S, double Kcont, int *foundnan) {
   if (ctx && ctx->P.xper) return MIC_ERR_BC;  // grids periodic in x: the marker path only
   if (!ctx || (!S && !ctx->solution)) return MIC_ERR_ARG;
@@ -302,14 +313,8 @@ extern "C" int mic_retrieve_solutions(mic_ctx *ctx, const double *S, double Kcon
   // S = NULL: the solution mic_linear_solve left on the device
   if (S)
     MIC_CUDA_TRY(cudaMemcpyAsync(ctx->solution, S, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, ctx->stream));
-  {
-    MIC_KERNEL(ctx, "k_retrieve");
-    const int64_t full = grid_for(nn, 256), wave = 2 * (int64_t)sm_count(ctx);
-    launch_after(k_retrieve, (unsigned)(full < wave ? full : wave), 256, 0, ctx->stream, ctx->P, ctx->solution, Kcont,
-                 ctx->nodal[MIC_NF_P], ctx->nodal[MIC_NF_VX], ctx->nodal[MIC_NF_VY]);
-  }
-  MIC_CUDA_TRY(cudaGetLastError());
-  if (S) MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // the caller may reuse S on return
+  if (const int e = mic_retrieve_launch(ctx, Kcont)) return e;
+  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // the caller may reuse S on return, and read the fields
   if (foundnan) *foundnan = 0;  // the reference checks for NaN only in its TEXTURE build
   return MIC_OK;
 }

@@ -279,6 +279,7 @@ int mic_words_out(mic_ctx *ctx, const void *dev, size_t bytes);
 int mic_strain_launch(mic_ctx *ctx, double dt);
 int mic_residual_launch(mic_ctx *ctx);                     // into the status
 void mic_residual_store(mic_ctx *ctx, int iter, double *residual);  // from the mirror
+int mic_retrieve_launch(mic_ctx *ctx, double Kcont);       // of the solution on the device
 int mic_limit_launch(mic_ctx *ctx, double factor);         // into h_words
 void mic_limit_result(const mic_ctx *ctx, double *dt);
 int mic_diagnostics_launch(mic_ctx *ctx, double dTbc, bool nusselt, bool vrms);  // into h_words[0], [1]

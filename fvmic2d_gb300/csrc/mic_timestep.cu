@@ -164,9 +164,7 @@ extern "C" int mic_subduction_timestep(mic_ctx *ctx, const mic_timestep_options 
       rep->Kbond = ctx->sys[0].Kbond;
       rep->Kcont = ctx->sys[0].Kcont;
     }
-    int fn = 0;
-    MIC_TRY(mic_retrieve_solutions(ctx, nullptr, rep->Kcont, &fn));
-    if (fn) return MIC_ERR_NAN;
+    MIC_TRY(mic_retrieve_launch(ctx, rep->Kcont));
     MIC_TRY(mic_nodal_stress_strain(ctx, displacementdt, gy));
     // (updateMarkerStrainPressure, the residual and the step limit: one wait for all three)
     MIC_TRY(mic_strain_launch(ctx, displacementdt));
