@@ -400,8 +400,9 @@ def roofline(prof, n, nodes, steps, hbm_peak, peak_src, law7=False):
     kern = sorted(prof.items(), key=lambda kv: -kv[1][0])
     # a kernel on the second stream (the first projection's partial sums) overlaps the yield pass:
     # its event span is not its own cost, so the dominant kernel is taken among the main stream's
-    main = [kv for kv in kern if not kv[0].startswith(("k_partials_basic<first>", "k_partials_centre<scalar>",
-                                                        "k_combine_scalar<-1>", "k_residual_weight"))]
+    main = [kv for kv in kern if not kv[0].startswith(("k_partials_basic<first>", "k_corners_basic<first>",
+                                                        "k_corners_centre<scalar>", "k_combine_scalar<-1>",
+                                                        "k_residual_weight"))]
     top_name, (top_ms, top_cnt) = (main or kern)[0]
     table = dict(KERNEL_BYTES, **(KERNEL_BYTES_LAW7 if law7 else {}))
     per_marker, per_node = table.get(top_name, (0, 0))

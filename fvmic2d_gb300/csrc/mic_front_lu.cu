@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstdio>
 #include <cstring>
 #include <iterator>
 #include <new>
@@ -1277,6 +1278,21 @@ size_t room(size_t bytes) { return ((bytes + 255) / 256) * 256; }
     if (launch_after(__VA_ARGS__) != cudaSuccess) return mic_fail_cuda(ctx, cudaGetLastError()); \
   } while (0)
 
+// a launch's name in the profile says which form ran
+template <int NB, int TR, int TC>
+const char *update_name() {
+  static char name[48];
+  static const int n = snprintf(name, sizeof(name), "k_front_update<%d,%d,%d>", NB, TR, TC);
+  return n > 0 ? name : "k_front_update";
+}
+template <int NB>
+const char *panel_name(int cl) {
+  static const char *const names[2][4] = {
+      {"k_front_panel<16>", "k_front_panel_cluster<16,2>", "k_front_panel_cluster<16,4>", "k_front_panel_cluster<16,8>"},
+      {"k_front_panel<32>", "k_front_panel_cluster<32,2>", "k_front_panel_cluster<32,4>", "k_front_panel_cluster<32,8>"}};
+  return names[NB == 32][cl == 8 ? 3 : cl == 4 ? 2 : cl == 2 ? 1 : 0];
+}
+
 struct Buffers {
   int *info;
   double *F[2], *U, *Lb;
@@ -1286,7 +1302,7 @@ struct Buffers {
 template <int NB, int TR, int TC, bool SOLVE>
 int update(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Buffers &B, double *F, int k0, int turn,
            int rows, int coff, int cols, cudaStream_t st) {
-  MIC_KERNEL_ON(ctx, "k_front_update", st);
+  MIC_KERNEL_ON(ctx, (update_name<NB, TR, TC>()), st);
   constexpr auto kernel = k_front_update<NB, TR, TC, SOLVE>;
   LU_LAUNCH(kernel, dim3(L.count, (rows + TR - 1) / TR, (cols + TC - 1) / TC), kUpdateThreads,
             (update_smem<NB, TR, TC, SOLVE>()), st, pl.d_fronts, L.first, k0, turn, coff, cols, F, B.U,
@@ -1310,7 +1326,7 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     const int share = (rows + cl - 1) / cl, threads = share <= 256 ? 256 : kPanelThreads;
     const size_t smem = (size_t)share * ((NB + 1) * sizeof(double) + kPanelBytes);
     {
-      MIC_KERNEL_ON(ctx, "k_front_panel", chain);
+      MIC_KERNEL_ON(ctx, panel_name<NB>(cl), chain);
       double *const Lb = B.Lb + turn * pl.nL;
       if (cl == 1) {
         LU_LAUNCH(k_front_panel<NB>, L.count, threads, smem, chain, pl.d_fronts, L.first, k0, turn, F, B.U, Lb, B.act,
@@ -1409,9 +1425,9 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     const Level &L = pl.levels[l];
     const double *Fin = B.F[(l + 1) & 1];
     if (L.small) {
-      MIC_KERNEL(ctx, "k_front_small");
       // (more warps where one front fills an SM's shared memory)
       const bool wide = L.smem_small > kMaxSmem / 2;
+      MIC_KERNEL(ctx, wide ? "k_front_small<512>" : "k_front_small<256>");
       const auto kernel = wide ? k_front_small<512> : k_front_small<256>;
       LU_LAUNCH(kernel, L.count, wide ? 512 : 256, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.act,
                 sys, Fin, B.F[l & 1], B.U, B.info);
@@ -1434,9 +1450,9 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
       LU_LAUNCH(k_front_border, dim3(L.count, (L.maxP + 7) / 8), 256, 0, ctx->stream, pl.d_fronts, L.first, pl.d_tab,
                 B.U, x);
     }
-    MIC_KERNEL(ctx, "k_front_back");
     const size_t smem = sizeof(double) * (apart ? L.maxP : L.maxC);
     const bool few = L.maxP <= 32;
+    MIC_KERNEL(ctx, few ? "k_front_back_small" : "k_front_back");
     const int threads = few ? (L.maxP <= 16 ? 128 : 256) : (L.maxP <= 64 ? 256 : 1024);
     const auto kernel = few ? k_front_back_small : k_front_back;
     LU_LAUNCH(kernel, L.count, threads, smem, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.U, x, apart ? 0 : 1);

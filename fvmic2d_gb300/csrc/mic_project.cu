@@ -781,7 +781,7 @@ int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cud
     const bool known = (ctx->wn_valid >> (stag == 0 ? 0 : 1)) & 1;
     if (stag == 0) {
       {
-        MIC_KERNEL_ON(ctx, "k_partials_basic<scalar>", s);
+        MIC_KERNEL_ON(ctx, "k_corners_basic_scalar", s);
         if (known)
           launch_after(k_corners_basic_scalar<false>, gb, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->part_b);
         else
@@ -794,7 +794,7 @@ int mic_project_scalar(mic_ctx *ctx, const double *v, int stag, double *out, cud
         launch_after(k_combine_scalar<0, false>, gn, 128, 0, s, ctx->P, ctx->part_b, nullptr, out);
     } else {
       {
-        MIC_KERNEL_ON(ctx, "k_partials_centre<scalar>", s);
+        MIC_KERNEL_ON(ctx, "k_corners_centre<scalar>", s);
         if (known)
           launch_after(k_corners_centre<false, false>, gc, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->part_c);
         else
@@ -896,7 +896,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   if (mode == 2) {
     const cudaStream_t s = st ? st : ctx->stream;
     {
-      MIC_KERNEL_ON(ctx, "k_partials_basic<first>", s);
+      MIC_KERNEL_ON(ctx, few ? "k_corners_basic<first>" : "k_partials_basic<first>", s);
       if (few)
         launch_after(k_corners_basic<kFirst>, g4, 128, 0, s, ctx->P, pv, ctx->quad_start, ctx->mat, ctx->part_b);
       else
@@ -915,7 +915,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[0], ctx->stream));
   MIC_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->aux_ev[0], 0));
   {
-    MIC_KERNEL_ON(ctx, "k_partials_centre", ctx->aux);
+    MIC_KERNEL_ON(ctx, few ? "k_corners_centre" : "k_partials_centre", ctx->aux);
     if (few)
       launch_after(k_corners_centre<true, true>, corners_centre_grid(ctx->P), 128, 0, ctx->aux, ctx->P, pv,
                    ctx->quad_start, ctx->part_c);
@@ -925,7 +925,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
   }
   MIC_CUDA_TRY(cudaEventRecord(ctx->aux_ev[1], ctx->aux));
   if (visc) {
-    MIC_KERNEL(ctx, "k_partials_basic<visc>");
+    MIC_KERNEL(ctx, few ? "k_corners_basic<visc>" : "k_partials_basic<visc>");
     if (few)
       launch_after(k_corners_basic<kVisc>, g4, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
                    ctx->part_b);
@@ -933,7 +933,7 @@ static int project_all2(mic_ctx *ctx, int mode, cudaStream_t st = nullptr) {
       launch_after(k_partials_basic<kVisc>, g1, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
                    ctx->part_b);
   } else {
-    MIC_KERNEL(ctx, "k_partials_basic");
+    MIC_KERNEL(ctx, few ? "k_corners_basic" : "k_partials_basic");
     if (few)
       launch_after(k_corners_basic<kFull>, g4, 128, 0, ctx->stream, ctx->P, pv, ctx->quad_start, ctx->mat,
                    ctx->part_b);
