@@ -1071,7 +1071,8 @@ struct Level {
   size_t smem_small;
 };
 
-constexpr size_t kMaxSmem = 227 * 1024 - 1024;  // dynamic shared memory (static parts stay below 1 KB)
+constexpr size_t kSmem = 227 * 1024;       // shared memory of a block
+constexpr size_t kMaxSmem = kSmem - 1024;  // of a small front (k_front_small's other arrays stay below 1 KB)
 constexpr int kUpdateThreads = 256;
 
 // Blocks a panel's rows are shared out between: as many as bring them to 112 a block while the fronts
@@ -1469,6 +1470,8 @@ cudaError_t allow(K *kernel, size_t bytes) {
 template <int NB>
 cudaError_t allow_panels() {
   constexpr size_t bytes = (size_t)kPanelRows * ((NB + 1) * sizeof(double) + kPanelBytes);
+  static_assert(bytes + kOffers * 8 * sizeof(PanelOffer<NB>) + 32 * sizeof(Offer) + NB * sizeof(int) + 256 <= kSmem,
+                "a full panel of a cluster of eight beside its offers");
   cudaError_t e = allow(k_front_panel<NB>, bytes);
   if (e == cudaSuccess) e = allow(k_front_panel_cluster<NB, 2>, bytes);
   if (e == cudaSuccess) e = allow(k_front_panel_cluster<NB, 4>, bytes);
@@ -1482,6 +1485,8 @@ cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
   if (e == cudaSuccess) e = allow_panels<16>();
   if (e == cudaSuccess) e = allow_panels<32>();
   if (e == cudaSuccess) e = allow(k_front_update<32, 128, 64, false>, update_smem<32, 128, 64, false>());
+  static_assert(64 * 1024 + (2 * 32 * 33 + 32 * 33 + 32 * 32 + 4 * 32 + 2 * 2 * 32) * sizeof(double) + 64 <= kSmem,
+                "a front's unknowns beside the triangles of its rows");
   if (e == cudaSuccess) e = allow(k_front_back, 64 * 1024);
   return e;
 }
@@ -1504,7 +1509,7 @@ static int ensure_plan(mic_ctx *ctx, mic_system_store &S, int dof) {
   int e;
   try {
     e = build_plan(*pl, dof, ctx->P.NX, ctx->P.NY, sm_count(ctx));
-  } catch (const std::bad_alloc &) {
+  } catch (...) {  // (no memory, or a size beyond what a vector holds)
     e = MIC_ERR_NOMEM;
   }
   if (e) {
