@@ -298,7 +298,7 @@ __global__ void __cluster_dims__(kTC, 1, 1) __launch_bounds__(kTThreads)
 
 // The clusters' sums in order and Adam (apply); in the last block the losses' sum.  A thread waits
 // for as many loads as there are clusters, so eight are in flight at a time.  (Done by the last
-// cluster of k_train_step instead, it measured 27 us a step against 22.)
+// cluster of k_train_fwdbwd instead, it measured 27 us a step against 22.)
 __global__ void k_train_reduce(float *p, const float *__restrict__ part, int nblocks, float *grad, float *m_, float *v_,
                                int step, float lr, int apply, const float *__restrict__ lpart, float *loss) {
   if (blockIdx.x == gridDim.x - 1) {
