@@ -117,15 +117,17 @@ __device__ __forceinline__ const double *child_row(const Front &k, int i, const 
 // columns; the warps that update column j + 1 also find its candidates.  Two barriers a step.
 // The step is bound by this chain (about 1 us) until a front exceeds some 50,000 multiply-adds,
 // then by the FP64 pipe.
-// Pivots are taken in groups of four columns.  A step updates the group's columns and, of the
-// others, row j alone; the rest follow once a group, each value's products summed before they are
-// subtracted, which leaves a quarter of the roundings at the value's size.  Error against a refined
-// solution of 513 x 129 temperatures (largest, of the largest value): 1.27e-15; 1.65e-15 without
-// groups, 1.24e-15 in an elimination of the band.  GB300, solves of 129 x 33 and 513 x 129 Stokes and
-// of 513 x 129 temperatures with groups of 1, 2, 4, 8 and 16, ms: 1.94, 2.01, 1.98, 2.01, 2.09; 38.0,
-// 39.2, 38.7, 38.9, 40.1; 4.60, 4.98, 4.78, 4.81, 5.09.
-constexpr int kGroupCols = 4;
-template <int kSmallThreads>
+// Pivots are taken in groups of columns.  A step updates the group's columns and, of the others, row j
+// alone; the rest follow once a group, each value's products summed before they are subtracted, which
+// leaves one rounding at the value's size a group.  Error against a refined solution of 513 x 129
+// temperatures (largest, of the largest value): 1.27e-15; 1.65e-15 without groups, 1.24e-15 in an
+// elimination of the band.  The subtraction is one FP64 operation more a group: eight columns where a
+// front fills an SM's shared memory and that operation bounds it, else four.  GB300, solves of 129 x
+// 33, 257 x 65 and 513 x 129 Stokes and of 513 x 129 temperatures with groups of 4 and 8, ms: 1.98,
+// 6.86, 38.3 and 4.69; 4 everywhere 1.98, 6.93, 38.5 and 4.72; 8 above 32 rows 1.98, 6.91, 38.4 and
+// 4.67.  Fronts of 32 rows at most have one warp's work in a step: 128 threads, so that more of them
+// share an SM (16,384 fronts: 197 us, 291 with 256 threads).
+template <int kSmallThreads, int kGroupCols>
 __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__restrict__ fr, int first,
                                                               const int *__restrict__ tab,
                                                               const int *__restrict__ act, SystemRows sys,
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
   constexpr int kSmallWarps = kSmallThreads / 32;
   extern __shared__ double A[];
   __shared__ Offer red[32];
-  __shared__ double s_rcp[kGroupCols];
+  __shared__ double s_rcp;
   const Front q = fr[first + blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int R = q.R, P = q.P, C = q.C, ld = C | 1;
@@ -200,44 +202,38 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
         A[j * ld + c] = up;
         A[p * ld + c] = dn;
         if (c == j) {
-          s_rcp[j - j0] = pivot_rcp(up);
+          s_rcp = pivot_rcp(up);
           if (up == 0.0) atomicMin(&info[0], tab[q.col + j]);
         }
       }
       __syncthreads();
-      const double rcp = s_rcp[j - j0];
+      const double rcp = s_rcp;
       const int n = R - j - 1, m = je - j - 1;  // rows below, columns of the group after j
       G = (n + 31) / 32;
-      const int SL = max(1, min(m, kSmallWarps / max(G, 1))), T1 = m > 0 ? G * SL : 0;
-      const int T2 = j > j0 ? (C - je + 31) / 32 : 0;
+      const int T1 = m > 0 ? G : 0, T2 = j > j0 ? (C - je + 31) / 32 : 0;
       const double *piv = A + j * ld;
       for (int t = warp; t < T1 + T2; t += kSmallWarps) {
-        if (t < T1) {  // rows below in the group's columns, the next column first, with its candidates
-          const int g = t % G, s = t / G, r = j + 1 + g * 32 + lane;
+        if (t < T1) {  // rows below: the multiplier, the group's columns, the next one first, with its candidates
+          const int r = j + 1 + t * 32 + lane;
           double *row = A + r * ld;
-          const double l = r < R ? row[j] * rcp : 0.0;
-          int c = j + 1 + s;
-          if (s == 0) {
-            double v = 0.0;
-            if (r < R) {
-              v = row[c] - l * piv[c];
-              row[c] = v;
-            }
-            const long long key = r < R ? pivot_key(v) : -2;
-            if (lane == warp_best(key)) red[g] = Offer{key, r};
-            c += SL;
+          double l = 0.0, v = 0.0;
+          if (r < R) {
+            l = row[j] * rcp;
+            v = row[j + 1] - l * piv[j + 1];
+            row[j] = l;
+            row[j + 1] = v;
           }
+          const long long key = r < R ? pivot_key(v) : -2;
+          if (lane == warp_best(key)) red[t] = Offer{key, r};
           if (r < R)
-            for (; c < je; c += SL) row[c] -= l * piv[c];
+            for (int c = j + 2; c < je; ++c) row[c] -= l * piv[c];
         } else {  // row j, a row of U, behind the group
           const int c = je + (t - T1) * 32 + lane;
-          const double l = j0 + lane < j ? piv[j0 + lane] * s_rcp[lane] : 0.0;
-          double sum = 0.0;
-          for (int k = 0; k < j - j0; ++k) {
-            const double lk = __shfl_sync(0xffffffffu, l, k);
-            if (c < C) sum += lk * A[(j0 + k) * ld + c];
+          if (c < C) {
+            double sum = 0.0;
+            for (int k = j0; k < j; ++k) sum += piv[k] * A[k * ld + c];
+            A[j * ld + c] -= sum;
           }
-          if (c < C) A[j * ld + c] -= sum;
         }
       }
       __syncthreads();
@@ -252,9 +248,10 @@ __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__re
       const double *u = A + j0 * ld;
       double l[kGroupCols];
 #pragma unroll
-      for (int k = 0; k < kGroupCols; ++k) {
-        l[k] = k < kk && r < R ? row[j0 + k] * s_rcp[k] : 0.0;
-      }
+      for (int k = 0; k < kGroupCols; ++k) l[k] = k < kk && r < R ? row[j0 + k] : 0.0;
+#pragma unroll
+      for (int k = 0; k < kGroupCols; ++k)
+        if (k == kk - 1) l[k] *= s_rcp;  // (the last column's: no step has formed it)
       const auto sum = [&](int c) {
         double a = 0.0;
         if (kk == kGroupCols) {
@@ -1426,12 +1423,12 @@ int solve_launches(mic_ctx *ctx, const mic_front_plan &pl, const Buffers &B, con
     const Level &L = pl.levels[l];
     const double *Fin = B.F[(l + 1) & 1];
     if (L.small) {
-      // (more warps where one front fills an SM's shared memory)
-      const bool wide = L.smem_small > kMaxSmem / 2;
-      MIC_KERNEL(ctx, wide ? "k_front_small<512>" : "k_front_small<256>");
-      const auto kernel = wide ? k_front_small<512> : k_front_small<256>;
-      LU_LAUNCH(kernel, L.count, wide ? 512 : 256, L.smem_small, ctx->stream, pl.d_fronts, L.first, pl.d_tab, B.act,
-                sys, Fin, B.F[l & 1], B.U, B.info);
+      // more warps where one front fills an SM's shared memory, fewer where all its rows are one warp's
+      const bool wide = L.smem_small > kMaxSmem / 2, tiny = L.maxR <= 32;
+      MIC_KERNEL(ctx, wide ? "k_front_small<512>" : tiny ? "k_front_small<128>" : "k_front_small<256>");
+      const auto kernel = wide ? k_front_small<512, 8> : tiny ? k_front_small<128, 4> : k_front_small<256, 4>;
+      LU_LAUNCH(kernel, L.count, wide ? 512 : tiny ? 128 : 256, L.smem_small, ctx->stream, pl.d_fronts, L.first,
+                pl.d_tab, B.act, sys, Fin, B.F[l & 1], B.U, B.info);
       continue;
     }
     {
@@ -1480,8 +1477,9 @@ cudaError_t allow_panels() {
 }
 
 cudaError_t allow_smem() {  // per device; cheap enough to set on every plan
-  cudaError_t e = allow(k_front_small<256>, kMaxSmem);
-  if (e == cudaSuccess) e = allow(k_front_small<512>, kMaxSmem);
+  cudaError_t e = allow(k_front_small<128, 4>, kMaxSmem);
+  if (e == cudaSuccess) e = allow(k_front_small<256, 4>, kMaxSmem);
+  if (e == cudaSuccess) e = allow(k_front_small<512, 8>, kMaxSmem);
   if (e == cudaSuccess) e = allow_panels<16>();
   if (e == cudaSuccess) e = allow_panels<32>();
   if (e == cudaSuccess) e = allow(k_front_update<32, 128, 64, false>, update_smem<32, 128, 64, false>());

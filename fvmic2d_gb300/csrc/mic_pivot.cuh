@@ -24,19 +24,16 @@ __device__ __forceinline__ void take_better(Offer &o, double a, int row) {
     o.row = row;
   }
 }
-// The lane with the warp's largest key, the first of equal ones.  One reduction of the high words;
-// where several lanes share the largest, another of their low words.  Twice a column on the chain of a
-// front's columns: GB300, solves of 129 x 33, 257 x 65 and 513 x 129 Stokes and of 513 x 129
-// temperatures 1.91, 6.68, 37.0 and 4.56 ms; 1.82, 6.53, 36.8 and 4.45 with the leading 21 bits and
-// the row in one integer, which takes rows for equal that differ by 2^-10.
+// The lane with the warp's largest key, the first of equal ones: the largest high word, then the
+// largest low word of the lanes that have it.  Twice a column on the chain of a front's columns.  GB300,
+// solves of 129 x 33 and 513 x 129 Stokes and of 513 x 129 temperatures: 1.96, 38.2 and 4.66 ms; with
+// the second reduction behind a branch (only where lanes share the high word) 1.99, 38.2 and 4.68; high
+// words alone 1.93, 38.2 and 4.63.  The leading 21 bits and the row in one integer, a single reduction,
+// would take rows for equal that differ by 2^-10.
 __device__ __forceinline__ int warp_best(long long key) {
   const int hi = (int)(key >> 32), top = __reduce_max_sync(0xffffffffu, hi);
-  unsigned lanes = __ballot_sync(0xffffffffu, hi == top);
-  if (lanes & (lanes - 1)) {  // (the same in every lane)
-    const unsigned lo = hi == top ? (unsigned)key : 0u, most = __reduce_max_sync(0xffffffffu, lo);
-    lanes &= __ballot_sync(0xffffffffu, lo == most);
-  }
-  return __ffs(lanes) - 1;
+  const unsigned lo = hi == top ? (unsigned)key : 0u, most = __reduce_max_sync(0xffffffffu, lo);
+  return __ffs(__ballot_sync(0xffffffffu, hi == top && lo == most)) - 1;
 }
 
 // a column whose best key is 0 or less (every a zero or NaN): the largest |a| of the rows not used, the
