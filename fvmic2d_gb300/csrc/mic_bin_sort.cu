@@ -396,11 +396,8 @@ __global__ void k_cell_start(const int *__restrict__ skey, int64_t n, int ncells
   const int64_t qmax = 4LL * ncells + 4;
   if (q > qmax) return;
   int64_t lo = 0, hi = n;
-  if (*lost) {
-    if (q == 0) *lost = (unsigned long long)n;
-    for (int64_t k = q; k < n; k += qmax + 1) perm[k] = (int)k;
-    hi = 0;
-  } else if (n > 0) {
+  const unsigned long long gave_up = *lost;  // (used at the end: the search ends whatever the keys are)
+  if (n > 0) {
     const int64_t g = q * n / (qmax + 1);  // in [0, n)
     if (skey[g] < q) {
       lo = g + 1;
@@ -432,6 +429,11 @@ __global__ void k_cell_start(const int *__restrict__ skey, int64_t n, int ncells
       lo = mid + 1;
     else
       hi = mid;
+  }
+  if (gave_up) {
+    if (q == 0) *lost = (unsigned long long)n;
+    for (int64_t k = q; k < n; k += qmax + 1) perm[k] = (int)k;
+    lo = 0;
   }
   if (qs) qs[q] = (int)lo;
   if ((q & 3) == 0) cs[q >> 2] = (int)lo;

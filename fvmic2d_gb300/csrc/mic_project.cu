@@ -997,7 +997,7 @@ extern "C" int mic_project_marker_field_to_nodes(mic_ctx *ctx, int off, const do
   }
   MIC_CUDA_TRY(cudaGetLastError());
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
+  return mic_sort_error(ctx);
 }
 
 // projectMarkersNodesFromScalar (markers.c:1507-1594): a per-marker array in the caller's order
@@ -1014,5 +1014,5 @@ extern "C" int mic_project_markers_nodes_from_scalar(mic_ctx *ctx, const double 
   }
   if ((e = mic_project_scalar(ctx, ctx->scr2, 0, ctx->nodal[out_field]))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
+  return mic_sort_error(ctx);
 }

@@ -34,8 +34,9 @@ enum {
   MIC_ERR_NOMEM = 3,      /* device or host allocation failed */
   MIC_ERR_CELL = 4,       /* impossible cell index (markers.c:74-77 aborts): a binning that gave up waiting for
                              its sort.  The markers keep their order and no cell holds any, so what a step
-                             computes after it is not valid; every call that waits for the device returns this
-                             code until the markers are uploaded or reset */
+                             computes after it is not valid: binning, steps, maxima, downloads, checkpoints,
+                             density control and the synchronize calls return this code until the markers are
+                             uploaded or reset */
   MIC_ERR_NAN = 5,        /* NaN strain-rate residual; updateMarkerStrainPressure.c:302-306 aborts */
   MIC_ERR_LAW = 6,        /* undefined viscosity law; viscosity.c:60-62 aborts */
   MIC_ERR_BC = 7,         /* unsupported boundary type, or a routine outside the marker path on a grid
