@@ -125,8 +125,8 @@ __device__ __forceinline__ const double *child_row(const Front &k, int i, const 
 // front fills an SM's shared memory and that operation bounds it, else four.  GB300, solves of 129 x
 // 33, 257 x 65 and 513 x 129 Stokes and of 513 x 129 temperatures with groups of 4 and 8, ms: 1.98,
 // 6.86, 38.3 and 4.69; 4 everywhere 1.98, 6.93, 38.5 and 4.72; 8 above 32 rows 1.98, 6.91, 38.4 and
-// 4.67.  Fronts of 32 rows at most have one warp's work in a step: 128 threads, so that more of them
-// share an SM (16,384 fronts: 197 us, 291 with 256 threads).
+// 4.67 (all with the search as it was, 1 to 2% slower).  Fronts of 32 rows at most have one warp's work
+// in a step: 128 threads, so that more of them share an SM (16,384 fronts: 197 us, 291 with 256).
 template <int kSmallThreads, int kGroupCols>
 __global__ void __launch_bounds__(kSmallThreads) k_front_small(const Front *__restrict__ fr, int first,
                                                               const int *__restrict__ tab,
@@ -498,8 +498,8 @@ __device__ __forceinline__ void solve_u12(double (*Us)[TC + 1], double (*L11)[NB
 // awaits nothing more (so the others' waits run out too), writes nothing of the panel, and counts
 // itself in info[1], which fails the solve.  What follows reads row lists that hold row numbers all
 // the same.  It stays until what the others have sent it has arrived.
-// GB300, us a panel on one SM and on a cluster: 27 and 22 of 330 rows, 33 and 22 of 645, 70 and 33
-// of 1,290.
+// GB300, us a panel of 16 columns on one SM and on a cluster (means over a level, events around each):
+// 30 and 28 from 330 rows down, 40 and 31 from 484, 37 and 29 from 645.
 constexpr int kOffers = 4;
 constexpr int kDrainPolls = 1 << 16;  // a millisecond for what is on its way already
 template <int NB>
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(256) k_front_solve(const Front *__restrict__ f
 // it, for one launch and one wait less; otherwise U12 is in U.  Columns coff .. coff + clen - 1 of
 // those right of the panel.
 // The chain's kernels (panels of 16 columns, the update of the next panel's) let each other's blocks
-// come early: 129 x 33 Stokes 1.85 -> 1.83 ms, 257 x 65 6.67 -> 6.57.
+// come early: 129 x 33 Stokes 1.98 -> 1.96 ms, 257 x 65 6.95 -> 6.84.
 template <int NB, int TR, int TC, bool SOLVE>
 constexpr int update_smem() {
   return (int)sizeof(double) * (NB * (TC + 1) + TR * (NB + 1) + (SOLVE ? NB * (NB + 1) : 0));
@@ -1075,8 +1075,9 @@ constexpr int kUpdateThreads = 256;
 // Blocks a panel's rows are shared out between: as many as bring them to 112 a block while the fronts
 // do not fill the SMs, and as many as shared memory asks for (a level's rows end at 4,056: the
 // solver's size limit).  GB300, solves of 129 x 33, 257 x 65 and 513 x 129 Stokes and of 513 x 129
-// temperatures, ms: one block always 2.11, 8.27, 41.3, 5.19; 64 rows 2.04, 7.62, 39.8, 4.87; 96 rows
-// 2.02, 7.60, 39.8, 4.86; 128 rows 2.04, 7.63, 39.8, 4.84; 256 rows 2.09, 8.00, 40.1, 5.16.
+// temperatures, ms: one block always 2.07, 7.69, 39.8, 5.17; 64 rows 2.05, 6.99, 38.4, 4.72; 96 rows
+// 1.97, 6.85, 38.3, 4.65; 112 rows 1.96, 6.84, 38.3, 4.67; 128 rows 1.96, 6.89, 38.3, 4.72; 256 rows
+// 2.06, 7.39, 38.7, 5.11.
 constexpr int kPanelRows = 800;
 int cluster_blocks(int fronts, int rows, int nsm) {
   int cl = 1;
@@ -1101,16 +1102,16 @@ namespace {
 // The level's form, by estimated time (us).  Small: a front's multiply-adds on one SM (2 per clock),
 // 1.1 us a column step, 6 us to load and store.  Large: per panel of 16 columns, 28 us for its
 // factorisation and the launches, and the update's 32 x 32 tiles (padding included) over all SMs at
-// 5.4 us a tile; 9 us for the gather.  Measured on the levels of five systems: the lines cross near
-// 60 fronts of 100 x 170 (241 us small, 230 large); 256 fronts of 52 x 90 take 81 us small and 280
-// large, 16 of 80 x 133 take 134 us small and 98 large.  With the small estimate a third higher 513 x
-// 129 Stokes take 37.5 ms instead of 36.9, with it a third lower 129 x 33 take 1.93 instead of 1.85.
+// 5.4 us a tile; 9 us for the gather.  The lines cross near 60 fronts of 100 x 170.  GB300, solves of
+// 129 x 33, 257 x 65 and 513 x 129 Stokes and of 129 x 33 and 513 x 129 temperatures, ms: 1.96, 6.84,
+// 38.3, 0.66, 4.67; with the small estimate a third higher 1.96, 7.00, 38.9, 0.65, 4.68, a third lower
+// 2.04, 6.84, 38.3, 0.89, 4.67.
 //
 // Columns of a panel: 16 where the chain of panels bounds the level, 32 where the updates do (twice
 // the multiply-adds for each value of the trailing rows read and written; the panels' own work and
 // the solve of U12 double).  By the level's first update at 2 multiply-adds per SM and clock, 16
-// columns deep: from 15 us 129 x 33 Stokes take 2.10 ms, from 40 us 1.85, with 16 always 1.84; 257 x
-// 65 6.87, 6.87 and 7.44; 513 x 129 37.6, 37.6 and 39.3, from 80 us 37.9.
+// columns deep: from 15 us 129 x 33 Stokes take 2.18 ms, from 40 us 1.96, with 16 always 1.95; 257 x
+// 65 6.82, 6.84 and 7.52; 513 x 129 38.3, 38.3 and 40.8, from 80 us 38.7.
 void plan_level(Level &L, const std::vector<Front> &fr, int nsm) {
   double total = 0, most = 0, large = 9.0;
   for (int i = L.first; i < L.first + L.count; ++i) {
@@ -1343,9 +1344,9 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     // multiply-adds under 50 us at 2 per SM and clock, or a panel that fits beside its blocks in an
     // SM's shared memory): it starts with the update of the next panel's columns.  Heavy: only after
     // that one, so that the panel, which may need an SM's whole shared memory, finds free SMs; behind
-    // a heavy update it would start when that ends (513 x 129 Stokes: 54.3 ms with every update
-    // light, 46.9 with the heavy ones whole before the next panel, 41.8 so; 513 x 129 temperatures
-    // with the line at 50 us and 200 rows 4.48, at 75 us and 400 rows 4.57).
+    // a heavy update it would start when that ends.  GB300, 257 x 65 and 513 x 129 Stokes and 513 x 129
+    // temperatures, ms: 6.84, 38.3, 4.67; every update light 7.06, 38.7, 4.81; the line at 75 us and
+    // 400 rows 6.89, 38.3, 4.77.
     const double us = (double)cols * below * NB * L.count / (2.0 * 1.9e3 * sm_count(ctx));
     const bool ahead = k0 + NB < L.maxP && cols > NB, light = us < 50.0 || rows < 200;
     const int near = ahead ? NB : 0, rest = cols - near;
@@ -1356,9 +1357,9 @@ int large_level(mic_ctx *ctx, const mic_front_plan &pl, const Level &L, const Bu
     }
     if (far) MIC_CUDA_TRY(cudaStreamWaitEvent(chain, ctx->lu_ev[1], 0));
     if (ahead) {
-      // on the chain: tiles as small as still get an SM each.  GB300: 64 rows always 1.97 ms for 129 x
-      // 33 Stokes, 7.48 for 257 x 65, 4.75 for 513 x 129 temperatures; up to one tile an SM 1.84, 7.45,
-      // 4.65; up to four 1.84, 7.62, 4.74
+      // on the chain: tiles as small as still get an SM each.  GB300: 64 rows always 2.07 ms for 129 x
+      // 33 Stokes, 6.95 for 257 x 65, 4.70 for 513 x 129 temperatures; up to one tile an SM 1.96, 6.84,
+      // 4.67; up to four 1.95, 6.92, 4.69
       const int at_once = sm_count(ctx);
       const auto tile = L.count * ((below + 15) / 16) <= at_once   ? update<NB, 16, 16, true>
                         : L.count * ((below + 31) / 32) <= at_once ? update<NB, 32, 16, true>
