@@ -526,7 +526,12 @@ __device__ __forceinline__ void centre_run(const Params &P, const int *__restric
   }
 }
 
-__global__ void __launch_bounds__(128) k_partials_centre(Params P, PartialView v, const int *__restrict__ qs,
+// Bound by the latency of a cell's chain of markers and by what L1 holds of the warps' markers: eight
+// blocks an SM, 64 registers.  With 48 (the compiler's choice without a bound, a spill in the loop) 300 x
+// 300 cells of 36 markers take 180 us for 147 and, beside the basic sums, the projection 290 for 256;
+// 700 x 700 of 16 550 for 520.  With seven blocks, 68 registers: 242 and 517, but 200 x 200 cells of 36 take
+// 141 for 126.
+__global__ void __launch_bounds__(128, 8) k_partials_centre(Params P, PartialView v, const int *__restrict__ qs,
                                                           double *__restrict__ part) {
   if (!after_previous()) return;
   __shared__ double sloc[12][128];
