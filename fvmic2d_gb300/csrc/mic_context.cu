@@ -824,21 +824,18 @@ int mic_clear(mic_ctx *ctx, const mic_clear_list &l) {
 
 int mic_words_out(mic_ctx *ctx, const void *dev, size_t bytes) { return words_out(ctx, dev, ctx->h_words, bytes); }
 
-static int status_to_host(mic_ctx *ctx) {
+int mic_fetch_status(mic_ctx *ctx) {
   if (const int e = words_out(ctx, ctx->d_status, ctx->h_status, sizeof(Status))) return e;
   MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return MIC_OK;
-}
-
-int mic_fetch_status(mic_ctx *ctx) {
-  const int e = status_to_host(ctx);
-  return e ? e : mic_sort_error(ctx);
+  return mic_sort_error(ctx);
 }
 
 extern "C" int mic_get_status(mic_ctx *ctx, mic_status *st) {
   if (!ctx || !st) return MIC_ERR_ARG;
   cudaSetDevice(ctx->device);
-  if (const int e = status_to_host(ctx)) return e;  // (the record itself: whatever it holds)
+  // (the record itself, whatever it holds; a copy, as nothing is to follow it on the stream)
+  MIC_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(Status), cudaMemcpyDeviceToHost, ctx->stream));
+  MIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   st->bad_cell = ctx->h_status->bad_cell;
   st->nan_residual = ctx->h_status->nan_residual;
   st->nan_dsxy = ctx->h_status->nan_dsxy;
